@@ -252,14 +252,85 @@ __global__ void __launch_bounds__(256) k_ae_e1_vol(const E1Vol a) {
     }
 }
 
+// out[(c * SC + j * SJ)] += sum over the block's 512 nodes of a[c] b[j], and
+// bias += the column sums of a (BIAS_A) or of b: the weight and bias
+// gradients of D1 (a = dy, b = g) and E1 (a = x, b = dh).  The nodes' 8 and
+// 16 values sit in shared memory, a node per row of an array padded so that
+// the 32-byte and 64-byte rows of consecutive nodes start in different banks.
+// Thread t owns a 2 x 4 tile of the 8 x 16 products (t & 15) over the nodes
+// congruent to t >> 4: two loads and eight multiply-adds per node, then a
+// shuffle, a pass through shared memory and one global atomic per product.
+// Bound by shared-memory latency; 136 shared atomics of every thread on the
+// same 136 words, which this replaces, took 675 us (D1) and 738 us (E1) for
+// 256 blocks; the kernels now take 11.7 us and 5.6 us.
+constexpr int kOutA = 12, kOutB = 20;   // row strides (floats)
+constexpr int kOutFloats = 512 * (kOutA + kOutB);
+
+template <bool BIAS_A, int SC, int SJ>
+__device__ __forceinline__ void block_outer(float *sm, float *gw, float *gb) {
+    const float *A = sm, *B = sm + 512 * kOutA;
+    const int t = threadIdx.x, c0 = (t & 3) * 2, j0 = ((t >> 2) & 3) * 4, grp = t >> 4;
+    float acc[2][4], sa[2] = {0.0f, 0.0f}, sb[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
+#pragma unroll 4
+    for (int k = 0; k < 32; k++) {
+        const int p = k * 16 + grp;
+        const float2 a = *reinterpret_cast<const float2 *>(A + p * kOutA + c0);
+        const float4 b = *reinterpret_cast<const float4 *>(B + p * kOutB + j0);
+        const float av[2] = {a.x, a.y}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[i][j] = __fmaf_rn(av[i], bv[j], acc[i][j]);
+        if (BIAS_A) {
+            sa[0] += av[0];
+            sa[1] += av[1];
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++) sb[j] += bv[j];
+        }
+    }
+    __syncthreads();   // every thread is done with A and B
+    // 16 groups -> 8 warps -> 1: slot (warp, tile) of 8 products and 4 sums
+    float *red = sm;
+    float v[12];
+#pragma unroll
+    for (int q = 0; q < 8; q++) v[q] = acc[q >> 2][q & 3];
+#pragma unroll
+    for (int q = 0; q < 4; q++) v[8 + q] = BIAS_A ? (q < 2 ? sa[q] : 0.0f) : sb[q];
+#pragma unroll
+    for (int q = 0; q < 12; q++) {
+        v[q] += __shfl_xor_sync(0xffffffffu, v[q], 16);
+        if (!(t & 16)) red[((t >> 5) * 16 + (t & 15)) * 13 + q] = v[q];
+    }
+    __syncthreads();
+    for (int o = t; o < 16 * 12; o += 256) {
+        const int tile = o / 12, q = o % 12;
+        float s = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 8; w++) s += red[(w * 16 + tile) * 13 + q];
+        const int c = (tile & 3) * 2, j = (tile >> 2) * 4;
+        if (q < 8) atomicAdd(gw + (c + (q >> 2)) * SC + (j + (q & 3)) * SJ, s);
+        else if (BIAS_A) {
+            if (j == 0 && q < 10) atomicAdd(gb + c + (q - 8), s);
+        } else if (c == 0) {
+            atomicAdd(gb + j + (q - 8), s);
+        }
+    }
+}
+
 struct D1Args {
     int nb;
     const __nv_bfloat16 *g1;      // [nbp*512 x 16]
     const float *v1, *c1;         // D1: W [8 x 16] (bf16 values), b [8]
     const float *xn;              // normalized target
     float *recon;                 // normalized reconstruction, or null
+    int recon16;                  // 1: recon is 16-byte aligned
     __nv_bfloat16 *dg1;           // gradient at D2's output (gated)
-    float *gd1;                   // D1 gradient (W then b, 136 floats)
+    float *gd1;                   // D1 gradient (W then b, 136 floats), or null: no gradients
     double *loss;                 // sum of squared errors, slot *step - step0
     const int *step;
     int step0;
@@ -271,12 +342,11 @@ struct D1Args {
 // and bias gradients and the gated gradient at D2's output.
 // loss = sum_b w_b |e_b|^2 / (W * 4096), W = sum_b w_b.
 __global__ void __launch_bounds__(256) k_ae_d1(const D1Args a) {
-    __shared__ float sg[136];
+    extern __shared__ float sm[];
     __shared__ float red[8];
     const int b = blockIdx.x, t = threadIdx.x;
     if (b >= a.nb) return;
-    for (int i = t; i < 136; i += 256) sg[i] = 0.0f;
-    __syncthreads();
+    float *A = sm, *B = sm + 512 * kOutA;
     float lsum = 0.0f;
     const float W = a.wsum ? a.wsum[*a.step - a.step0] : (float)gridDim.x;
     const float wb = a.wrow ? a.wrow[b] : 1.0f;
@@ -284,35 +354,50 @@ __global__ void __launch_bounds__(256) k_ae_d1(const D1Args a) {
 #pragma unroll 1
     for (int r = 0; r < 2; r++) {
         const int p = t + 256 * r;
-        float g[16], y[8];
+        float g[16], y[8], x[8];
+        const float4 *xp = reinterpret_cast<const float4 *>(a.xn + (long)b * kAePts + p * 8);
+        *reinterpret_cast<float4 *>(x) = xp[0];
+        *reinterpret_cast<float4 *>(x + 4) = xp[1];
         d1_node(a.v1, a.c1, a.g1 + ((long)b * 512 + p) * 16, g, y);
         float dy[8];
 #pragma unroll
         for (int c = 0; c < 8; c++) {
-            const long o = (long)b * kAePts + p * 8 + c;
-            const float d = y[c] - a.xn[o];
+            const float d = y[c] - x[c];
             lsum += d * d;
             dy[c] = 2.0f * d * gsc;
-            if (a.recon) a.recon[o] = y[c];
         }
+        if (a.recon) {   // the caller's buffer: 4-byte aligned
+            float *rp = a.recon + (long)b * kAePts + p * 8;
+            if (a.recon16) {
+                reinterpret_cast<float4 *>(rp)[0] = make_float4(y[0], y[1], y[2], y[3]);
+                reinterpret_cast<float4 *>(rp)[1] = make_float4(y[4], y[5], y[6], y[7]);
+            } else {
 #pragma unroll
-        for (int c = 0; c < 8; c++) {
-#pragma unroll
-            for (int j = 0; j < 16; j++) atomicAdd(&sg[c * 16 + j], dy[c] * g[j]);
-            atomicAdd(&sg[128 + c], dy[c]);
+                for (int c = 0; c < 8; c++) rp[c] = y[c];
+            }
         }
-        uint4 o4[2];
-        __nv_bfloat16 *ob = reinterpret_cast<__nv_bfloat16 *>(o4);
+        if (a.gd1) {
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-            float acc = 0.0f;
+            for (int c = 0; c < 2; c++)
+                reinterpret_cast<float4 *>(A + p * kOutA)[c] =
+                    make_float4(dy[4 * c], dy[4 * c + 1], dy[4 * c + 2], dy[4 * c + 3]);
 #pragma unroll
-            for (int c = 0; c < 8; c++) acc += a.v1[c * 16 + j] * dy[c];
-            ob[j] = __float2bfloat16_rn(g[j] > 0.0f ? acc : kLeak * acc);
+            for (int c = 0; c < 4; c++)
+                reinterpret_cast<float4 *>(B + p * kOutB)[c] =
+                    make_float4(g[4 * c], g[4 * c + 1], g[4 * c + 2], g[4 * c + 3]);
+            uint4 o4[2];
+            __nv_bfloat16 *ob = reinterpret_cast<__nv_bfloat16 *>(o4);
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                float acc = 0.0f;
+#pragma unroll
+                for (int c = 0; c < 8; c++) acc += a.v1[c * 16 + j] * dy[c];
+                ob[j] = __float2bfloat16_rn(g[j] > 0.0f ? acc : kLeak * acc);
+            }
+            uint4 *dst = reinterpret_cast<uint4 *>(a.dg1 + ((long)b * 512 + p) * 16);
+            dst[0] = o4[0];
+            dst[1] = o4[1];
         }
-        uint4 *dst = reinterpret_cast<uint4 *>(a.dg1 + ((long)b * 512 + p) * 16);
-        dst[0] = o4[0];
-        dst[1] = o4[1];
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
@@ -324,7 +409,7 @@ __global__ void __launch_bounds__(256) k_ae_d1(const D1Args a) {
         const double Wd = a.wsum ? (double)a.wsum[*a.step - a.step0] : (double)gridDim.x;
         atomicAdd(a.loss + (*a.step - a.step0), tot * wb / Wd);
     }
-    for (int i = t; i < 136; i += 256) atomicAdd(&a.gd1[i], sg[i]);
+    if (a.gd1) block_outer<true, 16, 1>(sm, a.gd1, a.gd1 + 128);
 }
 
 // D1 of a snapshot's blocks with the weights passed by value, unscaled and
@@ -488,30 +573,29 @@ __global__ void __launch_bounds__(256) k_ae_escape_copy(const int *esc, const __
 // E1 weight and bias gradients from the normalized input and the gated
 // gradient at E1's output.
 __global__ void __launch_bounds__(256) k_ae_e1_bwd(const float *xn, const __nv_bfloat16 *dh1, float *ge1, int nb) {
-    __shared__ float sg[144];
+    extern __shared__ float sm[];
     const int b = blockIdx.x, t = threadIdx.x;
     if (b >= nb) return;
-    for (int i = t; i < 144; i += 256) sg[i] = 0.0f;
-    __syncthreads();
-#pragma unroll 1
+    float *A = sm, *B = sm + 512 * kOutA;
+#pragma unroll
     for (int r = 0; r < 2; r++) {
         const int p = t + 256 * r;
-        float x8[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) x8[j] = bf16r(xn[(long)b * kAePts + p * 8 + j]);
+        const float4 *xp = reinterpret_cast<const float4 *>(xn + (long)b * kAePts + p * 8);
+        const float4 x0 = xp[0], x1 = xp[1];
+        float4 *ap = reinterpret_cast<float4 *>(A + p * kOutA);
+        ap[0] = make_float4(bf16r(x0.x), bf16r(x0.y), bf16r(x0.z), bf16r(x0.w));
+        ap[1] = make_float4(bf16r(x1.x), bf16r(x1.y), bf16r(x1.z), bf16r(x1.w));
         const uint4 *src = reinterpret_cast<const uint4 *>(dh1 + ((long)b * 512 + p) * 16);
-        uint4 q[2] = {src[0], src[1]};
+        const uint4 q[2] = {src[0], src[1]};
         const __nv_bfloat16 *qb = reinterpret_cast<const __nv_bfloat16 *>(q);
+        float4 *bp = reinterpret_cast<float4 *>(B + p * kOutB);
 #pragma unroll
-        for (int c = 0; c < 16; c++) {
-            const float d = __bfloat162float(qb[c]);
-#pragma unroll
-            for (int j = 0; j < 8; j++) atomicAdd(&sg[c * 8 + j], d * x8[j]);
-            atomicAdd(&sg[128 + c], d);
-        }
+        for (int c = 0; c < 4; c++)
+            bp[c] = make_float4(__bfloat162float(qb[4 * c]), __bfloat162float(qb[4 * c + 1]),
+                                __bfloat162float(qb[4 * c + 2]), __bfloat162float(qb[4 * c + 3]));
     }
     __syncthreads();
-    for (int i = t; i < 144; i += 256) atomicAdd(&ge1[i], sg[i]);
+    block_outer<false, 1, 8>(sm, ge1, ge1 + 128);   // W1[j * 8 + c]
 }
 
 // grad[n*K + k] += sum_m dy[m*N + n] * x[m*K + k] over this split's rows.
@@ -671,6 +755,7 @@ struct geo_ae {
     // training scratch
     int trows = 0;
     DevBuf xn, dg1, dg2, dg3, dz, dh3, dh2, dh1, wrow;
+    DevBuf ev;                                 // evaluation: loss (double), zero step counter
     // escape settings
     float tau = 0.05f, frac = 0.03f;
     DevBuf resall, err2, norm2;
@@ -826,7 +911,6 @@ static D1Args d1_args(geo_ae *ae, int nb) {
     a.g1 = bf(ae->g1);
     a.v1 = ae->small.as<float>() + 128;
     a.c1 = ae->params.as<float>() + ae->off.b[7];
-    a.step = ae->step.as<int>();
     return a;
 }
 
@@ -950,22 +1034,37 @@ int ae_decode_volume(geo_ae *ae, const AeVolume &v, const void *code, const floa
     return check_launch("ae_d1");
 }
 
+// Dynamic shared memory of the kernels that end in block_outer (64 KB).
+static int outer_smem() {
+    static bool set = false;
+    if (set) return GEO_OK;
+    GEO_CUDA(cudaFuncSetAttribute(k_ae_d1, cudaFuncAttributeMaxDynamicSharedMemorySize, kOutFloats * 4));
+    GEO_CUDA(cudaFuncSetAttribute(k_ae_e1_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, kOutFloats * 4));
+    set = true;
+    return GEO_OK;
+}
+
 // Forward (+ backward when grads are wanted) over `rows` blocks already
-// loaded by k_ae_e1 (xn filled); loss slot from the step counter.
-static int train_pass(geo_ae *ae, int rows, double *loss, const float *wsum, int step0, float *recon, bool backward,
-                      cudaStream_t s) {
+// loaded by k_ae_e1 (xn filled); loss slot *step - step0.
+static int train_pass(geo_ae *ae, int rows, double *loss, const float *wsum, const int *step, int step0, float *recon,
+                      bool backward, cudaStream_t s) {
     GEO_TRY(encode_rows(ae, rows, bf(ae->z), s));
     GEO_TRY(decode_rows(ae, rows, bf(ae->z), s));
     D1Args a = d1_args(ae, rows);
     a.xn = ae->xn.as<float>();
     a.recon = recon;
-    a.dg1 = bf(ae->dg1);
-    a.gd1 = ae->grad.as<float>() + ae->off.w[7];
+    a.recon16 = (reinterpret_cast<uintptr_t>(recon) & 15) == 0;
+    if (backward) {
+        a.dg1 = bf(ae->dg1);
+        a.gd1 = ae->grad.as<float>() + ae->off.w[7];
+    }
     a.loss = loss;
+    a.step = step;
     a.step0 = step0;
     a.wrow = wsum ? ae->wrow.as<float>() : nullptr;
     a.wsum = wsum;
-    k_ae_d1<<<rows, 256, 0, s>>>(a);
+    GEO_TRY(outer_smem());
+    k_ae_d1<<<rows, 256, kOutFloats * 4, s>>>(a);
     GEO_TRY(check_launch("ae_d1_train"));
     if (!backward) return GEO_OK;
     GEO_TRY(level_bwd(ae, 6, rows, bf(ae->dg1), bf(ae->g2), bf(ae->dg2), bf(ae->g2), s));   // D2
@@ -974,7 +1073,7 @@ static int train_pass(geo_ae *ae, int rows, double *loss, const float *wsum, int
     GEO_TRY(level_bwd(ae, 3, rows, bf(ae->dz), bf(ae->h3), bf(ae->dh3), bf(ae->h3), s));    // E4
     GEO_TRY(level_bwd(ae, 2, rows, bf(ae->dh3), bf(ae->h2), bf(ae->dh2), bf(ae->h2), s));   // E3
     GEO_TRY(level_bwd(ae, 1, rows, bf(ae->dh2), bf(ae->h1), bf(ae->dh1), bf(ae->h1), s));   // E2
-    k_ae_e1_bwd<<<rows, 256, 0, s>>>(ae->xn.as<float>(), bf(ae->dh1), ae->grad.as<float>() + ae->off.w[0], rows);
+    k_ae_e1_bwd<<<rows, 256, kOutFloats * 4, s>>>(ae->xn.as<float>(), bf(ae->dh1), ae->grad.as<float>() + ae->off.w[0], rows);
     return check_launch("ae_e1_bwd");
 }
 
@@ -1131,16 +1230,22 @@ extern "C" int geo_ae_eval(geo_ae *ae, const float *blocks, int nb, float *recon
     if (nb % 128) return fail(GEO_ERR_ARG, "block count must be a multiple of 128");
     cudaStream_t s = (cudaStream_t)stream;
     GEO_TRY(ensure_train(ae, nb));
-    DevBuf in, rec, dl;
+    DevBuf in, rec;
     const float *src = blocks;
     if (mem != GEO_MEM_DEVICE) {
         GEO_TRY(in.alloc((size_t)nb * kAePts * 4));
         GEO_CUDA(cudaMemcpyAsync(in.p, blocks, (size_t)nb * kAePts * 4, cudaMemcpyHostToDevice, s));
         src = in.as<float>();
     }
-    GEO_TRY(rec.alloc((size_t)nb * kAePts * 4));
-    GEO_TRY(dl.alloc(16));
-    GEO_TRY(dl.zero(s));
+    // device callers take the reconstruction straight from D1; the loss and
+    // a zero step counter (the loss slot) share one small buffer
+    float *prec = mem == GEO_MEM_DEVICE ? recon : nullptr;
+    if (recon && !prec) {
+        GEO_TRY(rec.alloc((size_t)nb * kAePts * 4));
+        prec = rec.as<float>();
+    }
+    if (!ae->ev.p) GEO_TRY(ae->ev.alloc(16));
+    GEO_TRY(ae->ev.zero(s));
     GEO_CUDA(cudaMemsetAsync(ae->grad.p, 0, ae->off.total * 4, s));
     GEO_CUDA(cudaMemsetAsync(ae->err.p, 0, 4, s));
     E1Args a = e1_args(ae, nb);
@@ -1148,16 +1253,13 @@ extern "C" int geo_ae_eval(geo_ae *ae, const float *blocks, int nb, float *recon
     a.xn = ae->xn.as<float>();
     k_ae_e1<<<nb, 256, 0, s>>>(a);
     GEO_TRY(check_launch("ae_e1"));
-    int h_step = 0;
-    GEO_CUDA(cudaMemcpyAsync(&h_step, ae->step.p, 4, cudaMemcpyDeviceToHost, s));
-    GEO_CUDA(cudaStreamSynchronize(s));
-    GEO_TRY(train_pass(ae, nb, dl.as<double>(), nullptr, h_step, rec.as<float>(), grad != nullptr, s));
-    GEO_TRY(ae_check_err(ae, s));
+    GEO_TRY(train_pass(ae, nb, ae->ev.as<double>(), nullptr, ae->ev.as<int>() + 2, 0, prec, grad != nullptr, s));
     const cudaMemcpyKind k = mem == GEO_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    if (recon) GEO_CUDA(cudaMemcpyAsync(recon, rec.p, (size_t)nb * kAePts * 4, k, s));
-    if (grad) GEO_CUDA(cudaMemcpyAsync(grad, ae->grad.p, ae->off.total * 4, k, s));
     double l = 0;
-    GEO_CUDA(cudaMemcpyAsync(&l, dl.p, 8, cudaMemcpyDeviceToHost, s));
+    GEO_CUDA(cudaMemcpyAsync(&l, ae->ev.p, 8, cudaMemcpyDeviceToHost, s));
+    GEO_TRY(ae_check_err(ae, s));
+    if (recon && prec != recon) GEO_CUDA(cudaMemcpyAsync(recon, prec, (size_t)nb * kAePts * 4, k, s));
+    if (grad) GEO_CUDA(cudaMemcpyAsync(grad, ae->grad.p, ae->off.total * 4, k, s));
     GEO_CUDA(cudaStreamSynchronize(s));
     if (loss) *loss = l / kAePts;
     return GEO_OK;
@@ -1204,7 +1306,8 @@ extern "C" int geo_ae_train(geo_ae *ae, int iters, int batch, float lr, float *l
         a.step0 = step0;
         k_ae_e1<<<batch, 256, 0, s>>>(a);
         GEO_TRY(check_launch("ae_e1"));
-        GEO_TRY(train_pass(ae, batch, dloss.as<double>(), dwsum.as<float>(), step0, nullptr, true, s));
+        GEO_TRY(train_pass(ae, batch, dloss.as<double>(), dwsum.as<float>(), ae->step.as<int>(), step0, nullptr, true,
+                           s));
         k_ae_adam<<<152 * 4, 256, 0, s>>>(ae->params.as<float>(), ae->grad.as<float>(), ae->m1.as<float>(),
                                           ae->m2.as<float>(), ae->off.total, ae->step.as<int>(), step0,
                                           dlr.as<float>());
