@@ -15,10 +15,10 @@
 // Training (one CUDA graph per iteration): the same forward on blocks drawn
 // from a store of solver snapshots (k_ae_e1, weights read from the device
 // copy that Adam updates inside the graph), the loss and the D1 backward in
-// k_ae_d1, per level the weight gradient (k_ae_wgrad, CUDA cores, fp32), the
-// bias gradient (k_ae_colsum) and the input gradient (tc_gemm against the
-// transposed weights, the activation derivative fused as a gate), E1's
-// weight gradient (k_ae_e1_bwd), then Adam and the bf16 repack.
+// k_ae_d1, per level the input gradient (tc_gemm against the transposed
+// weights, the activation derivative fused as a gate), then every level's
+// weight gradient (tc_wgrad) and bias gradient (k_ae_colsum) in one launch
+// each, E1's weight gradient (k_ae_e1_bwd), Adam and the bf16 repack.
 #include "ae.cuh"
 #include "tc_gemm.cuh"
 #include "fd3d.cuh"
@@ -598,55 +598,43 @@ __global__ void __launch_bounds__(256) k_ae_e1_bwd(const float *xn, const __nv_b
     block_outer<false, 1, 8>(sm, ge1, ge1 + 128);   // W1[j * 8 + c]
 }
 
-// grad[n*K + k] += sum_m dy[m*N + n] * x[m*K + k] over this split's rows.
-__global__ void __launch_bounds__(256) k_ae_wgrad(const __nv_bfloat16 *dy, const __nv_bfloat16 *x, float *grad, int M,
-                                                  int N, int K, int rows) {
-    __shared__ float ys[32][64];
-    __shared__ float xs[32][65];
-    const int k0 = blockIdx.x * 64, n0 = blockIdx.y * 64;
-    const int mb = blockIdx.z * rows, me = min(M, mb + rows);
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float acc[4][4];
+// Bias gradients of the GEMM levels in one launch: gb[n] += sum over the
+// rows of dy[m*N + n].  A thread sums 8 columns (one 16-byte load per row)
+// over every (256 / (N/8))-th row of its block's range, the block reduces
+// through shared memory and adds N values.  Latency-bound (4 MB of reads at
+// 256 blocks); one launch for the six levels instead of one each.
+struct ColsumLevel {
+    const __nv_bfloat16 *dy;
+    float *gb;
+    int M, N, base, ctas;
+};
+struct ColsumArgs {
+    ColsumLevel it[6];
+};
+
+__global__ void __launch_bounds__(256) k_ae_colsum(const ColsumArgs g) {
+    __shared__ float red[256 * 8];
+    int l = 0;
+    while (l < 5 && (int)blockIdx.x >= g.it[l + 1].base) l++;
+    const ColsumLevel &w = g.it[l];
+    const int rel = (int)blockIdx.x - w.base, t = threadIdx.x;
+    const int m0 = (int)((long)w.M * rel / w.ctas), m1 = (int)((long)w.M * (rel + 1) / w.ctas);
+    const int cg = w.N / 8, per = 256 / cg, col = t % cg, r0 = t / cg;   // N <= 2048, a multiple of 64
+    float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int m = m0 + r0; m < m1; m += per) {
+        const uint4 q = *reinterpret_cast<const uint4 *>(w.dy + (long)m * w.N + col * 8);
+        const __nv_bfloat16 *h = reinterpret_cast<const __nv_bfloat16 *>(&q);
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
-    for (int m0 = mb; m0 < me; m0 += 32) {
-        for (int i = threadIdx.x; i < 32 * 64; i += 256) {
-            const int r = i >> 6, c = i & 63, m = m0 + r;
-            ys[r][c] = m < me ? __bfloat162float(dy[(long)m * N + n0 + c]) : 0.0f;
-            xs[r][c] = m < me ? __bfloat162float(x[(long)m * K + k0 + c]) : 0.0f;
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int r = 0; r < 32; r++) {
-            float av[4], bv[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                av[i] = ys[r][ty * 4 + i];
-                bv[i] = xs[r][tx * 4 + i];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] += av[i] * bv[j];
-        }
-        __syncthreads();
+        for (int j = 0; j < 8; j++) s[j] += __bfloat162float(h[j]);
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) atomicAdd(&grad[(long)(n0 + ty * 4 + i) * K + k0 + tx * 4 + j], acc[i][j]);
-}
-
-// gb[n] += sum_m dy[m*N + n] over this split's rows.
-__global__ void __launch_bounds__(256) k_ae_colsum(const __nv_bfloat16 *dy, float *gb, int M, int N, int rows) {
-    const int n = blockIdx.x * 256 + threadIdx.x;
-    if (n >= N) return;
-    const int mb = blockIdx.y * rows, me = min(M, mb + rows);
-    float s = 0.0f;
-    for (int m = mb; m < me; m++) s += __bfloat162float(dy[(long)m * N + n]);
-    atomicAdd(&gb[n], s);
+    for (int j = 0; j < 8; j++) red[t * 8 + j] = s[j];
+    __syncthreads();
+    for (int n = t; n < w.N; n += 256) {
+        float v = 0.0f;
+        for (int r = 0; r < per; r++) v += red[r * w.N + n];
+        atomicAdd(w.gb + n, v);
+    }
 }
 
 // Adam (bias-corrected) with the step's learning rate from lrs[*step - step0].
@@ -840,43 +828,51 @@ static int level(geo_ae *ae, int l, int rows, const __nv_bfloat16 *in, __nv_bflo
     return tc_gemm(g, s);
 }
 
-// Backward through GEMM level l: weight and bias gradients, and (if din)
-// the input gradient gated by the input activation (null gate: linear).
-static int level_bwd(geo_ae *ae, int l, int rows, const __nv_bfloat16 *dout, const __nv_bfloat16 *in,
-                     __nv_bfloat16 *din, const __nv_bfloat16 *gate, cudaStream_t s) {
+// Input gradient of GEMM level l, gated by the input activation (null gate:
+// linear).
+static int level_bwd(geo_ae *ae, int l, int rows, const __nv_bfloat16 *dout, __nv_bfloat16 *din,
+                     const __nv_bfloat16 *gate, cudaStream_t s) {
     const AeLayer &L = kAeNet[l];
-    const int M = rows * L.rows;
-    float *gw = ae->grad.as<float>() + ae->off.w[l], *gbias = ae->grad.as<float>() + ae->off.b[l];
-    {
-        const int tiles = (L.K / 64) * (L.N / 64);
-        int splits = (2 * 152 * 2 + tiles - 1) / tiles;
-        splits = std::max(1, std::min(splits, M / 32));
-        const int rws = ((M + splits - 1) / splits + 31) / 32 * 32;
-        splits = (M + rws - 1) / rws;
-        k_ae_wgrad<<<dim3(L.K / 64, L.N / 64, splits), 256, 0, s>>>(dout, in, gw, M, L.N, L.K, rws);
-        GEO_TRY(check_launch("ae_wgrad"));
+    TcGemm g{};
+    g.M = rows * L.rows;
+    g.N = L.K;
+    g.K = L.N;
+    g.A = dout;
+    g.B = bf(ae->wtb) + ae->off.wb[l];
+    g.gate = gate;
+    g.out = din;
+    g.err = ae->err.as<int>();
+    return tc_gemm(g, s);
+}
+
+// Weight and bias gradients of the GEMM levels 1..6 from their output
+// gradients dout[l] and inputs in[l]: one launch each.
+static int wgrads(geo_ae *ae, int rows, const __nv_bfloat16 *const *dout, const __nv_bfloat16 *const *in,
+                  cudaStream_t s) {
+    TcWgradLevel lv[6];
+    ColsumArgs c{};
+    int base = 0;
+    for (int q = 0; q < 6; q++) {
+        const int l = q + 1;
+        const AeLayer &L = kAeNet[l];
+        const int M = rows * L.rows;
+        float *gw = ae->grad.as<float>() + ae->off.w[l];
+        // the 128-row operand is dY, or X where dY has only 64 columns
+        const bool xa = L.N % 128 != 0;
+        lv[q] = TcWgradLevel{M, xa ? in[l] : dout[l], xa ? dout[l] : in[l], xa ? L.K : L.N, xa ? L.N : L.K, gw,
+                             xa ? 1L : (long)L.K, xa ? (long)L.K : 1L};
+        ColsumLevel &k = c.it[q];
+        k.dy = dout[l];
+        k.gb = ae->grad.as<float>() + ae->off.b[l];
+        k.M = M;
+        k.N = L.N;
+        k.base = base;
+        k.ctas = std::max(1, std::min(M / 16, 64));
+        base += k.ctas;
     }
-    {
-        const int cb = (L.N + 255) / 256;
-        int splits = std::max(1, std::min(M / 64, (152 * 8) / cb));
-        const int rws = (M + splits - 1) / splits;
-        splits = (M + rws - 1) / rws;
-        k_ae_colsum<<<dim3(cb, splits), 256, 0, s>>>(dout, gbias, M, L.N, rws);
-        GEO_TRY(check_launch("ae_colsum"));
-    }
-    if (din) {
-        TcGemm g{};
-        g.M = M;
-        g.N = L.K;
-        g.K = L.N;
-        g.A = dout;
-        g.B = bf(ae->wtb) + ae->off.wb[l];
-        g.gate = gate;
-        g.out = din;
-        g.err = ae->err.as<int>();
-        GEO_TRY(tc_gemm(g, s));
-    }
-    return GEO_OK;
+    GEO_TRY(tc_wgrad(lv, 6, ae->err.as<int>(), s));
+    k_ae_colsum<<<base, 256, 0, s>>>(c);
+    return check_launch("ae_colsum");
 }
 
 // Encoder levels E2..E4 from h1 into `code` (rows x 512 bf16).
@@ -1067,12 +1063,15 @@ static int train_pass(geo_ae *ae, int rows, double *loss, const float *wsum, con
     k_ae_d1<<<rows, 256, kOutFloats * 4, s>>>(a);
     GEO_TRY(check_launch("ae_d1_train"));
     if (!backward) return GEO_OK;
-    GEO_TRY(level_bwd(ae, 6, rows, bf(ae->dg1), bf(ae->g2), bf(ae->dg2), bf(ae->g2), s));   // D2
-    GEO_TRY(level_bwd(ae, 5, rows, bf(ae->dg2), bf(ae->g3), bf(ae->dg3), bf(ae->g3), s));   // D3
-    GEO_TRY(level_bwd(ae, 4, rows, bf(ae->dg3), bf(ae->z), bf(ae->dz), nullptr, s));        // D4
-    GEO_TRY(level_bwd(ae, 3, rows, bf(ae->dz), bf(ae->h3), bf(ae->dh3), bf(ae->h3), s));    // E4
-    GEO_TRY(level_bwd(ae, 2, rows, bf(ae->dh3), bf(ae->h2), bf(ae->dh2), bf(ae->h2), s));   // E3
-    GEO_TRY(level_bwd(ae, 1, rows, bf(ae->dh2), bf(ae->h1), bf(ae->dh1), bf(ae->h1), s));   // E2
+    GEO_TRY(level_bwd(ae, 6, rows, bf(ae->dg1), bf(ae->dg2), bf(ae->g2), s));   // D2
+    GEO_TRY(level_bwd(ae, 5, rows, bf(ae->dg2), bf(ae->dg3), bf(ae->g3), s));   // D3
+    GEO_TRY(level_bwd(ae, 4, rows, bf(ae->dg3), bf(ae->dz), nullptr, s));       // D4
+    GEO_TRY(level_bwd(ae, 3, rows, bf(ae->dz), bf(ae->dh3), bf(ae->h3), s));    // E4
+    GEO_TRY(level_bwd(ae, 2, rows, bf(ae->dh3), bf(ae->dh2), bf(ae->h2), s));   // E3
+    GEO_TRY(level_bwd(ae, 1, rows, bf(ae->dh2), bf(ae->dh1), bf(ae->h1), s));   // E2
+    const __nv_bfloat16 *dout[7] = {nullptr, bf(ae->dh2), bf(ae->dh3), bf(ae->dz), bf(ae->dg3), bf(ae->dg2), bf(ae->dg1)};
+    const __nv_bfloat16 *in[7] = {nullptr, bf(ae->h1), bf(ae->h2), bf(ae->h3), bf(ae->z), bf(ae->g3), bf(ae->g2)};
+    GEO_TRY(wgrads(ae, rows, dout, in, s));
     k_ae_e1_bwd<<<rows, 256, kOutFloats * 4, s>>>(ae->xn.as<float>(), bf(ae->dh1), ae->grad.as<float>() + ae->off.w[0], rows);
     return check_launch("ae_e1_bwd");
 }

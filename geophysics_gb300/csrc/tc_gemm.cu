@@ -260,6 +260,176 @@ int tc_gemm(const TcGemm &g, cudaStream_t s) {
     return launch_bn_k<64>(g, s);
 }
 
+// ---------------------------------------------------------- weight gradients
+// dW = dY^T X of every codec level in one launch.  The contraction runs over
+// the rows, which are the slow dimension of both operands in memory, so both
+// are handed to tcgen05.mma MN-major: a TMA box of 64 rows x 64 columns is a
+// swizzled operand slice as it lies.  A CTA owns a 128 x (64 or 128) tile of
+// one level's dW and a range of 64-row slices (three-stage TMA ring, the same
+// roles and bounded waits as k_tc_gemm) and adds its tile to the gradient
+// with vector reductions.  The levels have 1 to 64 tiles and 4 to 256 slices
+// at 256 blocks; the slices of a tile are split so that each level fills the
+// chip once (kWgradCtas), and all levels share the launch, which leaves one
+// partial wave instead of six.  Bound by latency and by the reductions (a
+// few MB into L2), not by the tensor cores (7 GFLOP, 4 us at peak).
+// 256 blocks: 19.7 us, against 197 us for six CUDA-core launches.
+struct WgradItem {
+    float *out;
+    long sa, sb;
+    int base, tb, splits, slices, bn;   // first CTA, tiles along b, splits, slices in all, tile width
+};
+struct WgradArgs {
+    CUtensorMap ta[kWgradMax], tb[kWgradMax];
+    WgradItem it[kWgradMax];
+    int n;
+    int *err;
+};
+
+constexpr int kWgStages = 3, kWgBox = 64 * 128, kWgA = 2 * kWgBox, kWgStage = 4 * kWgBox;
+constexpr size_t kWgSmem = (size_t)kWgStages * kWgStage + 1024 + 128;
+constexpr int kWgradCtas = 128;
+static_assert(2 * kWgSmem <= 232448 && 2 * 128 <= 512, "two CTAs per SM");
+
+__device__ __forceinline__ void red_add4(float *p, float a, float b, float c, float d) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d)
+                 : "memory");
+}
+
+__global__ void __launch_bounds__(128, 2) k_tc_wgrad(const __grid_constant__ WgradArgs g) {
+    extern __shared__ unsigned char smem_raw[];
+    uint8_t *sm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint64_t *full = reinterpret_cast<uint64_t *>(sm + (size_t)kWgStages * kWgStage);
+    uint64_t *empty = full + kWgStages;
+    uint64_t *done = empty + kWgStages;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(done + 1);
+    __shared__ int s_abort;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int l = 0;
+    while (l + 1 < g.n && (int)blockIdx.x >= g.it[l + 1].base) l++;
+    const WgradItem &w = g.it[l];
+    const int rel = (int)blockIdx.x - w.base, tile = rel / w.splits, sp = rel % w.splits;
+    const int a0 = (tile / w.tb) * 128, b0 = (tile % w.tb) * w.bn;
+    const int s0 = (int)((long)w.slices * sp / w.splits), nk = (int)((long)w.slices * (sp + 1) / w.splits) - s0;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kWgStages; s++) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(done, 1);
+        s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    if (warp == 0) tmem_alloc(tslot, 128);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tslot;
+    const int nbox = w.bn / 64;
+
+    if (warp == 0 && lane == 0) {
+        int issued = 0;
+        for (int kb = 0; kb < nk; kb++) {
+            const int s = kb % kWgStages;
+            if (kb >= kWgStages && !mbar_wait(&empty[s], ((kb / kWgStages) - 1) & 1)) {
+                s_abort = 1;
+                break;
+            }
+            uint8_t *st = sm + s * kWgStage;
+            const int m = (s0 + kb) * 64;
+            mbar_expect_tx(&full[s], (2 + nbox) * kWgBox);
+            tma2(st, &g.ta[l], a0, m, &full[s]);
+            tma2(st + kWgBox, &g.ta[l], a0 + 64, m, &full[s]);
+            for (int q = 0; q < nbox; q++) tma2(st + kWgA + q * kWgBox, &g.tb[l], b0 + 64 * q, m, &full[s]);
+            issued = kb + 1;
+        }
+        if (*(volatile int *)&s_abort)
+            for (int kb = issued > kWgStages ? issued - kWgStages : 0; kb < issued; kb++)
+                mbar_wait(&full[kb % kWgStages], (kb / kWgStages) & 1);
+    } else if (warp == 1 && lane == 0) {
+        const uint32_t idesc = idesc_bf16_f32_mn(128, w.bn);
+        for (int kb = 0; kb < nk; kb++) {
+            const int s = kb % kWgStages;
+            if (!mbar_wait(&full[s], (kb / kWgStages) & 1)) {
+                s_abort = 1;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t pa = su32(sm + s * kWgStage), pb = pa + kWgA;
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                mma_bf16(tmem, sdesc_mn128(pa + k * 2048, kWgBox), sdesc_mn128(pb + k * 2048, kWgBox), idesc,
+                         (kb | k) != 0);
+            mma_commit(&empty[s]);
+        }
+        mma_commit(done);
+    }
+    __syncwarp();
+
+    if (!mbar_wait(done, 0)) s_abort = 1;
+    tc_fence_after();
+    const bool ok = !*(volatile int *)&s_abort;
+    float *row = w.out + (long)(a0 + warp * 32 + lane) * w.sa + (long)b0 * w.sb;
+#pragma unroll 1
+    for (int c0 = 0; c0 < w.bn; c0 += 16) {
+        uint32_t r[16];
+        tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
+        if (!ok) continue;
+        if (w.sb == 1) {
+#pragma unroll
+            for (int j = 0; j < 16; j += 4)
+                red_add4(row + c0 + j, __uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
+                         __uint_as_float(r[j + 3]));
+        } else {
+#pragma unroll
+            for (int j = 0; j < 16; j++) atomicAdd(row + (long)(c0 + j) * w.sb, __uint_as_float(r[j]));
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (s_abort && threadIdx.x == 0) atomicExch(g.err, 2);
+    if (warp == 0) tmem_dealloc(tmem, 128);
+}
+
+int tc_wgrad(const TcWgradLevel *lv, int n, int *err, cudaStream_t s) {
+    if (n < 1 || n > kWgradMax || !err) return fail(GEO_ERR_ARG, "tc_wgrad: 1 to %d levels", kWgradMax);
+    WgradArgs g;
+    int base = 0;
+    for (int l = 0; l < n; l++) {
+        const TcWgradLevel &L = lv[l];
+        if (L.M <= 0 || L.M % 64 || L.wa % 128 || (L.wb != 64 && L.wb % 128) || !L.A || !L.B || !L.out ||
+            (L.sa != 1 && L.sb != 1) || (L.sa * L.sb) % 4)
+            return fail(GEO_ERR_ARG, "tc_wgrad: bad level (M=%d wa=%d wb=%d)", L.M, L.wa, L.wb);
+        if ((reinterpret_cast<uintptr_t>(L.A) | reinterpret_cast<uintptr_t>(L.B) |
+             reinterpret_cast<uintptr_t>(L.out)) & 15)
+            return fail(GEO_ERR_ARG, "tc_wgrad: operands must be 16-byte aligned");
+        GEO_TRY(encode_bf16_2d(&g.ta[l], L.A, L.M, L.wa, 64));
+        GEO_TRY(encode_bf16_2d(&g.tb[l], L.B, L.M, L.wb, 64));
+        WgradItem &w = g.it[l];
+        w.out = L.out;
+        w.sa = L.sa;
+        w.sb = L.sb;
+        w.bn = L.wb == 64 ? 64 : 128;
+        w.tb = L.wb / w.bn;
+        w.slices = L.M / 64;
+        const int tiles = (L.wa / 128) * w.tb;
+        w.splits = (kWgradCtas + tiles - 1) / tiles;
+        if (w.splits > w.slices) w.splits = w.slices;
+        w.base = base;
+        base += tiles * w.splits;
+    }
+    g.n = n;
+    g.err = err;
+    static bool attr = false;
+    if (!attr) {
+        GEO_CUDA(cudaFuncSetAttribute(k_tc_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgSmem));
+        attr = true;
+    }
+    k_tc_wgrad<<<base, 128, kWgSmem, s>>>(g);
+    return check_launch("tc_wgrad");
+}
+
 }  // namespace geo
 
 // C-ABI entry for tests and callers with their own bf16 operands (device

@@ -23,4 +23,17 @@ constexpr float kLeak = 0.1f;
 
 int tc_gemm(const TcGemm &g, cudaStream_t s);
 
+// Weight gradients of up to kWgradMax levels in one launch: for each,
+// out[a*sa + b*sb] += sum over m < M of A[m*wa + a] * B[m*wb + b].
+struct TcWgradLevel {
+    int M;                            // rows, M % 64 == 0
+    const __nv_bfloat16 *A, *B;       // [M x wa], [M x wb] row-major
+    int wa, wb;                       // wa % 128 == 0, wb == 64 or wb % 128 == 0
+    float *out;                       // fp32, accumulated into; 16-byte aligned
+    long sa, sb;                      // one of them 1
+};
+constexpr int kWgradMax = 6;
+
+int tc_wgrad(const TcWgradLevel *lv, int n, int *err, cudaStream_t s);
+
 }  // namespace geo

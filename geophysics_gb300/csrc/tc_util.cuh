@@ -91,9 +91,29 @@ __device__ __forceinline__ uint64_t sdesc_k128(uint32_t saddr) {
     return d;
 }
 
+// Shared-memory descriptor of an operand stored contraction-row by
+// contraction-row (MN-major): TMA boxes of 64 bf16 columns (one 128-byte
+// swizzled line per contraction row), 8-row groups 1024 B apart (stride
+// byte offset), further 64-column boxes `box_bytes` apart (leading byte
+// offset).  Stepping 16 contraction rows adds 2048 B to the start address.
+__device__ __forceinline__ uint64_t sdesc_mn128(uint32_t saddr, uint32_t box_bytes) {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)(box_bytes >> 4) << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;            // descriptor version
+    d |= (uint64_t)2 << 61;            // 128-byte swizzle
+    return d;
+}
+
 // Instruction descriptor, kind::f16: D f32, A and B bf16, both K-major.
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+
+// The same with both operands MN-major (transpose bits 15 and 16).
+__host__ __device__ constexpr uint32_t idesc_bf16_f32_mn(int M, int N) {
+    return idesc_bf16_f32(M, N) | (1u << 15) | (1u << 16);
 }
 
 // D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.

@@ -58,6 +58,24 @@ def test_codec_forward_and_gradients_match_oracle(geo):
     print("codec gradient worst rel-L2 per tensor: %.3g" % worst)
 
 
+# weight gradients of every level from 2 to 40 row slices per split, and
+# E2's transposed tile: against the numpy oracle (bf16 activations, tolerance
+# as above)
+@pytest.mark.parametrize("nb", [128, 256, 640])
+def test_codec_gradients_over_batch_sizes(geo, nb):
+    from oracle import ae_oracle as A
+    codec = geo.Codec(seed=11)
+    blocks = wave_blocks(nb, 23)
+    _, loss, g = codec.eval(blocks)
+    lo, go = A.backward(codec.params(), blocks)
+    codec.close()
+    assert abs(loss - lo) <= 3e-3 * lo
+    for l, (ow, ob) in enumerate(A.offsets()[0]):
+        N, K, _, _ = A.LAYERS[l]
+        for q, n in ((ow, N * K), (ob, N)):
+            assert rel_l2(g[q:q + n], go[q:q + n]) < 3e-3, (nb, l)
+
+
 @pytest.mark.parametrize("mode", [0, 1])
 def test_rtm3d_snapshot_method_bit_exact(geo, orc, mode):
     v, e, d = random_model_3d(20, 17, 23, seed=11)
