@@ -32,6 +32,8 @@ constexpr int kGM = 128, kGK = 64;
 // is then padded so that no more CTAs fit than tensor memory holds
 // accumulators for (512 columns per SM), so no allocation ever waits.
 constexpr int default_stages(int bn) { return bn >= 256 ? 2 : (bn >= 128 ? 3 : 4); }
+// GEMMs of few tiles take narrow ones with a deep ring instead (launch_bn_k).
+constexpr int kDeepStages = 8;
 constexpr size_t kSmSmem = 233472;      // shared memory per SM
 constexpr size_t kCtaReserve = 1024;    // reserved per resident CTA
 
@@ -51,8 +53,8 @@ struct GemmShape {
     static constexpr size_t kSmem = kRing > kFloor ? kRing : kFloor;
     static_assert(kA % 1024 == 0 && kB % 1024 == 0, "swizzle atoms stay 1024-byte aligned");
     static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "UMMA N for M = 128");
-    static_assert(ST >= 1 && ST <= default_stages(BN), "stage count");
-    static_assert(2 * kSmem <= 232448, "two CTAs per SM");
+    static_assert(ST >= 1 && (ST <= default_stages(BN) || ST == kDeepStages), "stage count");
+    static_assert((ST == kDeepStages ? 1 : 2) * kSmem <= 232448, "two CTAs per SM, or one with the deep ring");
     static_assert((kSmSmem / (kSmem + kCtaReserve)) * kCols <= 512, "resident CTAs' accumulators fit in TMEM");
 };
 
@@ -236,10 +238,22 @@ static int launch_bn(const TcGemm &g, cudaStream_t s) {
     return check_launch("tc_gemm");
 }
 
+// Tile width: the widest that divides N and leaves a tile for every SM,
+// else 64.  A training batch of 256 blocks has 4 to 32 tiles of width 256
+// (E4: 4 CTAs walking 32 K slices each behind a two-slot ring), so the chip
+// idles and a slice costs a full memory latency; with width 64 and, where
+// no more than one CTA lands on an SM anyway, an eight-slot ring, the ten
+// input and output GEMMs of such an evaluation take 80 us instead of
+// 145 us.  From 152 tiles on the wide tile's fewer operand reads win
+// (k_tc_gemm<256> at 24 576 blocks: 90 us a level).
+constexpr long kFewTiles = 152;
+
 // stages = K slices, up to the tile width's default
 template <int BN>
 static int launch_bn_k(const TcGemm &g, cudaStream_t s) {
     const int nk = g.K / kGK;
+    if constexpr (BN == 64)
+        if (nk > 4 && (long)(g.M / kGM) * (g.N / BN) <= kFewTiles) return launch_bn<BN, kDeepStages>(g, s);
     if constexpr (default_stages(BN) >= 4)
         if (nk >= 4) return launch_bn<BN, 4>(g, s);
     if constexpr (default_stages(BN) >= 3)
@@ -255,8 +269,9 @@ int tc_gemm(const TcGemm &g, cudaStream_t s) {
     const uintptr_t al = reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B) |
                          reinterpret_cast<uintptr_t>(g.out) | reinterpret_cast<uintptr_t>(g.gate);
     if (al & 15) return fail(GEO_ERR_ARG, "tc_gemm: operands must be 16-byte aligned");
-    if (g.N % 256 == 0) return launch_bn_k<256>(g, s);
-    if (g.N % 128 == 0) return launch_bn_k<128>(g, s);
+    const long mt = g.M / kGM;
+    if (g.N % 256 == 0 && mt * (g.N / 256) >= kFewTiles) return launch_bn_k<256>(g, s);
+    if (g.N % 128 == 0 && mt * (g.N / 128) >= kFewTiles) return launch_bn_k<128>(g, s);
     return launch_bn_k<64>(g, s);
 }
 

@@ -58,6 +58,21 @@ def test_codec_forward_and_gradients_match_oracle(geo):
     print("codec gradient worst rel-L2 per tensor: %.3g" % worst)
 
 
+# the widest tile from 152 tiles on, one tile fewer (64 wide, eight-slot
+# ring), and every stage count of the wide tiles
+@pytest.mark.parametrize("M,N,K", [(19456, 256, 64), (19456, 256, 512), (19328, 256, 512), (19456, 128, 64),
+                                   (19456, 128, 128), (19456, 128, 320), (9728, 512, 128), (19456, 64, 320)])
+def test_tc_gemm_tile_width_rule(geo, M, N, K):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    A = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    B = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    ref = A.double() @ B.double().T
+    out = geo.tc_gemm_bf16(A, B)
+    # K fp32 additions of products of size |a||b|
+    assert (out - ref).abs().max().item() <= 1e-5 * ref.abs().max().item()
+
+
 # weight gradients of every level from 2 to 40 row slices per split, and
 # E2's transposed tile: against the numpy oracle (bf16 activations, tolerance
 # as above)
