@@ -5,6 +5,7 @@
 // (velocity, stress) covering every shot's tiles; the time loops are
 // captured once into CUDA graphs and replayed.
 #include "geo_internal.h"
+#include "model2d.cuh"
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -25,174 +26,236 @@ static int sm_count() {
     return n;
 }
 
-// Host-side working set of one shot (window) plus its device buffers.
-struct ShotHost {
-    int nx, nz, npd, nnx, nnz;
-    Variant var;
-    std::vector<float> vp, e2, d2, cx1, cx2, cz1, cz2, ax1, ax2, az1, az2;
-    std::vector<double> kz, kx;     // MPI exact form: the chains' double factors per point
-    Taper2D taper;
-    std::vector<float> te2, td2;
-    std::vector<double> tkz, tkx;   // the same on the taper box
-    int ixs, izs;
-    float mu_v;
-    DevBuf d_model, d_k, d_prof, d_taper, d_tk, d_fields, d_rec, d_edge, d_img, d_adcig;
+// One shot's window of the model and its source.
+struct ShotGeom {
+    int nx, col0;        // window width, model column of window column 0
+    float srcx, srcz;    // source position inside the window, 1-based
 };
 
-// Build the propagation coefficients of one (padded) window from its
-// unpadded model; Variant picks the reference program's formulas.
-static void build_shot_host(ShotHost &h, Variant var, int nx, int nz, int npd, float dx, float dz, float dt,
-                            const float *v, const float *e, const float *d, float srcx, float srcz, bool taper,
-                            bool fast = false) {
-    h.var = var;
-    h.nx = nx; h.nz = nz; h.npd = npd;
-    h.nnx = nx + 2 * npd; h.nnz = nz + 2 * npd;
-    const size_t n = (size_t)h.nnx * h.nnz;
-    std::vector<float> pv(n), pe(n), pd(n);
-    pad_model_2d(nx, nz, npd, v, pv.data());
-    pad_model_2d(nx, nz, npd, e, pe.data());
-    pad_model_2d(nx, nz, npd, d, pd.data());
-    float vpmax = v[0];
-    for (size_t k = 0; k < (size_t)nx * nz; k++) vpmax = std::max(vpmax, v[k]);
-    const float d0 = sponge_d0(var, 2, vpmax, pv[(size_t)h.nnx * h.nnz / 2], npd, dx, dx, dz);
-    h.cx1.resize(h.nnx); h.cx2.resize(h.nnx); h.ax1.resize(h.nnx); h.ax2.resize(h.nnx);
-    h.cz1.resize(h.nnz); h.cz2.resize(h.nnz); h.az1.resize(h.nnz); h.az2.resize(h.nnz);
-    sponge_profiles(var, nx, npd, dt, d0, h.cx1.data(), h.cx2.data(), h.ax1.data(), h.ax2.data());
-    sponge_profiles(var, nz, npd, dt, d0, h.cz1.data(), h.cz2.data(), h.az1.data(), h.az2.data());
-    // source cell: (int)(fs+0.5)+npd-1 (CPU_vti2dfd_kernels.c:65-66)
-    h.ixs = (int)(srcx + 0.5) + npd - 1;
-    h.izs = (int)(srcz + 0.5) + npd - 1;
-    h.vp.resize(n); h.e2.resize(n); h.d2.resize(n);
+// The shots of one run on the device: model and state in one allocation,
+// the profiles and taper boxes in another.
+struct ShotSet {
+    Variant var;
+    int nz, npd, nnz;
+    bool taper;
+    std::vector<ShotGeom> G;
+    std::vector<Shot2D> S;
+    RawStats st;
+    float v00, e00;               // model values at unpadded (0, 0)
+    std::vector<float> mu_v;      // MPI mute velocity of each shot
+    Arena mem;
+    Blob small;
+    size_t o_amp = 0, o_on = 0;
+    // cleared state: fields of side 0 of every shot, then of side 1, images
+    // and gathers, records
+    size_t z_side0 = 0, z_side1 = 0, z_img = 0, z_rec = 0, z_end = 0;
+    int clear(size_t from, size_t to, cudaStream_t s) {
+        if (to > from) GEO_CUDA(cudaMemsetAsync(mem.buf.as<char>() + from, 0, to - from, s));
+        return GEO_OK;
+    }
+    static constexpr int kPick = 3 + 3 * kTB * kTB;   // centre v, v(1,1), e(1,1); v, e, d on the taper box
+    void source(int k, int &ixs, int &izs) const {
+        // source cell: (int)(fs+0.5)+npd-1 (CPU_vti2dfd_kernels.c:65-66)
+        ixs = (int)(G[k].srcx + 0.5) + npd - 1;
+        izs = (int)(G[k].srcz + 0.5) + npd - 1;
+    }
+    // CPU/MPI circle centre = the source cell; GPU form centre is
+    // (fs+(is-1)ds+npd, zs+npd), one cell right/down of it
+    void centre(int k, int &cx, int &cz) const {
+        source(k, cx, cz);
+        if (var == V_GPU) {
+            cx++;
+            cz++;
+        }
+    }
+    int read(const Raw2D &raw, cudaStream_t s);
+    int build(const Raw2D &raw, float dx, float dz, float dt, const std::vector<float> &amp,
+              const std::vector<uint8_t> &on, int nfields, int nt, bool edges, bool image, bool adcig, bool fast,
+              cudaStream_t s);
+};
+
+// The model values the set-up formulas read, with the model check.
+int ShotSet::read(const Raw2D &raw, cudaStream_t s) {
+    std::vector<unsigned long long> pick;
+    pick.reserve(2 + G.size() * kPick);
+    pick.push_back(raw_at(0, raw, 0, 0));
+    pick.push_back(raw_at(1, raw, 0, 0));
+    for (size_t k = 0; k < G.size(); k++) {
+        const int nx = G[k].nx, nnx = nx + 2 * npd;
+        auto at = [&](int a, int ix, int iz) {   // padded position
+            const int sx = std::min(std::max(ix - npd, 0), nx - 1) + G[k].col0;
+            const int sz = std::min(std::max(iz - npd, 0), nz - 1);
+            return raw_at(a, raw, std::min(sx, raw.nx - 1), sz);
+        };
+        const size_t c = (size_t)nnx * nnz / 2;
+        pick.push_back(at(0, (int)(c / nnz), (int)(c % nnz)));
+        pick.push_back(at(0, 1 + npd, 1 + npd));
+        pick.push_back(at(1, 1 + npd, 1 + npd));
+        int cx, cz;
+        centre(k, cx, cz);
+        for (int a = 0; a < 3; a++)
+            for (int b = 0; b < kTB * kTB; b++)
+                pick.push_back(taper ? at(a, cx - kTB / 2 + b / kTB, cz - kTB / 2 + b % kTB) : 0);
+    }
+    GEO_TRY(raw_stats(raw, pick, st, s));
+    v00 = st.val[0];
+    e00 = st.val[1];
+    return GEO_OK;
+}
+
+// Propagation coefficients and state of every shot; var picks the reference
+// program's formulas.
+int ShotSet::build(const Raw2D &raw, float dx, float dz, float dt, const std::vector<float> &amp,
+                   const std::vector<uint8_t> &on, int nfields, int nt, bool edges, bool image, bool adcig, bool fast,
+                   cudaStream_t s) {
+    const int ns = (int)G.size();
     // the MPI program's pz and qx chains are
     //   (double)(az2*pz) - (double)(az1*vp) * pow(1+2del,0.5) * (double)dtz * (double)zz
     // (and with ax, dtx, xx for qx), evaluated left to right; every factor but
     // zz is fixed for the shot, so the product of the first three is formed
-    // here once, in the same order and precision, and the kernel issues one
-    // double multiply and one double subtraction per chain
+    // once, in the same order and precision (ModelJob::kz), and the kernel
+    // issues one double multiply and one double subtraction per chain.  The
+    // program's pow runs on the host, once per model point.
     const bool kchain = var == V_MPI && !fast;
     const double ddtx = (double)(dt / dx), ddtz = (double)(dt / dz);
+    S.assign(ns, Shot2D{});
+    mu_v.resize(ns);
+    DevBuf d_pw;
     if (kchain) {
-        h.kz.resize(n);
-        h.kx.resize(n);
+        const size_t n0 = (size_t)raw.nx * raw.nz;
+        std::vector<float> hd(n0);
+        std::vector<double> pw(n0);
+        GEO_CUDA(cudaMemcpyAsync(hd.data(), raw.a[2], n0 * 4, cudaMemcpyDeviceToHost, s));
+        GEO_CUDA(cudaStreamSynchronize(s));
+        host_pow_half(hd.data(), n0, pw.data());
+        GEO_TRY(d_pw.alloc(n0 * 8));
+        GEO_CUDA(cudaMemcpyAsync(d_pw.p, pw.data(), n0 * 8, cudaMemcpyHostToDevice, s));
+        GEO_CUDA(cudaStreamSynchronize(s));   // pw is freed below
     }
-    for (size_t k = 0; k < n; k++) {
-        // MPI program: vp <- rho*vp^2 with rho == 1 (Toa_rtm_vti_adcig_cdp.c:641)
-        h.vp[k] = (var == V_MPI) ? 1.0f * (pv[k] * pv[k]) : pv[k];
-        h.e2[k] = 1 + 2 * pe[k];
-        h.d2[k] = sqrtf(1 + 2 * pd[k]);
-        if (kchain) {
-            const double pw = std::pow((double)(1 + 2 * pd[k]), 0.5);
-            const size_t ix = k / h.nnz, iz = k % h.nnz;
-            h.kz[k] = (double)(h.az1[iz] * h.vp[k]) * pw * ddtz;
-            h.kx[k] = (double)(h.ax1[ix] * h.vp[k]) * pw * ddtx;
+    struct Off {
+        size_t prof[8], te2, td2, tkz, tkx;
+    };
+    std::vector<Off> off(ns);
+    for (int k = 0; k < ns; k++) {
+        const ShotGeom &g = G[k];
+        const int nnx = g.nx + 2 * npd;
+        const float *val = st.val.data() + 2 + (size_t)k * kPick;
+        float vpmax = 0.0f;
+        for (int c = 0; c < g.nx; c++) vpmax = std::max(vpmax, st.colmax[std::min(c + g.col0, raw.nx - 1)]);
+        const float d0 = sponge_d0(var, 2, vpmax, val[0], npd, dx, dx, dz);
+        mu_v[k] = val[1] * sqrtf(1 + 2 * val[2]);
+        std::vector<float> p[8];
+        for (int q = 0; q < 8; q++) p[q].resize(q < 4 ? nnx : nnz);
+        sponge_profiles(var, g.nx, npd, dt, d0, p[0].data(), p[1].data(), p[2].data(), p[3].data());
+        sponge_profiles(var, nz, npd, dt, d0, p[4].data(), p[5].data(), p[6].data(), p[7].data());
+        for (int q = 0; q < 8; q++) off[k].prof[q] = small.put(p[q]);
+        Shot2D &h = S[k];
+        source(k, h.ixs, h.izs);
+        h.tx0 = h.tz0 = -100000;
+        if (!taper) continue;
+        int cx, cz;
+        centre(k, cx, cz);
+        Taper2D tp;
+        const float *vbox = val + 3;
+        sv_taper_2d(var, nnx, nnz, cx, cz, vbox + kTB * kTB, vbox + 2 * kTB * kTB, tp);
+        h.tx0 = tp.x0;
+        h.tz0 = tp.z0;
+        std::vector<float> te2(kTB * kTB, 1.0f), td2(kTB * kTB, 1.0f);
+        for (int b = 0; b < kTB * kTB; b++) {
+            te2[b] = 1 + 2 * tp.e[b];
+            td2[b] = sqrtf(1 + 2 * tp.d[b]);
         }
+        off[k].te2 = small.put(te2);
+        off[k].td2 = small.put(td2);
+        if (!kchain) continue;
+        std::vector<double> tkz(kTB * kTB, 0.0), tkx(kTB * kTB, 0.0);
+        for (int b = 0; b < kTB * kTB; b++) {
+            const int ix = tp.x0 + b / kTB, iz = tp.z0 + b % kTB;
+            if (ix < 0 || ix >= nnx || iz < 0 || iz >= nnz) continue;
+            const double pw = std::pow((double)(1 + 2 * tp.d[b]), 0.5);
+            const float vpk = 1.0f * (vbox[b] * vbox[b]);
+            tkz[b] = (double)(p[6][iz] * vpk) * pw * ddtz;
+            tkx[b] = (double)(p[2][ix] * vpk) * pw * ddtx;
+        }
+        off[k].tkz = small.put(tkz);
+        off[k].tkx = small.put(tkx);
     }
-    h.mu_v = pv[(size_t)(1 + npd) * h.nnz + 1 + npd] * sqrtf(1 + 2 * pe[(size_t)(1 + npd) * h.nnz + 1 + npd]);
-    if (taper) {
-        // CPU/MPI circle centre = the source cell; GPU form centre is
-        // (fs+(is-1)ds+npd, zs+npd), one cell right/down of it
-        const int cx = (var == V_GPU) ? h.ixs + 1 : h.ixs, cz = (var == V_GPU) ? h.izs + 1 : h.izs;
-        sv_taper_2d(var, h.nnx, h.nnz, npd, cx, cz, pe.data(), pd.data(), h.taper);
-        h.te2.assign(kTB * kTB, 1.0f); h.td2.assign(kTB * kTB, 1.0f);
-        if (kchain) {
-            h.tkz.assign(kTB * kTB, 0.0);
-            h.tkx.assign(kTB * kTB, 0.0);
-        }
-        for (int k = 0; k < kTB * kTB; k++) {
-            const float ee = h.taper.e[k], dd = h.taper.d[k];
-            h.te2[k] = 1 + 2 * ee;
-            h.td2[k] = sqrtf(1 + 2 * dd);
-            const int ix = h.taper.x0 + k / kTB, iz = h.taper.z0 + k % kTB;
-            if (kchain && ix >= 0 && ix < h.nnx && iz >= 0 && iz < h.nnz) {
-                const double pw = std::pow((double)(1 + 2 * dd), 0.5);
-                const float vpk = h.vp[(size_t)ix * h.nnz + iz];
-                h.tkz[k] = (double)(h.az1[iz] * vpk) * pw * ddtz;
-                h.tkx[k] = (double)(h.ax1[ix] * vpk) * pw * ddtx;
+    o_amp = small.put(amp);
+    o_on = small.put(on);
+    GEO_TRY(small.upload(s));
+    // two passes: sizes, then addresses
+    std::vector<ModelJob> jobs(ns);
+    for (int pass = 0; pass < 2; pass++) {
+        z_side0 = 0;
+        for (int f = 0; f < nfields; f++) {
+            if (f == 1) z_side1 = mem.off;
+            for (int k = 0; k < ns; k++) {
+                const size_t n = (size_t)(G[k].nx + 2 * npd) * nnz;
+                float **dst[8] = {&S[k].u[f], &S[k].w[f], &S[k].P[f], &S[k].Q[f],
+                                  &S[k].px[f], &S[k].pz[f], &S[k].qx[f], &S[k].qz[f]};
+                for (auto d : dst) *d = mem.take<float>(n);
             }
         }
-    }
-}
-
-// Upload one shot and fill its device descriptor.
-static int upload_shot(ShotHost &h, Shot2D &S, int nfields, int nt, bool records, bool edges, bool image,
-                       float dtx, float dtz, cudaStream_t s) {
-    const size_t n = (size_t)h.nnx * h.nnz;
-    GEO_TRY(h.d_model.alloc(3 * n * 4));
-    float *m = h.d_model.as<float>();
-    GEO_CUDA(cudaMemcpyAsync(m, h.vp.data(), n * 4, cudaMemcpyHostToDevice, s));
-    GEO_CUDA(cudaMemcpyAsync(m + n, h.e2.data(), n * 4, cudaMemcpyHostToDevice, s));
-    GEO_CUDA(cudaMemcpyAsync(m + 2 * n, h.d2.data(), n * 4, cudaMemcpyHostToDevice, s));
-    if (!h.kz.empty()) {
-        GEO_TRY(h.d_k.alloc(2 * n * 8));
-        GEO_CUDA(cudaMemcpyAsync(h.d_k.p, h.kz.data(), n * 8, cudaMemcpyHostToDevice, s));
-        GEO_CUDA(cudaMemcpyAsync(h.d_k.as<double>() + n, h.kx.data(), n * 8, cudaMemcpyHostToDevice, s));
-    }
-    const size_t np = 4 * (size_t)h.nnx + 4 * (size_t)h.nnz;
-    GEO_TRY(h.d_prof.alloc(np * 4));
-    float *pr = h.d_prof.as<float>();
-    const std::vector<float> *prof[8] = {&h.cx1, &h.cx2, &h.ax1, &h.ax2, &h.cz1, &h.cz2, &h.az1, &h.az2};
-    size_t o = 0;
-    const float *dp[8];
-    for (int k = 0; k < 8; k++) {
-        GEO_CUDA(cudaMemcpyAsync(pr + o, prof[k]->data(), prof[k]->size() * 4, cudaMemcpyHostToDevice, s));
-        dp[k] = pr + o;
-        o += prof[k]->size();
-    }
-    memset(&S, 0, sizeof S);
-    S.nnx = h.nnx; S.nnz = h.nnz; S.npd = h.npd; S.nx = h.nx; S.nz = h.nz;
-    S.dtx = dtx; S.dtz = dtz;
-    S.cx1 = dp[0]; S.cx2 = dp[1]; S.ax1 = dp[2]; S.ax2 = dp[3];
-    S.cz1 = dp[4]; S.cz2 = dp[5]; S.az1 = dp[6]; S.az2 = dp[7];
-    S.vp = m; S.e2 = m + n; S.d2 = m + 2 * n;
-    S.kz = h.kz.empty() ? nullptr : h.d_k.as<double>();
-    S.kx = h.kz.empty() ? nullptr : h.d_k.as<double>() + n;
-    if (!h.te2.empty()) {
-        GEO_TRY(h.d_taper.alloc(2 * kTB * kTB * 4));
-        GEO_CUDA(cudaMemcpyAsync(h.d_taper.p, h.te2.data(), kTB * kTB * 4, cudaMemcpyHostToDevice, s));
-        GEO_CUDA(cudaMemcpyAsync(h.d_taper.as<float>() + kTB * kTB, h.td2.data(), kTB * kTB * 4, cudaMemcpyHostToDevice, s));
-        if (!h.tkz.empty()) {
-            GEO_TRY(h.d_tk.alloc(2 * kTB * kTB * 8));
-            GEO_CUDA(cudaMemcpyAsync(h.d_tk.p, h.tkz.data(), kTB * kTB * 8, cudaMemcpyHostToDevice, s));
-            GEO_CUDA(cudaMemcpyAsync(h.d_tk.as<double>() + kTB * kTB, h.tkx.data(), kTB * kTB * 8,
-                                     cudaMemcpyHostToDevice, s));
+        if (nfields < 2) z_side1 = mem.off;
+        z_img = mem.off;
+        for (int k = 0; k < ns; k++) {
+            const size_t m = (size_t)G[k].nx * nz;
+            if (image) {
+                S[k].mig = mem.take<float>(m);
+                S[k].ill = mem.take<float>(m);
+            }
+            if (adcig) S[k].adcig = mem.take<float>(kAdcigAngles * m);
         }
-        S.tx0 = h.taper.x0; S.tz0 = h.taper.z0;
-        S.te2 = h.d_taper.as<float>(); S.td2 = h.d_taper.as<float>() + kTB * kTB;
-        S.tkz = h.tkz.empty() ? nullptr : h.d_tk.as<double>();
-        S.tkx = h.tkz.empty() ? nullptr : h.d_tk.as<double>() + kTB * kTB;
-    } else {
-        S.tx0 = -100000; S.tz0 = -100000;
+        z_rec = mem.off;
+        for (int k = 0; k < ns; k++) {
+            S[k].rec_p = mem.take<float>((size_t)nt * G[k].nx);
+            S[k].rec_q = edges ? mem.take<float>((size_t)nt * G[k].nx) : nullptr;
+        }
+        z_end = mem.off;
+        for (int k = 0; k < ns; k++) {
+            const int nnx = G[k].nx + 2 * npd;
+            const size_t n = (size_t)nnx * nnz, L = 2 * (size_t)G[k].nx + 2 * (size_t)nz;
+            ModelJob &j = jobs[k];
+            j.nx = G[k].nx; j.nz = nz; j.npd = npd; j.ldz = nnz; j.col0 = G[k].col0;
+            j.vp2 = var == V_MPI;   // vp <- rho*vp^2 with rho == 1 (Toa_rtm_vti_adcig_cdp.c:641)
+            j.vp = mem.take<float>(n);
+            j.e2 = mem.take<float>(n);
+            j.d2 = kchain ? nullptr : mem.take<float>(n);
+            j.rad = nullptr;
+            j.kz = kchain ? mem.take<double>(n) : nullptr;
+            j.kx = kchain ? mem.take<double>(n) : nullptr;
+            j.pw = d_pw.as<double>();
+            j.ddtx = ddtx; j.ddtz = ddtz;
+            if (edges) {
+                S[k].edge_p = mem.take<float>((size_t)nt * L);
+                S[k].edge_q = mem.take<float>((size_t)nt * L);
+            }
+        }
+        if (pass == 0) GEO_TRY(mem.alloc());
     }
-    S.ixs = h.ixs; S.izs = h.izs;
-    GEO_TRY(h.d_fields.alloc((size_t)8 * nfields * n * 4));
-    GEO_TRY(h.d_fields.zero(s));
-    float *f = h.d_fields.as<float>();
-    for (int k = 0; k < nfields; k++) {
-        float *b = f + (size_t)8 * k * n;
-        S.u[k] = b; S.w[k] = b + n; S.P[k] = b + 2 * n; S.Q[k] = b + 3 * n;
-        S.px[k] = b + 4 * n; S.pz[k] = b + 5 * n; S.qx[k] = b + 6 * n; S.qz[k] = b + 7 * n;
+    for (int k = 0; k < ns; k++) {
+        Shot2D &h = S[k];
+        h.nnx = G[k].nx + 2 * npd; h.nnz = nnz; h.npd = npd; h.nx = G[k].nx; h.nz = nz;
+        h.dtx = dt / dx; h.dtz = dt / dz;
+        const float **dp[8] = {&h.cx1, &h.cx2, &h.ax1, &h.ax2, &h.cz1, &h.cz2, &h.az1, &h.az2};
+        for (int q = 0; q < 8; q++) *dp[q] = small.at<float>(off[k].prof[q]);
+        ModelJob &j = jobs[k];
+        j.ax1 = h.ax1;
+        j.az1 = h.az1;
+        h.vp = j.vp; h.e2 = j.e2; h.d2 = j.d2; h.kz = j.kz; h.kx = j.kx;
+        if (taper) {
+            h.te2 = small.at<float>(off[k].te2);
+            h.td2 = small.at<float>(off[k].td2);
+            if (kchain) {
+                h.tkz = small.at<double>(off[k].tkz);
+                h.tkx = small.at<double>(off[k].tkx);
+            }
+        }
+        h.rec_iz = npd;
+        h.rec_scale = 1.0f;
     }
-    S.rec_iz = h.npd;
-    S.rec_scale = 1.0f;
-    if (records) {
-        GEO_TRY(h.d_rec.alloc((size_t)2 * nt * h.nx * 4));
-        GEO_TRY(h.d_rec.zero(s));
-        S.rec_p = h.d_rec.as<float>();
-        S.rec_q = S.rec_p + (size_t)nt * h.nx;
-    }
-    if (edges) {
-        const size_t L = 2 * (size_t)h.nx + 2 * (size_t)h.nz;
-        GEO_TRY(h.d_edge.alloc((size_t)2 * nt * L * 4));
-        S.edge_p = h.d_edge.as<float>();
-        S.edge_q = S.edge_p + (size_t)nt * L;
-    }
-    if (image) {
-        GEO_TRY(h.d_img.alloc((size_t)2 * h.nx * h.nz * 4));
-        GEO_TRY(h.d_img.zero(s));
-        S.mig = h.d_img.as<float>();
-        S.ill = S.mig + (size_t)h.nx * h.nz;
-    }
-    return GEO_OK;
+    GEO_TRY(launch_model2d(raw, jobs, s));
+    return clear(0, z_end, s);
 }
 
 // Work list: item -> shot.  Tiles are 32 (z) x by (x).
@@ -382,18 +445,6 @@ static int autotune(Batch2D &B, int nf, int key_nx, int key_nz, cudaStream_t s, 
     return GEO_OK;
 }
 
-static int host_model(const float *v, const float *e, const float *d, size_t n, int mem, cudaStream_t s,
-                      std::vector<float> &hv, std::vector<float> &he, std::vector<float> &hd) {
-    hv.resize(n); he.resize(n); hd.resize(n);
-    const cudaMemcpyKind k = mem == GEO_MEM_DEVICE ? cudaMemcpyDeviceToHost : cudaMemcpyHostToHost;
-    if (mem != GEO_MEM_DEVICE && mem != GEO_MEM_HOST) return fail(GEO_ERR_ARG, "bad mem kind");
-    GEO_CUDA(cudaMemcpyAsync(hv.data(), v, n * 4, k, s));
-    GEO_CUDA(cudaMemcpyAsync(he.data(), e, n * 4, k, s));
-    GEO_CUDA(cudaMemcpyAsync(hd.data(), d, n * 4, k, s));
-    GEO_CUDA(cudaStreamSynchronize(s));
-    return check_model(hv.data(), he.data(), hd.data(), n);
-}
-
 // Event-ordered hand-off between the caller's stream and a private one.
 struct SideStream {
     cudaStream_t cs = nullptr;
@@ -429,36 +480,38 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
     const int nnx = D.nx + 2 * D.npd, nnz = D.nz + 2 * D.npd;
     if (D.rec_iz < 4 || D.rec_iz >= nnz - 4) return fail(GEO_ERR_ARG, "receiver row outside grid");
     cudaStream_t s = (cudaStream_t)stream;
-    std::vector<float> hv, he, hd;
-    GEO_TRY(host_model(v, e, d, (size_t)D.nx * D.nz, mem, s, hv, he, hd));
     const Variant var = (Variant)D.variant;
-    {
-        const auto mm = std::minmax_element(hv.begin(), hv.end());
-        GEO_TRY(check_stability(var, 2, *mm.first, *mm.second, D.dt, D.dx, D.dx, D.dz, D.favg));
-    }
-    const float fsx = D.fs + (D.is - 1) * D.ds;
-    ShotHost h;
-    const bool taper = var == V_MPI || D.sv;
-    build_shot_host(h, var, D.nx, D.nz, D.npd, D.dx, D.dz, D.dt, hv.data(), he.data(), hd.data(), fsx, D.zs, taper);
-    if (h.ixs < 4 || h.ixs >= nnx - 4 || h.izs < 4 || h.izs >= nnz - 4)
-        return fail(GEO_ERR_ARG, "source outside the updated grid");
-    if (var == V_CPU || var == V_MPI)
-        if (h.ixs - 3 < 0 || h.ixs + 3 >= nnx || h.izs - 3 < 0 || h.izs + 3 >= nnz)
-            return fail(GEO_ERR_ARG, "source window outside grid");
     SideStream ss;
     GEO_TRY(ss.open(s));
-    Batch2D B;
-    B.variant = var;
-    B.S.resize(1);
-    GEO_TRY(upload_shot(h, B.S[0], 1, D.nt, true, false, false, D.dt / D.dx, D.dt / D.dz, ss.cs));
-    B.S[0].rec_iz = D.rec_iz;
-    B.S[0].rec_scale = D.rec_scale;
-    B.S[0].rec_q = nullptr;
-    const bool persistent = !(snap && snap_every > 0);
-    GEO_TRY(B.upload(persistent ? 16 : 8, 8, ss.cs));
+    Raw2D raw;
+    GEO_TRY(raw.open(D.nx, D.nz, v, e, d, nullptr, mem, ss.cs));
+    const bool taper = var == V_MPI || D.sv;
+    ShotSet X;
+    X.var = var;
+    X.nz = D.nz; X.npd = D.npd; X.nnz = nnz;
+    X.taper = taper;
+    X.G = {ShotGeom{D.nx, 0, D.fs + (D.is - 1) * D.ds, D.zs}};
+    GEO_TRY(X.read(raw, ss.cs));
+    GEO_TRY(check_stability(var, 2, X.st.vmin, X.st.vmax, D.dt, D.dx, D.dx, D.dz, D.favg));
+    int ixs, izs;
+    X.source(0, ixs, izs);
+    if (ixs < 4 || ixs >= nnx - 4 || izs < 4 || izs >= nnz - 4)
+        return fail(GEO_ERR_ARG, "source outside the updated grid");
+    if (var == V_CPU || var == V_MPI)
+        if (ixs - 3 < 0 || ixs + 3 >= nnx || izs - 3 < 0 || izs + 3 >= nnz)
+            return fail(GEO_ERR_ARG, "source window outside grid");
     std::vector<float> amp;
     std::vector<uint8_t> on;
     source_amplitudes(var, D.nt, D.dt, D.favg, D.pfac, D.wtype, amp, on);
+    GEO_TRY(X.build(raw, D.dx, D.dz, D.dt, amp, on, 1, D.nt, false, false, false, false, ss.cs));
+    const float *d_amp = X.small.at<float>(X.o_amp);
+    const unsigned char *d_on = X.small.at<unsigned char>(X.o_on);
+    Batch2D B;
+    B.variant = var;
+    B.S = X.S;
+    B.S[0].rec_iz = D.rec_iz;
+    B.S[0].rec_scale = D.rec_scale;
+    const bool persistent = !(snap && snap_every > 0);
     auto step = [&](int it) -> int {
         Step2D st{};
         st.it = it;
@@ -469,6 +522,11 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
         GEO_TRY(B.vel(st, ss.cs));
         return B.stress(PH_FWD, st, ss.cs);
     };
+    DevBuf d_sync;
+    GEO_TRY(d_sync.alloc(8));
+    GEO_TRY(d_sync.zero(ss.cs));
+    unsigned *bar = d_sync.as<unsigned>();
+    int *errw = d_sync.as<int>() + 1;
     const size_t nn = (size_t)nnx * nnz;
     Watchdog wd;
     GEO_TRY(wd.open());
@@ -478,17 +536,9 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
     // between snapshots, when the grid fits on the device that way
     bool tiled = false;
     if (var == V_CPU || var == V_GPU) {
-        DevBuf xch, d_amp, d_on, d_sync;
+        DevBuf xch;
         GEO_TRY(xch.alloc(8 * nn * 4));
         GEO_TRY(xch.zero(ss.cs));
-        GEO_TRY(d_amp.alloc((size_t)D.nt * 4));
-        GEO_TRY(d_on.alloc((size_t)D.nt));
-        GEO_TRY(d_sync.alloc(8));
-        GEO_TRY(d_sync.zero(ss.cs));
-        GEO_CUDA(cudaMemcpyAsync(d_amp.p, amp.data(), (size_t)D.nt * 4, cudaMemcpyHostToDevice, ss.cs));
-        GEO_CUDA(cudaMemcpyAsync(d_on.p, on.data(), (size_t)D.nt, cudaMemcpyHostToDevice, ss.cs));
-        unsigned *bar = d_sync.as<unsigned>();
-        int *errw = d_sync.as<int>() + 1;
         for (int it0 = 0; it0 < D.nt;) {
             int it1 = it0 + 1;
             if (snap && snap_every > 0)
@@ -496,8 +546,7 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
             else
                 it1 = D.nt;
             bool fits = false;
-            GEO_TRY(launch_fd2d_tile(var, B.S[0], xch.as<float>(), d_amp.as<float>(), d_on.as<unsigned char>(),
-                                     taper ? 1 : 0, it0, it1, bar, errw, &fits, ss.cs));
+            GEO_TRY(launch_fd2d_tile(var, B.S[0], xch.as<float>(), d_amp, d_on, taper ? 1 : 0, it0, it1, bar, errw, &fits, ss.cs));
             if (!fits) {   // decided by the grid alone, so on the first run of steps
                 if (tiled) return fail(GEO_ERR_CUDA, "2D shot: tile-resident launch refused mid-run");
                 break;
@@ -507,7 +556,7 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
             if (snap && snap_every > 0 && it % snap_every == 0)
                 GEO_CUDA(cudaMemcpyAsync(snap + (size_t)(it / snap_every) * nn, B.S[0].P[0], nn * 4, ksnap, ss.cs));
             if (wd.every > 0) {
-                GEO_TRY(launch_watch_shots(B.d_S.as<Shot2D>(), 1, 1, wd.d, it + 1, ss.cs));
+                GEO_TRY(wd.scan(B.S[0].P[0], nn, it + 1, ss.cs));
                 if (wd.tripped()) break;
             }
             it0 = it1;
@@ -520,6 +569,7 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
             if (wd.every > 0) GEO_TRY(wd.scan(B.S[0].rec_p, (size_t)D.nx * D.nt, D.nt, ss.cs));
         }
     }
+    if (!tiled) GEO_TRY(B.upload(persistent ? 16 : 8, 8, ss.cs));
     if (!tiled && snap && snap_every > 0) {
         for (int it = 0; it < D.nt; it++) {
             GEO_TRY(step(it));
@@ -533,20 +583,13 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
     } else if (!tiled) {
         // the whole shot in one cooperative launch (grid barriers between the
         // half-steps, bounded waits reported through an error word)
-        DevBuf d_amp, d_on, d_sync;
-        GEO_TRY(d_amp.alloc((size_t)D.nt * 4));
-        GEO_TRY(d_on.alloc((size_t)D.nt));
-        GEO_TRY(d_sync.alloc(8));
-        GEO_TRY(d_sync.zero(ss.cs));
-        GEO_CUDA(cudaMemcpyAsync(d_amp.p, amp.data(), (size_t)D.nt * 4, cudaMemcpyHostToDevice, ss.cs));
-        GEO_CUDA(cudaMemcpyAsync(d_on.p, on.data(), (size_t)D.nt, cudaMemcpyHostToDevice, ss.cs));
         Persist2D a{};
         a.nt = D.nt;
         a.taper = taper ? 1 : 0;
-        a.amp = d_amp.as<float>();
-        a.on = d_on.as<unsigned char>();
-        a.bar = d_sync.as<unsigned>();
-        a.err = d_sync.as<int>() + 1;
+        a.amp = d_amp;
+        a.on = d_on;
+        a.bar = bar;
+        a.err = errw;
         GEO_TRY(launch_fd2d_shot(var, B.d_S.as<Shot2D>(), B.d_items.as<int>(), (int)B.items.size(), B.by, a, ss.cs));
         int err = 0;
         GEO_CUDA(cudaMemcpyAsync(&err, a.err, 4, cudaMemcpyDeviceToHost, ss.cs));
@@ -562,15 +605,11 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
     DevBuf mlo, mhi, out;
     if (D.mute_tt > 0) {
         std::vector<int> lo, hi;
-        // vp[1]*sqrtf(1+2*eps[1]) of the padded model (GPU_vti2dfd_kernels.cu:167)
-        {
-            std::vector<float> pv((size_t)nnx * nnz), pe((size_t)nnx * nnz);
-            pad_model_2d(D.nx, D.nz, D.npd, hv.data(), pv.data());
-            pad_model_2d(D.nx, D.nz, D.npd, he.data(), pe.data());
-            const float mu_v = pv[1] * sqrtf(1 + 2 * pe[1]);
-            mute_window_gpu2d(D.nx, D.nt, D.dt, D.favg, D.dx, D.dz, (int)D.fs, (int)D.ds, (int)D.zs, D.is, mu_v,
-                              D.mute_tt, lo, hi);
-        }
+        // vp[1]*sqrtf(1+2*eps[1]) of the padded model (GPU_vti2dfd_kernels.cu:167):
+        // the sponge is at least five cells wide, so the model's first cell
+        const float mu_v = X.v00 * sqrtf(1 + 2 * X.e00);
+        mute_window_gpu2d(D.nx, D.nt, D.dt, D.favg, D.dx, D.dz, (int)D.fs, (int)D.ds, (int)D.zs, D.is, mu_v, D.mute_tt,
+                          lo, hi);
         GEO_TRY(mlo.alloc(lo.size() * 4));
         GEO_TRY(mhi.alloc(hi.size() * 4));
         GEO_CUDA(cudaMemcpyAsync(mlo.p, lo.data(), lo.size() * 4, cudaMemcpyHostToDevice, ss.cs));
@@ -611,58 +650,41 @@ extern "C" int geo_rtm2d_batch_adcig(const geo_rtm2d_desc *desc, const float *v,
     if (D.mode != GEO_MODE_EXACT && D.mode != GEO_MODE_FAST) return fail(GEO_ERR_ARG, "bad mode %d", D.mode);
     const int fast = D.mode == GEO_MODE_FAST;
     cudaStream_t s = (cudaStream_t)stream;
-    std::vector<float> hv, he, hd;
-    GEO_TRY(host_model(v, e, d, (size_t)D.nx * D.nz, mem, s, hv, he, hd));
     SideStream ss;
     GEO_TRY(ss.open(s));
+    Raw2D raw;
+    GEO_TRY(raw.open(D.nx, D.nz, v, e, d, nullptr, mem, ss.cs));
     const float dt = D.dt_ms / 1000;
     const int nt = D.nt, nz = D.nz, npd = D.npd;
-    {
-        const auto mm = std::minmax_element(hv.begin(), hv.end());
-        GEO_TRY(check_stability(V_MPI, 2, *mm.first, *mm.second, dt, D.dx, D.dx, D.dz, D.favg));
-    }
-    std::vector<std::unique_ptr<ShotHost>> H(D.ns);
-    Batch2D B;
-    B.variant = V_MPI;
-    B.S.resize(D.ns);
+    ShotSet X;
+    X.var = V_MPI;
+    X.nz = nz; X.npd = npd; X.nnz = nz + 2 * npd;
+    X.taper = true;
     int maxline = 0;
     for (int k = 0; k < D.ns; k++) {
         const int nxs = D.shot_nxs[k], kk = D.shot_x[k];
-        // window column c <- model column c + k - nxs/2, clamped into the pad
-        std::vector<float> wv((size_t)nxs * nz), we((size_t)nxs * nz), wd((size_t)nxs * nz);
-        for (int c = 0; c < nxs; c++) {
-            int col = c + kk - nxs / 2;
-            col = std::min(col, D.nx - 1);
-            memcpy(&wv[(size_t)c * nz], &hv[(size_t)col * nz], nz * 4);
-            memcpy(&we[(size_t)c * nz], &he[(size_t)col * nz], nz * 4);
-            memcpy(&wd[(size_t)c * nz], &hd[(size_t)col * nz], nz * 4);
-        }
-        H[k].reset(new ShotHost());
+        // window column c <- model column c + k - nxs/2, clamped into the pad;
         // shot position inside its window: fs = nxs/2+1, ds = 0
-        build_shot_host(*H[k], V_MPI, nxs, nz, npd, D.dx, D.dz, dt, wv.data(), we.data(), wd.data(),
-                        (float)(nxs / 2 + 1), (float)D.zs, true, fast != 0);
-        GEO_TRY(upload_shot(*H[k], B.S[k], 2, nt, true, true, true, dt / D.dx, dt / D.dz, ss.cs));
-        if (adcig) {
-            GEO_TRY(H[k]->d_adcig.alloc((size_t)kAdcigAngles * nxs * nz * 4));
-            B.S[k].adcig = H[k]->d_adcig.as<float>();
-        }
+        X.G.push_back(ShotGeom{nxs, kk - nxs / 2, (float)(nxs / 2 + 1), (float)D.zs});
         maxline = std::max(maxline, 2 * nxs + 2 * nz);
     }
+    GEO_TRY(X.read(raw, ss.cs));
+    GEO_TRY(check_stability(V_MPI, 2, X.st.vmin, X.st.vmax, dt, D.dx, D.dx, D.dz, D.favg));
+    std::vector<float> amp;
+    std::vector<uint8_t> on;
+    source_amplitudes(V_MPI, nt, dt, D.favg, D.pfac, 1, amp, on);
+    GEO_TRY(X.build(raw, D.dx, D.dz, dt, amp, on, 2, nt, true, true, adcig != nullptr, fast != 0, ss.cs));
+    Batch2D B;
+    B.variant = V_MPI;
+    B.S = X.S;
     // tile shape: caller's choice or the autotuner's
     int by = D.tile_x, bps = 8;
     if (by != 4 && by != 8) GEO_TRY(autotune(B, 2, D.nx, D.nz, ss.cs, &by, &bps));
     GEO_TRY(B.upload(by, bps, ss.cs));
     // the autotuner stepped the state: start from zero again
-    for (int k = 0; k < D.ns; k++) {
-        GEO_TRY(H[k]->d_fields.zero(ss.cs));
-        GEO_TRY(H[k]->d_img.zero(ss.cs));
-        if (adcig) GEO_TRY(H[k]->d_adcig.zero(ss.cs));
-    }
+    GEO_TRY(X.clear(X.z_side0, X.z_rec, ss.cs));
     if (adcig) GEO_TRY(load_adcig_tables(ss.cs));
 
-    std::vector<float> amp;
-    std::vector<uint8_t> on;
-    source_amplitudes(V_MPI, nt, dt, D.favg, D.pfac, 1, amp, on);
     // non-finite detector: every wd.every steps (and the last) the graphs
     // scan every shot's P; the verdict follows each pass
     Watchdog wd;
@@ -705,18 +727,22 @@ extern "C" int geo_rtm2d_batch_adcig(const geo_rtm2d_desc *desc, const float *v,
     }
     GEO_TRY(wd.verdict(ss.cs, "batched 2D RTM forward pass"));
     // mute both records (tt = 285) and restart the source side from zero
-    std::vector<DevBuf> mute(D.ns);
+    std::vector<int> mute;
     for (int k = 0; k < D.ns; k++) {
         const int nxs = D.shot_nxs[k];
         std::vector<int> lo, hi;
-        mute_window_mpi(nxs, nt, D.dt_ms, D.favg, D.dx, D.dz, nxs / 2 + 1, 0, D.zs, k + 1, H[k]->mu_v, 285, lo, hi);
-        GEO_TRY(mute[k].alloc(hi.size() * 4));
-        GEO_CUDA(cudaMemcpyAsync(mute[k].p, hi.data(), hi.size() * 4, cudaMemcpyHostToDevice, ss.cs));
-        GEO_TRY(launch_mute_records(B.S[k].rec_p, nxs, nt, nullptr, mute[k].as<int>(), ss.cs));
-        GEO_TRY(launch_mute_records(B.S[k].rec_q, nxs, nt, nullptr, mute[k].as<int>(), ss.cs));
-        const size_t n = (size_t)H[k]->nnx * H[k]->nnz;
-        GEO_CUDA(cudaMemsetAsync(B.S[k].u[0], 0, 8 * n * 4, ss.cs));
+        mute_window_mpi(nxs, nt, D.dt_ms, D.favg, D.dx, D.dz, nxs / 2 + 1, 0, D.zs, k + 1, X.mu_v[k], 285, lo, hi);
+        mute.insert(mute.end(), hi.begin(), hi.end());
     }
+    DevBuf d_mute;
+    GEO_TRY(d_mute.alloc(mute.size() * 4));
+    GEO_CUDA(cudaMemcpyAsync(d_mute.p, mute.data(), mute.size() * 4, cudaMemcpyHostToDevice, ss.cs));
+    for (int k = 0, o = 0; k < D.ns; o += D.shot_nxs[k++]) {
+        const int *hi = d_mute.as<int>() + o;
+        GEO_TRY(launch_mute_records(B.S[k].rec_p, D.shot_nxs[k], nt, nullptr, hi, ss.cs));
+        GEO_TRY(launch_mute_records(B.S[k].rec_q, D.shot_nxs[k], nt, nullptr, hi, ss.cs));
+    }
+    GEO_TRY(X.clear(X.z_side0, X.z_side1, ss.cs));
     // backward: inject, both propagations, fused imaging
     {
         Graph G;

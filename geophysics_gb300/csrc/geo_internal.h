@@ -91,10 +91,6 @@ struct Watchdog {
     int verdict(cudaStream_t s, const char *what);
 };
 
-// Edge-replicate an nx*nz model into its padded (nx+2npd)*(nz+2npd) form.
-void pad_model_2d(int nx, int nz, int npd, const float *in, float *out);
-// Same for 3D, reference layout iz + nz*(ix + nx*iy).
-
 float sponge_d0(Variant v, int dims, float vpmax, float vcenter, int npd, float dx, float dy, float dz);
 // coff1/coff2 on half cells (velocities), acoff1/acoff2 on integer cells
 // (stresses); arrays of n+2npd.
@@ -108,8 +104,8 @@ struct Taper2D {
     int x0 = 0, z0 = 0, n = 0;            // box origin (padded) and size
     std::vector<float> e, d;              // tapered values on the box
 };
-void sv_taper_2d(Variant v, int nnx, int nnz, int npd, int ixs_center, int izs_center,
-                 const float *e_pad, const float *d_pad, Taper2D &out);
+void sv_taper_2d(Variant v, int nnx, int nnz, int ixs_center, int izs_center, const float *e_box, const float *d_box,
+                 Taper2D &out);
 
 // Per-trace direct-wave mute window [lo, hi) of samples to zero.
 void mute_window_gpu2d(int nx, int nt, float dt, float favg, float dx, float dz, int fs, int ds,
@@ -132,9 +128,6 @@ int adcig_angle_tables(int nangle, int dangle, float *thr, float *cs, cudaStream
 // Raw float32 files: read exactly n values; write n values at a byte offset.
 int read_floats(const char *fn, size_t n, std::vector<float> &out);
 int write_at(FILE *fp, size_t offset_bytes, const float *a, size_t n);
-
-// Model sanity: finite, velocity > 0.
-int check_model(const float *v, const float *e, const float *d, size_t n);
 
 // ------------------------------------------------------------ 2D device side
 constexpr int kTB = 31;  // taper box edge (circle radius 15)

@@ -39,6 +39,7 @@
 #include "adcig.cuh"
 #include "tti2d.cuh"
 #include "gridsync.cuh"
+#include "model2d.cuh"
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -301,9 +302,15 @@ __global__ void __launch_bounds__(256, 4) k_grtm_bwd(const GCoop a) {
     }
 }
 
-__global__ void k_g_mask(float *rec, const uint8_t *keep, long n) {
-    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x)
-        if (!keep[k]) rec[k] = 0.0f;
+// Zero samples lo <= it < hi of every trace, as flat positions ix*nt + it of
+// the trace-major record inside it (the record itself is time-major).
+__global__ void k_g_mute(float *rec, const int *lo, const int *hi, int nx, int nt) {
+    const int it = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int ix = blockIdx.y; ix < nx; ix += gridDim.y) {
+        if (it < lo[ix] || it >= hi[ix]) continue;
+        const long j = (long)ix * nt + it;
+        if (j < (long)nx * nt) rec[(j % nt) * nx + j / nt] = 0.0f;
+    }
 }
 
 // gathers [ixa][ia][iz] /= ill[ixa*dcdp][iz]
@@ -383,12 +390,7 @@ static int gpu_adcig_tables(int nangle, int dangle, cudaStream_t s) {
 }
 
 // readFile's checks (:930-965): grid spacing for the frequency, dt, dispersion, stability.
-static int gpu_rtm_checks(const geo_rtm2d_gpu_desc &D, const std::vector<float> &v) {
-    float vmin = 999999.9f, vmax = -999999.9f;
-    for (float x : v) {
-        vmin = std::min(vmin, x);
-        vmax = std::max(vmax, x);
-    }
+static int gpu_rtm_checks(const geo_rtm2d_gpu_desc &D, float vmin, float vmax) {
     const float H_min = D.dx < D.dz ? D.dx : D.dz;
     const float dt_max = (float)(0.5 * H_min / vmin), dxz_max = (float)(vmax / D.favg * 0.2);
     if (dxz_max < D.dz || dxz_max < D.dx) return fail(GEO_ERR_CFL, "grid spacing too coarse for favg (redefine dx, dz)");
@@ -426,30 +428,37 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
     const int nx = D.nx, nz = D.nz, npml = D.npml, nt = D.nt, nnx = nx + 2 * npml, nnz = nz + 2 * npml;
     const size_t n0 = (size_t)nx * nz, n = (size_t)nnx * nnz;
     cudaStream_t s = (cudaStream_t)stream;
-    std::vector<float> hv(n0), he(n0), hd(n0), ht(prog.tti ? n0 : 0);
-    const float *src[4] = {v, e, d, theta};
-    float *dst[4] = {hv.data(), he.data(), hd.data(), ht.data()};
-    for (int k = 0; k < (prog.tti ? 4 : 3); k++) {
-        if (mem == GEO_MEM_DEVICE) GEO_CUDA(cudaMemcpyAsync(dst[k], src[k], n0 * 4, cudaMemcpyDeviceToHost, s));
-        else memcpy(dst[k], src[k], n0 * 4);
+    Raw2D raw;
+    GEO_TRY(raw.open(nx, nz, v, e, d, prog.tti ? theta : nullptr, mem, s));
+    // the values the host formulas read: vp at the padded centre (d0), vp and
+    // eps at padded index 1 (the mute: the model's first cell, the sponge
+    // being at least five wide), eps and del on every shot's SV taper box
+    // (centre fs+(is-1)ds+npml, zs+npml)
+    const int TR = prog.taper_R, tr = prog.taper_r, nb = 2 * TR + 1;
+    auto at = [&](int a, int ix, int iz) {   // padded position
+        return raw_at(a, raw, std::min(std::max(ix - npml, 0), nx - 1), std::min(std::max(iz - npml, 0), nz - 1));
+    };
+    std::vector<unsigned long long> pick;
+    pick.push_back(at(0, (int)(n / 2 / nnz), (int)(n / 2 % nnz)));
+    pick.push_back(at(0, 0, 1));
+    pick.push_back(at(1, 0, 1));
+    for (int is = 1; is <= D.ns; is++) {
+        const int cx = D.fs + (is - 1) * D.ds + npml, cz = D.zs + npml;
+        for (int b = 0; b < nb * nb; b++) {
+            pick.push_back(at(1, cx - TR + b / nb, cz - TR + b % nb));
+            pick.push_back(at(2, cx - TR + b / nb, cz - TR + b % nb));
+        }
     }
-    GEO_CUDA(cudaStreamSynchronize(s));
-    GEO_TRY(check_model(hv.data(), he.data(), hd.data(), n0));
-    if (prog.tti)
-        for (size_t k = 0; k < n0; k++)
-            if (!std::isfinite(ht[k])) return fail(GEO_ERR_MODEL, "theta[%zu] not finite", k);
-    if (prog.checks) GEO_TRY(gpu_rtm_checks(D, hv));
+    RawStats rs;
+    GEO_TRY(raw_stats(raw, pick, rs, s));
+    if (prog.checks) GEO_TRY(gpu_rtm_checks(D, rs.vmin, rs.vmax));
     for (int is = 1; is <= D.ns; is++) {
         const int ixs = D.fs + (is - 1) * D.ds + npml - 1, izs = D.zs + npml - 1;
         if (ixs < 4 || ixs >= nnx - 4 || izs < 4 || izs >= nnz - 4) return fail(GEO_ERR_ARG, "shot %d outside the grid", is);
     }
-    std::vector<float> pv(n), pe(n), pd(n);
-    pad_model_2d(nx, nz, npml, hv.data(), pv.data());
-    pad_model_2d(nx, nz, npml, he.data(), pe.data());
-    pad_model_2d(nx, nz, npml, hd.data(), pd.data());
     // get_d0 and initial_coffe of the program (VTI :110-118; TTI :230-233, :289-320)
     const Variant sp = prog.tti ? V_TTIRTM : V_GPU;
-    const float d0 = sponge_d0(sp, 2, 0.0f, pv[n / 2], npml, D.dx, D.dx, D.dz);
+    const float d0 = sponge_d0(sp, 2, 0.0f, rs.val[0], npml, D.dx, D.dx, D.dz);
     std::vector<float> prof(4 * (size_t)(nnx + nnz));
     float *q = prof.data();
     sponge_profiles(sp, nx, npml, D.dt, d0, q, q + nnx, q + 2 * nnx, q + 3 * nnx);
@@ -458,93 +467,107 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
     std::vector<float> amp;
     std::vector<uint8_t> on;
     source_amplitudes(V_GPU, nt, D.dt, D.favg, D.pfac, D.wtype, amp, on);
-    // untapered 1+2eps, sqrtf(1+2del)
-    std::vector<float> e2(n), d2(n);
-    for (size_t k = 0; k < n; k++) {
-        e2[k] = 1 + 2 * pe[k];
-        d2[k] = sqrtf(1 + 2 * pd[k]);
+    Blob small;
+    const size_t o_prof = small.put(prof), o_amp = small.put(amp), o_on = small.put(on);
+    // tapered 1+2eps, sqrtf(1+2del) of every shot's box
+    std::vector<size_t> o_te2(D.ns), o_td2(D.ns);
+    for (int is = 1; is <= D.ns; is++) {
+        std::vector<float> te2(nb * nb), td2(nb * nb);
+        const float *box = rs.val.data() + 3 + (size_t)(is - 1) * 2 * nb * nb;
+        for (int b = 0; b < nb * nb; b++) {
+            const int rx = b / nb - TR, rz = b % nb - TR, q2 = rx * rx + rz * rz;
+            float ee = box[2 * b], dd = box[2 * b + 1];
+            if (q2 <= tr * tr) {
+                ee = dd = 0.0f;
+            } else if (q2 <= TR * TR) {
+                const double gq = 0.5 * (1 - std::cos(kPiGui * ((sqrtf((float)q2) - tr) * 4.0 / (TR * 3.0 - 1))));
+                ee = (float)(gq * ee);
+                dd = (float)(gq * dd);
+            }
+            te2[b] = 1 + 2 * ee;
+            td2[b] = sqrtf(1 + 2 * dd);
+        }
+        o_te2[is - 1] = small.put(te2);
+        o_td2[is - 1] = small.put(td2);
     }
-    // tilt in radians as read_file converts it (theta *= pi/180); its cos and
-    // sin are formed on the device below, as the program's kernels form them
-    std::vector<float> ct;
-    float mu_v = pv[1] * sqrtf(1 + 2 * pe[1]);   // direct-wave velocity of the VTI program's mute
-    if (prog.tti) {
-        std::vector<float> pt(n);
-        pad_model_2d(nx, nz, npml, ht.data(), pt.data());
-        ct.resize(n);
-        for (size_t k = 0; k < n; k++) ct[k] = (float)((double)pt[k] * (kPiGui / 180.0));
-    }
+    GEO_TRY(small.upload(s));
+    float mu_v = rs.val[1] * sqrtf(1 + 2 * rs.val[2]);   // direct-wave velocity of the VTI program's mute
     const int L = 2 * nx + 2 * nz;
-
-    DevBuf dvp, dprof, de2, dd2, dte2, dtd2, fs_, fr_, ring, rec, mig, ill, ag, lap, stk, mkeep, trs, dct, dst_;
-    GEO_TRY(dvp.alloc(n * 4));
-    if (prog.tti) {
-        GEO_TRY(dct.alloc(n * 4));
-        GEO_TRY(dst_.alloc(n * 4));
-        GEO_CUDA(cudaMemcpyAsync(dct.p, ct.data(), n * 4, cudaMemcpyHostToDevice, s));
-        GEO_TRY(launch_tilt_trig(dct.as<float>(), dst_.as<float>(), n, s));
-        // mute_directwave of the TTI program: vp[1]*(1+(sqrtf(1+2 eps[1])-1)*cos(theta[1]))
-        float c1 = 0.0f;
-        GEO_CUDA(cudaMemcpyAsync(&c1, dct.as<float>() + 1, 4, cudaMemcpyDeviceToHost, s));
-        GEO_CUDA(cudaStreamSynchronize(s));
-        mu_v = pv[1] * (1 + (sqrtf(1 + 2 * pe[1]) - 1) * c1);
-    }
-    GEO_TRY(dprof.alloc(prof.size() * 4));
-    GEO_TRY(de2.alloc(n * 4));
-    GEO_TRY(dd2.alloc(n * 4));
-    GEO_TRY(dte2.alloc(n * 4));
-    GEO_TRY(dtd2.alloc(n * 4));
-    GEO_TRY(fs_.alloc(8 * n * 4));
-    GEO_TRY(fr_.alloc(8 * n * 4));
-    GEO_TRY(ring.alloc((size_t)2 * nt * L * 4));
-    GEO_TRY(rec.alloc((size_t)nt * nx * 4));
-    GEO_TRY(mig.alloc(n0 * 4));
-    GEO_TRY(ill.alloc(n0 * 4));
-    GEO_TRY(mkeep.alloc((size_t)nt * nx));
     const int nxa = nx / dcdp;
     const size_t nag = (size_t)D.nangle * nz * nxa;
-    if (adcigs || stk_lap) {
-        GEO_TRY(ag.alloc(nag * 4));
-        GEO_TRY(ag.zero(s));
-        GEO_TRY(gpu_adcig_tables(D.nangle, D.dangle, s));
+    const bool gathers = adcigs || stk_lap;
+    // one allocation; the state a shot starts from is cleared together
+    Arena ar;
+    float *fS = nullptr, *fR = nullptr, *rec = nullptr, *ring = nullptr, *mig = nullptr, *ill = nullptr, *ag = nullptr;
+    float *dvp = nullptr, *de2 = nullptr, *dd2 = nullptr, *dte2 = nullptr, *dtd2 = nullptr, *dct = nullptr, *dsn = nullptr;
+    float *lap = nullptr, *stk = nullptr, *trs = nullptr;
+    int *mlo = nullptr;
+    unsigned *sync = nullptr;
+    size_t shot_end = 0, clear_end = 0;
+    for (int pass = 0; pass < 2; pass++) {
+        fS = ar.take<float>(8 * n);
+        fR = ar.take<float>(8 * n);
+        rec = ar.take<float>((size_t)nt * nx);
+        ring = ar.take<float>((size_t)2 * nt * L);
+        shot_end = ar.off;
+        mig = ar.take<float>(n0);
+        ill = ar.take<float>(n0);
+        if (gathers) ag = ar.take<float>(nag);
+        sync = ar.take<unsigned>(2);
+        clear_end = ar.off;
+        dvp = ar.take<float>(n);
+        de2 = ar.take<float>(n);
+        dd2 = ar.take<float>(n);
+        dte2 = ar.take<float>(n);
+        dtd2 = ar.take<float>(n);
+        if (prog.tti) {
+            dct = ar.take<float>(n);
+            dsn = ar.take<float>(n);
+        }
+        lap = ar.take<float>(n0);
+        if (stk_lap) stk = ar.take<float>(n0);
+        if (shots || obs) trs = ar.take<float>((size_t)nt * nx);
+        mlo = ar.take<int>(2 * (size_t)nx);
+        if (pass == 0) GEO_TRY(ar.alloc());
     }
-    GEO_CUDA(cudaMemcpyAsync(dvp.p, pv.data(), n * 4, cudaMemcpyHostToDevice, s));
-    GEO_CUDA(cudaMemcpyAsync(dprof.p, prof.data(), prof.size() * 4, cudaMemcpyHostToDevice, s));
-    GEO_CUDA(cudaMemcpyAsync(de2.p, e2.data(), n * 4, cudaMemcpyHostToDevice, s));
-    GEO_CUDA(cudaMemcpyAsync(dd2.p, d2.data(), n * 4, cudaMemcpyHostToDevice, s));
-    GEO_TRY(mig.zero(s));
-    GEO_TRY(ill.zero(s));
+    GEO_CUDA(cudaMemsetAsync(ar.buf.p, 0, clear_end, s));
+    ModelJob job{};
+    job.nx = nx; job.nz = nz; job.npd = npml; job.ldz = nnz;
+    job.vp = dvp; job.e2 = de2; job.d2 = dd2; job.rad = dct;
+    GEO_TRY(launch_model2d(raw, {job}, s));
+    if (prog.tti) {
+        // tilt in radians as read_file converts it (theta *= pi/180); its cos
+        // and sin as the program's kernels form them
+        GEO_TRY(launch_tilt_trig(dct, dsn, n, s));
+        // mute_directwave of the TTI program: vp[1]*(1+(sqrtf(1+2 eps[1])-1)*cos(theta[1]))
+        float c1 = 0.0f;
+        GEO_CUDA(cudaMemcpyAsync(&c1, dct + 1, 4, cudaMemcpyDeviceToHost, s));
+        GEO_CUDA(cudaStreamSynchronize(s));
+        mu_v = rs.val[1] * (1 + (sqrtf(1 + 2 * rs.val[2]) - 1) * c1);
+    }
+    if (gathers) GEO_TRY(gpu_adcig_tables(D.nangle, D.dangle, s));
     GRtm g{};
     g.nnx = nnx; g.nnz = nnz; g.nx = nx; g.nz = nz; g.npml = npml; g.nangle = D.nangle; g.dcdp = dcdp;
-    g.ct = dct.as<float>();
-    g.st = dst_.as<float>();
+    g.ct = dct;
+    g.st = dsn;
     g.dtx = D.dt / D.dx;
     g.dtz = D.dt / D.dz;
-    const float *pp = dprof.as<float>();
+    const float *pp = small.at<float>(o_prof);
     g.cx1 = pp; g.cx2 = pp + nnx; g.ax1 = pp + 2 * nnx; g.ax2 = pp + 3 * nnx;
     pp += 4 * nnx;
     g.cz1 = pp; g.cz2 = pp + nnz; g.az1 = pp + 2 * nnz; g.az2 = pp + 3 * nnz;
-    g.vp = dvp.as<float>();
-    auto fields = [&](DevBuf &b) {
+    g.vp = dvp;
+    auto fields = [&](float *p) {
         GField f;
-        float *p = b.as<float>();
         f.u = p; f.w = p + n; f.P = p + 2 * n; f.Q = p + 3 * n;
         f.px = p + 4 * n; f.pz = p + 5 * n; f.qx = p + 6 * n; f.qz = p + 7 * n;
         return f;
     };
-    const GField S = fields(fs_), R = fields(fr_);
-    float *bp = ring.as<float>(), *bq = bp + (size_t)nt * L;
+    const GField S = fields(fS), R = fields(fR);
+    float *bp = ring, *bq = bp + (size_t)nt * L;
     const int gi = grid_of_n((long)n0);
     const cudaMemcpyKind kout = mem == GEO_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
     const cudaMemcpyKind kin = mem == GEO_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    if (shots || obs) GEO_TRY(trs.alloc((size_t)nt * nx * 4));
-    DevBuf d_amp, d_on, d_sync;
-    GEO_TRY(d_amp.alloc((size_t)nt * 4));
-    GEO_TRY(d_on.alloc((size_t)nt));
-    GEO_TRY(d_sync.alloc(8));
-    GEO_TRY(d_sync.zero(s));
-    GEO_CUDA(cudaMemcpyAsync(d_amp.p, amp.data(), (size_t)nt * 4, cudaMemcpyHostToDevice, s));
-    GEO_CUDA(cudaMemcpyAsync(d_on.p, on.data(), (size_t)nt, cudaMemcpyHostToDevice, s));
     GCoop a{};
     a.g = g;
     a.tg = tti_grid(g);
@@ -552,17 +575,17 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
     a.R = R;
     a.tS = tti_field(S);
     a.tR = tti_field(R);
-    a.amp = d_amp.as<float>();
-    a.on = d_on.as<unsigned char>();
-    a.rec = rec.as<float>();
+    a.amp = small.at<float>(o_amp);
+    a.on = small.at<unsigned char>(o_on);
+    a.rec = rec;
     a.bp = bp;
     a.bq = bq;
-    a.ill = ill.as<float>();
-    a.mig = mig.as<float>();
-    a.adcig = ag.p ? ag.as<float>() : nullptr;
+    a.ill = ill;
+    a.mig = mig;
+    a.adcig = ag;
     a.L = L;
-    a.bar = d_sync.as<unsigned>();
-    a.err = d_sync.as<int>() + 1;
+    a.bar = sync;
+    a.err = reinterpret_cast<int *>(sync) + 1;
     // every block resident at once (the grid barrier needs it; the
     // cooperative launch checks it), threads striding over the points
     const void *kf = prog.tti ? (const void *)k_grtm_fwd<true> : (const void *)k_grtm_fwd<false>;
@@ -592,37 +615,17 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
     Watchdog wd;
     GEO_TRY(wd.open());
     for (int is = 1; is <= D.ns; is++) {
-        // SV taper box of this shot (centre fs+(is-1)ds+npml, zs+npml)
-        std::vector<float> te2(e2), td2(d2);
-        {
-            const int TR = prog.taper_R, tr = prog.taper_r;
-            const int cx = D.fs + (is - 1) * D.ds + npml, cz = D.zs + npml, R2 = TR * TR, r2 = tr * tr;
-            for (int ix = std::max(0, cx - TR); ix <= std::min(nnx - 1, cx + TR); ix++)
-                for (int iz = std::max(0, cz - TR); iz <= std::min(nnz - 1, cz + TR); iz++) {
-                    const int rx = ix - cx, rz = iz - cz, q2 = rx * rx + rz * rz;
-                    if (q2 > R2) continue;
-                    const size_t id = (size_t)ix * nnz + iz;
-                    float ee = 0.0f, dd = 0.0f;
-                    if (q2 > r2) {
-                        const double gq = 0.5 * (1 - std::cos(kPiGui * ((sqrtf((float)q2) - tr) * 4.0 / (TR * 3.0 - 1))));
-                        ee = (float)(gq * pe[id]);
-                        dd = (float)(gq * pd[id]);
-                    }
-                    te2[id] = 1 + 2 * ee;
-                    td2[id] = sqrtf(1 + 2 * dd);
-                }
-        }
-        GEO_CUDA(cudaMemcpyAsync(dte2.p, te2.data(), n * 4, cudaMemcpyHostToDevice, s));
-        GEO_CUDA(cudaMemcpyAsync(dtd2.p, td2.data(), n * 4, cudaMemcpyHostToDevice, s));
-        GEO_TRY(fs_.zero(s));
-        GEO_TRY(fr_.zero(s));
-        GEO_TRY(rec.zero(s));
-        GEO_TRY(ring.zero(s));
+        // the shot's tapered model: the untapered one with its box replaced
+        GEO_CUDA(cudaMemcpyAsync(dte2, de2, n * 4, cudaMemcpyDeviceToDevice, s));
+        GEO_CUDA(cudaMemcpyAsync(dtd2, dd2, n * 4, cudaMemcpyDeviceToDevice, s));
+        GEO_TRY(launch_box2d(dte2, dtd2, nnx, nnz, D.fs + (is - 1) * D.ds + npml - TR, D.zs + npml - TR, nb,
+                             small.at<float>(o_te2[is - 1]), small.at<float>(o_td2[is - 1]), s));
+        if (is > 1) GEO_CUDA(cudaMemsetAsync(ar.buf.p, 0, shot_end, s));
         a.ixs = D.fs + (is - 1) * D.ds + npml - 1;
         a.izs = D.zs + npml - 1;
         a.src = (long)a.ixs * nnz + a.izs;
-        a.e2 = dte2.as<float>();
-        a.d2 = dtd2.as<float>();
+        a.e2 = dte2;
+        a.d2 = dtd2;
         // runs of steps between the watchdog's scans, one launch each
         for (int it0 = 0; it0 < nt;) {
             int it1 = it0 + 1;
@@ -640,36 +643,32 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
         // ix whose window holds it -- past nt that lands on later traces.
         // TTI program: one thread per sample, bounded.
         {
-            std::vector<uint8_t> keep((size_t)nt * nx, 1);   // time-major
+            std::vector<int> lohi(2 * (size_t)nx);
             const int nt512 = prog.mute_overrun ? (nt + 511) / 512 * 512 : nt;
             for (int ix = 0; ix < nx; ix++) {
                 const float mu_x = D.dx * std::abs(ix - D.fs - (is - 1) * D.ds), mu_z = D.dz * D.zs;
                 const float mu_t0 = sqrtf((float)(std::pow(mu_x, 2) + std::pow(mu_z, 2))) / mu_v;
                 const int mu_t = (int)(2.0 / (D.dt * D.favg));
                 const int mu_nt = (int)(mu_t0 / D.dt) + mu_t + D.mute_tt;
-                const int first = std::max(0, (int)(mu_t0 / D.dt) - D.mute_tt + 1);
-                for (int it = first; it < std::min(mu_nt, nt512); it++) {
-                    const long j = (long)ix * nt + it;          // trace-major flat index
-                    if (j >= (long)nx * nt) break;
-                    keep[(size_t)(j % nt) * nx + (size_t)(j / nt)] = 0;
-                }
+                lohi[ix] = std::max(0, (int)(mu_t0 / D.dt) - D.mute_tt + 1);
+                lohi[nx + ix] = std::min(mu_nt, nt512);
             }
-            GEO_CUDA(cudaMemcpyAsync(mkeep.p, keep.data(), keep.size(), cudaMemcpyHostToDevice, s));
-            k_g_mask<<<grid_of_n((long)nt * nx), 256, 0, s>>>(rec.as<float>(), mkeep.as<uint8_t>(), (long)nt * nx);
+            GEO_CUDA(cudaMemcpyAsync(mlo, lohi.data(), lohi.size() * 4, cudaMemcpyHostToDevice, s));
+            k_g_mute<<<dim3((nt512 + 255) / 256, std::min(nx, 65535)), 256, 0, s>>>(rec, mlo, mlo + nx, nx, nt);
             GEO_TRY(check_launch("grtm_mute"));
             GEO_CUDA(cudaStreamSynchronize(s));
         }
         if (shots) {
-            GEO_TRY(launch_transpose_records(rec.as<float>(), trs.as<float>(), nx, nt, s));
-            GEO_CUDA(cudaMemcpyAsync(shots + (size_t)(is - 1) * nx * nt, trs.p, (size_t)nx * nt * 4, kout, s));
+            GEO_TRY(launch_transpose_records(rec, trs, nx, nt, s));
+            GEO_CUDA(cudaMemcpyAsync(shots + (size_t)(is - 1) * nx * nt, trs, (size_t)nx * nt * 4, kout, s));
         }
         if (obs) {
             // observed shot (trace-major nx*nt) replaces the modelled record
-            GEO_CUDA(cudaMemcpyAsync(trs.p, obs + (size_t)(is - 1) * nx * nt, (size_t)nx * nt * 4, kin, s));
-            GEO_TRY(launch_transpose_records(trs.as<float>(), rec.as<float>(), nt, nx, s));
+            GEO_CUDA(cudaMemcpyAsync(trs, obs + (size_t)(is - 1) * nx * nt, (size_t)nx * nt * 4, kin, s));
+            GEO_TRY(launch_transpose_records(trs, rec, nt, nx, s));
         }
-        a.e2 = de2.as<float>();
-        a.d2 = dd2.as<float>();
+        a.e2 = de2;
+        a.d2 = dd2;
         // runs of steps between the watchdog's scans (after backward step
         // it when (nt - it) is a multiple of the interval), one launch each
         for (int hi = nt - 1; hi >= 0;) {
@@ -689,21 +688,19 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
         GEO_CUDA(cudaStreamSynchronize(s));
         if (err) return fail(GEO_ERR_CUDA, "2D RTM: a grid barrier wait timed out");
     }
-    GEO_TRY(launch_normalize_image(mig.as<float>(), ill.as<float>(), n0, s));
-    GEO_TRY(lap.alloc(n0 * 4));
-    GEO_TRY(launch_laplace2d(nx, nz, mig.as<float>(), lap.as<float>(), s));
-    GEO_CUDA(cudaMemcpyAsync(mig_lap, lap.p, n0 * 4, kout, s));
-    if (illum) GEO_CUDA(cudaMemcpyAsync(illum, ill.p, n0 * 4, kout, s));
-    if (ag.p) {
-        k_g_adcig_norm<<<grid_of_n((long)nag), 256, 0, s>>>(ag.as<float>(), ill.as<float>(), nxa, nz, D.nangle, dcdp);
+    GEO_TRY(launch_normalize_image(mig, ill, n0, s));
+    GEO_TRY(launch_laplace2d(nx, nz, mig, lap, s));
+    GEO_CUDA(cudaMemcpyAsync(mig_lap, lap, n0 * 4, kout, s));
+    if (illum) GEO_CUDA(cudaMemcpyAsync(illum, ill, n0 * 4, kout, s));
+    if (gathers) {
+        k_g_adcig_norm<<<grid_of_n((long)nag), 256, 0, s>>>(ag, ill, nxa, nz, D.nangle, dcdp);
         GEO_TRY(check_launch("grtm_adcig_norm"));
-        if (adcigs) GEO_CUDA(cudaMemcpyAsync(adcigs, ag.p, nag * 4, kout, s));
+        if (adcigs) GEO_CUDA(cudaMemcpyAsync(adcigs, ag, nag * 4, kout, s));
         if (stk_lap) {
-            GEO_TRY(stk.alloc(n0 * 4));
-            k_g_stack_angles<<<gi, 256, 0, s>>>(ag.as<float>(), stk.as<float>(), nx, nz, D.nangle);
+            k_g_stack_angles<<<gi, 256, 0, s>>>(ag, stk, nx, nz, D.nangle);
             GEO_TRY(check_launch("grtm_stack_angles"));
-            GEO_TRY(launch_laplace2d(nx, nz, stk.as<float>(), lap.as<float>(), s));
-            GEO_CUDA(cudaMemcpyAsync(stk_lap, lap.p, n0 * 4, kout, s));
+            GEO_TRY(launch_laplace2d(nx, nz, stk, lap, s));
+            GEO_CUDA(cudaMemcpyAsync(stk_lap, lap, n0 * 4, kout, s));
         }
     }
     GEO_CUDA(cudaStreamSynchronize(s));

@@ -57,20 +57,6 @@ void DevBuf::release() {
     bytes = 0;
 }
 
-// ---------------------------------------------------------------- padding
-// pad_vv: left/right columns first, then top/bottom rows over the full
-// width, so corners take the corner value (CPU_vti2dfd_kernels.c:221-246).
-void pad_model_2d(int nx, int nz, int npd, const float *in, float *out) {
-    const int nnx = nx + 2 * npd, nnz = nz + 2 * npd;
-    for (int ix = 0; ix < nnx; ix++) {
-        int sx = ix < npd ? 0 : (ix >= npd + nx ? nx - 1 : ix - npd);
-        for (int iz = 0; iz < nnz; iz++) {
-            int sz = iz < npd ? 0 : (iz >= npd + nz ? nz - 1 : iz - npd);
-            out[(size_t)ix * nnz + iz] = in[(size_t)sx * nz + sz];
-        }
-    }
-}
-
 // ---------------------------------------------------------------- sponge
 // d0 (CPU_vti2dfd_kernels.c:192; Toa_rtm_vti_adcig_cdp.c:1346;
 // GPU_vti2dfd_kernels.cu:105; GPU_vti3dfd_kernels.cu:205).
@@ -157,10 +143,8 @@ void source_amplitudes(Variant v, int nt, float dt, float favg, float pfac, int 
 // eps=del=0 inside CR*CR/16 (integer), cosine ramp outside
 // (CPU_vti2dfd_kernels.c:136-156).  GPU form: R=15, r=4, ramp on sqrtf of
 // the radius (GPU_vti2dfd_kernels.cu:260-278).  Only the kTB*kTB box around
-// the centre can change.
-void sv_taper_2d(Variant v, int nnx, int nnz, int npd, int cx, int cz, const float *e_pad,
-                 const float *d_pad, Taper2D &out) {
-    (void)npd;
+// the centre can change; e_box and d_box hold its padded eps and del.
+void sv_taper_2d(Variant v, int nnx, int nnz, int cx, int cz, const float *e_box, const float *d_box, Taper2D &out) {
     out.n = kTB;
     out.x0 = cx - kTB / 2;
     out.z0 = cz - kTB / 2;
@@ -170,9 +154,8 @@ void sv_taper_2d(Variant v, int nnx, int nnz, int npd, int cx, int cz, const flo
         for (int bz = 0; bz < kTB; bz++) {
             const int ix = out.x0 + bx, iz = out.z0 + bz;
             if (ix < 0 || ix >= nnx || iz < 0 || iz >= nnz) continue;
-            const size_t id = (size_t)ix * nnz + iz;
             const int rx = ix - cx, rz = iz - cz, r2 = rx * rx + rz * rz;
-            float e = e_pad[id], d = d_pad[id];
+            float e = e_box[bx * kTB + bz], d = d_box[bx * kTB + bz];
             if (v == V_CPU || v == V_MPI) {
                 const double pi = (v == V_MPI) ? kPiMpi : kPiGui;
                 const int CR = 15;
@@ -271,15 +254,6 @@ void mute_window_3d_band(int nx, int ny, int nt, float dt, float favg, float dx,
             lo[(size_t)iy * nx + ix] = a < 0 ? 0 : (a < nt ? a : nt);
             hi[(size_t)iy * nx + ix] = mu_nt < 0 ? 0 : (mu_nt < nt ? mu_nt : nt);
         }
-}
-
-int check_model(const float *v, const float *e, const float *d, size_t n) {
-    for (size_t i = 0; i < n; i++) {
-        if (!std::isfinite(v[i]) || !(v[i] > 0.0f)) return fail(GEO_ERR_MODEL, "velocity[%zu]=%g", i, v[i]);
-        if (!std::isfinite(e[i]) || !std::isfinite(d[i])) return fail(GEO_ERR_MODEL, "eps/del[%zu] not finite", i);
-        if (1 + 2 * d[i] < 0) return fail(GEO_ERR_MODEL, "1+2*delta[%zu] < 0", i);
-    }
-    return GEO_OK;
 }
 
 }  // namespace geo

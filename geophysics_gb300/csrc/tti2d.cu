@@ -21,6 +21,7 @@
 #include "geo_internal.h"
 #include <algorithm>
 #include "tti2d.cuh"
+#include "model2d.cuh"
 #include "gridsync.cuh"
 #include <cmath>
 #include <vector>
@@ -113,57 +114,30 @@ extern "C" int geo_tti2d_shot(const geo_fd2d_desc *desc, const float *v, const f
     if (snap && snap_every < 1) return fail(GEO_ERR_ARG, "snap_every must be >= 1");
     const int nx = D.nx, nz = D.nz, npd = D.npd, nt = D.nt;
     const int nnx = nx + 2 * npd, nnz = nz + 2 * npd;
-    const size_t n0 = (size_t)nx * nz, n = (size_t)nnx * nnz;
+    const size_t n = (size_t)nnx * nnz;
     if (D.rec_iz < 0 || D.rec_iz >= nnz) return fail(GEO_ERR_ARG, "receiver row outside the grid");
     cudaStream_t s = (cudaStream_t)stream;
-    std::vector<float> hv(n0), he(n0), hd(n0), ht(n0);
-    const float *src[4] = {v, e, d, theta};
-    float *dst[4] = {hv.data(), he.data(), hd.data(), ht.data()};
-    for (int k = 0; k < 4; k++) {
-        if (mem == GEO_MEM_DEVICE) GEO_CUDA(cudaMemcpyAsync(dst[k], src[k], n0 * 4, cudaMemcpyDeviceToHost, s));
-        else std::copy(src[k], src[k] + n0, dst[k]);
-    }
-    GEO_CUDA(cudaStreamSynchronize(s));
-    GEO_TRY(check_model(hv.data(), he.data(), hd.data(), n0));
-    for (size_t k = 0; k < n0; k++)
-        if (!std::isfinite(ht[k])) return fail(GEO_ERR_MODEL, "theta[%zu] not finite", k);
-    std::vector<float> pv(n), pe(n), pd(n), pt(n);
-    pad_model_2d(nx, nz, npd, hv.data(), pv.data());
-    pad_model_2d(nx, nz, npd, he.data(), pe.data());
-    pad_model_2d(nx, nz, npd, hd.data(), pd.data());
-    pad_model_2d(nx, nz, npd, ht.data(), pt.data());
+    Raw2D raw;
+    GEO_TRY(raw.open(nx, nz, v, e, d, theta, mem, s));
     // source cell (add_source :71-72), shot is 1-based
     const float fsx = D.fs + (D.is - 1) * D.ds;
     const int ixs = (int)(fsx + 0.5f) + npd - 1, izs = (int)(D.zs + 0.5f) + npd - 1;
+    // SV taper centre (fs+(is-1)ds+npml, zs+npml) (:131-132): one cell right/down of the source cell
+    const int cx = ixs + 1, cz = izs + 1;
+    std::vector<unsigned long long> pick;
+    auto at = [&](int a, int ix, int iz) {   // padded position
+        return raw_at(a, raw, std::min(std::max(ix - npd, 0), nx - 1), std::min(std::max(iz - npd, 0), nz - 1));
+    };
+    pick.push_back(at(0, (int)(n / 2 / nnz), (int)(n / 2 % nnz)));
+    if (D.sv)
+        for (int a = 1; a <= 2; a++)
+            for (int b = 0; b < kTB * kTB; b++) pick.push_back(at(a, cx - kTB / 2 + b / kTB, cz - kTB / 2 + b % kTB));
+    RawStats rs;
+    GEO_TRY(raw_stats(raw, pick, rs, s));
     if (ixs < 4 || ixs >= nnx - 4 || izs < 4 || izs >= nnz - 4) return fail(GEO_ERR_ARG, "source outside the grid");
-    if (D.sv) {
-        // centre (fs+(is-1)ds+npml, zs+npml) (:131-132): one cell right/down of the source cell
-        Taper2D tp;
-        sv_taper_2d(V_GPU, nnx, nnz, npd, ixs + 1, izs + 1, pe.data(), pd.data(), tp);
-        for (int bx = 0; bx < tp.n; bx++)
-            for (int bz = 0; bz < tp.n; bz++) {
-                const int ix = tp.x0 + bx, iz = tp.z0 + bz;
-                if (ix < 0 || ix >= nnx || iz < 0 || iz >= nnz) continue;
-                pe[(size_t)ix * nnz + iz] = tp.e[bx * tp.n + bz];
-                pd[(size_t)ix * nnz + iz] = tp.d[bx * tp.n + bz];
-            }
-    }
-    // model arrays: vp, 1+2eps, sqrtf(1+2del), and the tilt in radians as
-    // read_file converts it (:235), whose cos and sin are then formed on the
-    // device (launch_tilt_trig) as the program's kernels form them
-    std::vector<float> model(5 * n);
-    for (size_t k = 0; k < n; k++) {
-        model[k] = pv[k];
-        model[n + k] = 1 + 2 * pe[k];
-        model[2 * n + k] = sqrtf(1 + 2 * pd[k]);
-        model[3 * n + k] = (float)((double)pt[k] * (kPiGui / 180.0));
-    }
-    {
-        const auto mm = std::minmax_element(pv.begin(), pv.end());
-        GEO_TRY(check_stability(V_GPU, 2, *mm.first, *mm.second, D.dt, D.dx, D.dx, D.dz, D.favg));
-    }
+    GEO_TRY(check_stability(V_GPU, 2, rs.vmin, rs.vmax, D.dt, D.dx, D.dx, D.dz, D.favg));
     // sponge (get_d0 :186-189 from the padded centre velocity; initial_coffe :227-271)
-    const float d0 = sponge_d0(V_GPU, 2, 0.0f, pv[n / 2], npd, D.dx, D.dx, D.dz);
+    const float d0 = sponge_d0(V_GPU, 2, 0.0f, rs.val[0], npd, D.dx, D.dx, D.dz);
     std::vector<float> prof(4 * (size_t)(nnx + nnz));
     float *q = prof.data();
     sponge_profiles(V_GPU, nx, npd, D.dt, d0, q, q + nnx, q + 2 * nnx, q + 3 * nnx);
@@ -172,58 +146,78 @@ extern "C" int geo_tti2d_shot(const geo_fd2d_desc *desc, const float *v, const f
     std::vector<float> amp;
     std::vector<uint8_t> on;
     source_amplitudes(V_GPU, nt, D.dt, D.favg, D.pfac, D.wtype, amp, on);
-
-    DevBuf dm, dprof, df, drec;
-    GEO_TRY(dm.alloc(5 * n * 4));
-    GEO_TRY(dprof.alloc(prof.size() * 4));
-    GEO_TRY(df.alloc(8 * n * 4));
-    GEO_TRY(drec.alloc((size_t)nx * nt * 4));
-    GEO_CUDA(cudaMemcpyAsync(dm.p, model.data(), 5 * n * 4, cudaMemcpyHostToDevice, s));
-    GEO_TRY(launch_tilt_trig(dm.as<float>() + 3 * n, dm.as<float>() + 4 * n, n, s));
-    GEO_CUDA(cudaMemcpyAsync(dprof.p, prof.data(), prof.size() * 4, cudaMemcpyHostToDevice, s));
-    GEO_TRY(df.zero(s));
-    GEO_TRY(drec.zero(s));
+    Blob small;
+    const size_t o_prof = small.put(prof), o_amp = small.put(amp), o_on = small.put(on);
+    size_t o_te2 = 0, o_td2 = 0;
+    Taper2D tp;
+    if (D.sv) {
+        sv_taper_2d(V_GPU, nnx, nnz, cx, cz, rs.val.data() + 1, rs.val.data() + 1 + kTB * kTB, tp);
+        std::vector<float> te2(kTB * kTB), td2(kTB * kTB);
+        for (int b = 0; b < kTB * kTB; b++) {
+            te2[b] = 1 + 2 * tp.e[b];
+            td2[b] = sqrtf(1 + 2 * tp.d[b]);
+        }
+        o_te2 = small.put(te2);
+        o_td2 = small.put(td2);
+    }
+    GEO_TRY(small.upload(s));
+    // one allocation: the cleared state (fields, record, barrier and error
+    // words), then vp, 1+2eps, sqrtf(1+2del) and the tilt in radians as
+    // read_file converts it (:235), whose cos and sin are formed on the
+    // device (launch_tilt_trig) as the program's kernels form them
+    Arena ar;
+    float *fb = nullptr, *drec = nullptr, *model = nullptr;
+    unsigned *sync = nullptr;
+    size_t clear = 0;
+    for (int pass = 0; pass < 2; pass++) {
+        fb = ar.take<float>(8 * n);
+        drec = ar.take<float>((size_t)nx * nt);
+        sync = ar.take<unsigned>(2);
+        clear = ar.off;
+        model = ar.take<float>(5 * n);
+        if (pass == 0) GEO_TRY(ar.alloc());
+    }
+    GEO_CUDA(cudaMemsetAsync(ar.buf.p, 0, clear, s));
+    ModelJob job{};
+    job.nx = nx; job.nz = nz; job.npd = npd; job.ldz = nnz;
+    job.vp = model; job.e2 = model + n; job.d2 = model + 2 * n; job.rad = model + 3 * n;
+    GEO_TRY(launch_model2d(raw, {job}, s));
+    if (D.sv)
+        GEO_TRY(launch_box2d(job.e2, job.d2, nnx, nnz, tp.x0, tp.z0, kTB, small.at<float>(o_te2), small.at<float>(o_td2),
+                             s));
+    GEO_TRY(launch_tilt_trig(model + 3 * n, model + 4 * n, n, s));
     TtiGrid g{};
     g.nnx = nnx;
     g.nnz = nnz;
     g.dtx = D.dt / D.dx;
     g.dtz = D.dt / D.dz;
-    const float *pp = dprof.as<float>();
+    const float *pp = small.at<float>(o_prof);
     g.cx1 = pp; g.cx2 = pp + nnx; g.ax1 = pp + 2 * nnx; g.ax2 = pp + 3 * nnx;
     pp += 4 * nnx;
     g.cz1 = pp; g.cz2 = pp + nnz; g.az1 = pp + 2 * nnz; g.az2 = pp + 3 * nnz;
-    const float *m = dm.as<float>();
-    g.vp = m; g.ct = m + 3 * n; g.st = m + 4 * n;
-    const float *e2 = m + n, *d2 = m + 2 * n;
-    float *fb = df.as<float>();
+    g.vp = model; g.ct = model + 3 * n; g.st = model + 4 * n;
+    const float *e2 = model + n, *d2 = model + 2 * n;
     TtiField f;
     f.u = fb; f.w = fb + n; f.px = fb + 2 * n; f.pz = fb + 3 * n; f.qx = fb + 4 * n; f.qz = fb + 5 * n;
     f.P = fb + 6 * n; f.Q = fb + 7 * n;
     const cudaMemcpyKind kout = mem == GEO_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    DevBuf d_amp, d_on, d_sync;
-    GEO_TRY(d_amp.alloc((size_t)nt * 4));
-    GEO_TRY(d_on.alloc((size_t)nt));
-    GEO_TRY(d_sync.alloc(8));
-    GEO_TRY(d_sync.zero(s));
-    GEO_CUDA(cudaMemcpyAsync(d_amp.p, amp.data(), (size_t)nt * 4, cudaMemcpyHostToDevice, s));
-    GEO_CUDA(cudaMemcpyAsync(d_on.p, on.data(), (size_t)nt, cudaMemcpyHostToDevice, s));
     TtiShot a{};
     a.g = g;
     a.f = f;
     a.e2 = e2;
     a.d2 = d2;
-    a.amp = d_amp.as<float>();
-    a.on = d_on.as<unsigned char>();
+    a.amp = small.at<float>(o_amp);
+    a.on = small.at<unsigned char>(o_on);
     a.src = (long)ixs * nnz + izs;
     a.ixs = ixs;
     a.izs = izs;
-    a.rec = drec.as<float>();
+    a.rec = drec;
     a.nx = nx;
     a.npd = npd;
     a.rec_iz = D.rec_iz;
     a.nt = nt;
-    a.bar = d_sync.as<unsigned>();
-    a.err = d_sync.as<int>() + 1;
+    a.bar = sync;
+    a.err = reinterpret_cast<int *>(sync) + 1;
     // every block resident at once (the grid barrier needs it; the
     // cooperative launch checks it), threads striding over the points
     int dev = 0, sms = 0, occ = 0, coop = 0;
@@ -265,7 +259,7 @@ extern "C" int geo_tti2d_shot(const geo_fd2d_desc *desc, const float *v, const f
     GEO_CUDA(cudaStreamSynchronize(s));
     if (err) return fail(GEO_ERR_CUDA, "2D TTI shot: a grid barrier wait timed out");
     GEO_TRY(wd.verdict(s, "2D TTI shot"));
-    GEO_CUDA(cudaMemcpyAsync(shot, drec.p, (size_t)nx * nt * 4, kout, s));
+    GEO_CUDA(cudaMemcpyAsync(shot, drec, (size_t)nx * nt * 4, kout, s));
     GEO_CUDA(cudaStreamSynchronize(s));
     return GEO_OK;
 }

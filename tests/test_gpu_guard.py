@@ -148,3 +148,28 @@ def test_cpu_program_limits(geo):
     assert ei.value.status == GEO_ERR_CFL
     out = geo.fd2d_shot(v, e, d, nt=20, variant="gpu", **dict(KW2, favg=150.0))
     assert np.isfinite(out).all()
+
+
+@pytest.mark.parametrize("array,value,text", [(0, np.nan, "velocity[37]"), (0, -1.0, "velocity[37]"),
+                                              (1, np.inf, "eps/del[37]"), (2, -0.6, "1+2*delta[37]"),
+                                              (3, np.nan, "theta[37]")])
+def test_2d_model_check_names_the_first_bad_cell(geo, array, value, text):
+    """Every 2D entry point, host and device arrays: the first failing cell
+    (a later one fails too) is reported and nothing runs."""
+    import torch
+    nx, nz = 21, 19
+    m = [np.full((nx, nz), x, np.float32) for x in (2000.0, 0.1, 0.05, 20.0)]
+    m[array].reshape(-1)[[37, 300]] = value
+    kw = dict(nt=5, dx=10.0, dz=10.0, dt=np.float32(1e-3), favg=20.0)
+    calls = [lambda a: geo.tti2d_shot(*a, npd=8, fs=10, zs=3, **kw), lambda a: geo.rtm2d_tti(*a, npml=8, fs=10, **kw)]
+    if array < 3:
+        calls += [lambda a: geo.fd2d_shot(*a[:3], npd=8, fs=10, zs=3, **kw),
+                  lambda a: geo.rtm2d_gpu(*a[:3], npml=8, fs=10, **kw),
+                  lambda a: geo.rtm2d_batch(*a[:3], npd=8, nt=5, dx=10.0, dz=10.0, dt_ms=1.0, favg=20.0, pfac=10.0,
+                                            zs=3, shot_x=[10], shot_nxs=[9])]
+    for dev in (False, True):
+        a = [torch.from_numpy(x).cuda() for x in m] if dev else m
+        for call in calls:
+            with pytest.raises(geo.GeoError) as err:
+                call(a)
+            assert text in str(err.value), str(err.value)
