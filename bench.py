@@ -742,9 +742,8 @@ def run_rtm2d_case(args):
     """Batched 2D RTM: 128 shots on a 2401x601 layered + random-field model
     (10 m), aperture widths odd in 401..1199 (seeded), sources evenly over
     x = 601..1801, 3000 steps at dt 1 ms, 20 Hz, every node of the window
-    recorded; per-shot image, stacked, adjoint Laplacian.  One persistent
-    launch per half-step over all shots' tiles, the time loop in CUDA graphs,
-    tiles from the autotuner.  cpu: the oracle's MPI-program restatement of
+    recorded; per-shot image, stacked, adjoint Laplacian.  One launch
+    per time step over all shots, the time loop in CUDA graphs.  cpu: the oracle's MPI-program restatement of
     one shot on one core (sample: 300 steps of the widest window)."""
     import numpy as np
     import torch
@@ -760,7 +759,7 @@ def run_rtm2d_case(args):
     xs = np.round(np.linspace(601, 1801, ns)).astype(int)
     kw = dict(npd=npd, nt=nt, dx=10.0, dz=10.0, dt_ms=1.0, favg=20.0, pfac=10.0, zs=5, shot_x=xs, shot_nxs=widths)
     tv, te, td = (torch.from_numpy(a).cuda() for a in (v, e, d))
-    geo.rtm2d_batch(tv, te, td, **dict(kw, nt=100))  # warm-up: autotune + graphs on a short run
+    geo.rtm2d_batch(tv, te, td, **dict(kw, nt=100))  # warm-up: a short run
     torch.cuda.synchronize()
     t0 = time.perf_counter()
     img = geo.rtm2d_batch(tv, te, td, **kw)

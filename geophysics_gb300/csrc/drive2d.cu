@@ -1,17 +1,13 @@
-// 2D drivers: single-shot forward modelling and batched RTM.
-//
-// Both build per-shot Shot2D descriptors and step them with the batched
-// kernels of fd2d.cu.  A batch time step is one persistent launch per phase
-// (velocity, stress) covering every shot's tiles; the time loops are
-// captured once into CUDA graphs and replayed.
+// 2D drivers: single-shot forward modelling (half-step, persistent and
+// tile-resident kernels of fd2d.cu) and batched RTM (fused steps of
+// march2d.cu over every shot, the time loops captured once into CUDA graphs
+// and replayed).
 #include "geo_internal.h"
 #include "model2d.cuh"
+#include "march2d.cuh"
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <map>
-#include <memory>
-#include <tuple>
 
 namespace geo {
 
@@ -39,20 +35,11 @@ struct ShotSet {
     int nz, npd, nnz;
     bool taper;
     std::vector<ShotGeom> G;
-    std::vector<Shot2D> S;
     RawStats st;
     float v00, e00;               // model values at unpadded (0, 0)
     std::vector<float> mu_v;      // MPI mute velocity of each shot
     Arena mem;
     Blob small;
-    size_t o_amp = 0, o_on = 0;
-    // cleared state: fields of side 0 of every shot, then of side 1, images
-    // and gathers, records
-    size_t z_side0 = 0, z_side1 = 0, z_img = 0, z_rec = 0, z_end = 0;
-    int clear(size_t from, size_t to, cudaStream_t s) {
-        if (to > from) GEO_CUDA(cudaMemsetAsync(mem.buf.as<char>() + from, 0, to - from, s));
-        return GEO_OK;
-    }
     static constexpr int kPick = 3 + 3 * kTB * kTB;   // centre v, v(1,1), e(1,1); v, e, d on the taper box
     void source(int k, int &ixs, int &izs) const {
         // source cell: (int)(fs+0.5)+npd-1 (CPU_vti2dfd_kernels.c:65-66)
@@ -69,9 +56,14 @@ struct ShotSet {
         }
     }
     int read(const Raw2D &raw, cudaStream_t s);
-    int build(const Raw2D &raw, float dx, float dz, float dt, const std::vector<float> &amp,
-              const std::vector<uint8_t> &on, int nfields, int nt, bool edges, bool image, bool adcig, bool fast,
-              cudaStream_t s);
+    // profiles and taper box of shot k: offsets in `small`
+    struct Off {
+        size_t xprof, zprof, te2, td2, tpw;   // xprof cx1 cx2 ax1 ax2; zprof cz1 cz2 az1 az2, ldz each
+        Taper2D box;
+        std::vector<float> vbox;              // v on the taper box
+        std::vector<float> p[8];
+    };
+    void tables(int k, float dx, float dz, float dt, int ldz, Off &o);
 };
 
 // The model values the set-up formulas read, with the model check.
@@ -103,12 +95,54 @@ int ShotSet::read(const Raw2D &raw, cudaStream_t s) {
     return GEO_OK;
 }
 
-// Propagation coefficients and state of every shot; var picks the reference
-// program's formulas.
-int ShotSet::build(const Raw2D &raw, float dx, float dz, float dt, const std::vector<float> &amp,
-                   const std::vector<uint8_t> &on, int nfields, int nt, bool edges, bool image, bool adcig, bool fast,
-                   cudaStream_t s) {
-    const int ns = (int)G.size();
+// The sponge profiles (of pitch ldz along z, ones beyond nnz), taper box and
+// mute velocity of shot k; var picks the reference program's formulas.
+void ShotSet::tables(int k, float dx, float dz, float dt, int ldz, Off &o) {
+    const ShotGeom &g = G[k];
+    const int nnx = g.nx + 2 * npd;
+    const float *val = st.val.data() + 2 + (size_t)k * kPick;
+    float vpmax = 0.0f;
+    for (int c = 0; c < g.nx; c++) vpmax = std::max(vpmax, st.colmax[std::min(c + g.col0, (int)st.colmax.size() - 1)]);
+    const float d0 = sponge_d0(var, 2, vpmax, val[0], npd, dx, dx, dz);
+    mu_v.resize(G.size());
+    mu_v[k] = val[1] * sqrtf(1 + 2 * val[2]);
+    for (int q = 0; q < 8; q++) o.p[q].assign(q < 4 ? nnx : ldz, 1.0f);
+    sponge_profiles(var, g.nx, npd, dt, d0, o.p[0].data(), o.p[1].data(), o.p[2].data(), o.p[3].data());
+    sponge_profiles(var, nz, npd, dt, d0, o.p[4].data(), o.p[5].data(), o.p[6].data(), o.p[7].data());
+    std::vector<float> px, pz;
+    for (int q = 0; q < 4; q++) {
+        px.insert(px.end(), o.p[q].begin(), o.p[q].end());
+        pz.insert(pz.end(), o.p[4 + q].begin(), o.p[4 + q].end());
+    }
+    o.xprof = small.put(px);
+    o.zprof = small.put(pz);
+    if (!taper) return;
+    int cx, cz;
+    centre(k, cx, cz);
+    const float *vbox = val + 3;
+    o.vbox.assign(vbox, vbox + kTB * kTB);
+    sv_taper_2d(var, nnx, nnz, cx, cz, vbox + kTB * kTB, vbox + 2 * kTB * kTB, o.box);
+    std::vector<float> te2(kTB * kTB), td2(kTB * kTB);
+    for (int b = 0; b < kTB * kTB; b++) {
+        te2[b] = 1 + 2 * o.box.e[b];
+        td2[b] = sqrtf(1 + 2 * o.box.d[b]);
+    }
+    o.te2 = small.put(te2);
+    o.td2 = small.put(td2);
+}
+
+// One shot on the device for the single-shot kernels.
+struct SingleShot {
+    ShotSet X;
+    Shot2D S{};
+    size_t o_amp = 0, o_on = 0;
+    int build(const Raw2D &raw, float dx, float dz, float dt, const std::vector<float> &amp,
+              const std::vector<uint8_t> &on, int nt, cudaStream_t s);
+};
+
+int SingleShot::build(const Raw2D &raw, float dx, float dz, float dt, const std::vector<float> &amp,
+                      const std::vector<uint8_t> &on, int nt, cudaStream_t s) {
+    const int nx = X.G[0].nx, nz = X.nz, npd = X.npd, nnx = nx + 2 * npd, nnz = X.nnz;
     // the MPI program's pz and qx chains are
     //   (double)(az2*pz) - (double)(az1*vp) * pow(1+2del,0.5) * (double)dtz * (double)zz
     // (and with ax, dtx, xx for qx), evaluated left to right; every factor but
@@ -116,146 +150,206 @@ int ShotSet::build(const Raw2D &raw, float dx, float dz, float dt, const std::ve
     // once, in the same order and precision (ModelJob::kz), and the kernel
     // issues one double multiply and one double subtraction per chain.  The
     // program's pow runs on the host, once per model point.
-    const bool kchain = var == V_MPI && !fast;
+    const bool mpi = X.var == V_MPI;
     const double ddtx = (double)(dt / dx), ddtz = (double)(dt / dz);
-    S.assign(ns, Shot2D{});
-    mu_v.resize(ns);
     DevBuf d_pw;
-    if (kchain) {
-        const size_t n0 = (size_t)raw.nx * raw.nz;
-        std::vector<float> hd(n0);
-        std::vector<double> pw(n0);
-        GEO_CUDA(cudaMemcpyAsync(hd.data(), raw.a[2], n0 * 4, cudaMemcpyDeviceToHost, s));
-        GEO_CUDA(cudaStreamSynchronize(s));
-        host_pow_half(hd.data(), n0, pw.data());
-        GEO_TRY(d_pw.alloc(n0 * 8));
-        GEO_CUDA(cudaMemcpyAsync(d_pw.p, pw.data(), n0 * 8, cudaMemcpyHostToDevice, s));
-        GEO_CUDA(cudaStreamSynchronize(s));   // pw is freed below
-    }
-    struct Off {
-        size_t prof[8], te2, td2, tkz, tkx;
-    };
-    std::vector<Off> off(ns);
-    for (int k = 0; k < ns; k++) {
-        const ShotGeom &g = G[k];
-        const int nnx = g.nx + 2 * npd;
-        const float *val = st.val.data() + 2 + (size_t)k * kPick;
-        float vpmax = 0.0f;
-        for (int c = 0; c < g.nx; c++) vpmax = std::max(vpmax, st.colmax[std::min(c + g.col0, raw.nx - 1)]);
-        const float d0 = sponge_d0(var, 2, vpmax, val[0], npd, dx, dx, dz);
-        mu_v[k] = val[1] * sqrtf(1 + 2 * val[2]);
-        std::vector<float> p[8];
-        for (int q = 0; q < 8; q++) p[q].resize(q < 4 ? nnx : nnz);
-        sponge_profiles(var, g.nx, npd, dt, d0, p[0].data(), p[1].data(), p[2].data(), p[3].data());
-        sponge_profiles(var, nz, npd, dt, d0, p[4].data(), p[5].data(), p[6].data(), p[7].data());
-        for (int q = 0; q < 8; q++) off[k].prof[q] = small.put(p[q]);
-        Shot2D &h = S[k];
-        source(k, h.ixs, h.izs);
-        h.tx0 = h.tz0 = -100000;
-        if (!taper) continue;
-        int cx, cz;
-        centre(k, cx, cz);
-        Taper2D tp;
-        const float *vbox = val + 3;
-        sv_taper_2d(var, nnx, nnz, cx, cz, vbox + kTB * kTB, vbox + 2 * kTB * kTB, tp);
-        h.tx0 = tp.x0;
-        h.tz0 = tp.z0;
-        std::vector<float> te2(kTB * kTB, 1.0f), td2(kTB * kTB, 1.0f);
-        for (int b = 0; b < kTB * kTB; b++) {
-            te2[b] = 1 + 2 * tp.e[b];
-            td2[b] = sqrtf(1 + 2 * tp.d[b]);
-        }
-        off[k].te2 = small.put(te2);
-        off[k].td2 = small.put(td2);
-        if (!kchain) continue;
+    if (mpi) GEO_TRY(upload_pow_half(raw, d_pw, s));
+    ShotSet::Off o;
+    X.tables(0, dx, dz, dt, nnz, o);
+    size_t o_tkz = 0, o_tkx = 0;
+    if (mpi && X.taper) {
         std::vector<double> tkz(kTB * kTB, 0.0), tkx(kTB * kTB, 0.0);
         for (int b = 0; b < kTB * kTB; b++) {
-            const int ix = tp.x0 + b / kTB, iz = tp.z0 + b % kTB;
+            const int ix = o.box.x0 + b / kTB, iz = o.box.z0 + b % kTB;
             if (ix < 0 || ix >= nnx || iz < 0 || iz >= nnz) continue;
-            const double pw = std::pow((double)(1 + 2 * tp.d[b]), 0.5);
-            const float vpk = 1.0f * (vbox[b] * vbox[b]);
-            tkz[b] = (double)(p[6][iz] * vpk) * pw * ddtz;
-            tkx[b] = (double)(p[2][ix] * vpk) * pw * ddtx;
+            const double pw = std::pow((double)(1 + 2 * o.box.d[b]), 0.5);
+            const float vpk = 1.0f * (o.vbox[b] * o.vbox[b]);
+            tkz[b] = (double)(o.p[6][iz] * vpk) * pw * ddtz;
+            tkx[b] = (double)(o.p[2][ix] * vpk) * pw * ddtx;
         }
-        off[k].tkz = small.put(tkz);
-        off[k].tkx = small.put(tkx);
+        o_tkz = X.small.put(tkz);
+        o_tkx = X.small.put(tkx);
     }
-    o_amp = small.put(amp);
-    o_on = small.put(on);
-    GEO_TRY(small.upload(s));
-    // two passes: sizes, then addresses
-    std::vector<ModelJob> jobs(ns);
-    for (int pass = 0; pass < 2; pass++) {
-        z_side0 = 0;
-        for (int f = 0; f < nfields; f++) {
-            if (f == 1) z_side1 = mem.off;
-            for (int k = 0; k < ns; k++) {
-                const size_t n = (size_t)(G[k].nx + 2 * npd) * nnz;
-                float **dst[8] = {&S[k].u[f], &S[k].w[f], &S[k].P[f], &S[k].Q[f],
-                                  &S[k].px[f], &S[k].pz[f], &S[k].qx[f], &S[k].qz[f]};
-                for (auto d : dst) *d = mem.take<float>(n);
-            }
+    o_amp = X.small.put(amp);
+    o_on = X.small.put(on);
+    GEO_TRY(X.small.upload(s));
+    const size_t n = (size_t)nnx * nnz;
+    ModelJob j{};
+    size_t clear = 0;
+    for (int pass = 0; pass < 2; pass++) {   // sizes, then addresses
+        float **dst[8] = {&S.u, &S.w, &S.P, &S.Q, &S.px, &S.pz, &S.qx, &S.qz};
+        for (auto d : dst) *d = X.mem.take<float>(n);
+        S.rec_p = X.mem.take<float>((size_t)nt * nx);
+        clear = X.mem.off;
+        j.vp = X.mem.take<float>(n);
+        j.e2 = X.mem.take<float>(n);
+        if (mpi) {
+            j.kz = X.mem.take<double>(n);
+            j.kx = X.mem.take<double>(n);
+        } else {
+            j.d2 = X.mem.take<float>(n);
         }
-        if (nfields < 2) z_side1 = mem.off;
-        z_img = mem.off;
+        if (pass == 0) GEO_TRY(X.mem.alloc());
+    }
+    S.nnx = nnx; S.nnz = nnz; S.npd = npd; S.nx = nx; S.nz = nz;
+    S.dtx = dt / dx; S.dtz = dt / dz;
+    const float *xp = X.small.at<float>(o.xprof), *zp = X.small.at<float>(o.zprof);
+    S.cx1 = xp; S.cx2 = xp + nnx; S.ax1 = xp + 2 * nnx; S.ax2 = xp + 3 * nnx;
+    S.cz1 = zp; S.cz2 = zp + nnz; S.az1 = zp + 2 * nnz; S.az2 = zp + 3 * nnz;
+    X.source(0, S.ixs, S.izs);
+    S.tx0 = S.tz0 = -100000;
+    if (X.taper) {
+        S.tx0 = o.box.x0;
+        S.tz0 = o.box.z0;
+        S.te2 = X.small.at<float>(o.te2);
+        S.td2 = X.small.at<float>(o.td2);
+        if (mpi) {
+            S.tkz = X.small.at<double>(o_tkz);
+            S.tkx = X.small.at<double>(o_tkx);
+        }
+    }
+    S.rec_iz = npd;
+    S.rec_scale = 1.0f;
+    j.nx = nx; j.nz = nz; j.npd = npd; j.ldz = nnz;
+    j.vp2 = mpi;   // vp <- rho*vp^2 with rho == 1 (Toa_rtm_vti_adcig_cdp.c:641)
+    j.pw = d_pw.as<double>();
+    j.ax1 = S.ax1; j.az1 = S.az1;
+    j.ddtx = ddtx; j.ddtz = ddtz;
+    S.vp = j.vp; S.e2 = j.e2; S.d2 = j.d2; S.kz = j.kz; S.kx = j.kx;
+    GEO_TRY(launch_model2d(raw, {j}, s));
+    GEO_CUDA(cudaMemsetAsync(X.mem.buf.p, 0, clear, s));
+    return GEO_OK;
+}
+
+// The shots of a batched RTM on the device for the fused steps.
+struct MarchBatch {
+    ShotSet X;
+    std::vector<March2D> M;
+    DevBuf d_M, d_items[2];
+    std::vector<int4> items[2];   // forward, backward
+    bool fast = false, wide = false, adcig = false;
+    int build(const Raw2D &raw, float dx, float dz, float dt, int nt, cudaStream_t s);
+    int clear_side(int k, int slots, cudaStream_t s) {
+        GEO_CUDA(cudaMemsetAsync(M[k].f, 0, (size_t)slots * M[k].n * 4, s));
+        return GEO_OK;
+    }
+    int work(bool backward);
+    int step(bool backward, const MarchStep &st, cudaStream_t s) {
+        return launch_march2d(backward, fast, adcig, wide, d_M.as<March2D>(), d_items[backward].as<int4>(),
+                              (int)items[backward].size(), st, s);
+    }
+};
+
+// Strips of at most 120 depths and chunks of columns.  A chunk repeats 14
+// columns' worth of P and 7 of u, so long chunks save work; short ones
+// balance it, since warps on a wavefront's rim take longer (ziv.cuh).  Four
+// waves of warps, within 8 and 48 columns: 16 shots of 401-1199 columns x 601
+// take 182 us a forward and 328 us a backward step with chunks of about 12,
+// 200 and 376 us with one wave (35 and 70 columns).
+int MarchBatch::work(bool backward) {
+    const int nnz = X.nnz, depths = nnz - 8, ns = (int)M.size();
+    const int strips = (depths + 119) / 120, len = ((depths + strips - 1) / strips + 3) / 4 * 4;
+    long cols = 0;
+    for (int k = 0; k < ns; k++) cols += (long)strips * (M[k].nnx - 8);
+    int res = 0;
+    GEO_TRY(march2d_resident(backward, fast, adcig, &res));
+    const int chunk = (int)std::min(48L, std::max(8L, cols / (4L * res)));
+    std::vector<int4> &v = items[backward];
+    v.clear();
+    for (int k = 0; k < ns; k++) {
+        const int w = M[k].nnx - 8, nc = std::max(1, (w + chunk / 2) / chunk);
+        for (int t = 0; t < strips; t++)
+            for (int c = 0; c < nc; c++)
+                v.push_back(make_int4(k | (len / 4) << 24, t * len, 4 + (int)((long)w * c / nc), 4 + (int)((long)w * (c + 1) / nc)));
+    }
+    return GEO_OK;
+}
+
+int MarchBatch::build(const Raw2D &raw, float dx, float dz, float dt, int nt, cudaStream_t s) {
+    const int ns = (int)X.G.size(), npd = X.npd, nz = X.nz, nnz = X.nnz, ldz = (nnz + 3) / 4 * 4;
+    DevBuf d_pw;
+    if (!fast) GEO_TRY(upload_pow_half(raw, d_pw, s));
+    std::vector<ShotSet::Off> off(ns);
+    std::vector<size_t> o_tpw2(ns), o_tpw(ns);
+    for (int k = 0; k < ns; k++) {
+        X.tables(k, dx, dz, dt, ldz, off[k]);
+        if (fast) continue;
+        std::vector<double> pw(kTB * kTB);
+        std::vector<float> p2(2 * kTB * kTB);
+        for (int b = 0; b < kTB * kTB; b++) {
+            pw[b] = std::pow((double)(1 + 2 * off[k].box.d[b]), 0.5);
+            p2[2 * b] = (float)pw[b];
+            p2[2 * b + 1] = (float)(pw[b] - (double)p2[2 * b]);
+        }
+        o_tpw[k] = X.small.put(pw);
+        o_tpw2[k] = X.small.put(p2);
+    }
+    GEO_TRY(X.small.upload(s));
+    M.assign(ns, March2D{});
+    std::vector<ModelJob> jobs(ns, ModelJob{});
+    for (int pass = 0; pass < 2; pass++) {   // sizes, then addresses
         for (int k = 0; k < ns; k++) {
-            const size_t m = (size_t)G[k].nx * nz;
-            if (image) {
-                S[k].mig = mem.take<float>(m);
-                S[k].ill = mem.take<float>(m);
-            }
-            if (adcig) S[k].adcig = mem.take<float>(kAdcigAngles * m);
+            const int nx = X.G[k].nx, nnx = nx + 2 * npd;
+            const size_t n = (size_t)nnx * ldz, L = 2 * (size_t)nx + 2 * (size_t)nz;
+            March2D &m = M[k];
+            m.n = (unsigned)n;
+            if ((double)MS_SLOTS * n >= 4294967296.0) wide = true;
+            m.f = X.mem.take<float>((fast ? MS_PL : MS_SLOTS) * n);
+            if (!fast) m.pw = jobs[k].pwd = X.mem.take<double>(n);
+            if (adcig) m.adcig = X.mem.take<float>((size_t)kAdcigAngles * nx * nz);
+            m.rec_p = X.mem.take<float>((size_t)nt * nx);
+            m.rec_q = X.mem.take<float>((size_t)nt * nx);
+            m.edge_p = X.mem.take<float>((size_t)nt * L);
+            m.edge_q = X.mem.take<float>((size_t)nt * L);
         }
-        z_rec = mem.off;
-        for (int k = 0; k < ns; k++) {
-            S[k].rec_p = mem.take<float>((size_t)nt * G[k].nx);
-            S[k].rec_q = edges ? mem.take<float>((size_t)nt * G[k].nx) : nullptr;
-        }
-        z_end = mem.off;
-        for (int k = 0; k < ns; k++) {
-            const int nnx = G[k].nx + 2 * npd;
-            const size_t n = (size_t)nnx * nnz, L = 2 * (size_t)G[k].nx + 2 * (size_t)nz;
-            ModelJob &j = jobs[k];
-            j.nx = G[k].nx; j.nz = nz; j.npd = npd; j.ldz = nnz; j.col0 = G[k].col0;
-            j.vp2 = var == V_MPI;   // vp <- rho*vp^2 with rho == 1 (Toa_rtm_vti_adcig_cdp.c:641)
-            j.vp = mem.take<float>(n);
-            j.e2 = mem.take<float>(n);
-            j.d2 = kchain ? nullptr : mem.take<float>(n);
-            j.rad = nullptr;
-            j.kz = kchain ? mem.take<double>(n) : nullptr;
-            j.kx = kchain ? mem.take<double>(n) : nullptr;
-            j.pw = d_pw.as<double>();
-            j.ddtx = ddtx; j.ddtz = ddtz;
-            if (edges) {
-                S[k].edge_p = mem.take<float>((size_t)nt * L);
-                S[k].edge_q = mem.take<float>((size_t)nt * L);
-            }
-        }
-        if (pass == 0) GEO_TRY(mem.alloc());
+        X.mem.take<float>(1024);   // the last column's rows run past it
+        if (pass == 0) GEO_TRY(X.mem.alloc());
     }
     for (int k = 0; k < ns; k++) {
-        Shot2D &h = S[k];
-        h.nnx = G[k].nx + 2 * npd; h.nnz = nnz; h.npd = npd; h.nx = G[k].nx; h.nz = nz;
-        h.dtx = dt / dx; h.dtz = dt / dz;
-        const float **dp[8] = {&h.cx1, &h.cx2, &h.ax1, &h.ax2, &h.cz1, &h.cz2, &h.az1, &h.az2};
-        for (int q = 0; q < 8; q++) *dp[q] = small.at<float>(off[k].prof[q]);
-        ModelJob &j = jobs[k];
-        j.ax1 = h.ax1;
-        j.az1 = h.az1;
-        h.vp = j.vp; h.e2 = j.e2; h.d2 = j.d2; h.kz = j.kz; h.kx = j.kx;
-        if (taper) {
-            h.te2 = small.at<float>(off[k].te2);
-            h.td2 = small.at<float>(off[k].td2);
-            if (kchain) {
-                h.tkz = small.at<double>(off[k].tkz);
-                h.tkx = small.at<double>(off[k].tkx);
-            }
+        March2D &m = M[k];
+        const int nx = X.G[k].nx;
+        m.nnx = nx + 2 * npd; m.nnz = nnz; m.ldz = ldz; m.npd = npd; m.nx = nx; m.nz = nz;
+        m.dtx = dt / dx; m.dtz = dt / dz;
+        const float *xp = X.small.at<float>(off[k].xprof);
+        m.cx1 = xp; m.cx2 = xp + m.nnx; m.ax1 = xp + 2 * m.nnx; m.ax2 = xp + 3 * m.nnx;
+        m.cz1 = X.small.at<float>(off[k].zprof);
+        m.tx0 = off[k].box.x0;
+        m.tz0 = off[k].box.z0;
+        m.te2 = X.small.at<float>(off[k].te2);
+        m.td2 = X.small.at<float>(off[k].td2);
+        if (!fast) {
+            m.tpw = X.small.at<double>(o_tpw[k]);
+            m.tpw2 = X.small.at<float2>(o_tpw2[k]);
         }
-        h.rec_iz = npd;
-        h.rec_scale = 1.0f;
+        X.source(k, m.ixs, m.izs);
+        ModelJob &j = jobs[k];
+        const size_t n = m.n;
+        j.nx = nx; j.nz = nz; j.npd = npd; j.ldz = ldz; j.col0 = X.G[k].col0;
+        j.vp2 = 1;   // vp <- rho*vp^2 with rho == 1 (Toa_rtm_vti_adcig_cdp.c:641)
+        j.vp = m.f + MS_VP * n;
+        j.e2 = m.f + MS_E2 * n;
+        if (fast) {
+            j.d2 = m.f + MS_D2 * n;
+        } else {
+            j.ph = m.f + MS_D2 * n;
+            j.pl = m.f + MS_PL * n;
+            j.pw = d_pw.as<double>();
+        }
+        // the model's slots, whose pitch columns beyond nnz are never used, stay as allocated
+        GEO_TRY(clear_side(k, MS_STATE, s));
+        if (adcig) GEO_CUDA(cudaMemsetAsync(m.adcig, 0, (size_t)kAdcigAngles * nx * nz * 4, s));
+        GEO_CUDA(cudaMemsetAsync(m.rec_p, 0, (size_t)nt * nx * 4, s));
+        GEO_CUDA(cudaMemsetAsync(m.rec_q, 0, (size_t)nt * nx * 4, s));
     }
     GEO_TRY(launch_model2d(raw, jobs, s));
-    return clear(0, z_end, s);
+    GEO_TRY(d_M.alloc(ns * sizeof(March2D)));
+    GEO_CUDA(cudaMemcpyAsync(d_M.p, M.data(), ns * sizeof(March2D), cudaMemcpyHostToDevice, s));
+    for (int b = 0; b < 2; b++) {
+        GEO_TRY(work(b));
+        GEO_TRY(d_items[b].alloc(items[b].size() * sizeof(int4)));
+        GEO_CUDA(cudaMemcpyAsync(d_items[b].p, items[b].data(), items[b].size() * sizeof(int4), cudaMemcpyHostToDevice, s));
+    }
+    return GEO_OK;
 }
 
 // Work list: item -> shot.  Tiles are 32 (z) x by (x).
@@ -289,72 +383,8 @@ struct Batch2D {
     int vel(Step2D st, cudaStream_t s) {
         return launch_vel2d(variant, d_S.as<Shot2D>(), d_items.as<int>(), (int)items.size(), by, grid, st, s);
     }
-    int stress(int phase, Step2D st, cudaStream_t s) {
-        return launch_stress2d(variant, phase, d_S.as<Shot2D>(), d_items.as<int>(), (int)items.size(), by, grid, st, s);
-    }
-
-    // Skewed schedule (MPI form, two or more shots): the shots are split
-    // into groups A = [0, split) and B = [split, ns) of about equal tiles,
-    // B half a step behind A, so that every launch pairs one group's stress
-    // tiles with the other's velocity tiles (launch_mix2d).  Every shot
-    // still runs velocity then stress of each step in order.  Tables, as
-    // (shot | kind << 30, tile) items with the kinds interleaved:
-    //   VA: velocity of A;  MX: stress of A + velocity of B;
-    //   MY: velocity of A + stress of B;  SB: stress of B.
-    enum { VA = 0, MX = 1, MY = 2, SB = 3 };
-    DevBuf d_mix;
-    int split = 0, mix_n[4] = {0, 0, 0, 0};
-    size_t mix_o[4] = {0, 0, 0, 0};
-    int build_mix(cudaStream_t s) {
-        const int ns = (int)S.size();
-        std::vector<long> tiles(ns);
-        long total = 0;
-        for (int k = 0; k < ns; k++) {
-            tiles[k] = (long)S[k].ntz * ((S[k].nnx + by - 1) / by);
-            total += tiles[k];
-        }
-        long acc = 0;
-        split = 1;
-        for (int k = 0; k < ns - 1; k++) {
-            acc += tiles[k];
-            split = k + 1;
-            if (2 * acc >= total) break;
-        }
-        auto list = [&](int k0, int k1, int kind) {
-            std::vector<int2> v;
-            for (int k = k0; k < k1; k++)
-                for (long t = 0; t < tiles[k]; t++) v.push_back(make_int2(k | (kind << 30), (int)t));
-            return v;
-        };
-        auto merge = [](const std::vector<int2> &a, const std::vector<int2> &b) {
-            std::vector<int2> v;
-            v.reserve(a.size() + b.size());
-            size_t i = 0, j = 0;
-            while (i < a.size() || j < b.size()) {
-                if (j >= b.size() || (i < a.size() && i * b.size() <= j * a.size())) v.push_back(a[i++]);
-                else v.push_back(b[j++]);
-            }
-            return v;
-        };
-        const std::vector<int2> vA = list(0, split, 0), sA = list(0, split, 1), vB = list(split, ns, 0),
-                                sB = list(split, ns, 1);
-        const std::vector<int2> tab[4] = {vA, merge(sA, vB), merge(vA, sB), sB};
-        size_t off = 0;
-        for (int t = 0; t < 4; t++) {
-            mix_o[t] = off;
-            mix_n[t] = (int)tab[t].size();
-            off += tab[t].size();
-        }
-        GEO_TRY(d_mix.alloc(off * sizeof(int2)));
-        for (int t = 0; t < 4; t++)
-            GEO_CUDA(cudaMemcpyAsync(d_mix.as<int2>() + mix_o[t], tab[t].data(), tab[t].size() * sizeof(int2),
-                                     cudaMemcpyHostToDevice, s));
-        GEO_CUDA(cudaStreamSynchronize(s));
-        return GEO_OK;
-    }
-    int mix(int table, int phase, int fast, Step2D sv, Step2D ss, cudaStream_t s) {
-        return launch_mix2d(phase, fast, d_S.as<Shot2D>(), d_mix.as<int2>() + mix_o[table], mix_n[table], by, grid,
-                            sv, ss, s);
+    int stress(Step2D st, cudaStream_t s) {
+        return launch_stress2d(variant, d_S.as<Shot2D>(), d_items.as<int>(), (int)items.size(), by, grid, st, s);
     }
 };
 
@@ -390,58 +420,6 @@ static int capture(Graph &G, cudaStream_t cs, F &&body) {
     if (e != cudaSuccess) return fail(GEO_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
     G.g = g;
     GEO_CUDA(cudaGraphInstantiate(&G.x, g, 0));
-    return GEO_OK;
-}
-
-// Autotuner: time a few forward steps for each (rows per tile, blocks per
-// SM) candidate on the real batch and keep the fastest.  Results are cached
-// per (grid extents, shot count, device) for the life of the process.
-static std::map<std::tuple<int, int, int, int>, std::pair<int, int>> g_tune_cache;
-
-static int autotune(Batch2D &B, int nf, int key_nx, int key_nz, cudaStream_t s, int *by_out, int *bps_out) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    auto key = std::make_tuple(key_nx, key_nz, (int)B.S.size() * 16 + nf, dev);
-    auto it = g_tune_cache.find(key);
-    if (it != g_tune_cache.end()) {
-        *by_out = it->second.first;
-        *bps_out = it->second.second;
-        return GEO_OK;
-    }
-    const int bys[] = {4, 8};
-    const int bpss[] = {4, 8, 16};
-    float best = 1e30f;
-    int bb = 8, bp = 8;
-    cudaEvent_t a, b;
-    GEO_CUDA(cudaEventCreate(&a));
-    GEO_CUDA(cudaEventCreate(&b));
-    Step2D st{};
-    st.nf = nf;
-    for (int by : bys)
-        for (int bps : bpss) {
-            GEO_TRY(B.upload(by, bps, s));
-            GEO_TRY(B.vel(st, s));
-            GEO_TRY(B.stress(PH_BWD, st, s));
-            GEO_CUDA(cudaEventRecord(a, s));
-            for (int k = 0; k < 4; k++) {
-                GEO_TRY(B.vel(st, s));
-                GEO_TRY(B.stress(PH_BWD, st, s));
-            }
-            GEO_CUDA(cudaEventRecord(b, s));
-            GEO_CUDA(cudaEventSynchronize(b));
-            float ms = 0;
-            GEO_CUDA(cudaEventElapsedTime(&ms, a, b));
-            if (ms < best) {
-                best = ms;
-                bb = by;
-                bp = bps;
-            }
-        }
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    g_tune_cache[key] = {bb, bp};
-    *by_out = bb;
-    *bps_out = bp;
     return GEO_OK;
 }
 
@@ -486,7 +464,8 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
     Raw2D raw;
     GEO_TRY(raw.open(D.nx, D.nz, v, e, d, nullptr, mem, ss.cs));
     const bool taper = var == V_MPI || D.sv;
-    ShotSet X;
+    SingleShot shot1;
+    ShotSet &X = shot1.X;
     X.var = var;
     X.nz = D.nz; X.npd = D.npd; X.nnz = nnz;
     X.taper = taper;
@@ -503,12 +482,12 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
     std::vector<float> amp;
     std::vector<uint8_t> on;
     source_amplitudes(var, D.nt, D.dt, D.favg, D.pfac, D.wtype, amp, on);
-    GEO_TRY(X.build(raw, D.dx, D.dz, D.dt, amp, on, 1, D.nt, false, false, false, false, ss.cs));
-    const float *d_amp = X.small.at<float>(X.o_amp);
-    const unsigned char *d_on = X.small.at<unsigned char>(X.o_on);
+    GEO_TRY(shot1.build(raw, D.dx, D.dz, D.dt, amp, on, D.nt, ss.cs));
+    const float *d_amp = X.small.at<float>(shot1.o_amp);
+    const unsigned char *d_on = X.small.at<unsigned char>(shot1.o_on);
     Batch2D B;
     B.variant = var;
-    B.S = X.S;
+    B.S = {shot1.S};
     B.S[0].rec_iz = D.rec_iz;
     B.S[0].rec_scale = D.rec_scale;
     const bool persistent = !(snap && snap_every > 0);
@@ -518,9 +497,8 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
         st.amp = amp[it];
         st.src_on = on[it];
         st.taper = taper ? 1 : 0;
-        st.nf = 1;
         GEO_TRY(B.vel(st, ss.cs));
-        return B.stress(PH_FWD, st, ss.cs);
+        return B.stress(st, ss.cs);
     };
     DevBuf d_sync;
     GEO_TRY(d_sync.alloc(8));
@@ -554,9 +532,9 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
             tiled = true;
             const int it = it1 - 1;
             if (snap && snap_every > 0 && it % snap_every == 0)
-                GEO_CUDA(cudaMemcpyAsync(snap + (size_t)(it / snap_every) * nn, B.S[0].P[0], nn * 4, ksnap, ss.cs));
+                GEO_CUDA(cudaMemcpyAsync(snap + (size_t)(it / snap_every) * nn, B.S[0].P, nn * 4, ksnap, ss.cs));
             if (wd.every > 0) {
-                GEO_TRY(wd.scan(B.S[0].P[0], nn, it + 1, ss.cs));
+                GEO_TRY(wd.scan(B.S[0].P, nn, it + 1, ss.cs));
                 if (wd.tripped()) break;
             }
             it0 = it1;
@@ -574,9 +552,9 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
         for (int it = 0; it < D.nt; it++) {
             GEO_TRY(step(it));
             if (it % snap_every == 0)
-                GEO_CUDA(cudaMemcpyAsync(snap + (size_t)(it / snap_every) * nn, B.S[0].P[0], nn * 4, ksnap, ss.cs));
+                GEO_CUDA(cudaMemcpyAsync(snap + (size_t)(it / snap_every) * nn, B.S[0].P, nn * 4, ksnap, ss.cs));
             if (wd.every > 0 && ((it + 1) % wd.every == 0 || it == D.nt - 1)) {
-                GEO_TRY(launch_watch_shots(B.d_S.as<Shot2D>(), 1, 1, wd.d, it + 1, ss.cs));
+                GEO_TRY(wd.scan(B.S[0].P, nn, it + 1, ss.cs));
                 if (wd.tripped()) break;
             }
         }
@@ -597,7 +575,7 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
         if (err) return fail(GEO_ERR_CUDA, "2D shot: a grid barrier wait timed out");
         // the shot ran in one launch: scan its final P and its record
         if (wd.every > 0) {
-            GEO_TRY(launch_watch_shots(B.d_S.as<Shot2D>(), 1, 1, wd.d, D.nt, ss.cs));
+            GEO_TRY(wd.scan(B.S[0].P, nn, D.nt, ss.cs));
             GEO_TRY(wd.scan(B.S[0].rec_p, (size_t)D.nx * D.nt, D.nt, ss.cs));
         }
     }
@@ -656,7 +634,10 @@ extern "C" int geo_rtm2d_batch_adcig(const geo_rtm2d_desc *desc, const float *v,
     GEO_TRY(raw.open(D.nx, D.nz, v, e, d, nullptr, mem, ss.cs));
     const float dt = D.dt_ms / 1000;
     const int nt = D.nt, nz = D.nz, npd = D.npd;
-    ShotSet X;
+    MarchBatch B;
+    B.fast = fast != 0;
+    B.adcig = adcig != nullptr;
+    ShotSet &X = B.X;
     X.var = V_MPI;
     X.nz = nz; X.npd = npd; X.nnz = nz + 2 * npd;
     X.taper = true;
@@ -673,53 +654,42 @@ extern "C" int geo_rtm2d_batch_adcig(const geo_rtm2d_desc *desc, const float *v,
     std::vector<float> amp;
     std::vector<uint8_t> on;
     source_amplitudes(V_MPI, nt, dt, D.favg, D.pfac, 1, amp, on);
-    GEO_TRY(X.build(raw, D.dx, D.dz, dt, amp, on, 2, nt, true, true, adcig != nullptr, fast != 0, ss.cs));
-    Batch2D B;
-    B.variant = V_MPI;
-    B.S = X.S;
-    // tile shape: caller's choice or the autotuner's
-    int by = D.tile_x, bps = 8;
-    if (by != 4 && by != 8) GEO_TRY(autotune(B, 2, D.nx, D.nz, ss.cs, &by, &bps));
-    GEO_TRY(B.upload(by, bps, ss.cs));
-    // the autotuner stepped the state: start from zero again
-    GEO_TRY(X.clear(X.z_side0, X.z_rec, ss.cs));
-    if (adcig) GEO_TRY(load_adcig_tables(ss.cs));
-
+    GEO_TRY(B.build(raw, D.dx, D.dz, dt, nt, ss.cs));
+    GEO_TRY(load_march_tables(adcig != nullptr, ss.cs));
+    const March2D *d_M = B.d_M.as<March2D>();
     // non-finite detector: every wd.every steps (and the last) the graphs
     // scan every shot's P; the verdict follows each pass
     Watchdog wd;
     GEO_TRY(wd.open());
-    auto watch = [&](int k, bool last, int nf) -> int {
+    auto watch = [&](int k, bool last, int nf, int lev) -> int {
         if (wd.every <= 0 || ((k + 1) % wd.every && !last)) return GEO_OK;
-        return launch_watch_shots(B.d_S.as<Shot2D>(), D.ns, nf, wd.d, k + 1, ss.cs);
+        return launch_march_watch(d_M, D.ns, nf, lev, wd.d, k + 1, ss.cs);
     };
-    // forward: source side only, with records and edge lines; with two or
-    // more shots on the skewed schedule (Batch2D::build_mix)
-    const bool skew = D.ns >= 2;
-    if (skew) GEO_TRY(B.build_mix(ss.cs));
-    auto fwd_st = [&](int it) {
-        Step2D st{};
-        st.it = it; st.amp = amp[it]; st.src_on = on[it]; st.taper = 1; st.nf = 1; st.fast = fast;
+    DevBuf d_err;
+    GEO_TRY(d_err.alloc(4));
+    GEO_TRY(d_err.zero(ss.cs));
+    auto step = [&](int it, int k) {   // k-th step of its pass
+        MarchStep st{};
+        st.it = it;
+        st.lev = k & 1;
+        st.inject = -1;
+        st.err = d_err.as<int>();
+        st.ddtx = (double)(dt / D.dx);
+        st.ddtz = (double)(dt / D.dz);
+        st.dhx = (float)st.ddtx; st.dlx = (float)(st.ddtx - (double)st.dhx);
+        st.dhz = (float)st.ddtz; st.dlz = (float)(st.ddtz - (double)st.dhz);
         return st;
     };
+    // forward: source side only, with records and edge lines
     {
         Graph G;
         GEO_TRY(capture(G, ss.cs, [&]() -> int {
-            if (skew) {
-                GEO_TRY(B.mix(Batch2D::VA, PH_FWD, fast, fwd_st(0), fwd_st(0), ss.cs));
-                for (int it = 0; it < nt; it++) {
-                    GEO_TRY(B.mix(Batch2D::MX, PH_FWD, fast, fwd_st(it), fwd_st(it), ss.cs));
-                    if (it + 1 < nt) GEO_TRY(B.mix(Batch2D::MY, PH_FWD, fast, fwd_st(it + 1), fwd_st(it), ss.cs));
-                    else GEO_TRY(B.mix(Batch2D::SB, PH_FWD, fast, fwd_st(it), fwd_st(it), ss.cs));
-                    GEO_TRY(watch(it, it == nt - 1, 1));
-                }
-                return GEO_OK;
-            }
             for (int it = 0; it < nt; it++) {
-                const Step2D st = fwd_st(it);
-                GEO_TRY(B.vel(st, ss.cs));
-                GEO_TRY(B.stress(PH_FWD, st, ss.cs));
-                GEO_TRY(watch(it, it == nt - 1, 1));
+                MarchStep st = step(it, it);
+                st.amp = amp[it];
+                st.src_on = on[it];
+                GEO_TRY(B.step(false, st, ss.cs));
+                GEO_TRY(watch(it, it == nt - 1, 1, st.lev ^ 1));
             }
             return GEO_OK;
         }));
@@ -739,65 +709,54 @@ extern "C" int geo_rtm2d_batch_adcig(const geo_rtm2d_desc *desc, const float *v,
     GEO_CUDA(cudaMemcpyAsync(d_mute.p, mute.data(), mute.size() * 4, cudaMemcpyHostToDevice, ss.cs));
     for (int k = 0, o = 0; k < D.ns; o += D.shot_nxs[k++]) {
         const int *hi = d_mute.as<int>() + o;
-        GEO_TRY(launch_mute_records(B.S[k].rec_p, D.shot_nxs[k], nt, nullptr, hi, ss.cs));
-        GEO_TRY(launch_mute_records(B.S[k].rec_q, D.shot_nxs[k], nt, nullptr, hi, ss.cs));
+        GEO_TRY(launch_mute_records(B.M[k].rec_p, D.shot_nxs[k], nt, nullptr, hi, ss.cs));
+        GEO_TRY(launch_mute_records(B.M[k].rec_q, D.shot_nxs[k], nt, nullptr, hi, ss.cs));
+        GEO_TRY(B.clear_side(k, MS_SIDE, ss.cs));
     }
-    GEO_TRY(X.clear(X.z_side0, X.z_side1, ss.cs));
-    // backward: inject, both propagations, fused imaging
+    // backward: both propagations with fused imaging; each step's lines and
+    // records go into the level it reads, the first by a launch of its own,
+    // the others as the step before stores that level
     {
         Graph G;
-        auto bwd_st = [&](int it) {
-            Step2D st{};
-            st.it = it; st.nf = 2; st.fast = fast;
-            return st;
-        };
-        const Shot2D *dA = B.d_S.as<Shot2D>(), *dB = dA + B.split;
-        const int nA = B.split, nB = D.ns - B.split;
         GEO_TRY(capture(G, ss.cs, [&]() -> int {
-            if (skew) {
-                GEO_TRY(launch_inject2d(dA, nA, maxline, nt - 1, ss.cs));
-                GEO_TRY(B.mix(Batch2D::VA, PH_BWD, fast, bwd_st(nt - 1), bwd_st(nt - 1), ss.cs));
-                for (int it = nt - 1; it >= 0; it--) {
-                    GEO_TRY(launch_inject2d(dB, nB, maxline, it, ss.cs));
-                    GEO_TRY(B.mix(Batch2D::MX, PH_BWD, fast, bwd_st(it), bwd_st(it), ss.cs));
-                    if (it > 0) {
-                        GEO_TRY(launch_inject2d(dA, nA, maxline, it - 1, ss.cs));
-                        GEO_TRY(B.mix(Batch2D::MY, PH_BWD, fast, bwd_st(it - 1), bwd_st(it), ss.cs));
-                    } else {
-                        GEO_TRY(B.mix(Batch2D::SB, PH_BWD, fast, bwd_st(it), bwd_st(it), ss.cs));
-                    }
-                    GEO_TRY(watch(nt - 1 - it, it == 0, 2));
-                }
-                return GEO_OK;
-            }
+            GEO_TRY(launch_march_inject(d_M, D.ns, maxline, nt - 1, 0, ss.cs));
             for (int it = nt - 1; it >= 0; it--) {
-                GEO_TRY(launch_inject2d(B.d_S.as<Shot2D>(), D.ns, maxline, it, ss.cs));
-                const Step2D st = bwd_st(it);
-                GEO_TRY(B.vel(st, ss.cs));
-                GEO_TRY(B.stress(PH_BWD, st, ss.cs));
-                GEO_TRY(watch(nt - 1 - it, it == 0, 2));
+                MarchStep st = step(it, nt - 1 - it);
+                st.inject = it - 1;
+                GEO_TRY(B.step(true, st, ss.cs));
+                GEO_TRY(watch(nt - 1 - it, it == 0, 2, st.lev ^ 1));
             }
             return GEO_OK;
         }));
         GEO_TRY(G.launch(ss.cs));
     }
+    int gave_up = 0;
+    GEO_CUDA(cudaMemcpyAsync(&gave_up, d_err.p, 4, cudaMemcpyDeviceToHost, ss.cs));
     GEO_TRY(wd.verdict(ss.cs, "batched 2D RTM backward pass"));
+    GEO_CUDA(cudaStreamSynchronize(ss.cs));
+    if (gave_up) return fail(GEO_ERR_CUDA, "batched 2D RTM: a pipeline wait timed out");
     // normalise per shot, stack in shot order, Laplacian
-    std::vector<const float *> imgs(D.ns);
+    std::vector<float *> imgs(2 * (size_t)D.ns);   // images, then illuminations
     std::vector<int> offs(D.ns), wid(D.ns);
-    for (int k = 0; k < D.ns; k++) {
-        GEO_TRY(launch_normalize_image(B.S[k].mig, B.S[k].ill, (size_t)D.shot_nxs[k] * nz, ss.cs));
-        imgs[k] = B.S[k].mig;
-        offs[k] = D.shot_x[k] - D.shot_nxs[k] / 2 - 1;
-        wid[k] = D.shot_nxs[k];
+    Arena out;
+    for (int pass = 0; pass < 2; pass++) {
+        for (int k = 0; k < D.ns; k++) {
+            const size_t m = (size_t)D.shot_nxs[k] * nz;
+            imgs[k] = out.take<float>(m);
+            imgs[D.ns + k] = out.take<float>(m);
+            offs[k] = D.shot_x[k] - D.shot_nxs[k] / 2 - 1;
+            wid[k] = D.shot_nxs[k];
+        }
+        if (pass == 0) GEO_TRY(out.alloc());
     }
     DevBuf d_imgs, d_offs, d_wid, stack, lap;
-    GEO_TRY(d_imgs.alloc(D.ns * sizeof(float *)));
+    GEO_TRY(d_imgs.alloc(2 * D.ns * sizeof(float *)));
     GEO_TRY(d_offs.alloc(D.ns * 4));
     GEO_TRY(d_wid.alloc(D.ns * 4));
-    GEO_CUDA(cudaMemcpyAsync(d_imgs.p, imgs.data(), D.ns * sizeof(float *), cudaMemcpyHostToDevice, ss.cs));
+    GEO_CUDA(cudaMemcpyAsync(d_imgs.p, imgs.data(), 2 * D.ns * sizeof(float *), cudaMemcpyHostToDevice, ss.cs));
     GEO_CUDA(cudaMemcpyAsync(d_offs.p, offs.data(), D.ns * 4, cudaMemcpyHostToDevice, ss.cs));
     GEO_CUDA(cudaMemcpyAsync(d_wid.p, wid.data(), D.ns * 4, cudaMemcpyHostToDevice, ss.cs));
+    GEO_TRY(launch_march_image(d_M, D.ns, d_imgs.as<float *>(), d_imgs.as<float *>() + D.ns, ss.cs));
     const size_t nimg = (size_t)D.nx * nz;
     GEO_TRY(stack.alloc(nimg * 4));
     GEO_TRY(stack.zero(ss.cs));
@@ -818,8 +777,8 @@ extern "C" int geo_rtm2d_batch_adcig(const geo_rtm2d_desc *desc, const float *v,
         std::vector<const float *> ap((size_t)kAdcigAngles * D.ns);
         for (int q = 0; q < D.ns; q++) {
             const size_t m = (size_t)D.shot_nxs[q] * nz;
-            GEO_TRY(launch_normalize_planes(B.S[q].adcig, B.S[q].ill, m, kAdcigAngles, ss.cs));
-            for (int ia = 0; ia < kAdcigAngles; ia++) ap[(size_t)ia * D.ns + q] = B.S[q].adcig + ia * m;
+            GEO_TRY(launch_normalize_planes(B.M[q].adcig, imgs[D.ns + q], m, kAdcigAngles, ss.cs));
+            for (int ia = 0; ia < kAdcigAngles; ia++) ap[(size_t)ia * D.ns + q] = B.M[q].adcig + ia * m;
         }
         GEO_TRY(d_aptr.alloc(ap.size() * sizeof(float *)));
         GEO_CUDA(cudaMemcpyAsync(d_aptr.p, ap.data(), ap.size() * sizeof(float *), cudaMemcpyHostToDevice, ss.cs));
@@ -835,7 +794,7 @@ extern "C" int geo_rtm2d_batch_adcig(const geo_rtm2d_desc *desc, const float *v,
         size_t o = 0;
         for (int q = 0; q < D.ns; q++) {
             const size_t m = (size_t)D.shot_nxs[q] * nz;
-            GEO_CUDA(cudaMemcpyAsync(per_shot + o, B.S[q].mig, m * 4, k, ss.cs));
+            GEO_CUDA(cudaMemcpyAsync(per_shot + o, imgs[q], m * 4, k, ss.cs));
             o += m;
         }
     }

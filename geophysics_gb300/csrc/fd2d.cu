@@ -1,9 +1,8 @@
-// 2D VTI staggered-grid kernels, batched over shots.
+// 2D VTI staggered-grid kernels of single-shot forward modelling.
 //
-// One launch updates every shot of a batch: the grid is persistent (a
-// multiple of the SM count) and walks the list of (shot, tile) work items,
-// so uneven aperture windows share one launch.  A tile is 32 z-points (one
-// warp, z contiguous in memory) by `blockDim.y` x-columns.
+// The half-step kernels walk a shot's tiles with a persistent grid; a tile
+// is 32 z-points (one warp, z contiguous in memory) by `blockDim.y`
+// x-columns.
 //
 // Arithmetic keeps the reference's operation order exactly (the library is
 // compiled with contraction off), so results are bit-identical to the
@@ -76,28 +75,7 @@ __device__ __forceinline__ float tap(const float *a, long idx, long src, float a
     return v;
 }
 
-// Poynting-vector angle gathers (RTM_corr_adcig, Toa_rtm_vti_adcig_cdp.c:1004-1068):
-// per image point the angle bin ia of the opening angle between the source
-// and receiver Poynting vectors, and adcig[ia] += gP*sP*cos(ia)^3.  The
-// program bins with (int)(float)(0.5*acosf(a1)*180/pi); that bin is a
-// non-increasing function of the float a1, so the host finds, with the same
-// libm, the largest a1 of every bin count (c_adthr[k-1]: largest a1 whose
-// bin is >= k) and the kernel counts thresholds instead of calling acosf.
-__constant__ float c_adthr[kAdcigAngles];
-__constant__ double c_adw[kAdcigAngles];
-
-__device__ __forceinline__ int adcig_bin(float a1) {
-    if (!(a1 >= -1.0f && a1 <= 1.0f)) return 0;
-    int lo = 0, hi = kAdcigAngles;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (a1 <= c_adthr[mid - 1]) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo == kAdcigAngles ? kAdcigAngles - 1 : lo;   // ia == 90 -> 89
-}
-
-// Velocity update of one updated point (ix, iz) of a shot, every field.
+// Velocity update of one updated point (ix, iz) of a shot.
 template <int VARIANT, bool NC>
 __device__ __forceinline__ void vel_point(const Shot2D &sh, int ix, int iz, const Step2D &st) {
     const int nnz = sh.nnz;
@@ -105,27 +83,24 @@ __device__ __forceinline__ void vel_point(const Shot2D &sh, int ix, int iz, cons
     const bool pt_src = VARIANT == V_GPU && st.src_on;
     const long src = (long)sh.ixs * nnz + sh.izs;
     const bool near = pt_src && ((iz == sh.izs && abs(ix - sh.ixs) <= 4) || (ix == sh.ixs && abs(iz - sh.izs) <= 4));
-    for (int f = 0; f < st.nf; f++) {
-        const float *P = sh.P[f], *Q = sh.Q[f];
-        float xx = 0.0f, zz = 0.0f;
-        if (near) {
+    const float *P = sh.P, *Q = sh.Q;
+    float xx = 0.0f, zz = 0.0f;
+    if (near) {
 #pragma unroll
-            for (int im = 0; im < 4; im++) {
-                xx += c_fd[im] * (tap<true, NC>(P, id + (im + 1) * nnz, src, st.amp) - tap<true, NC>(P, id - im * nnz, src, st.amp));
-                zz += c_fd[im] * (tap<true, NC>(Q, id + im + 1, src, st.amp) - tap<true, NC>(Q, id - im, src, st.amp));
-            }
-        } else {
-#pragma unroll
-            for (int im = 0; im < 4; im++) {
-                xx += c_fd[im] * (ldf<NC>(P + id + (im + 1) * nnz) - ldf<NC>(P + id - im * nnz));
-                zz += c_fd[im] * (ldf<NC>(Q + id + im + 1) - ldf<NC>(Q + id - im));
-            }
+        for (int im = 0; im < 4; im++) {
+            xx += c_fd[im] * (tap<true, NC>(P, id + (im + 1) * nnz, src, st.amp) - tap<true, NC>(P, id - im * nnz, src, st.amp));
+            zz += c_fd[im] * (tap<true, NC>(Q, id + im + 1, src, st.amp) - tap<true, NC>(Q, id - im, src, st.amp));
         }
-        float *u = sh.u[f], *w = sh.w[f];
-        // u1 = coffx2*u0 - coffx1*dtx*xx (the MPI copy's extra *rho is *1.0f)
-        u[id] = sh.cx2[ix] * u[id] - sh.cx1[ix] * sh.dtx * xx;
-        w[id] = sh.cz2[iz] * w[id] - sh.cz1[iz] * sh.dtz * zz;
+    } else {
+#pragma unroll
+        for (int im = 0; im < 4; im++) {
+            xx += c_fd[im] * (ldf<NC>(P + id + (im + 1) * nnz) - ldf<NC>(P + id - im * nnz));
+            zz += c_fd[im] * (ldf<NC>(Q + id + im + 1) - ldf<NC>(Q + id - im));
+        }
     }
+    // u1 = coffx2*u0 - coffx1*dtx*xx (the MPI copy's extra *rho is *1.0f)
+    sh.u[id] = sh.cx2[ix] * sh.u[id] - sh.cx1[ix] * sh.dtx * xx;
+    sh.w[id] = sh.cz2[iz] * sh.w[id] - sh.cz1[iz] * sh.dtz * zz;
 }
 
 template <int VARIANT>
@@ -138,20 +113,16 @@ __global__ void __launch_bounds__(256) k_vel2d(const Shot2D *__restrict__ shots,
     }
 }
 
-// Stress update of one updated point (ix, iz) of a shot, every field, and
-// the phase's epilogue (records and edge lines forward; image, illumination
-// and gathers backward).
-template <int VARIANT, int PHASE, bool NC, bool FAST = false>
+// Stress update of one updated point (ix, iz) of a shot, with the record.
+template <int VARIANT, bool NC>
 __device__ __forceinline__ void stress_point(const Shot2D &sh, int ix, int iz, const Step2D &st) {
     const int nnz = sh.nnz;
     const long id = (long)ix * nnz + iz;
     const float vp = __ldg(sh.vp + id);
-    // the MPI form's exact arithmetic carries its pz and qx chains in double
-    // (their fixed factors kz, kx formed per shot on the host in the
-    // program's order); its fast form (FAST, a separate instantiation so
-    // that no double operation is issued) uses the FP32 sqrtf(1+2del) of
-    // the others
-    constexpr bool dpw = VARIANT == V_MPI && !FAST;
+    // the MPI form's arithmetic carries its pz and qx chains in double
+    // (their fixed factors kz, kx formed once per shot in the program's
+    // order)
+    constexpr bool dpw = VARIANT == V_MPI;
     float e2 = __ldg(sh.e2 + id), d2 = 0.0f;
     double kz = 0.0, kx = 0.0;
     if (dpw) {
@@ -173,112 +144,60 @@ __device__ __forceinline__ void stress_point(const Shot2D &sh, int ix, int iz, c
         }
     }
     const float ax1 = sh.ax1[ix], ax2 = sh.ax2[ix], az1 = sh.az1[iz], az2 = sh.az2[iz];
-    // Gaussian source window value (CPU/MPI forward), added after the split sum.
-    float s = 0.0f;
-    if ((VARIANT == V_CPU || VARIANT == V_MPI) && PHASE == PH_FWD && st.src_on) {
-        const int rx = ix - sh.ixs, rz = iz - sh.izs;
-        if (rx >= -3 && rx <= 3 && rz >= -3 && rz <= 3)
-            s = (float)((double)st.amp * c_gauss[(rx + 3) * 7 + (rz + 3)]);
-    }
-    float Pn[2], Qn[2];
-    for (int f = 0; f < st.nf; f++) {
-        const float *u = sh.u[f], *w = sh.w[f];
-        float xx = 0.0f, zz = 0.0f;
+    float xx = 0.0f, zz = 0.0f;
 #pragma unroll
-        for (int im = 0; im < 4; im++) {
-            xx += c_fd[im] * (ldf<NC>(u + id + im * nnz) - ldf<NC>(u + id - (im + 1) * nnz));
-            zz += c_fd[im] * (ldf<NC>(w + id + im) - ldf<NC>(w + id - im - 1));
-        }
-        float px = sh.px[f][id], pz = sh.pz[f][id], qx = sh.qx[f][id], qz = sh.qz[f][id];
-        if (VARIANT == V_MPI) {
-            px = ax2 * px - ax1 * vp * e2 * sh.dtx * xx;
-            if (dpw) {
-                // the conversions on the integer pipe (softcvt.cuh): same bits
-                pz = d2f_rn(f2d_exact(az2 * pz) - kz * f2d_exact(zz));
-                qx = d2f_rn(f2d_exact(ax2 * qx) - kx * f2d_exact(xx));
-            } else {
-                pz = az2 * pz - az1 * vp * d2 * sh.dtz * zz;
-                qx = ax2 * qx - ax1 * vp * d2 * sh.dtx * xx;
-            }
-            qz = az2 * qz - az1 * vp * sh.dtz * zz;
-        } else {
-            px = ax2 * px - ax1 * vp * vp * e2 * sh.dtx * xx;
-            pz = az2 * pz - az1 * vp * vp * d2 * sh.dtz * zz;
-            qx = ax2 * qx - ax1 * vp * vp * d2 * sh.dtx * xx;
-            qz = az2 * qz - az1 * vp * vp * sh.dtz * zz;
-        }
-        sh.px[f][id] = px; sh.pz[f][id] = pz; sh.qx[f][id] = qx; sh.qz[f][id] = qz;
-        float P, Q;
-        if ((VARIANT == V_CPU || VARIANT == V_MPI) && PHASE == PH_FWD) {
-            P = px + pz + s;
-            Q = qx + qz + s;
-        } else {
-            P = px + pz;
-            Q = qx + qz;
-        }
-        sh.P[f][id] = P;
-        sh.Q[f][id] = Q;
-        Pn[f] = P; Qn[f] = Q;
+    for (int im = 0; im < 4; im++) {
+        xx += c_fd[im] * (ldf<NC>(sh.u + id + im * nnz) - ldf<NC>(sh.u + id - (im + 1) * nnz));
+        zz += c_fd[im] * (ldf<NC>(sh.w + id + im) - ldf<NC>(sh.w + id - im - 1));
     }
-    const int gx = ix - sh.npd, gz = iz - sh.npd;
-    if (PHASE == PH_FWD) {
-        // receiver gather at rec_iz, time-major
-        if (iz == sh.rec_iz && gx >= 0 && gx < sh.nx) {
-            const float r = sh.rec_scale == 2.0f ? Pn[0] + Pn[0] : Pn[0] * sh.rec_scale;
-            sh.rec_p[(long)st.it * sh.nx + gx] = r;
-            if (sh.rec_q) sh.rec_q[(long)st.it * sh.nx + gx] = Qn[0];
-        }
-        // interior-edge lines for the boundary-driven reconstruction
-        // (Toa_rtm_vti_adcig_cdp.c:668-683): top, bottom, left, right
-        if (sh.edge_p && gx >= 0 && gx < sh.nx && gz >= 0 && gz < sh.nz) {
-            const long L = 2L * sh.nx + 2L * sh.nz, b = (long)st.it * L;
-            if (gz == 0) { sh.edge_p[b + gx] = Pn[0]; sh.edge_q[b + gx] = Qn[0]; }
-            if (gz == sh.nz - 1) { sh.edge_p[b + sh.nx + gx] = Pn[0]; sh.edge_q[b + sh.nx + gx] = Qn[0]; }
-            if (gx == 0) { sh.edge_p[b + 2 * sh.nx + gz] = Pn[0]; sh.edge_q[b + 2 * sh.nx + gz] = Qn[0]; }
-            if (gx == sh.nx - 1) { sh.edge_p[b + 2 * sh.nx + sh.nz + gz] = Pn[0]; sh.edge_q[b + 2 * sh.nx + sh.nz + gz] = Qn[0]; }
-        }
-    } else if (st.nf == 2 && gx >= 0 && gx < sh.nx && gz >= 0 && gz < sh.nz) {
-        // zero-lag cross-correlation image and source illumination
-        // (Toa_rtm_vti_adcig_cdp.c:1067-1076): the illumination sum is
-        // formed in double, as pow() returns it, and a zero becomes 1
-        const long o = (long)gx * sh.nz + gz;
-        const float sv = Pn[0];
-        float ill;
-        if (FAST) ill = sh.ill[o] + sv * sv;
-        else {
-            const double svd = f2d_exact(sv);
-            ill = d2f_rn(f2d_exact(sh.ill[o]) + svd * svd);
-        }
-        if (ill == 0.0f) ill = 1.0f;
-        sh.ill[o] = ill;
-        sh.mig[o] = sh.mig[o] + Pn[1] * sv;
-        if (sh.adcig) {
-            // Poynting vectors from the new P,Q and u,w of both fields
-            const float sx = -Pn[0] * sh.u[0][id], sz = -Qn[0] * sh.w[0][id];
-            const float gx = Pn[1] * sh.u[1][id], gz = Qn[1] * sh.w[1][id];
-            const float b1 = sx * sx + sz * sz, b2 = gx * gx + gz * gz, a = sx * gx + sz * gz;
-            const float a1 = (float)((double)a / ((double)sqrtf(b1 * b2) + 0.0000000000001));
-            const int ia = adcig_bin(a1);
-            float *ag = sh.adcig + (long)ia * sh.nx * sh.nz + o;
-            *ag = d2f_rn(f2d_exact(*ag) + f2d_exact(Pn[1] * sv) * c_adw[ia]);
-        }
+    float px = sh.px[id], pz = sh.pz[id], qx = sh.qx[id], qz = sh.qz[id];
+    if (VARIANT == V_MPI) {
+        px = ax2 * px - ax1 * vp * e2 * sh.dtx * xx;
+        // the conversions on the integer pipe (softcvt.cuh): same bits
+        pz = d2f_rn(f2d_exact(az2 * pz) - kz * f2d_exact(zz));
+        qx = d2f_rn(f2d_exact(ax2 * qx) - kx * f2d_exact(xx));
+        qz = az2 * qz - az1 * vp * sh.dtz * zz;
+    } else {
+        px = ax2 * px - ax1 * vp * vp * e2 * sh.dtx * xx;
+        pz = az2 * pz - az1 * vp * vp * d2 * sh.dtz * zz;
+        qx = ax2 * qx - ax1 * vp * vp * d2 * sh.dtx * xx;
+        qz = az2 * qz - az1 * vp * vp * sh.dtz * zz;
     }
+    sh.px[id] = px; sh.pz[id] = pz; sh.qx[id] = qx; sh.qz[id] = qz;
+    float P = px + pz, Q = qx + qz;
+    if (VARIANT == V_CPU || VARIANT == V_MPI) {
+        // Gaussian source window, added after the split sum
+        float s = 0.0f;
+        if (st.src_on) {
+            const int rx = ix - sh.ixs, rz = iz - sh.izs;
+            if (rx >= -3 && rx <= 3 && rz >= -3 && rz <= 3)
+                s = (float)((double)st.amp * c_gauss[(rx + 3) * 7 + (rz + 3)]);
+        }
+        P = P + s;
+        Q = Q + s;
+    }
+    sh.P[id] = P;
+    sh.Q[id] = Q;
+    // receiver gather at rec_iz, time-major
+    const int gx = ix - sh.npd;
+    if (iz == sh.rec_iz && gx >= 0 && gx < sh.nx)
+        sh.rec_p[(long)st.it * sh.nx + gx] = sh.rec_scale == 2.0f ? P + P : P * sh.rec_scale;
 }
 
-template <int VARIANT, int PHASE, bool FAST = false>
+template <int VARIANT>
 __global__ void __launch_bounds__(256) k_stress2d(const Shot2D *__restrict__ shots, const int *__restrict__ item_shot,
                                                   int nitems, Step2D st) {
     for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
         Tile2D t;
         if (!locate(shots, item_shot, item, t)) continue;
-        stress_point<VARIANT, PHASE, true, FAST>(*t.sh, t.ix, t.iz, st);
+        stress_point<VARIANT, true>(*t.sh, t.ix, t.iz, st);
     }
 }
 
 // ------------------------------------------------------ persistent shot
 // A whole single-shot forward run in one cooperative launch: per step the
 // velocity half-step over every tile, a grid barrier, the stress half-step
-// (records, edge lines), a grid barrier.  Same per-point arithmetic as the
+// with the record, a grid barrier.  Same per-point arithmetic as the
 // per-half-step kernels; neighbours' values are read through L2.
 template <int VARIANT>
 __global__ void __launch_bounds__(512) k_fd2d_shot(const Shot2D *__restrict__ shots,
@@ -290,8 +209,6 @@ __global__ void __launch_bounds__(512) k_fd2d_shot(const Shot2D *__restrict__ sh
         st.amp = a.amp[it];
         st.src_on = a.on[it];
         st.taper = a.taper;
-        st.nf = 1;
-        st.fast = 0;  // the single-shot forms have no double chains
         for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
             Tile2D t;
             if (locate(shots, item_shot, item, t)) vel_point<VARIANT, false>(*t.sh, t.ix, t.iz, st);
@@ -299,7 +216,7 @@ __global__ void __launch_bounds__(512) k_fd2d_shot(const Shot2D *__restrict__ sh
         if (!grid_barrier(a.bar, ++k * gridDim.x, a.err)) return;
         for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
             Tile2D t;
-            if (locate(shots, item_shot, item, t)) stress_point<VARIANT, PH_FWD, false>(*t.sh, t.ix, t.iz, st);
+            if (locate(shots, item_shot, item, t)) stress_point<VARIANT, false>(*t.sh, t.ix, t.iz, st);
         }
         if (!grid_barrier(a.bar, ++k * gridDim.x, a.err)) return;
     }
@@ -381,14 +298,14 @@ __global__ void __launch_bounds__(512) k_fd2d_tile(const TileShot2D a) {
             const int ix = x0 + cx, iz = z0 + lz, o = cx * TZ + lz;
             const bool in = ix < nnx && iz < nnz;
             const long id = (long)ix * nnz + iz;
-            ph(cx, lz) = in ? sh.P[0][id] : 0.0f;
-            qh(cx, lz) = in ? sh.Q[0][id] : 0.0f;
-            uh(cx, lz) = in ? sh.u[0][id] : 0.0f;
-            wh(cx, lz) = in ? sh.w[0][id] : 0.0f;
-            PX[o] = in ? sh.px[0][id] : 0.0f;
-            PZ[o] = in ? sh.pz[0][id] : 0.0f;
-            QX[o] = in ? sh.qx[0][id] : 0.0f;
-            QZ[o] = in ? sh.qz[0][id] : 0.0f;
+            ph(cx, lz) = in ? sh.P[id] : 0.0f;
+            qh(cx, lz) = in ? sh.Q[id] : 0.0f;
+            uh(cx, lz) = in ? sh.u[id] : 0.0f;
+            wh(cx, lz) = in ? sh.w[id] : 0.0f;
+            PX[o] = in ? sh.px[id] : 0.0f;
+            PZ[o] = in ? sh.pz[id] : 0.0f;
+            QX[o] = in ? sh.qx[id] : 0.0f;
+            QZ[o] = in ? sh.qz[id] : 0.0f;
             float e2 = in ? sh.e2[id] : 0.0f, d2 = in ? sh.d2[id] : 0.0f;
             if (a.taper) {
                 const int bx = ix - sh.tx0, bz = iz - sh.tz0;
@@ -519,14 +436,14 @@ __global__ void __launch_bounds__(512) k_fd2d_tile(const TileShot2D a) {
             const int ix = x0 + cx, iz = z0 + lz, o = cx * TZ + lz;
             if (ix >= nnx || iz >= nnz) continue;
             const long id = (long)ix * nnz + iz;
-            sh.P[0][id] = ph(cx, lz);
-            sh.Q[0][id] = qh(cx, lz);
-            sh.u[0][id] = uh(cx, lz);
-            sh.w[0][id] = wh(cx, lz);
-            sh.px[0][id] = PX[o];
-            sh.pz[0][id] = PZ[o];
-            sh.qx[0][id] = QX[o];
-            sh.qz[0][id] = QZ[o];
+            sh.P[id] = ph(cx, lz);
+            sh.Q[id] = qh(cx, lz);
+            sh.u[id] = uh(cx, lz);
+            sh.w[id] = wh(cx, lz);
+            sh.px[id] = PX[o];
+            sh.pz[id] = PZ[o];
+            sh.qx[id] = QX[o];
+            sh.qz[id] = QZ[o];
         }
 }
 
@@ -617,60 +534,10 @@ int launch_fd2d_tile(int variant, const Shot2D &sh, float *xch, const float *amp
     return check_launch("fd2d_tile");
 }
 
-// Boundary-driven reconstruction and receiver injection before step it of
-// the backward pass (Toa_rtm_vti_adcig_cdp.c:914-927 and 953-957): the saved
-// interior-edge lines go into the source-side P,Q (corners end with the
-// left/right values, as the reference's loop order leaves them) and the
-// muted surface records into the receiver-side P,Q at the surface row.
-__global__ void k_inject2d(const Shot2D *__restrict__ shots, int maxline, int it) {
-    const Shot2D &sh = shots[blockIdx.y];
-    const int nx = sh.nx, nz = sh.nz, npd = sh.npd, nnz = sh.nnz;
-    const long L = 2L * nx + 2L * nz;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < L; k += gridDim.x * blockDim.x) {
-        int ix, iz;
-        if (k < nx) { ix = npd + k; iz = npd; if (k == 0 || k == nx - 1) goto rec; }
-        else if (k < 2 * nx) { ix = npd + k - nx; iz = npd + nz - 1; if (k - nx == 0 || k - nx == nx - 1) goto rec; }
-        else if (k < 2 * nx + nz) { ix = npd; iz = npd + k - 2 * nx; }
-        else { ix = npd + nx - 1; iz = npd + k - 2 * nx - nz; }
-        {
-            const long id = (long)ix * nnz + iz;
-            sh.P[0][id] = sh.edge_p[(long)it * L + k];
-            sh.Q[0][id] = sh.edge_q[(long)it * L + k];
-        }
-    rec:
-        if (k < nx) {
-            const long id = (long)(npd + k) * nnz + npd;
-            sh.P[1][id] = sh.rec_p[(long)it * nx + k];
-            sh.Q[1][id] = sh.rec_q[(long)it * nx + k];
-        }
-    }
-    (void)maxline;
-}
-
 template <int V>
 static void vel_dispatch(const Shot2D *d_shots, const int *d_item_shot, int nitems, dim3 grid, dim3 block,
                          Step2D st, cudaStream_t s) {
     k_vel2d<V><<<grid, block, 0, s>>>(d_shots, d_item_shot, nitems, st);
-}
-
-// Wavefield watchdog over a batch: block row y scans shot y's P of sides
-// 0..nf-1 and sets *flag to tag (first writer wins) on a NaN or +-Inf.
-__global__ void k_watch_shots(const Shot2D *__restrict__ S, int nf, int *flag, int tag) {
-    const Shot2D &sh = S[blockIdx.y];
-    const size_t n = (size_t)sh.nnx * sh.nnz;
-    bool bad = false;
-    for (int f = 0; f < nf; f++) {
-        const float *P = sh.P[f];
-        for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
-            bad |= !(fabsf(P[k]) <= FLT_MAX);
-    }
-    if (__syncthreads_or(bad) && threadIdx.x == 0) atomicCAS(flag, 0, tag);
-}
-
-int launch_watch_shots(const Shot2D *d_shots, int ns, int nf, int *flag, int tag, cudaStream_t s) {
-    if (!flag || ns < 1) return GEO_OK;
-    k_watch_shots<<<dim3(64, ns), 256, 0, s>>>(d_shots, nf, flag, tag);
-    return check_launch("watch_shots");
 }
 
 int launch_vel2d(int variant, const Shot2D *d_shots, const int *d_item_shot, int nitems, int by, int grid,
@@ -684,119 +551,16 @@ int launch_vel2d(int variant, const Shot2D *d_shots, const int *d_item_shot, int
     return check_launch("vel2d");
 }
 
-int launch_stress2d(int variant, int phase, const Shot2D *d_shots, const int *d_item_shot, int nitems, int by,
-                    int grid, Step2D st, cudaStream_t s) {
+int launch_stress2d(int variant, const Shot2D *d_shots, const int *d_item_shot, int nitems, int by, int grid,
+                    Step2D st, cudaStream_t s) {
     GEO_TRY(ensure_gauss());
     dim3 block(32, by), g(grid);
-#define GEO_STRESS(V, PH) k_stress2d<V, PH><<<g, block, 0, s>>>(d_shots, d_item_shot, nitems, st)
-#define GEO_STRESS_MPI(PH) \
-    (st.fast ? k_stress2d<V_MPI, PH, true><<<g, block, 0, s>>>(d_shots, d_item_shot, nitems, st) \
-             : k_stress2d<V_MPI, PH, false><<<g, block, 0, s>>>(d_shots, d_item_shot, nitems, st))
-    if (phase == PH_FWD) {
-        switch (variant) {
-            case V_CPU: GEO_STRESS(V_CPU, PH_FWD); break;
-            case V_GPU: GEO_STRESS(V_GPU, PH_FWD); break;
-            default: GEO_STRESS_MPI(PH_FWD); break;
-        }
-    } else {
-        switch (variant) {
-            case V_CPU: GEO_STRESS(V_CPU, PH_BWD); break;
-            case V_GPU: GEO_STRESS(V_GPU, PH_BWD); break;
-            default: GEO_STRESS_MPI(PH_BWD); break;
-        }
+    switch (variant) {
+        case V_CPU: k_stress2d<V_CPU><<<g, block, 0, s>>>(d_shots, d_item_shot, nitems, st); break;
+        case V_GPU: k_stress2d<V_GPU><<<g, block, 0, s>>>(d_shots, d_item_shot, nitems, st); break;
+        default: k_stress2d<V_MPI><<<g, block, 0, s>>>(d_shots, d_item_shot, nitems, st); break;
     }
-#undef GEO_STRESS_MPI
-#undef GEO_STRESS
     return check_launch("stress2d");
-}
-
-int launch_inject2d(const Shot2D *d_shots, int nshots, int maxline, int it, cudaStream_t s) {
-    dim3 g((maxline + 255) / 256, nshots);
-    k_inject2d<<<g, 256, 0, s>>>(d_shots, maxline, it);
-    return check_launch("inject2d");
-}
-
-// One launch that runs velocity tiles of some shots and stress tiles of
-// others (the MPI form of the batched RTM).  Each item is (shot | kind << 30,
-// tile): kind 0 a velocity tile at step st_v, kind 1 a stress tile at st_s.
-// The caller keeps the two kinds on disjoint shots, so the read-only path
-// stays valid for both.  The exact form's stress tiles are bound by the FP64
-// pipe and the velocity tiles by memory, so a launch that holds both keeps
-// both busy on every SM.
-template <int PHASE, bool FAST>
-__global__ void __launch_bounds__(256) k_mix2d(const Shot2D *__restrict__ shots, const int2 *__restrict__ items,
-                                               int nitems, Step2D st_v, Step2D st_s) {
-    for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
-        const int2 e = items[item];
-        const int kind = e.x >> 30;
-        const Shot2D &sh = shots[e.x & ((1 << 30) - 1)];
-        const int tz = e.y % sh.ntz, tx = e.y / sh.ntz;
-        const int iz = tz * 32 + threadIdx.x, ix = tx * blockDim.y + threadIdx.y;
-        if (ix < 4 || ix >= sh.nnx - 4 || iz < 4 || iz >= sh.nnz - 4) continue;
-        if (kind == 0) vel_point<V_MPI, true>(sh, ix, iz, st_v);
-        else stress_point<V_MPI, PHASE, true, FAST>(sh, ix, iz, st_s);
-    }
-}
-
-int launch_mix2d(int phase, int fast, const Shot2D *d_shots, const int2 *d_items, int nitems, int by, int grid,
-                 Step2D st_v, Step2D st_s, cudaStream_t s) {
-    if (nitems < 1) return GEO_OK;
-    GEO_TRY(ensure_gauss());
-    dim3 block(32, by), g(grid < nitems ? grid : nitems);
-    if (phase == PH_FWD) {
-        if (fast) k_mix2d<PH_FWD, true><<<g, block, 0, s>>>(d_shots, d_items, nitems, st_v, st_s);
-        else k_mix2d<PH_FWD, false><<<g, block, 0, s>>>(d_shots, d_items, nitems, st_v, st_s);
-    } else {
-        if (fast) k_mix2d<PH_BWD, true><<<g, block, 0, s>>>(d_shots, d_items, nitems, st_v, st_s);
-        else k_mix2d<PH_BWD, false><<<g, block, 0, s>>>(d_shots, d_items, nitems, st_v, st_s);
-    }
-    return check_launch("mix2d");
-}
-
-// The MPI program's bin of one cosine a1 (before its 90 -> 89 clamp).
-static int ref_adcig_bin(float a1) {
-    const float a2 = (float)(0.5 * std::acos(a1) * 180 / kPiMpi);
-    return (int)(a2 / 1.0);
-}
-
-static uint32_t order_key(float f) {
-    uint32_t b;
-    memcpy(&b, &f, 4);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-
-static float key_float(uint32_t k) {
-    const uint32_t b = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
-    float f;
-    memcpy(&f, &b, 4);
-    return f;
-}
-
-int load_adcig_tables(cudaStream_t s) {
-    static float thr[kAdcigAngles];
-    static double w[kAdcigAngles];
-    static bool built = false;
-    if (!built) {
-        const uint32_t lo = order_key(-1.0f), hi = order_key(1.0f);
-        for (int k = 1; k <= kAdcigAngles; k++) {
-            if (ref_adcig_bin(-1.0f) < k) {
-                thr[k - 1] = -2.0f;   // no cosine reaches this bin
-                continue;
-            }
-            uint32_t a = lo, b = hi;  // ref_adcig_bin(key_float(a)) >= k
-            while (a < b) {
-                const uint32_t m = a + (b - a + 1) / 2;
-                if (ref_adcig_bin(key_float(m)) >= k) a = m;
-                else b = m - 1;
-            }
-            thr[k - 1] = key_float(a);
-        }
-        for (int ia = 0; ia < kAdcigAngles; ia++) w[ia] = std::pow(std::cos(ia * kPiMpi / 180.0), 3);
-        built = true;
-    }
-    GEO_CUDA(cudaMemcpyToSymbolAsync(c_adthr, thr, sizeof thr, 0, cudaMemcpyHostToDevice, s));
-    GEO_CUDA(cudaMemcpyToSymbolAsync(c_adw, w, sizeof w, 0, cudaMemcpyHostToDevice, s));
-    return GEO_OK;
 }
 
 }  // namespace geo

@@ -132,7 +132,7 @@ int write_at(FILE *fp, size_t offset_bytes, const float *a, size_t n);
 // ------------------------------------------------------------ 2D device side
 constexpr int kTB = 31;  // taper box edge (circle radius 15)
 
-// Per-shot descriptor read by the batched 2D kernels (device memory).
+// A single shot's descriptor (device memory).
 struct Shot2D {
     int nnx, nnz, npd, nx, nz;
     float dtx, dtz;
@@ -146,13 +146,10 @@ struct Shot2D {
     const float *te2, *td2;
     const double *tkz, *tkx;
     int ixs, izs;                   // source cell (padded)
-    float *u[2], *w[2], *P[2], *Q[2], *px[2], *pz[2], *qx[2], *qz[2];
+    float *u, *w, *P, *Q, *px, *pz, *qx, *qz;
     int rec_iz;                     // receiver row
     float rec_scale;
-    float *rec_p, *rec_q;           // time-major records nt x nx
-    float *edge_p, *edge_q;         // time-major edge lines nt x (2nx+2nz)
-    float *mig, *ill;               // image and source illumination nx*nz
-    float *adcig;                   // Poynting angle gathers [90][nx][nz], or null
+    float *rec_p;                   // time-major record nt x nx
     int tile_base, ntz;             // first work item, tiles along z
 };
 
@@ -161,11 +158,7 @@ struct Step2D {
     float amp;        // pfac*w(t) this step (0 when off)
     int src_on;       // source active this step
     int taper;        // use the taper box for eps/del
-    int nf;           // fields updated (1: s only, 2: s and g)
-    int fast;         // MPI form: double-precision chains in FP32
 };
-
-enum Phase2D { PH_FWD = 0, PH_BWD = 1 };
 
 // A whole single-shot forward run in one cooperative launch (launch_fd2d_shot).
 struct Persist2D {
@@ -186,25 +179,16 @@ int launch_fd2d_tile(int variant, const Shot2D &sh, float *xch, const float *amp
 
 int launch_vel2d(int variant, const Shot2D *d_shots, const int *d_item_shot, int nitems, int by,
                  int grid, Step2D st, cudaStream_t s);
-int launch_stress2d(int variant, int phase, const Shot2D *d_shots, const int *d_item_shot, int nitems,
-                    int by, int grid, Step2D st, cudaStream_t s);
-int launch_inject2d(const Shot2D *d_shots, int nshots, int maxline, int it, cudaStream_t s);
-// Velocity tiles (kind 0, step st_v) and stress tiles (kind 1, step st_s)
-// of disjoint shots in one launch, MPI form (fd2d.cu, k_mix2d).
-int launch_mix2d(int phase, int fast, const Shot2D *d_shots, const int2 *d_items, int nitems, int by, int grid,
-                 Step2D st_v, Step2D st_s, cudaStream_t s);
+int launch_stress2d(int variant, const Shot2D *d_shots, const int *d_item_shot, int nitems, int by, int grid,
+                    Step2D st, cudaStream_t s);
 int launch_mute_records(float *rec, int nx, int nt, const int *lo, const int *hi, cudaStream_t s);
 // cos and sin of n tilt angles in radians on the device, as the 2D TTI
 // programs form them (in place: th_cos holds the angles, then the cosines).
 int launch_tilt_trig(float *th_cos, float *sn, size_t n, cudaStream_t s);
-// Watchdog scan of the P fields (sides 0..nf-1) of ns shots (fd2d.cu).
-int launch_watch_shots(const Shot2D *d_shots, int ns, int nf, int *flag, int tag, cudaStream_t s);
 int launch_transpose_records(const float *tm, float *out, int ntr, int nt, cudaStream_t s);
 int launch_normalize_image(float *mig, const float *ill, size_t n, cudaStream_t s);
 // a[p*n + k] /= ill[k] for p < planes.
 int launch_normalize_planes(float *a, const float *ill, size_t n, int planes, cudaStream_t s);
-// Angle-bin thresholds and cos^3 weights of the Poynting ADCIG into constant memory.
-int load_adcig_tables(cudaStream_t s);
 constexpr int kAdcigAngles = 90;
 int launch_stack_image(float *full, int nz, const float *const *imgs, const int *offsets,
                        const int *widths, int nshots, int nx, cudaStream_t s);

@@ -87,6 +87,13 @@ __global__ void __launch_bounds__(256) k_model2d(const RawView r, const __grid_c
             j.e2[o] = 1 + 2 * r.a[1][src];
             if (j.d2) j.d2[o] = sqrtf(1 + 2 * r.a[2][src]);
             if (j.rad) j.rad[o] = (float)((double)r.a[3][src] * (kPiGui / 180.0));
+            if (j.pwd) {
+                const double pw = j.pw[src];
+                const float h = (float)pw;
+                j.pwd[o] = pw;
+                j.ph[o] = h;
+                j.pl[o] = (float)(pw - (double)h);
+            }
             if (j.kz) {
                 const double pw = j.pw[src];
                 j.kz[o] = (double)(j.az1[iz] * vp) * pw * j.ddtz;
@@ -186,7 +193,7 @@ int launch_model2d(const Raw2D &r, const std::vector<ModelJob> &jobs, cudaStream
     return GEO_OK;
 }
 
-void host_pow_half(const float *del, size_t n, double *out) {
+static void host_pow_half(const float *del, size_t n, double *out) {
     auto part = [&](size_t a, size_t b) {
         for (size_t k = a; k < b; k++) out[k] = std::pow((double)(1 + 2 * del[k]), 0.5);
     };
@@ -204,6 +211,19 @@ void host_pow_half(const float *del, size_t n, double *out) {
     }
     part(done, n);
     for (std::thread &t : th) t.join();
+}
+
+int upload_pow_half(const Raw2D &r, DevBuf &out, cudaStream_t s) {
+    const size_t n = (size_t)r.nx * r.nz;
+    std::vector<float> hd(n);
+    std::vector<double> pw(n);
+    GEO_CUDA(cudaMemcpyAsync(hd.data(), r.a[2], n * 4, cudaMemcpyDeviceToHost, s));
+    GEO_CUDA(cudaStreamSynchronize(s));
+    host_pow_half(hd.data(), n, pw.data());
+    GEO_TRY(out.alloc(n * 8));
+    GEO_CUDA(cudaMemcpyAsync(out.p, pw.data(), n * 8, cudaMemcpyHostToDevice, s));
+    GEO_CUDA(cudaStreamSynchronize(s));   // pw is freed on return
+    return GEO_OK;
 }
 
 int launch_box2d(float *e2, float *d2, int nnx, int nnz, int x0, int z0, int nb, const float *te2, const float *td2,

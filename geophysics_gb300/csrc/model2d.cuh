@@ -88,11 +88,15 @@ struct ModelJob {
     const double *pw;
     const float *ax1, *az1;
     double ddtx, ddtz;
+    // pw on the padded grid and its split into two floats
+    double *pwd;
+    float *ph, *pl;
 };
 int launch_model2d(const Raw2D &r, const std::vector<ModelJob> &jobs, cudaStream_t s);
 
-// pow(1 + 2 del, 0.5) of n values with the host's pow, over host threads.
-void host_pow_half(const float *del, size_t n, double *out);
+// pow(1 + 2 del, 0.5) of every model point with the host's pow (over host
+// threads), on the device.
+int upload_pow_half(const Raw2D &r, DevBuf &out, cudaStream_t s);
 
 // e2, d2 on the box (x0.., z0..) of edge nb from te2, td2 (nb*nb), clipped
 // to the nnx x nnz grid.

@@ -277,10 +277,10 @@ extern "C" int geo_fd2d_shot_noalloc(const geo_fd2d_desc *desc, const float *v, 
     H.vp = vp; H.e2 = e2; H.d2 = d2; H.kz = nullptr; H.kx = nullptr;
     H.tx0 = tx0; H.tz0 = tz0; H.te2 = taper; H.td2 = taper + kTB * kTB; H.tkz = nullptr; H.tkx = nullptr;
     H.ixs = ixs; H.izs = izs;
-    H.u[0] = fields; H.w[0] = fields + n; H.P[0] = fields + 2 * n; H.Q[0] = fields + 3 * n;
-    H.px[0] = fields + 4 * n; H.pz[0] = fields + 5 * n; H.qx[0] = fields + 6 * n; H.qz[0] = fields + 7 * n;
+    H.u = fields; H.w = fields + n; H.P = fields + 2 * n; H.Q = fields + 3 * n;
+    H.px = fields + 4 * n; H.pz = fields + 5 * n; H.qx = fields + 6 * n; H.qz = fields + 7 * n;
     H.rec_iz = D.rec_iz; H.rec_scale = D.rec_scale;
-    H.rec_p = rec; H.rec_q = nullptr;
+    H.rec_p = rec;
     H.tile_base = 0; H.ntz = (nnz + 31) / 32;
     // from pageable memory: the copy has taken H before it returns
     GEO_CUDA(cudaMemcpyAsync(dshot, &H, sizeof(Shot2D), cudaMemcpyHostToDevice, s));
@@ -291,9 +291,9 @@ extern "C" int geo_fd2d_shot_noalloc(const geo_fd2d_desc *desc, const float *v, 
     const int grid = ntiles < sms * 8 ? ntiles : sms * 8;
     for (int it = 0; it < D.nt; it++) {
         Step2D st{};
-        st.it = it; st.amp = h_amp[it]; st.src_on = h_on[it]; st.taper = D.sv ? 1 : 0; st.nf = 1;
+        st.it = it; st.amp = h_amp[it]; st.src_on = h_on[it]; st.taper = D.sv ? 1 : 0;
         GEO_TRY(launch_vel2d(var, dshot, items, ntiles, by, grid, st, s));
-        GEO_TRY(launch_stress2d(var, PH_FWD, dshot, items, ntiles, by, grid, st, s));
+        GEO_TRY(launch_stress2d(var, dshot, items, ntiles, by, grid, st, s));
     }
     if (D.mute_tt > 0) {
         // GPU-form direct-wave mute (GPU_vti2dfd_kernels.cu:151-174)

@@ -256,8 +256,8 @@ int geo_rtm3d_adcig(const geo_rtm3d_desc *desc, const float *v, const float *e, 
 /* 2D RTM with the MPI CPU program's semantics on per-shot aperture windows
  * (2D-vti-fd+rtm-mpi/Toa_rtm_vti_adcig_cdp.c:295-392 with
  * model_vti_get_boundry :483 and RTM_corr_adcig :739).  All shots run
- * together: each time step is one persistent launch over every shot's
- * tiles, and the time loop is replayed from a CUDA graph.  The stacked image
+ * together: each time step is one launch over every shot, and the time
+ * loop is replayed from a CUDA graph.  The stacked image
  * is formed in shot order and optionally passed through the adjoint
  * Laplacian (laplac2_lop adj=1). */
 typedef struct geo_rtm2d_desc {
@@ -269,7 +269,7 @@ typedef struct geo_rtm2d_desc {
     const int *shot_x;       /* ns source x positions k (1-based), host      */
     const int *shot_nxs;     /* ns odd window widths, host                   */
     int   laplace;           /* apply the adjoint Laplacian to the stack     */
-    int   tile_z, tile_x;    /* 0 = autotuned                                */
+    int   tile_z, tile_x;    /* accepted; the fused step chooses its own work */
     int   mode;              /* GEO_MODE_EXACT (0): the program's arithmetic,
                                 bit for bit, with its double-precision chains;
                                 GEO_MODE_FAST: those chains in FP32 (pz, qx

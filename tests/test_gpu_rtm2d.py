@@ -36,6 +36,23 @@ def test_rtm2d_batch_bit_exact(geo, orc, tile_x):
     assert np.array_equal(raw, acc)
 
 
+# the fused step's strips (120 depths, the last of the grid short, a pitch
+# beyond nnz) and chunks (windows of 3 columns, of one and of several chunks)
+@pytest.mark.parametrize("nz,npd,widths", [(107, 10, [3, 17]), (108, 10, [41]), (109, 10, [5, 9, 61]),
+                                           (113, 10, [31, 33]), (229, 9, [25, 101]), (31, 7, [3])])
+def test_rtm2d_batch_strip_and_chunk_edges(geo, orc, nz, npd, widths):
+    v, e, d = model(103, nz)
+    xs = [52 + 3 * k if w < 90 else 52 for k, w in enumerate(widths)]
+    kw = dict(npd=npd, nt=420, dx=10.0, dz=10.0, dt_ms=1.0, favg=25.0, pfac=1000.0)
+    img, per = geo.rtm2d_batch(v, e, d, zs=2, shot_x=xs, shot_nxs=widths, per_shot=True, laplace=False, **kw)
+    acc = np.zeros(v.shape, np.float32)
+    for k, (x, w) in enumerate(zip(xs, widths)):
+        mo, off, _ = orc.rtm2d_mpi_shot(v, e, d, fs_sxd=x, ds_sxd=0, zs_sxd=2, is_=k + 1, nxs=w, **kw)
+        assert np.array_equal(per[k], mo), (nz, w)
+        orc.stack2d(acc, mo, off)
+    assert np.abs(acc).max() > 0 and np.array_equal(img, acc)
+
+
 def test_rtm2d_batch_fast_mode_within_rounding(geo, orc):
     """The fast mode forms the program's double-precision chains in FP32.
     Both modes are FP32 roundings of one computation whose image is a small
