@@ -239,7 +239,7 @@ static Fused3D make_fused(const geo_fd3d_plan *p, int f) {
     r.cy1 = g.cy1; r.cy2 = g.cy2; r.ay1 = g.ay1; r.ay2 = g.ay2;
     r.cz1 = g.cz1; r.cz2 = g.cz2; r.az1 = g.az1; r.az2 = g.az2;
     r.m0 = g.vp; r.m1 = g.e2; r.m2 = g.d2;
-    r.P0 = g.P; r.Q0 = g.Q;
+    r.P0 = g.P; r.Q0 = g.Q; r.v0 = g.v;
     const int n = 1 - F.cur;
     r.u1 = F.lev[n][0].as<float>(); r.v1 = F.lev[n][1].as<float>(); r.w1 = F.lev[n][2].as<float>();
     r.P1 = F.lev[n][3].as<float>(); r.Q1 = F.lev[n][4].as<float>();
@@ -259,24 +259,22 @@ static int alloc_fields(geo_fd3d_plan *p, int f) {
     for (int c = 0; c < 2; c++) {
         StepMaps &M = F.maps[c];
         const int nz = p->nnz, ld = p->ldz, nx = p->nnx, ny = p->nny;
-        GEO_TRY(encode_map(&M.m[0], F.lev[c][3].as<float>(), nz, ld, nx, ny, kTZ, kTXF + 14));  // P halo
-        GEO_TRY(encode_map(&M.m[1], F.lev[c][3].as<float>(), nz, ld, nx, ny, kTZ, kTXF));       // P own
-        GEO_TRY(encode_map(&M.m[2], F.lev[c][4].as<float>(), nz, ld, nx, ny, 48, kTXF));        // Q
-        GEO_TRY(encode_map(&M.m[3], F.lev[c][0].as<float>(), nz, ld, nx, ny, kTZ, kTXF + 8));   // u
-        GEO_TRY(encode_map(&M.m[4], F.lev[c][2].as<float>(), nz, ld, nx, ny, 48, kTXF));        // w
-        GEO_TRY(encode_map(&M.m[5], F.lev[c][1].as<float>(), nz, ld, nx, ny, kTZ, kTXF));       // v
-        const DevBuf *own[9] = {&p->vp, &p->e2, &p->d2, &F.px, &F.py, &F.pz, &F.qx, &F.qy, &F.qz};
-        for (int r = 0; r < 9; r++) GEO_TRY(encode_map(&M.m[6 + r], own[r]->as<float>(), nz, ld, nx, ny, kTZ, kTXF));
+        GEO_TRY(encode_map(&M.m[0], F.lev[c][3].as<float>(), nz, ld, nx, ny, kTZ, kFX + 14));  // P halo
+        GEO_TRY(encode_map(&M.m[1], F.lev[c][4].as<float>(), nz, ld, nx, ny, 48, kFX));        // Q
+        GEO_TRY(encode_map(&M.m[2], F.lev[c][0].as<float>(), nz, ld, nx, ny, kTZ, kFX + 8));   // u
+        GEO_TRY(encode_map(&M.m[3], F.lev[c][2].as<float>(), nz, ld, nx, ny, 48, kFX));        // w
+        const DevBuf *model[3] = {&p->vp, &p->e2, &p->d2};
+        for (int r = 0; r < 3; r++) GEO_TRY(encode_map(&M.m[4 + r], model[r]->as<float>(), nz, ld, nx, ny, kTZ, kFX));
     }
     return GEO_OK;
 }
 
-// y chunking: a block marches over one chunk of y planes and recomputes 14
-// warm-up planes of its queues, so more chunks mean more blocks in flight at
-// different depths (better DRAM and L2 spread, shorter tails) at the price of
-// the warm-up.  The best count varies with the grid (measured on GB300: 4
-// for 480^3, 6 for 592x592x464, 8 for 272^3), so set_model times the
-// candidates (autotune_chunks); this is the starting guess.
+// y chunking: a block marches over one chunk of y planes after filling its
+// queues (14 planes of P, 7 of v), so more chunks mean more blocks in flight
+// and shorter tails at the price of the fill.  The best count varies with
+// the grid (measured on GB300: 8-12 for 480^3, 6-12 for 216x200x184, 12-16
+// for 161x133x147), so set_model times the candidates (autotune_chunks);
+// this is the starting guess.
 static void set_chunks(geo_fd3d_plan *p, int c) {
     const int planes = p->nny - 8, ntiles = p->ntz * p->ntx;
     c = std::max(1, std::min(c, planes / 8));
@@ -351,8 +349,8 @@ static int autotune_chunks(geo_fd3d_plan *p, cudaStream_t s) {
     float best = 1e30f;
     int best_c = 4;
     const int planes = p->nny - 8;
-    for (int c : {2, 3, 4, 5, 6, 8, 10}) {
-        if (planes / c < 16) break;
+    for (int c : {2, 4, 6, 8, 10, 12, 16}) {
+        if (planes / c < 8) break;
         set_chunks(p, c);
         int rc = step3d(p, 0, st, s);
         if (rc == GEO_OK && cudaEventRecord(a, s) != cudaSuccess) rc = fail(GEO_ERR_CUDA, "event record");
@@ -534,7 +532,7 @@ int plan3d_create(geo_fd3d_plan **out, const geo_fd3d_desc *desc, int nfs) {
         return fail(GEO_ERR_ARG, "grid of %zu points per field exceeds 2^31", (size_t)d.nx * d.ny * d.nz);
     }
     p->ntz = (p->nnz + kTZ - 1) / kTZ;
-    p->ntx = (p->nnx + kTXF - 1) / kTXF;
+    p->ntx = (p->nnx + kFX - 1) / kFX;
     const size_t n = p->nalloc, ntr = (size_t)d.nrx * d.nry;
     int st = GEO_OK;
     DevBuf *model[3] = {&p->vp, &p->e2, &p->d2};

@@ -29,6 +29,7 @@ struct StepArgs3D {
     float *ill;                 // interior illumination += P^2+Q^2 (or null)
     float *mig;                 // interior image += other_P * P (or null)
     const float *other_P;       // the source-side field's P (same layout)
+    bool img_vec;               // ill and mig take 16-byte accesses (set by the launch)
 };
 
 // One 3D TTI step (tti3d.cu): g describes the grid, its profiles and the

@@ -6,20 +6,35 @@
 // updates the stresses, so u,v,w never make a round trip through HBM between
 // the two half-steps of the reference (GPU_vti3dfd_kernels.cu:90-201).
 //
-// Each thread owns two adjacent x columns at one depth (lane = z), so the
-// x taps of the two columns share shared-memory loads and the per-plane
-// bookkeeping is paid once per two points.
+// Each of the 256 threads owns two consecutive depths of one x column and
+// moves them as one 8-byte vector: a tap along x is one shared-memory load
+// for two points, the eight taps along z are five, and addresses, predicates
+// and loop bookkeeping are paid once per two points.  The y taps come from
+// two register queues (P of planes y .. y+7, the new v of planes y-4 .. y+3).
 //
-// Data movement: every read goes through TMA (cp.async.bulk.tensor) into a
-// 3-stage shared-memory pipeline, one mbarrier per stage.  Iteration i
-// brings the own-column box of P at plane ybase+i (feeding an 8-deep
-// register queue for dP/dy), v at plane ybase+i-4, and for the stress plane
-// y = ybase+i-7 the x-halo box of P (its own columns an L2 hit: fetched 7
-// planes earlier), Q and w with a z halo, u with an x halo, the model and,
-// where the tile touches the sponge, the split stresses.  Writes are plain
-// coalesced stores to the next level (u,v,w,P,Q ping-pong between steps;
-// split stresses in place).
+// Data movement: the boxes with halos and the model of a plane go through
+// TMA (cp.async.bulk.tensor) into a 3-stage shared-memory pipeline, one
+// mbarrier per stage; the thread's own P seven planes ahead and v three
+// planes ahead are loaded into registers one plane early, the split stresses
+// (sponge planes of the fast form, every plane of the exact form) at the
+// start of their plane.  The rebuilt u and w tiles are double-buffered, so a
+// plane has one block barrier, after which the previous plane's stage is
+// refilled.  A chunk's queues are filled by plain loads, all in flight
+// together, before the march.  Writes go to the next level (u,v,w,P,Q
+// ping-pong between steps; split stresses in place).
 //
+// Measured per step against one depth and two columns per thread with every
+// array in the TMA stages and two barriers a plane: 400^3 + 40 fast 1.557 ->
+// 1.395 ms (8.4 GB of DRAM traffic: 6.0 TB/s), exact 1.780 -> 1.736 ms;
+// 176x160x144 + 20 with imaging 0.184 -> 0.137 ms; 121x93x107 + 20 exact 83
+// -> 62 us.  The fast form is bound by DRAM at the large size (halos miss L2:
+// 1.24x the algorithmic bytes), by issue and latency at the small ones (240^3:
+// 333 thread instructions a point, issue 58%, DRAM 64% busy).  Four depths
+// per thread (128 threads, 168 registers, 12 warps an SM) took 1.53 ms, 190
+// and 100 us: half the instructions' latency is exposed; capped at 128
+// registers, or at 80 with two depths, it spills and the spills miss L1 (2.0
+// ms and more).  32 columns a tile: 1.45 ms; two stages 1.55 ms; four 1.39.
+
 // Arithmetic: GEO_MODE_EXACT keeps the reference's operation chain (no
 // contraction) and is bit-identical to it; GEO_MODE_FAST uses fused
 // multiply-adds at fixed places and the premultiplied model (A,B,C), the
@@ -29,29 +44,25 @@
 #include "fd3d_fused.cuh"
 #include "tc_util.cuh"
 #include <cudaTypedefs.h>
+#include <type_traits>
 
 namespace geo {
 
 __constant__ float cf_fd[4] = {1.196289f, -0.0797526f, 0.009570313f, -0.0006975447f};
 
 // stage layout (floats)
-constexpr int OFF_PO = 0;                 // P own box, plane y+7
-constexpr int OFF_V = OFF_PO + kOB;       // v own box, plane y+3
-constexpr int OFF_PH = OFF_V + kOB;       // P x-halo box, stress plane
+constexpr int OFF_PH = 0;                 // P x-halo box, stress plane
 constexpr int OFF_Q = OFF_PH + kPB;
 constexpr int OFF_U = OFF_Q + kQB;
 constexpr int OFF_W = OFF_U + kUB;
 constexpr int OFF_M = OFF_W + kQB;        // vp,e2,d2 or A,B,C
-constexpr int OFF_S = OFF_M + 3 * kOB;    // px py pz qx qy qz
-static_assert(OFF_S + 6 * kOB == kStageFloats, "stage layout");
-static_assert((OFF_V * 4) % 128 == 0 && (OFF_PH * 4) % 128 == 0 && (OFF_Q * 4) % 128 == 0 &&
-                  (OFF_U * 4) % 128 == 0 && (OFF_W * 4) % 128 == 0 && (OFF_M * 4) % 128 == 0 &&
-                  (OFF_S * 4) % 128 == 0 && (kStageFloats * 4) % 128 == 0,
+static_assert(OFF_M + 3 * kOB == kStageFloats, "stage layout");
+static_assert((OFF_Q * 4) % 128 == 0 && (OFF_U * 4) % 128 == 0 && (OFF_W * 4) % 128 == 0 && (OFF_M * 4) % 128 == 0 &&
+                  (kStageFloats * 4) % 128 == 0,
               "TMA destinations must stay 128-byte aligned");
-static_assert(kFusedSmem * 2 + 2048 <= 233472, "two blocks per SM must fit in shared memory");
+static_assert((kFusedSmem + 1024 + 64) * kFusedBlocks <= 233472, "blocks per SM must fit in shared memory");
 
 // mbarrier helpers with bounded waits (2 s), shared with the codec kernels
-using tc::gtimer;
 using tc::mbar_expect_tx;
 using tc::mbar_init;
 using tc::mbar_wait;
@@ -63,6 +74,61 @@ __device__ __forceinline__ void tma3(float *dst, const CUtensorMap *map, int c0,
             "r"(su32(dst)),
         "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(su32(bar))
         : "memory");
+}
+
+namespace {
+
+constexpr unsigned kFull = (1u << kW) - 1;
+
+// kW consecutive depths, moved as one vector.
+struct FV {
+    float v[kW];
+};
+using VecT = std::conditional_t<kW == 4, float4, float2>;
+template <class T>
+__device__ __forceinline__ FV unpack(const T &t) {
+    FV r;
+    r.v[0] = t.x;
+    r.v[1] = t.y;
+    if constexpr (kW == 4) {
+        r.v[2] = t.z;
+        r.v[3] = t.w;
+    }
+    return r;
+}
+__device__ __forceinline__ FV ld_s(const float *p) { return unpack(*reinterpret_cast<const VecT *>(p)); }
+__device__ __forceinline__ FV ld_g(const float *p, bool on) {
+    VecT t{};
+    if (on) t = __ldg(reinterpret_cast<const VecT *>(p));
+    return unpack(t);
+}
+// data this launch also writes (own points only): a plain load
+__device__ __forceinline__ FV ld_rw(const float *p) { return unpack(*reinterpret_cast<const VecT *>(p)); }
+template <class T = VecT>
+__device__ __forceinline__ void st_v(float *p, const FV &a) {
+    T t;
+    t.x = a.v[0];
+    t.y = a.v[1];
+    if constexpr (kW == 4) {
+        t.z = a.v[2];
+        t.w = a.v[3];
+    }
+    *reinterpret_cast<T *>(p) = t;
+}
+__device__ __forceinline__ void push(FV *q, const FV &a) {
+#pragma unroll
+    for (int k = 0; k < 7; k++) q[k] = q[k + 1];
+    q[7] = a;
+}
+// a where the point is updated, else b
+__device__ __forceinline__ FV pick(unsigned m, const FV &a, const FV &b) {
+    FV r = a;
+    if (m != kFull) {
+#pragma unroll
+        for (int j = 0; j < kW; j++)
+            if (!(m >> j & 1u)) r.v[j] = b.v[j];
+    }
+    return r;
 }
 
 // 8-tap staggered derivative sum_m c_m (a_m - b_m).  EXACT: the reference's
@@ -84,6 +150,38 @@ __device__ __forceinline__ float deriv(float a0, float b0, float a1, float b1, f
     return d;
 }
 
+// Derivative over eight vectors a(-3) .. a(+4) (forward stagger) or, shifted
+// by one, a(-4) .. a(+3) (backward).
+template <int MODE>
+__device__ __forceinline__ FV deriv8(const FV *q) {
+    FV r;
+#pragma unroll
+    for (int j = 0; j < kW; j++)
+        r.v[j] = deriv<MODE>(q[4].v[j], q[3].v[j], q[5].v[j], q[2].v[j], q[6].v[j], q[1].v[j], q[7].v[j], q[0].v[j]);
+    return r;
+}
+
+// Derivative along z of the kW depths at p; SHIFT 1: taps +1..+4 minus
+// 0..-3 (forward), 0: 0..+3 minus -1..-4.  mid: the vector at p, if the
+// caller has it in registers.
+template <int MODE, int SHIFT>
+__device__ __forceinline__ FV derivz(const float *p, const FV &mid) {
+    float e[8 + kW];
+#pragma unroll
+    for (int k = 0; k < 8 + kW; k += kW) {
+        const FV t = k == 4 ? mid : ld_s(p + k - 4);
+#pragma unroll
+        for (int j = 0; j < kW; j++) e[k + j] = t.v[j];
+    }
+    FV r;
+#pragma unroll
+    for (int j = 0; j < kW; j++) {
+        const float *q = e + 4 + j + SHIFT;
+        r.v[j] = deriv<MODE>(q[0], q[-1], q[1], q[-2], q[2], q[-3], q[3], q[-4]);
+    }
+    return r;
+}
+
 // Velocity update: c2*old - k1*d with k1 = c1*dt.
 template <int MODE>
 __device__ __forceinline__ float vel_update(float c2, float old, float k1, float d) {
@@ -91,210 +189,233 @@ __device__ __forceinline__ float vel_update(float c2, float old, float k1, float
     return c2 * old - k1 * d;
 }
 
-// Derivative along a shared-memory line: taps p[(m+1)*s] - p[-m*s].
-template <int MODE>
-__device__ __forceinline__ float dline_fwd(const float *p, int s) {
-    return deriv<MODE>(p[s], p[0], p[2 * s], p[-s], p[3 * s], p[-2 * s], p[4 * s], p[-3 * s]);
-}
-// Taps p[m*s] - p[-(m+1)*s].
-template <int MODE>
-__device__ __forceinline__ float dline_bwd(const float *p, int s) {
-    return deriv<MODE>(p[0], p[-s], p[s], p[-2 * s], p[2 * s], p[-3 * s], p[3 * s], p[-4 * s]);
-}
-
-template <int MODE>
-__global__ void __launch_bounds__(kTZ *kWarps, 2)
+template <int MODE, bool RTM>
+__global__ void __launch_bounds__(kFusedThreads, kFusedBlocks)
     k_fused3d(const __grid_constant__ StepMaps tm, const Fused3D g, const StepArgs3D st) {
     extern __shared__ unsigned char smem_raw[];
     float *base = reinterpret_cast<float *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
     float *stages = base;
-    float *utile = stages + kStages * kStageFloats;
-    float *wtile = utile + kUTile;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(wtile + kWTile);
+    float *utiles = stages + kStages * kStageFloats;   // two of each tile
+    float *wtiles = utiles + 2 * kUTile;
+    float *zprof = wtiles + 2 * kWTile;                // cz1*dtz, cz2, az1, az2 on the tile's 32 depths
+    uint64_t *bar = reinterpret_cast<uint64_t *>(zprof + 4 * kTZ);
     __shared__ int s_abort;
 
-    const int lane = threadIdx.x, wy = threadIdx.y, tid = wy * 32 + lane;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tile = blockIdx.x % g.ntiles, chunk = blockIdx.x / g.ntiles;
-    // consecutive blocks are z neighbours (measured on GB300: 25% faster
-    // than x neighbours at 480^3)
-    const int z0 = (tile % g.ntz) * kTZ, x0 = (tile / g.ntz) * kTXF;
+    // consecutive blocks are z neighbours
+    const int z0 = (tile % g.ntz) * kTZ, x0 = (tile / g.ntz) * kFX;
     const int ylo = 4 + chunk * g.chunk;
     const int yhi = min(ylo + g.chunk, g.nny - 4);
-    // iteration i brings P(ybase+i) into the queue, computes v(ybase+i-4)
-    // (i >= 7) and the stresses of plane ybase+i-7 (i >= 14)
-    const int ybase = ylo - 7;
-    const int NI = (yhi - ylo) + 14;
-    const bool xz_inside = x0 >= g.npd && x0 + kTXF <= g.npd + g.nx && z0 >= g.npd && z0 + kTZ <= g.npd + g.nz;
-    auto needs_split = [&](int y) {
-        return MODE == GEO_MODE_EXACT || !xz_inside || y < g.npd || y >= g.npd + g.ny;
-    };
+    const int NI = yhi - ylo;
+    const bool xz_inside = x0 >= g.npd && x0 + kFX <= g.npd + g.nx && z0 >= g.npd && z0 + kTZ <= g.npd + g.nz;
 
     if (tid == 0) {
         for (int s = 0; s < kStages; s++) mbar_init(&bar[s], 1);
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (tid < kTZ) {
+        const int z = min(z0 + tid, g.nnz - 1);
+        zprof[tid] = g.cz1[z] * g.dtz;
+        zprof[kTZ + tid] = g.cz2[z];
+        zprof[2 * kTZ + tid] = g.az1[z];
+        zprof[3 * kTZ + tid] = g.az2[z];
+    }
     __syncthreads();
 
-    // Loads of iteration i into stage i % kStages, spread over lane 0 of warps
-    // 0-3 (one per SM sub-partition).  The expected byte count may be posted
-    // after a copy completes: the phase cannot finish before warp 0 arrives.
-    auto issue = [&](int i) {
-        const int s = i % kStages;
-        const int y = ybase + i - 7;
+    // Boxes of plane ylo + i into stage s, spread over the warps'
+    // first lanes.  The expected byte count may be posted after a copy
+    // completes: the phase cannot finish before warp 0 arrives.
+    auto issue = [&](int i, int s) {
+        const int y = ylo + i;
         float *sp = stages + s * kStageFloats;
-        const bool sv = i >= 7, ss = i >= 14, split = ss && needs_split(y);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        if (wy == 0) {
-            uint32_t bytes = kOB * 4;
-            if (sv) bytes += kOB * 4;
-            if (ss) bytes += (kPB + kQB + kUB + kQB + 3 * kOB) * 4;
-            if (split) bytes += 6 * kOB * 4;
-            mbar_expect_tx(&bar[s], bytes);
-            tma3(sp + OFF_PO, &tm.m[1], z0, x0, ybase + i, &bar[s]);
-            if (sv) tma3(sp + OFF_V, &tm.m[5], z0, x0, y + 3, &bar[s]);
-        } else if (wy == 1) {
-            if (ss) {
-                tma3(sp + OFF_PH, &tm.m[0], z0, x0 - 7, y, &bar[s]);
-                tma3(sp + OFF_Q, &tm.m[2], z0 - 8, x0, y, &bar[s]);
-            }
-        } else if (wy == 2) {
-            if (ss) {
-                tma3(sp + OFF_U, &tm.m[3], z0, x0 - 4, y, &bar[s]);
-                tma3(sp + OFF_W, &tm.m[4], z0 - 8, x0, y, &bar[s]);
-                for (int r = 0; r < 3; r++) tma3(sp + OFF_M + r * kOB, &tm.m[6 + r], z0, x0, y, &bar[s]);
-            }
-        } else {
-            if (split)
-                for (int r = 0; r < 6; r++) tma3(sp + OFF_S + r * kOB, &tm.m[9 + r], z0, x0, y, &bar[s]);
+        if (warp == 0) {
+            mbar_expect_tx(&bar[s], kStageFloats * 4);
+            tma3(sp + OFF_PH, &tm.m[0], z0, x0 - 7, y, &bar[s]);
+            tma3(sp + OFF_Q, &tm.m[1], z0 - 8, x0, y, &bar[s]);
+        } else if (warp == 1) {
+            tma3(sp + OFF_U, &tm.m[2], z0, x0 - 4, y, &bar[s]);
+            tma3(sp + OFF_W, &tm.m[3], z0 - 8, x0, y, &bar[s]);
+        } else if (warp == 2) {
+            for (int r = 0; r < 3; r++) tma3(sp + OFF_M + r * kOB, &tm.m[4 + r], z0, x0, y, &bar[s]);
         }
     };
-    if (lane == 0 && wy < 4)
-        for (int i = 0; i < kStages && i < NI; i++) issue(i);
+    if (lane == 0)
+        for (int i = 0; i < kStages && i < NI; i++) issue(i, i);
 
-    // ---- per-thread constants: columns ca = 2*wy and ca+1, depth zo
-    const int ca = 2 * wy, xa = x0 + ca, zo = z0 + lane;
-    const bool z_upd = zo >= 4 && zo < g.nnz - 4;
-    const bool upd_a = z_upd && xa >= 4 && xa < g.nnx - 4, upd_b = z_upd && xa + 1 >= 4 && xa + 1 < g.nnx - 4;
-    const bool z_in = zo >= g.npd && zo < g.npd + g.nz;
-    const bool in_a = z_in && xa >= g.npd && xa < g.npd + g.nx, in_b = z_in && xa + 1 >= g.npd && xa + 1 < g.npd + g.nx;
-    const int xca = min(max(xa, 0), g.nnx - 1), xcb = min(max(xa + 1, 0), g.nnx - 1), zc = min(max(zo, 0), g.nnz - 1);
-    const float kxa = g.cx1[xca] * g.dtx, cx2a = g.cx2[xca], ax1a = g.ax1[xca], ax2a = g.ax2[xca];
-    const float kxb = g.cx1[xcb] * g.dtx, cx2b = g.cx2[xcb], ax1b = g.ax1[xcb], ax2b = g.ax2[xcb];
-    const float kz = g.cz1[zc] * g.dtz, cz2 = g.cz2[zc], az1 = g.az1[zc], az2 = g.az2[zc];
-    // receiver traces along x (or -1)
-    int rec_a = -1, rec_b = -1;
-    if (st.rec && zo == st.rec_iz) {
-        const int ra = xa - g.npd - st.rx0, rb = ra + 1;
-        if (ra >= 0 && ra % st.drx == 0 && ra / st.drx < st.nrx) rec_a = ra / st.drx;
-        if (rb >= 0 && rb % st.drx == 0 && rb / st.drx < st.nrx) rec_b = rb / st.drx;
-    }
-    // halo velocities: items 0-223 are u on the 7 halo columns (4 left, 3
-    // right), items 224-335 w on the 7 halo depths of each column (4 above, 3
-    // below); thread t takes items t and t+256
-    int h1_idx = 0, h1_src = 0, h2_idx = 0, h2_src = 0;  // tile index, tap origin
-    bool h1_upd = false, h2_upd = false;
-    float h1k = 0, h1c2 = 0, h2k = 0, h2c2 = 0;
-    const bool h1_u = tid < 224, h2_on = tid + 256 < 224 + 7 * kTXF;
-    {
-        auto setup = [&](int h, int &idx, int &src, bool &upd, float &k, float &c2) {
-            if (h < 224) {
-                const int hc = h >> 5, hl = h & 31;
-                const int c = hc < 4 ? hc : kTXF + hc;  // u tile / u box column
-                const int x = x0 - 4 + c, z = z0 + hl;
-                upd = x >= 4 && x < g.nnx - 4 && z >= 4 && z < g.nnz - 4;
-                const int xcl = min(max(x, 0), g.nnx - 1);
-                k = g.cx1[xcl] * g.dtx;
-                c2 = g.cx2[xcl];
-                idx = c * 32 + hl;                 // u tile and u box
-                src = (c + 3) * 32 + hl;           // P halo box
-            } else {
-                const int t = h - 224, col = t / 7, hh = t % 7;
-                const int qz = hh < 4 ? hh : kTZ + hh;  // w tile index (z0-4 origin)
-                const int z = z0 - 4 + qz, x = x0 + col;
-                upd = z >= 4 && z < g.nnz - 4 && x >= 4 && x < g.nnx - 4;
-                const int zcl = min(max(z, 0), g.nnz - 1);
-                k = g.cz1[zcl] * g.dtz;
-                c2 = g.cz2[zcl];
-                idx = col * 40 + qz;               // w tile
-                src = col * 48 + qz + 4;           // Q / w box
-            }
-        };
-        setup(tid, h1_idx, h1_src, h1_upd, h1k, h1c2);
-        if (h2_on) setup(tid + 256, h2_idx, h2_src, h2_upd, h2k, h2c2);
-    }
-    // element offsets fit in 32 bits (checked on the host)
-    const int sxy = (int)g.sxy, ldz = g.ldz;
-    const int col_a = zo + ldz * xa;   // own columns at y = 0 (b = a + ldz)
-    const int oa = ca * 32 + lane;     // column a in an own box (b = +32)
-    float qa[8], qb[8], pa[8], pb[8];  // v(y-4 .. y+3), P(y .. y+7) per column
+    // ---- the thread's column and depths
+    const int zl = tid % (kTZ / kW) * kW, c = tid / (kTZ / kW), xa = x0 + c, zo = z0 + zl;
+    const bool mem = xa < g.nnx && zo < g.ldz;   // its vector exists
+    unsigned um = 0;                             // updated depths
+    if (xa >= 4 && xa < g.nnx - 4)
 #pragma unroll
-    for (int k = 0; k < 8; k++) qa[k] = qb[k] = pa[k] = pb[k] = 0.0f;
-    uint32_t phase = 0;
-    // y-direction sponge factors (v plane y+3, stress plane y), loaded one
-    // iteration ahead so their latency hides behind a plane of work
-    auto ycoef = [&](int i, float &c1, float &c2, float &a1, float &a2) {
-        const int y = ybase + i - 7;
-        const int yv = min(max(y + 3, 0), g.nny - 1), ys = min(max(y, 0), g.nny - 1);
+        for (int j = 0; j < kW; j++) um |= (zo + j >= 4 && zo + j < g.nnz - 4 ? 1u : 0u) << j;
+    unsigned in4 = 0;                            // depths inside the physical box (x and z)
+    if (xa >= g.npd && xa < g.npd + g.nx)
+#pragma unroll
+        for (int j = 0; j < kW; j++) in4 |= (zo + j >= g.npd && zo + j < g.npd + g.nz ? 1u : 0u) << j;
+    const bool wr = um != 0;
+    const int xc = min(xa, g.nnx - 1);
+    const float kx = g.cx1[xc] * g.dtx, cx2 = g.cx2[xc], ax1 = g.ax1[xc], ax2 = g.ax2[xc];
+    // receiver trace along x (or -1) and depth within the vector
+    int rec_x = -1;
+    const int rec_j = st.rec_iz - zo;
+    if (st.rec && rec_j >= 0 && rec_j < kW) {
+        const int r = xa - g.npd - st.rx0;
+        if (r >= 0 && r % st.drx == 0 && r / st.drx < st.nrx && (um >> rec_j & 1u)) rec_x = r / st.drx;
+    }
+    // halo velocities: the first threads u on the 7 halo columns (4 left, 3
+    // right), threads of the upper half w on the four depths above and below
+    // each column
+    FV hk, hc2;
+    unsigned hm = 0;
+    int h_tile = 0, h_src = 0;
+    constexpr int kUTasks = 7 * kTZ / kW, kWGroups = 8 / kW, kHalf = kFusedThreads / 2;
+    static_assert(kUTasks <= kHalf && kFX * kWGroups <= kHalf, "halo tasks");
+    const bool hu = tid < kUTasks, hw = tid >= kHalf && tid < kHalf + kFX * kWGroups;
+    if (hu) {
+        const int hc = c, cc = hc < 4 ? hc : kFX + hc, x = x0 - 4 + cc, xcl = min(max(x, 0), g.nnx - 1);
+        if (x >= 4 && x < g.nnx - 4)
+            for (int j = 0; j < kW; j++) hm |= (zo + j >= 4 && zo + j < g.nnz - 4 ? 1u : 0u) << j;
+        for (int j = 0; j < kW; j++) {
+            hk.v[j] = g.cx1[xcl] * g.dtx;
+            hc2.v[j] = g.cx2[xcl];
+        }
+        h_tile = cc * kTZ + zl;          // u tile and u box
+        h_src = (cc + 3) * kTZ + zl;     // P halo box
+    } else {
+        const int t = (tid - kHalf + kFusedThreads) % (kFX * kWGroups), col = t / kWGroups, grp = t % kWGroups;
+        const int zr = grp < kWGroups / 2 ? grp * kW - 4 : kTZ + (grp - kWGroups / 2) * kW, x = x0 + col, z = z0 + zr;
+        for (int j = 0; j < kW; j++) {
+            if (x >= 4 && x < g.nnx - 4) hm |= (z + j >= 4 && z + j < g.nnz - 4 ? 1u : 0u) << j;
+            const int zcl = min(max(z + j, 0), g.nnz - 1);
+            hk.v[j] = g.cz1[zcl] * g.dtz;
+            hc2.v[j] = g.cz2[zcl];
+        }
+        h_tile = col * 40 + zr + 4;          // w tile
+        h_src = col * 48 + zr + 8;           // Q and w boxes
+    }
+    const int sxy = (int)g.sxy, own = zo + g.ldz * xa;   // element offsets fit in 32 bits (checked on the host)
+    // the step's point source, P,Q += amp before the velocity update
+    // (GPU_vti3dfd_kernels.cu:135), on this thread's own copy of P
+    const int src_j = st.src_on && xa == st.ixs ? st.izs - zo : -1;
+    auto add_source = [&](FV &a, int plane) {
+        if (src_j >= 0 && plane == st.iys)
+#pragma unroll
+            for (int j = 0; j < kW; j++)
+                if (j == src_j) a.v[j] += st.amp;
+    };
+
+    // ---- queues: P of planes ylo-1 .. ylo+6, the new v of ylo-4 .. ylo+2
+    FV p[8], q[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+#pragma unroll
+        for (int j = 0; j < kW; j++) p[k].v[j] = q[k].v[j] = 0.0f;
+    auto ld_P = [&](int y) { return ld_g(g.P0 + own + sxy * y, mem && y >= 0 && y < g.nny); };
+    auto ld_v = [&](int y) { return ld_g(g.v0 + own + sxy * y, mem && y >= 0 && y < g.nny); };
+    auto new_v = [&](const FV &vo, int yv, float cy1, float cy2) {
+        if (yv < 4 || yv >= g.nny - 4) return vo;
+        const float ky = cy1 * g.dty;
+        const FV d = deriv8<MODE>(p);
+        FV r;
+#pragma unroll
+        for (int j = 0; j < kW; j++) r.v[j] = vel_update<MODE>(cy2, vo.v[j], ky, d.v[j]);
+        return pick(um, r, vo);
+    };
+#pragma unroll
+    for (int k = 0; k < 7; k++) p[k + 1] = ld_P(ylo - 7 + k);
+    {
+        FV pn[7], vn[7];
+#pragma unroll
+        for (int k = 0; k < 7; k++) {
+            pn[k] = ld_P(ylo + k);
+            vn[k] = ld_v(ylo - 4 + k);
+        }
+#pragma unroll
+        for (int k = 0; k < 7; k++) add_source(p[k + 1], ylo - 7 + k);
+#pragma unroll
+        for (int k = 0; k < 7; k++) {
+            const int yv = ylo - 4 + k, yc = min(max(yv, 0), g.nny - 1);
+            add_source(pn[k], ylo + k);
+            push(p, pn[k]);
+            const FV t = new_v(vn[k], yv, g.cy1[yc], g.cy2[yc]);
+            push(q, t);
+            if (wr && yv >= ylo && yv < yhi) st_v(g.v1 + own + sxy * yv, t);
+        }
+    }
+    // one plane ahead: own P and v, y-direction sponge factors
+    FV nP = ld_P(ylo + 7), nv = ld_v(ylo + 3);
+    auto ycoef = [&](int y, float &c1, float &c2, float &a1, float &a2) {
+        const int yv = min(y + 3, g.nny - 1), ys = min(y, g.nny - 1);
         c1 = __ldg(g.cy1 + yv); c2 = __ldg(g.cy2 + yv); a1 = __ldg(g.ay1 + ys); a2 = __ldg(g.ay2 + ys);
     };
     float ncy1, ncy2, nay1, nay2;
-    ycoef(0, ncy1, ncy2, nay1, nay2);
+    ycoef(ylo, ncy1, ncy2, nay1, nay2);
 
-    for (int i = 0; i < NI; i++) {
+    int s = 0, off = own + sxy * ylo;   // stage and offset of the plane
+    unsigned par = 0;                   // parity of the stage's phase
+    for (int i = 0; i < NI; i++, s = s + 1 == kStages ? 0 : s + 1, par ^= s == 0, off += sxy) {
+        const int y = ylo + i;
         const float cy1 = ncy1, cy2 = ncy2, ay1 = nay1, ay2 = nay2;
-        if (i + 1 < NI) ycoef(i + 1, ncy1, ncy2, nay1, nay2);
-        const int s = i % kStages;
-        if (tid == 0 && !mbar_wait(&bar[s], (phase >> s) & 1u)) s_abort = 1;
-        phase ^= 1u << s;
-        __syncthreads();
-        if (s_abort) {
-            // a stage never completed: report, let copies in flight land
-            // (bounded), and leave
-            if (tid == 0) {
-                atomicExch(g.err, 1);
-                for (int k = 1; k < kStages; k++) {
-                    const int s2 = (s + k) % kStages;
-                    mbar_wait(&bar[s2], (phase >> s2) & 1u);
-                }
-            }
-            return;
+        const bool y_in = y >= g.npd && y < g.npd + g.ny;
+        const bool split = MODE == GEO_MODE_EXACT || !xz_inside || !y_in;   // this plane of the block
+        const unsigned in = y_in ? in4 : 0u;
+        const bool own_split = MODE == GEO_MODE_EXACT ? wr : wr && (um & ~in) != 0;
+        // own P seven and v three planes ahead, then the next plane's
+        FV pc = nP;
+        const FV vo = nv;
+        if (i + 1 < NI) {
+            nP = ld_P(y + 8);
+            nv = ld_v(y + 4);
+            ycoef(y + 1, ncy1, ncy2, nay1, nay2);
         }
-        // stage (i-1) % kStages is free now
-        if (lane == 0 && wy < 4 && i >= 1 && i - 1 + kStages < NI) issue(i - 1 + kStages);
-        float *sp = stages + s * kStageFloats;
-        const int y = ybase + i - 7;           // stress plane
-        const bool stress_plane = i >= 14;
-        // illumination / image inputs of the stress plane (RTM), loaded here
-        // so that their latency hides behind the plane's arithmetic
-        float pre_ill[2] = {0.0f, 0.0f}, pre_mig[2] = {0.0f, 0.0f}, pre_oth[2] = {0.0f, 0.0f};
-        if (stress_plane && (st.ill || st.mig) && y >= g.npd && y < g.npd + g.ny) {
+        FV S[6];
+        if (split && own_split) {
+            S[0] = ld_rw(g.px + off); S[1] = ld_rw(g.py + off); S[2] = ld_rw(g.pz + off);
+            S[3] = ld_rw(g.qx + off); S[4] = ld_rw(g.qy + off); S[5] = ld_rw(g.qz + off);
+        }
+        // illumination / image inputs (RTM), loaded here so that their latency
+        // hides behind the plane's arithmetic
+        FV ill, mig, oth;
+        const unsigned im = RTM ? in & um : 0u;
+        const bool imv = im == kFull && st.img_vec;
+        long io = 0;
+        if (RTM && im) {
+            io = (long)(zo - g.npd) + (long)g.nz * ((xa - g.npd) + (long)g.nx * (y - g.npd));
+            if (imv) {
+                if (st.ill) ill = ld_rw(st.ill + io);
+                if (st.mig) mig = ld_rw(st.mig + io);
+            } else {
 #pragma unroll
-            for (int cb = 0; cb < 2; cb++) {
-                if (!(cb ? in_b : in_a)) continue;
-                const long o = (long)(zo - g.npd) + (long)g.nz * ((xa + cb - g.npd) + (long)g.nx * (y - g.npd));
-                if (st.ill) pre_ill[cb] = st.ill[o];
-                if (st.mig) {
-                    pre_mig[cb] = st.mig[o];
-                    pre_oth[cb] = st.other_P[col_a + sxy * y + cb * ldz];
-                }
+                for (int j = 0; j < kW; j++)
+                    if (im >> j & 1u) {
+                        if (st.ill) ill.v[j] = st.ill[io + j];
+                        if (st.mig) mig.v[j] = st.mig[io + j];
+                    }
             }
+            if (st.mig) oth = ld_g(st.other_P + off, true);
         }
 
-        // point source, P,Q += amp before the velocity update
-        // (GPU_vti3dfd_kernels.cu:135): patch the shared copies holding the
-        // source cell; the own-point stress update reads P,Q from global.
-        if (st.src_on) {
-            const bool pO = st.iys == ybase + i && st.izs >= z0 && st.izs < z0 + kTZ && st.ixs >= x0 &&
-                            st.ixs < x0 + kTXF;
-            const bool pH = stress_plane && st.iys == y && st.izs >= z0 && st.izs < z0 + kTZ &&
-                            st.ixs >= x0 - 7 && st.ixs < x0 + kTXF + 7;
-            const bool pQ = stress_plane && st.iys == y && st.ixs >= x0 && st.ixs < x0 + kTXF &&
-                            st.izs >= z0 - 8 && st.izs < z0 + 40;
-            if (pO || pH || pQ) {
+        add_source(pc, y + 7);
+        push(p, pc);
+        {
+            const FV vn = new_v(vo, y + 3, cy1, cy2);
+            push(q, vn);
+            if (wr && y + 3 < yhi) st_v(g.v1 + off + 3 * sxy, vn);
+        }
+
+        if (!mbar_wait(&bar[s], par)) *(volatile int *)&s_abort = 1;
+        float *sp = stages + s * kStageFloats;
+        if (st.src_on && y == st.iys) {
+            // the shared copies that hold the source cell
+            const bool pH = st.izs >= z0 && st.izs < z0 + kTZ && st.ixs >= x0 - 7 && st.ixs < x0 + kFX + 7;
+            const bool pQ = st.ixs >= x0 && st.ixs < x0 + kFX && st.izs >= z0 - 8 && st.izs < z0 + 40;
+            if (pH || pQ) {
                 if (tid == 0) {
-                    if (pO) sp[OFF_PO + (st.ixs - x0) * 32 + (st.izs - z0)] += st.amp;
-                    if (pH) sp[OFF_PH + (st.ixs - (x0 - 7)) * 32 + (st.izs - z0)] += st.amp;
+                    if (pH) sp[OFF_PH + (st.ixs - (x0 - 7)) * kTZ + (st.izs - z0)] += st.amp;
                     if (pQ) sp[OFF_Q + (st.ixs - x0) * 48 + (st.izs - (z0 - 8))] += st.amp;
                     // these cells are later overwritten by the async proxy
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -302,174 +423,179 @@ __global__ void __launch_bounds__(kTZ *kWarps, 2)
                 __syncthreads();
             }
         }
-
-        // own-column P queues
+        float *ut = utiles + (i & 1) * kUTile, *wt = wtiles + (i & 1) * kWTile;
+        // own u: taps P(x-3 .. x+4) = P box columns c+4 .. c+11
+        FV un;
+        {
+            const float *ph = sp + OFF_PH + (c + 4) * kTZ + zl;
+            FV t[8];
 #pragma unroll
-        for (int k = 0; k < 7; k++) {
-            pa[k] = pa[k + 1];
-            pb[k] = pb[k + 1];
+            for (int k = 0; k < 8; k++) t[k] = ld_s(ph + k * kTZ);
+            const FV uo = ld_s(sp + OFF_U + (c + 4) * kTZ + zl), d = deriv8<MODE>(t);
+#pragma unroll
+            for (int j = 0; j < kW; j++) un.v[j] = vel_update<MODE>(cx2, uo.v[j], kx, d.v[j]);
+            un = pick(um, un, uo);
+            st_v(ut + (c + 4) * kTZ + zl, un);
+            if (wr) st_v(g.u1 + off, un);
         }
-        pa[7] = sp[OFF_PO + oa];
-        pb[7] = sp[OFF_PO + oa + 32];
-
-        // Both columns' updates are computed unconditionally and only the
-        // stores are predicated: one basic block per half-step lets the
-        // compiler interleave the two columns (measured at 400^3 + 40:
-        // 1.505 ms per step against 1.547 ms with per-column branches).
-        // v at plane yv = y+3 (taps P(yv-3 .. yv+4) = the queue), into the queues
-        if (i >= 7) {
-            const int yv = y + 3;
-            const float va = sp[OFF_V + oa], vb = sp[OFF_V + oa + 32];
-            float vna = va, vnb = vb;
-            if (yv >= 4 && yv < g.nny - 4) {
-                const float ky = cy1 * g.dty;
-                const int iv = col_a + sxy * yv;
-                const float ta = vel_update<MODE>(cy2, va, ky, deriv<MODE>(pa[4], pa[3], pa[5], pa[2], pa[6], pa[1], pa[7], pa[0]));
-                const float tb = vel_update<MODE>(cy2, vb, ky, deriv<MODE>(pb[4], pb[3], pb[5], pb[2], pb[6], pb[1], pb[7], pb[0]));
-                if (upd_a) g.v1[iv] = ta;
-                if (upd_b) g.v1[iv + ldz] = tb;
-                vna = upd_a ? ta : va;
-                vnb = upd_b ? tb : vb;
-            }
+        // own w
+        FV wn, qo;
+        {
+            const float *Q = sp + OFF_Q + c * 48 + zl + 8;
+            qo = ld_s(Q);
+            const FV wo = ld_s(sp + OFF_W + c * 48 + zl + 8);
+            const FV kz = ld_s(zprof + zl), cz2 = ld_s(zprof + kTZ + zl), d = derivz<MODE, 1>(Q, qo);
 #pragma unroll
-            for (int k = 0; k < 7; k++) {
-                qa[k] = qa[k + 1];
-                qb[k] = qb[k + 1];
-            }
-            qa[7] = vna;
-            qb[7] = vnb;
+            for (int j = 0; j < kW; j++) wn.v[j] = vel_update<MODE>(cz2.v[j], wo.v[j], kz.v[j], d.v[j]);
+            wn = pick(um, wn, wo);
+            st_v(wt + c * 40 + zl + 4, wn);
+            if (wr) st_v(g.w1 + off, wn);
         }
+        // halo u and w
+        if (hu) {
+            FV t[8], r;
+#pragma unroll
+            for (int k = 0; k < 8; k++) t[k] = ld_s(sp + OFF_PH + h_src + (k - 3) * kTZ);
+            const FV uo = ld_s(sp + OFF_U + h_tile), d = deriv8<MODE>(t);
+#pragma unroll
+            for (int j = 0; j < kW; j++) r.v[j] = vel_update<MODE>(hc2.v[j], uo.v[j], hk.v[j], d.v[j]);
+            st_v(ut + h_tile, pick(hm, r, uo));
+        } else if (hw) {
+            const float *Q = sp + OFF_Q + h_src;
+            const FV wo = ld_s(sp + OFF_W + h_src), d = derivz<MODE, 1>(Q, ld_s(Q));
+            FV r;
+#pragma unroll
+            for (int j = 0; j < kW; j++) r.v[j] = vel_update<MODE>(hc2.v[j], wo.v[j], hk.v[j], d.v[j]);
+            st_v(wt + h_tile, pick(hm, r, wo));
+        }
+        __syncthreads();
+        if (*(volatile int *)&s_abort) {
+            // a stage never completed: report, let copies in flight land
+            // (bounded), and leave
+            if (tid == 0) {
+                atomicExch(g.err, 1);
+                for (int k = 1; k < kStages; k++)
+                    if (i + k < NI && i + k < (i ? i + 2 : kStages)) mbar_wait(&bar[(i + k) % kStages], ((i + k) / kStages) & 1);
+            }
+            return;
+        }
+        // every thread is past plane i-1: its stage takes plane i+2
+        if (lane == 0 && i >= 1 && i - 1 + kStages < NI) issue(i - 1 + kStages, s == 0 ? kStages - 1 : s - 1);
 
-        if (stress_plane) {
-            const float *ph = sp + OFF_PH;
-            const int yoff = sxy * y;
-            // own u at u-tile columns ca+4, ca+5 (P-halo columns ca+7, ca+8):
-            // taps on P-halo columns ca+4 .. ca+12, shared by the two
-            {
-                float p[9];
+        // stresses
+        FV xx, zz;
+        {
+            FV t[8];
 #pragma unroll
-                for (int k = 0; k < 9; k++) p[k] = ph[(ca + 4 + k) * 32 + lane];
-                const float uoa = sp[OFF_U + (ca + 4) * 32 + lane], uob = sp[OFF_U + (ca + 5) * 32 + lane];
-                float una = uoa, unb = uob;
-                const int iu = col_a + yoff;
-                const float ta = vel_update<MODE>(cx2a, uoa, kxa, deriv<MODE>(p[4], p[3], p[5], p[2], p[6], p[1], p[7], p[0]));
-                const float tb = vel_update<MODE>(cx2b, uob, kxb, deriv<MODE>(p[5], p[4], p[6], p[3], p[7], p[2], p[8], p[1]));
-                if (upd_a) g.u1[iu] = ta;
-                if (upd_b) g.u1[iu + ldz] = tb;
-                una = upd_a ? ta : uoa;
-                unb = upd_b ? tb : uob;
-                utile[(ca + 4) * 32 + lane] = una;
-                utile[(ca + 5) * 32 + lane] = unb;
+            for (int k = 0; k < 8; k++) t[k] = k == 4 ? un : ld_s(ut + (c + k) * kTZ + zl);
+            xx = deriv8<MODE>(t);
+            zz = derivz<MODE, 0>(wt + c * 40 + zl + 4, wn);
+        }
+        const FV yy = deriv8<MODE>(q);
+        const float *M = sp + OFF_M + c * kTZ + zl;
+        const FV m0 = ld_s(M), m1 = ld_s(M + kOB), m2 = ld_s(M + 2 * kOB);
+        FV P, Q;
+        if (MODE == GEO_MODE_FAST) {
+            // m = A, B, C; inside the box all sponge factors are 1
+            FV p0 = p[0];
+            if (src_j >= 0 && src_j < kW && y == st.iys) {   // the stress update starts from the cell's own P, Q
+                const float ps = g.P0[own + src_j + sxy * y], qs = g.Q0[own + src_j + sxy * y];
+#pragma unroll
+                for (int j = 0; j < kW; j++)
+                    if (j == src_j) {
+                        p0.v[j] = ps;
+                        qo.v[j] = qs;
+                    }
             }
-            // own w at depth lane+4 of columns ca, ca+1
-            {
-                const float *Qa = sp + OFF_Q + ca * 48 + lane + 8, *Qb = Qa + 48;
-                const float woa = sp[OFF_W + ca * 48 + lane + 8], wob = sp[OFF_W + ca * 48 + 48 + lane + 8];
-                float wna = woa, wnb = wob;
-                const int iw = col_a + yoff;
-                const float ta = vel_update<MODE>(cz2, woa, kz, dline_fwd<MODE>(Qa, 1));
-                const float tb = vel_update<MODE>(cz2, wob, kz, dline_fwd<MODE>(Qb, 1));
-                if (upd_a) g.w1[iw] = ta;
-                if (upd_b) g.w1[iw + ldz] = tb;
-                wna = upd_a ? ta : woa;
-                wnb = upd_b ? tb : wob;
-                wtile[ca * 40 + lane + 4] = wna;
-                wtile[ca * 40 + 40 + lane + 4] = wnb;
+#pragma unroll
+            for (int j = 0; j < kW; j++) {
+                const float Ax = m0.v[j] * g.dtx, Ay = m0.v[j] * g.dty, Bz = m1.v[j] * g.dtz;
+                const float Bx = m1.v[j] * g.dtx, By = m1.v[j] * g.dty, Cz = m2.v[j] * g.dtz;
+                P.v[j] = __fmaf_rn(-Bz, zz.v[j], __fmaf_rn(-Ay, yy.v[j], __fmaf_rn(-Ax, xx.v[j], p0.v[j])));
+                Q.v[j] = __fmaf_rn(-Cz, zz.v[j], __fmaf_rn(-By, yy.v[j], __fmaf_rn(-Bx, xx.v[j], qo.v[j])));
             }
-            // halo u and w
-            {
-                if (h1_u) {
-                    const float uo = sp[OFF_U + h1_idx];
-                    utile[h1_idx] = h1_upd ? vel_update<MODE>(h1c2, uo, h1k, dline_fwd<MODE>(ph + h1_src, 32)) : uo;
+        }
+        if (split && own_split) {
+            const FV az1 = ld_s(zprof + 2 * kTZ + zl), az2 = ld_s(zprof + 3 * kTZ + zl);
+#pragma unroll
+            for (int j = 0; j < kW; j++) {
+                float px, py, pz, qx, qy, qz;
+                if (MODE == GEO_MODE_FAST) {
+                    const float Ax = m0.v[j] * g.dtx, Ay = m0.v[j] * g.dty, Bz = m1.v[j] * g.dtz;
+                    const float Bx = m1.v[j] * g.dtx, By = m1.v[j] * g.dty, Cz = m2.v[j] * g.dtz;
+                    px = __fmaf_rn(-(ax1 * Ax), xx.v[j], ax2 * S[0].v[j]);
+                    py = __fmaf_rn(-(ay1 * Ay), yy.v[j], ay2 * S[1].v[j]);
+                    pz = __fmaf_rn(-(az1.v[j] * Bz), zz.v[j], az2.v[j] * S[2].v[j]);
+                    qx = __fmaf_rn(-(ax1 * Bx), xx.v[j], ax2 * S[3].v[j]);
+                    qy = __fmaf_rn(-(ay1 * By), yy.v[j], ay2 * S[4].v[j]);
+                    qz = __fmaf_rn(-(az1.v[j] * Cz), zz.v[j], az2.v[j] * S[5].v[j]);
+                    // points of the vector inside the box keep the unsplit form
+                    if ((in & um) >> j & 1u) continue;
                 } else {
-                    const float wo = sp[OFF_W + h1_src];
-                    wtile[h1_idx] = h1_upd ? vel_update<MODE>(h1c2, wo, h1k, dline_fwd<MODE>(sp + OFF_Q + h1_src, 1)) : wo;
+                    // m = vp, 1+2eps, sqrtf(1+2del); the reference's chain
+                    const float vp = m0.v[j], e2 = m1.v[j], d2 = m2.v[j];
+                    px = ax2 * S[0].v[j] - ax1 * vp * vp * e2 * g.dtx * xx.v[j];
+                    py = ay2 * S[1].v[j] - ay1 * vp * vp * e2 * g.dty * yy.v[j];
+                    pz = az2.v[j] * S[2].v[j] - az1.v[j] * vp * vp * d2 * g.dtz * zz.v[j];
+                    qx = ax2 * S[3].v[j] - ax1 * vp * vp * d2 * g.dtx * xx.v[j];
+                    qy = ay2 * S[4].v[j] - ay1 * vp * vp * d2 * g.dty * yy.v[j];
+                    qz = az2.v[j] * S[5].v[j] - az1.v[j] * vp * vp * g.dtz * zz.v[j];
                 }
-                if (h2_on) {
-                    const float wo = sp[OFF_W + h2_src];
-                    wtile[h2_idx] = h2_upd ? vel_update<MODE>(h2c2, wo, h2k, dline_fwd<MODE>(sp + OFF_Q + h2_src, 1)) : wo;
+                if (um >> j & 1u) {
+                    S[0].v[j] = px; S[1].v[j] = py; S[2].v[j] = pz;
+                    S[3].v[j] = qx; S[4].v[j] = qy; S[5].v[j] = qz;
                 }
+                P.v[j] = px + py + pz;
+                Q.v[j] = qx + qy + qz;
             }
-            __syncthreads();
-
-            // stresses of columns a and b
-            float t[9];
+            st_v(g.px + off, S[0]); st_v(g.py + off, S[1]); st_v(g.pz + off, S[2]);
+            st_v(g.qx + off, S[3]); st_v(g.qy + off, S[4]); st_v(g.qz + off, S[5]);
+        }
+        if (!wr) continue;
+        if (um != kFull) {   // points off the updated grid keep their zeros
 #pragma unroll
-            for (int k = 0; k < 9; k++) t[k] = utile[(ca + k) * 32 + lane];
-            const bool y_in = y >= g.npd && y < g.npd + g.ny;
+            for (int j = 0; j < kW; j++)
+                if (!(um >> j & 1u)) P.v[j] = Q.v[j] = 0.0f;
+        }
+        st_v(g.P1 + off, P);
+        st_v(g.Q1 + off, Q);
+        if (rec_x >= 0) {
+            const int rr = y - g.npd - st.ry0;
+            if (rr >= 0 && rr % st.dry == 0 && rr / st.dry < st.nry) {
+                float a = P.v[0], b = Q.v[0];
 #pragma unroll
-            for (int cb = 0; cb < 2; cb++) {
-                const bool upd = cb ? upd_b : upd_a;
-                const float *q = cb ? qb : qa;
-                const int o = oa + 32 * cb;
-                const float m0 = sp[OFF_M + o], m1 = sp[OFF_M + kOB + o], m2 = sp[OFF_M + 2 * kOB + o];
-                const float yy = deriv<MODE>(q[4], q[3], q[5], q[2], q[6], q[1], q[7], q[0]);
-                const float xx = cb ? deriv<MODE>(t[5], t[4], t[6], t[3], t[7], t[2], t[8], t[1])
-                                    : deriv<MODE>(t[4], t[3], t[5], t[2], t[6], t[1], t[7], t[0]);
-                const float zz = dline_bwd<MODE>(wtile + (ca + cb) * 40 + lane + 4, 1);
-                const float ax1 = cb ? ax1b : ax1a, ax2 = cb ? ax2b : ax2a;
-                const int id = col_a + yoff + cb * ldz;
-                float P, Q;
-                if (MODE == GEO_MODE_FAST && (cb ? in_b : in_a) && y_in) {
-                    // m = A, B, C; all sponge factors are 1
-                    const float Ax = m0 * g.dtx, Ay = m0 * g.dty, Bz = m1 * g.dtz;
-                    const float Bx = m1 * g.dtx, By = m1 * g.dty, Cz = m2 * g.dtz;
-                    float p0 = cb ? pb[0] : pa[0], q0 = sp[OFF_Q + (ca + cb) * 48 + lane + 8];
-                    if (st.src_on && id == (int)st.src) {
-                        p0 = g.P0[id];
-                        q0 = g.Q0[id];
+                for (int j = 1; j < kW; j++)
+                    if (j == rec_j) {
+                        a = P.v[j];
+                        b = Q.v[j];
                     }
-                    P = __fmaf_rn(-Bz, zz, __fmaf_rn(-Ay, yy, __fmaf_rn(-Ax, xx, p0)));
-                    Q = __fmaf_rn(-Cz, zz, __fmaf_rn(-By, yy, __fmaf_rn(-Bx, xx, q0)));
-                } else {
-                    const float *S = sp + OFF_S + o;
-                    float px, py, pz, qx, qy, qz;
-                    if (MODE == GEO_MODE_FAST) {
-                        const float Ax = m0 * g.dtx, Ay = m0 * g.dty, Bz = m1 * g.dtz;
-                        const float Bx = m1 * g.dtx, By = m1 * g.dty, Cz = m2 * g.dtz;
-                        px = __fmaf_rn(-(ax1 * Ax), xx, ax2 * S[0]);
-                        py = __fmaf_rn(-(ay1 * Ay), yy, ay2 * S[kOB]);
-                        pz = __fmaf_rn(-(az1 * Bz), zz, az2 * S[2 * kOB]);
-                        qx = __fmaf_rn(-(ax1 * Bx), xx, ax2 * S[3 * kOB]);
-                        qy = __fmaf_rn(-(ay1 * By), yy, ay2 * S[4 * kOB]);
-                        qz = __fmaf_rn(-(az1 * Cz), zz, az2 * S[5 * kOB]);
-                    } else {
-                        // m = vp, 1+2eps, sqrtf(1+2del); the reference's chain
-                        const float vp = m0, e2 = m1, d2 = m2;
-                        px = ax2 * S[0] - ax1 * vp * vp * e2 * g.dtx * xx;
-                        py = ay2 * S[kOB] - ay1 * vp * vp * e2 * g.dty * yy;
-                        pz = az2 * S[2 * kOB] - az1 * vp * vp * d2 * g.dtz * zz;
-                        qx = ax2 * S[3 * kOB] - ax1 * vp * vp * d2 * g.dtx * xx;
-                        qy = ay2 * S[4 * kOB] - ay1 * vp * vp * d2 * g.dty * yy;
-                        qz = az2 * S[5 * kOB] - az1 * vp * vp * g.dtz * zz;
+                st.rec[(long)st.it * st.nrx * st.nry + rec_x + (long)st.nrx * (rr / st.dry)] = st.rec_pq ? a + b : a;
+            }
+        }
+        // RTM imaging epilogue on the physical box
+        // (cal_illumination / cal_migration, 3D RTM program :508-537)
+        if (RTM && im) {
+#pragma unroll
+            for (int j = 0; j < kW; j++) {
+                if (st.ill) ill.v[j] = ill.v[j] + (P.v[j] * P.v[j] + Q.v[j] * Q.v[j]);
+                if (st.mig) mig.v[j] = mig.v[j] + oth.v[j] * P.v[j];
+            }
+            if (imv) {
+                if (st.ill) st_v(st.ill + io, ill);
+                if (st.mig) st_v(st.mig + io, mig);
+            } else {
+#pragma unroll
+                for (int j = 0; j < kW; j++)
+                    if (im >> j & 1u) {
+                        if (st.ill) st.ill[io + j] = ill.v[j];
+                        if (st.mig) st.mig[io + j] = mig.v[j];
                     }
-                    if (upd) {
-                        g.px[id] = px; g.py[id] = py; g.pz[id] = pz;
-                        g.qx[id] = qx; g.qy[id] = qy; g.qz[id] = qz;
-                    }
-                    P = px + py + pz;
-                    Q = qx + qy + qz;
-                }
-                if (!upd) continue;
-                g.P1[id] = P;
-                g.Q1[id] = Q;
-                const int rix = cb ? rec_b : rec_a;
-                if (rix >= 0) {
-                    const int rr = y - g.npd - st.ry0;
-                    if (rr >= 0 && rr % st.dry == 0 && rr / st.dry < st.nry)
-                        st.rec[(long)st.it * st.nrx * st.nry + rix + (long)st.nrx * (rr / st.dry)] = st.rec_pq ? P + Q : P;
-                }
-                // RTM imaging epilogue on the physical box
-                // (cal_illumination / cal_migration, 3D RTM program :508-537)
-                if ((st.ill || st.mig) && (cb ? in_b : in_a) && y_in) {
-                    const long o = (long)(zo - g.npd) + (long)g.nz * ((xa + cb - g.npd) + (long)g.nx * (y - g.npd));
-                    if (st.ill) st.ill[o] = pre_ill[cb] + (P * P + Q * Q);
-                    if (st.mig) st.mig[o] = pre_mig[cb] + pre_oth[cb] * P;
-                }
             }
         }
     }
 }
+
+}  // namespace
 
 // ------------------------------------------------------------------ host
 static PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
@@ -498,23 +624,20 @@ int encode_map(CUtensorMap *map, const float *base, int nnz, int ldz, int nnx, i
 }
 
 int launch_fused3d(const StepMaps &maps, const Fused3D &g, int mode, const StepArgs3D &args, cudaStream_t s) {
-    static bool attr_set[2] = {false, false};
+    static bool attr_set[2][2];
     StepArgs3D st = args;
-    st.src = st.izs + (long)g.ldz * (st.ixs + (long)g.nnx * st.iys);
-    dim3 block(kTZ, kWarps), grid(g.nitems);
-    if (mode == GEO_MODE_FAST) {
-        if (!attr_set[0]) {
-            GEO_CUDA(cudaFuncSetAttribute(k_fused3d<GEO_MODE_FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFusedSmem));
-            attr_set[0] = true;
-        }
-        k_fused3d<GEO_MODE_FAST><<<grid, block, kFusedSmem, s>>>(maps, g, st);
-    } else {
-        if (!attr_set[1]) {
-            GEO_CUDA(cudaFuncSetAttribute(k_fused3d<GEO_MODE_EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFusedSmem));
-            attr_set[1] = true;
-        }
-        k_fused3d<GEO_MODE_EXACT><<<grid, block, kFusedSmem, s>>>(maps, g, st);
+    const bool rtm = st.ill || st.mig, fast = mode == GEO_MODE_FAST;
+    // 16-byte image accesses need aligned rows whose first depth sits on a vector
+    st.img_vec = g.npd % kW == 0 && g.nz % kW == 0 &&
+                 ((reinterpret_cast<uintptr_t>(st.ill) | reinterpret_cast<uintptr_t>(st.mig)) & (4 * kW - 1)) == 0;
+    const void *fn = fast ? (rtm ? (const void *)k_fused3d<GEO_MODE_FAST, true> : (const void *)k_fused3d<GEO_MODE_FAST, false>)
+                          : (rtm ? (const void *)k_fused3d<GEO_MODE_EXACT, true> : (const void *)k_fused3d<GEO_MODE_EXACT, false>);
+    if (!attr_set[fast][rtm]) {
+        GEO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFusedSmem));
+        attr_set[fast][rtm] = true;
     }
+    void *a[] = {(void *)&maps, (void *)&g, (void *)&st};
+    GEO_CUDA(cudaLaunchKernel(fn, dim3(g.nitems), dim3(kFusedThreads), a, kFusedSmem, s));
     return check_launch("fused3d");
 }
 

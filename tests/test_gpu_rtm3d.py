@@ -105,3 +105,28 @@ def test_rtm3d_receiver_grid(geo, orc, method):
         mig_o, _, _ = orc.rtm3d(v, e, d, snap_every=4, theta=th, phi=ph, **kw)
         mig = geo.rtm3d(v, e, d, mode="fast", method=method, snap_every=4, laplace=False, theta=th, phi=ph, **kw)
         assert np.array_equal(mig, mig_o), rel_l2(mig, mig_o)
+
+
+# vectors of two depths against the physical box: sponge widths and depth
+# counts of either parity (16-byte, 8-byte and scalar image accesses, vectors
+# that straddle the box edge), extents at the edges of the 32 x 16 tiles,
+# one chunk of planes and many
+@pytest.mark.parametrize("nx,ny,nz,npd,chunks", [(16, 9, 16, 8, "1"), (17, 10, 15, 9, "3"), (7, 21, 46, 7, "9"),
+                                                 (30, 8, 17, 10, "2"), (15, 12, 22, 5, "4")])
+def test_fused_step_vectors_and_tile_edges(geo, orc, monkeypatch, nx, ny, nz, npd, chunks):
+    monkeypatch.setenv("GEO_FD3D_CHUNKS", chunks)
+    v, e, d = random_model_3d(nx, ny, nz, seed=nx + nz)
+    kw = dict(KW, npd=npd, nt=90, fsx=nx // 2, fsy=ny // 2, fsz=nz // 2, dsx=1)
+    for mode in (0, 1):
+        mig_o, ill_o, _ = orc.rtm3d(v, e, d, mode=mode, **kw)
+        mig, ill = geo.rtm3d(v, e, d, mode=mode, laplace=False, illum=True, **kw)
+        assert np.abs(ill_o).max() > 0
+        assert np.array_equal(ill, ill_o) and np.array_equal(mig, mig_o), mode
+        fk = {k: kw[k] for k in ("npd", "nt", "dx", "dy", "dz", "dt", "favg", "pfac", "fsx", "fsy", "fsz")}
+        ref, P, Q = orc.fd3d(v, e, d, mode=mode, final=True, **fk)
+        plan = geo.FD3DPlan(nx=nx, ny=ny, nz=nz, mode=mode, **fk)
+        plan.set_model(v, e, d)
+        assert np.array_equal(plan.run_shot(0), ref)
+        a, b = plan.fields()
+        plan.close()
+        assert np.array_equal(a, P) and np.array_equal(b, Q)
