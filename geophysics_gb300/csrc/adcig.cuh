@@ -15,9 +15,14 @@
 // division, each within half an ulp), so when the float value lies farther
 // than 1e-6*(|a|+|t|) from the thresholds t on either side of it and farther
 // than 2e-6 from +-1, it gives the same decisions as the rounded double
-// quotient.  Otherwise -- and for a denominator outside [1e-30, 1e30], where
-// the float product could lose precision -- the double quotient is formed as
-// the programs form it.  Only a few points in a million take that path.
+// quotient.  A denominator below 1e-30, where the float product could lose
+// precision, is first scaled together with the dividend by 2^64, which is
+// exact (a dividend that overflows belongs to a quotient far above one, and
+// 0/0 is NaN either way).  Otherwise -- and above 1e30 -- the double quotient
+// is formed as the programs form it.  Only a few points in a million take
+// that path; when every point of a quiet wavefield took it (its denominators
+// are tiny or zero), the FP64 divisions took a third of a backward step
+// (1700x601 + 50, 70 angles: 82 us with them, 56 without).
 #pragma once
 
 namespace geo {
@@ -42,8 +47,9 @@ __device__ __forceinline__ bool angle_near(float a, float t) {
 // Bin of the pair (S.G, |S|^2, |G|^2), or -1 when the program adds nothing.
 __device__ __forceinline__ int poynting_bin(float dot, float b1, float b2, const float *thr, int na) {
     const float den = sqrtf(b1 * b2);
-    if (den >= 1e-30f && den <= 1e30f) {
-        const float a = dot / (den * 0.9f);
+    if (den <= 1e30f) {
+        const float up = den < 1e-30f ? 0x1p64f : 1.0f;
+        const float a = (dot * up) / (den * up * 0.9f);
         const float m = fabsf(a);
         if (!(m <= 1.0f + 2e-6f)) return -1;          // out of range (also inf, NaN)
         if (m < 1.0f - 2e-6f) {
