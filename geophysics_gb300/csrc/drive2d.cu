@@ -1,12 +1,15 @@
-// 2D drivers: single-shot forward modelling (half-step, persistent and
-// tile-resident kernels of fd2d.cu) and batched RTM (fused steps of
+// 2D drivers: single-shot forward modelling (fused steps of step2d.cu; the
+// MPI form the half-steps of fd2d.cu) and batched RTM (fused steps of
 // march2d.cu over every shot, the time loops captured once into CUDA graphs
 // and replayed).
 #include "geo_internal.h"
 #include "model2d.cuh"
 #include "march2d.cuh"
+#include "step2d.cuh"
 #include <algorithm>
 #include <cmath>
+#include <cstdio>
+#include <cstdlib>
 #include <cstring>
 
 namespace geo {
@@ -131,7 +134,7 @@ void ShotSet::tables(int k, float dx, float dz, float dt, int ldz, Off &o) {
     o.td2 = small.put(td2);
 }
 
-// One shot on the device for the single-shot kernels.
+// One shot of the MPI form on the device for the half-steps of fd2d.cu.
 struct SingleShot {
     ShotSet X;
     Shot2D S{};
@@ -150,26 +153,21 @@ int SingleShot::build(const Raw2D &raw, float dx, float dz, float dt, const std:
     // once, in the same order and precision (ModelJob::kz), and the kernel
     // issues one double multiply and one double subtraction per chain.  The
     // program's pow runs on the host, once per model point.
-    const bool mpi = X.var == V_MPI;
     const double ddtx = (double)(dt / dx), ddtz = (double)(dt / dz);
     DevBuf d_pw;
-    if (mpi) GEO_TRY(upload_pow_half(raw, d_pw, s));
+    GEO_TRY(upload_pow_half(raw, d_pw, s));
     ShotSet::Off o;
     X.tables(0, dx, dz, dt, nnz, o);
-    size_t o_tkz = 0, o_tkx = 0;
-    if (mpi && X.taper) {
-        std::vector<double> tkz(kTB * kTB, 0.0), tkx(kTB * kTB, 0.0);
-        for (int b = 0; b < kTB * kTB; b++) {
-            const int ix = o.box.x0 + b / kTB, iz = o.box.z0 + b % kTB;
-            if (ix < 0 || ix >= nnx || iz < 0 || iz >= nnz) continue;
-            const double pw = std::pow((double)(1 + 2 * o.box.d[b]), 0.5);
-            const float vpk = 1.0f * (o.vbox[b] * o.vbox[b]);
-            tkz[b] = (double)(o.p[6][iz] * vpk) * pw * ddtz;
-            tkx[b] = (double)(o.p[2][ix] * vpk) * pw * ddtx;
-        }
-        o_tkz = X.small.put(tkz);
-        o_tkx = X.small.put(tkx);
+    std::vector<double> tkz(kTB * kTB, 0.0), tkx(kTB * kTB, 0.0);
+    for (int b = 0; b < kTB * kTB; b++) {
+        const int ix = o.box.x0 + b / kTB, iz = o.box.z0 + b % kTB;
+        if (ix < 0 || ix >= nnx || iz < 0 || iz >= nnz) continue;
+        const double pw = std::pow((double)(1 + 2 * o.box.d[b]), 0.5);
+        const float vpk = 1.0f * (o.vbox[b] * o.vbox[b]);
+        tkz[b] = (double)(o.p[6][iz] * vpk) * pw * ddtz;
+        tkx[b] = (double)(o.p[2][ix] * vpk) * pw * ddtx;
     }
+    const size_t o_tkz = X.small.put(tkz), o_tkx = X.small.put(tkx);
     o_amp = X.small.put(amp);
     o_on = X.small.put(on);
     GEO_TRY(X.small.upload(s));
@@ -183,12 +181,8 @@ int SingleShot::build(const Raw2D &raw, float dx, float dz, float dt, const std:
         clear = X.mem.off;
         j.vp = X.mem.take<float>(n);
         j.e2 = X.mem.take<float>(n);
-        if (mpi) {
-            j.kz = X.mem.take<double>(n);
-            j.kx = X.mem.take<double>(n);
-        } else {
-            j.d2 = X.mem.take<float>(n);
-        }
+        j.kz = X.mem.take<double>(n);
+        j.kx = X.mem.take<double>(n);
         if (pass == 0) GEO_TRY(X.mem.alloc());
     }
     S.nnx = nnx; S.nnz = nnz; S.npd = npd; S.nx = nx; S.nz = nz;
@@ -197,28 +191,83 @@ int SingleShot::build(const Raw2D &raw, float dx, float dz, float dt, const std:
     S.cx1 = xp; S.cx2 = xp + nnx; S.ax1 = xp + 2 * nnx; S.ax2 = xp + 3 * nnx;
     S.cz1 = zp; S.cz2 = zp + nnz; S.az1 = zp + 2 * nnz; S.az2 = zp + 3 * nnz;
     X.source(0, S.ixs, S.izs);
-    S.tx0 = S.tz0 = -100000;
-    if (X.taper) {
-        S.tx0 = o.box.x0;
-        S.tz0 = o.box.z0;
-        S.te2 = X.small.at<float>(o.te2);
-        S.td2 = X.small.at<float>(o.td2);
-        if (mpi) {
-            S.tkz = X.small.at<double>(o_tkz);
-            S.tkx = X.small.at<double>(o_tkx);
-        }
-    }
-    S.rec_iz = npd;
-    S.rec_scale = 1.0f;
+    S.tx0 = o.box.x0;
+    S.tz0 = o.box.z0;
+    S.te2 = X.small.at<float>(o.te2);
+    S.tkz = X.small.at<double>(o_tkz);
+    S.tkx = X.small.at<double>(o_tkx);
     j.nx = nx; j.nz = nz; j.npd = npd; j.ldz = nnz;
-    j.vp2 = mpi;   // vp <- rho*vp^2 with rho == 1 (Toa_rtm_vti_adcig_cdp.c:641)
+    j.vp2 = 1;   // vp <- rho*vp^2 with rho == 1 (Toa_rtm_vti_adcig_cdp.c:641)
     j.pw = d_pw.as<double>();
     j.ax1 = S.ax1; j.az1 = S.az1;
     j.ddtx = ddtx; j.ddtz = ddtz;
-    S.vp = j.vp; S.e2 = j.e2; S.d2 = j.d2; S.kz = j.kz; S.kx = j.kx;
+    S.vp = j.vp; S.e2 = j.e2; S.kz = j.kz; S.kx = j.kx;
     GEO_TRY(launch_model2d(raw, {j}, s));
     GEO_CUDA(cudaMemsetAsync(X.mem.buf.p, 0, clear, s));
     return GEO_OK;
+}
+
+// One shot of the CPU or GPU form on the device for the fused steps of
+// step2d.cu.
+struct FusedShot {
+    ShotSet X;
+    SStep st{};
+    Fused2D plan;
+    size_t n = 0;                 // floats of an array
+    int build(const Raw2D &raw, float dx, float dz, float dt, const std::vector<float> &amp,
+              const std::vector<uint8_t> &on, int nt, cudaStream_t s);
+    const float *P() const { return st.f[0].P[st.lev]; }
+};
+
+int FusedShot::build(const Raw2D &raw, float dx, float dz, float dt, const std::vector<float> &amp,
+                     const std::vector<uint8_t> &on, int nt, cudaStream_t s) {
+    const int nx = X.G[0].nx, nz = X.nz, npd = X.npd, nnx = nx + 2 * npd, nnz = X.nnz, ldz = (nnz + 3) / 4 * 4;
+    ShotSet::Off o;
+    X.tables(0, dx, dz, dt, ldz, o);
+    const size_t o_amp = X.small.put(amp), o_on = X.small.put(on);
+    GEO_TRY(X.small.upload(s));
+    n = (size_t)nnx * ldz;
+    float *f = nullptr, *model = nullptr;
+    unsigned *sync = nullptr;
+    size_t clear = 0;
+    for (int pass = 0; pass < 2; pass++) {   // sizes, then addresses
+        f = X.mem.take<float>(12 * n);
+        st.rec = X.mem.take<float>((size_t)nt * nx);
+        sync = X.mem.take<unsigned>(2);
+        clear = X.mem.off;
+        model = X.mem.take<float>(3 * n);
+        if (pass == 0) GEO_TRY(X.mem.alloc());
+    }
+    SGrid &g = st.g;
+    g.nnx = nnx; g.nnz = nnz; g.ldz = ldz; g.npd = npd; g.nx = nx; g.nz = nz;
+    g.dtx = dt / dx; g.dtz = dt / dz;
+    const float *xp = X.small.at<float>(o.xprof);
+    g.cx1 = xp; g.cx2 = xp + nnx; g.ax1 = xp + 2 * nnx; g.ax2 = xp + 3 * nnx;
+    g.zp = X.small.at<float>(o.zprof);
+    step2d_fields(f, n, st.f[0]);
+    X.source(0, st.ixs, st.izs);
+    st.amp = X.small.at<float>(o_amp);
+    st.on = X.small.at<unsigned char>(o_on);
+    st.bar = sync;
+    st.err = reinterpret_cast<int *>(sync) + 1;
+    ModelJob j{};
+    j.nx = nx; j.nz = nz; j.npd = npd; j.ldz = ldz;
+    j.vp = model; j.e2 = model + n; j.d2 = model + 2 * n;
+    GEO_TRY(launch_model2d(raw, {j}, s));
+    if (X.taper)
+        GEO_TRY(launch_box2d(j.e2, j.d2, nnx, ldz, o.box.x0, o.box.z0, kTB, X.small.at<float>(o.te2),
+                             X.small.at<float>(o.td2), s));
+    GEO_CUDA(cudaMemsetAsync(X.mem.buf.p, 0, clear, s));
+    // GEO_FD2D_TILE=TZxTX: tiles of 16 columns from TX 16, of 8 below; a shape
+    // no block could hold with its whole state is refused as it always was
+    int tz = 0, tx = 0;
+    if (const char *e = getenv("GEO_FD2D_TILE"))
+        if (sscanf(e, "%dx%d", &tz, &tx) != 2 || tx < 4 || tx > 128) tx = 0;
+    GEO_TRY(plan.plan(X.var == V_CPU ? SK_CPU : SK_GPU, g, !tx ? 0 : tx < 16 ? 8 : 16));
+    if (tx && tz >= 32 && tz <= 256 && !(tz & (tz - 1)) && plan.stages == 1 && 11L * tx * tz + 21L * (tx + tz) > 56320)
+        return fail(GEO_ERR_ARG, "GEO_FD2D_TILE %dx%d: tile too large", tz, tx);
+    GEO_TRY(plan.maps(g, st.f[0], 0));
+    return plan.model(g, model);
 }
 
 // The shots of a batched RTM on the device for the fused steps.
@@ -367,7 +416,7 @@ struct Batch2D {
     std::vector<Shot2D> S;
     std::vector<int> items;
     DevBuf d_S, d_items;
-    int by = 8, grid = 1, variant = V_CPU;
+    int by = 8, grid = 1;
     int upload(int by_, int blocks_per_sm, cudaStream_t s) {
         by = by_;
         build_items(S, by, items);
@@ -381,10 +430,10 @@ struct Batch2D {
         return GEO_OK;
     }
     int vel(Step2D st, cudaStream_t s) {
-        return launch_vel2d(variant, d_S.as<Shot2D>(), d_items.as<int>(), (int)items.size(), by, grid, st, s);
+        return launch_vel2d(V_MPI, d_S.as<Shot2D>(), d_items.as<int>(), (int)items.size(), by, grid, st, s);
     }
     int stress(Step2D st, cudaStream_t s) {
-        return launch_stress2d(variant, d_S.as<Shot2D>(), d_items.as<int>(), (int)items.size(), by, grid, st, s);
+        return launch_stress2d(V_MPI, d_S.as<Shot2D>(), d_items.as<int>(), (int)items.size(), by, grid, st, s);
     }
 };
 
@@ -465,7 +514,8 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
     GEO_TRY(raw.open(D.nx, D.nz, v, e, d, nullptr, mem, ss.cs));
     const bool taper = var == V_MPI || D.sv;
     SingleShot shot1;
-    ShotSet &X = shot1.X;
+    FusedShot fused;
+    ShotSet &X = var == V_MPI ? shot1.X : fused.X;
     X.var = var;
     X.nz = D.nz; X.npd = D.npd; X.nnz = nnz;
     X.taper = taper;
@@ -482,75 +532,55 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
     std::vector<float> amp;
     std::vector<uint8_t> on;
     source_amplitudes(var, D.nt, D.dt, D.favg, D.pfac, D.wtype, amp, on);
-    GEO_TRY(shot1.build(raw, D.dx, D.dz, D.dt, amp, on, D.nt, ss.cs));
-    const float *d_amp = X.small.at<float>(shot1.o_amp);
-    const unsigned char *d_on = X.small.at<unsigned char>(shot1.o_on);
-    Batch2D B;
-    B.variant = var;
-    B.S = {shot1.S};
-    B.S[0].rec_iz = D.rec_iz;
-    B.S[0].rec_scale = D.rec_scale;
-    const bool persistent = !(snap && snap_every > 0);
-    auto step = [&](int it) -> int {
-        Step2D st{};
-        st.it = it;
-        st.amp = amp[it];
-        st.src_on = on[it];
-        st.taper = taper ? 1 : 0;
-        GEO_TRY(B.vel(st, ss.cs));
-        return B.stress(st, ss.cs);
-    };
-    DevBuf d_sync;
-    GEO_TRY(d_sync.alloc(8));
-    GEO_TRY(d_sync.zero(ss.cs));
-    unsigned *bar = d_sync.as<unsigned>();
-    int *errw = d_sync.as<int>() + 1;
     const size_t nn = (size_t)nnx * nnz;
+    const bool snaps = snap && snap_every > 0;
+    const cudaMemcpyKind ksnap = mem == GEO_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
     Watchdog wd;
     GEO_TRY(wd.open());
-    const cudaMemcpyKind ksnap = mem == GEO_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    // CPU and GPU forms: every block keeps its tile of the fields in shared
-    // memory for the run (launch_fd2d_tile), one launch per run of steps
-    // between snapshots, when the grid fits on the device that way
-    bool tiled = false;
-    if (var == V_CPU || var == V_GPU) {
-        DevBuf xch;
-        GEO_TRY(xch.alloc(8 * nn * 4));
-        GEO_TRY(xch.zero(ss.cs));
-        for (int it0 = 0; it0 < D.nt;) {
-            int it1 = it0 + 1;
-            if (snap && snap_every > 0)
-                while (it1 < D.nt && (it1 - 1) % snap_every != 0) it1++;
-            else
-                it1 = D.nt;
-            bool fits = false;
-            GEO_TRY(launch_fd2d_tile(var, B.S[0], xch.as<float>(), d_amp, d_on, taper ? 1 : 0, it0, it1, bar, errw, &fits, ss.cs));
-            if (!fits) {   // decided by the grid alone, so on the first run of steps
-                if (tiled) return fail(GEO_ERR_CUDA, "2D shot: tile-resident launch refused mid-run");
-                break;
-            }
-            tiled = true;
-            const int it = it1 - 1;
-            if (snap && snap_every > 0 && it % snap_every == 0)
-                GEO_CUDA(cudaMemcpyAsync(snap + (size_t)(it / snap_every) * nn, B.S[0].P, nn * 4, ksnap, ss.cs));
+    DevBuf d_sync;
+    Batch2D B;
+    float *rec = nullptr;
+    int *errw = nullptr;
+    if (var != V_MPI) {
+        GEO_TRY(fused.build(raw, D.dx, D.dz, D.dt, amp, on, D.nt, ss.cs));
+        SStep &st = fused.st;
+        rec = st.rec;
+        errw = st.err;
+        st.rec_iz = D.rec_iz;
+        st.rec_scale = D.rec_scale;
+        // one launch per run of steps between snapshots
+        for (st.it0 = 0; st.it0 < D.nt; st.it0 = st.it1) {
+            st.it1 = snaps ? st.it0 + 1 : D.nt;
+            while (st.it1 < D.nt && (st.it1 - 1) % snap_every != 0) st.it1++;
+            GEO_TRY(fused.plan.run(st, ss.cs));
+            st.lev = (st.lev + st.it1 - st.it0) & 1;
+            const int it = st.it1 - 1;
+            if (snaps && it % snap_every == 0)
+                GEO_CUDA(cudaMemcpy2DAsync(snap + (size_t)(it / snap_every) * nn, (size_t)nnz * 4, fused.P(),
+                                           (size_t)st.g.ldz * 4, (size_t)nnz * 4, nnx, ksnap, ss.cs));
             if (wd.every > 0) {
-                GEO_TRY(wd.scan(B.S[0].P, nn, it + 1, ss.cs));
+                GEO_TRY(wd.scan(fused.P(), fused.n, it + 1, ss.cs));
                 if (wd.tripped()) break;
             }
-            it0 = it1;
         }
-        if (tiled) {
-            int err = 0;
-            GEO_CUDA(cudaMemcpyAsync(&err, errw, 4, cudaMemcpyDeviceToHost, ss.cs));
-            GEO_CUDA(cudaStreamSynchronize(ss.cs));
-            if (err) return fail(GEO_ERR_CUDA, "2D shot: a grid barrier wait timed out");
-            if (wd.every > 0) GEO_TRY(wd.scan(B.S[0].rec_p, (size_t)D.nx * D.nt, D.nt, ss.cs));
-        }
-    }
-    if (!tiled) GEO_TRY(B.upload(persistent ? 16 : 8, 8, ss.cs));
-    if (!tiled && snap && snap_every > 0) {
-        for (int it = 0; it < D.nt; it++) {
-            GEO_TRY(step(it));
+    } else {
+        GEO_TRY(shot1.build(raw, D.dx, D.dz, D.dt, amp, on, D.nt, ss.cs));
+        GEO_TRY(d_sync.alloc(8));
+        GEO_TRY(d_sync.zero(ss.cs));
+        errw = d_sync.as<int>() + 1;
+        B.S = {shot1.S};
+        B.S[0].rec_iz = D.rec_iz;
+        B.S[0].rec_scale = D.rec_scale;
+        rec = B.S[0].rec_p;
+        GEO_TRY(B.upload(snaps ? 8 : 16, 8, ss.cs));
+        for (int it = 0; snaps && it < D.nt; it++) {
+            Step2D st{};
+            st.it = it;
+            st.amp = amp[it];
+            st.src_on = on[it];
+            st.taper = 1;
+            GEO_TRY(B.vel(st, ss.cs));
+            GEO_TRY(B.stress(st, ss.cs));
             if (it % snap_every == 0)
                 GEO_CUDA(cudaMemcpyAsync(snap + (size_t)(it / snap_every) * nn, B.S[0].P, nn * 4, ksnap, ss.cs));
             if (wd.every > 0 && ((it + 1) % wd.every == 0 || it == D.nt - 1)) {
@@ -558,26 +588,27 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
                 if (wd.tripped()) break;
             }
         }
-    } else if (!tiled) {
-        // the whole shot in one cooperative launch (grid barriers between the
-        // half-steps, bounded waits reported through an error word)
-        Persist2D a{};
-        a.nt = D.nt;
-        a.taper = taper ? 1 : 0;
-        a.amp = d_amp;
-        a.on = d_on;
-        a.bar = bar;
-        a.err = errw;
-        GEO_TRY(launch_fd2d_shot(var, B.d_S.as<Shot2D>(), B.d_items.as<int>(), (int)B.items.size(), B.by, a, ss.cs));
-        int err = 0;
-        GEO_CUDA(cudaMemcpyAsync(&err, a.err, 4, cudaMemcpyDeviceToHost, ss.cs));
-        GEO_CUDA(cudaStreamSynchronize(ss.cs));
-        if (err) return fail(GEO_ERR_CUDA, "2D shot: a grid barrier wait timed out");
-        // the shot ran in one launch: scan its final P and its record
-        if (wd.every > 0) {
-            GEO_TRY(wd.scan(B.S[0].P, nn, D.nt, ss.cs));
-            GEO_TRY(wd.scan(B.S[0].rec_p, (size_t)D.nx * D.nt, D.nt, ss.cs));
+        if (!snaps) {
+            // the whole shot in one cooperative launch (grid barriers between
+            // the half-steps, bounded waits reported through an error word)
+            Persist2D a{};
+            a.nt = D.nt;
+            a.taper = 1;
+            a.amp = X.small.at<float>(shot1.o_amp);
+            a.on = X.small.at<unsigned char>(shot1.o_on);
+            a.bar = d_sync.as<unsigned>();
+            a.err = errw;
+            GEO_TRY(launch_fd2d_shot(B.d_S.as<Shot2D>(), B.d_items.as<int>(), (int)B.items.size(), B.by, a, ss.cs));
         }
+    }
+    int err = 0;
+    GEO_CUDA(cudaMemcpyAsync(&err, errw, 4, cudaMemcpyDeviceToHost, ss.cs));
+    GEO_CUDA(cudaStreamSynchronize(ss.cs));
+    if (err) return fail(GEO_ERR_CUDA, "2D shot: a device-side wait timed out");
+    // what a launch left unscanned
+    if (wd.every > 0 && (var != V_MPI || !snaps)) {
+        if (var == V_MPI) GEO_TRY(wd.scan(B.S[0].P, nn, D.nt, ss.cs));
+        GEO_TRY(wd.scan(rec, (size_t)D.nx * D.nt, D.nt, ss.cs));
     }
     GEO_TRY(wd.verdict(ss.cs, "2D shot"));
     DevBuf mlo, mhi, out;
@@ -592,14 +623,14 @@ extern "C" int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const fl
         GEO_TRY(mhi.alloc(hi.size() * 4));
         GEO_CUDA(cudaMemcpyAsync(mlo.p, lo.data(), lo.size() * 4, cudaMemcpyHostToDevice, ss.cs));
         GEO_CUDA(cudaMemcpyAsync(mhi.p, hi.data(), hi.size() * 4, cudaMemcpyHostToDevice, ss.cs));
-        GEO_TRY(launch_mute_records(B.S[0].rec_p, D.nx, D.nt, mlo.as<int>(), mhi.as<int>(), ss.cs));
+        GEO_TRY(launch_mute_records(rec, D.nx, D.nt, mlo.as<int>(), mhi.as<int>(), ss.cs));
     }
     const size_t rbytes = (size_t)D.nx * D.nt * 4;
     if (mem == GEO_MEM_DEVICE) {
-        GEO_TRY(launch_transpose_records(B.S[0].rec_p, shot, D.nx, D.nt, ss.cs));
+        GEO_TRY(launch_transpose_records(rec, shot, D.nx, D.nt, ss.cs));
     } else {
         GEO_TRY(out.alloc(rbytes));
-        GEO_TRY(launch_transpose_records(B.S[0].rec_p, out.as<float>(), D.nx, D.nt, ss.cs));
+        GEO_TRY(launch_transpose_records(rec, out.as<float>(), D.nx, D.nt, ss.cs));
         GEO_CUDA(cudaMemcpyAsync(shot, out.p, rbytes, cudaMemcpyDeviceToHost, ss.cs));
     }
     GEO_CUDA(cudaStreamSynchronize(ss.cs));

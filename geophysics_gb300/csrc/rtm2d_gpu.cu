@@ -19,8 +19,8 @@
 // adcigs_illum :768), the adjoint Laplacian of the image and of the angle
 // stack (stk_adcigs :799).  The image kernels of the program run over
 // nnx*nnz threads on nx*nz arrays (an overrun); here they cover nx*nz.
-// Fields are single buffers updated in place (the program's u0 = u1
-// pointer assignment).
+// The VTI program's steps are those of step2d.cu; the TTI program's below
+// update single buffers in place (its u0 = u1 pointer assignment).
 //
 // The 2D TTI GPU RTM program (2D-tti-fd+rtm-cuda/
 // Toa_gpu_2dtti_rtm_adcigs_iorderfunciton.cu, main :500-800) has the same
@@ -40,6 +40,7 @@
 #include "tti2d.cuh"
 #include "gridsync.cuh"
 #include "model2d.cuh"
+#include "step2d.cuh"
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -77,7 +78,7 @@ static TtiField tti_field(const GField &f) {
     return t;
 }
 
-// Everything one persistent launch of a pass needs.
+// Everything one persistent launch of a TTI program's pass needs.
 struct GCoop {
     GRtm g;
     TtiGrid tg;
@@ -96,61 +97,6 @@ struct GCoop {
     unsigned *bar;               // grid-barrier arrival counter, zeroed before the launch
     int *err;                    // set when a barrier wait gave up
 };
-
-// The VTI program's update_vel (Toa_gpu2DvtiFdRtmAdcigsLaplace.cu:256-289)
-// at one point; SRC folds the step's point source (add_source :204, P,Q +=
-// amp at the source cell before the update) into the taps that read it.
-template <bool SRC>
-__device__ __forceinline__ void g_vel_at(const GRtm &g, const GField &f, long id, int ix, int iz, long src, float amp) {
-    const long s = g.nnz;
-    float xx = 0.0f, zz = 0.0f;
-#pragma unroll
-    for (int im = 0; im < 4; im++) {
-        xx += c_grtm[im] * (tti_tap<true, SRC>(f.P, id + (im + 1) * s, src, amp) - tti_tap<true, SRC>(f.P, id - im * s, src, amp));
-        zz += c_grtm[im] * (tti_tap<true, SRC>(f.Q, id + im + 1, src, amp) - tti_tap<true, SRC>(f.Q, id - im, src, amp));
-    }
-    f.u[id] = g.cx2[ix] * __ldcg(f.u + id) - g.cx1[ix] * g.dtx * xx;
-    f.w[id] = g.cz2[iz] * __ldcg(f.w + id) - g.cz1[iz] * g.dtz * zz;
-}
-
-// The VTI program's update_stress (:303-404) at one point; returns P and Q.
-__device__ __forceinline__ float2 g_stress_at(const GRtm &g, const GField &f, const float *e2, const float *d2,
-                                              long id, int ix, int iz) {
-    const long s = g.nnz;
-    float xx = 0.0f, zz = 0.0f;
-#pragma unroll
-    for (int im = 0; im < 4; im++) {
-        xx += c_grtm[im] * (__ldcg(f.u + id + im * s) - __ldcg(f.u + id - (im + 1) * s));
-        zz += c_grtm[im] * (__ldcg(f.w + id + im) - __ldcg(f.w + id - im - 1));
-    }
-    const float vp = g.vp[id];
-    const float px = g.ax2[ix] * __ldcg(f.px + id) - g.ax1[ix] * vp * vp * e2[id] * g.dtx * xx;
-    const float pz = g.az2[iz] * __ldcg(f.pz + id) - g.az1[iz] * vp * vp * d2[id] * g.dtz * zz;
-    const float qx = g.ax2[ix] * __ldcg(f.qx + id) - g.ax1[ix] * vp * vp * d2[id] * g.dtx * xx;
-    const float qz = g.az2[iz] * __ldcg(f.qz + id) - g.az1[iz] * vp * vp * g.dtz * zz;
-    f.px[id] = px; f.pz[id] = pz; f.qx[id] = qx; f.qz[id] = qz;
-    const float P = px + pz, Q = qx + qz;
-    f.P[id] = P;
-    f.Q[id] = Q;
-    return make_float2(P, Q);
-}
-
-// One program's velocity / stress update: the TTI program's
-// (Toa_gpu_2dtti_rtm_adcigs_iorderfunciton.cu:126-228) over the tilt field,
-// or the VTI program's.
-template <bool TTI, bool SRC>
-__device__ __forceinline__ void vel_at(const GCoop &a, const GField &f, const TtiField &tf, long id, int ix, int iz,
-                                       float amp) {
-    if constexpr (TTI) tti_vel_at<true, SRC>(a.tg, tf, c_grtm, id, ix, iz, a.src, amp);
-    else g_vel_at<SRC>(a.g, f, id, ix, iz, a.src, amp);
-}
-
-template <bool TTI>
-__device__ __forceinline__ float2 stress_at(const GCoop &a, const GField &f, const TtiField &tf, long id, int ix,
-                                            int iz) {
-    if constexpr (TTI) return tti_stress_at<true>(a.tg, tf, a.e2, a.d2, c_grtm, id, ix, iz);
-    else return g_stress_at(a.g, f, a.e2, a.d2, id, ix, iz);
-}
 
 // Position of (ix, iz) in the ring of wavefield_bndr (:532): rows npml-1
 // (top) and npml+nz+1 (bottom) over the nx interior columns, then columns
@@ -179,11 +125,9 @@ __device__ __forceinline__ bool g_updated(const GRtm &g, int ix, int iz) {
 // illumination (cal_illumination :654: ill += P*P + Q*Q, <= 0 -> 1), a grid
 // barrier.  The ring covers cells outside the updated band too (their
 // unchanged values).
-template <bool TTI>
 // Four blocks per SM (64 registers): the passes are bound by the latency of
-// their L2 round trips and the gathers' scattered updates, and at 1700x601
-// that ran the TTI program 1.3x and the VTI program 1.1x faster than with
-// the two blocks its 128 registers allowed.
+// their L2 round trips and the gathers' scattered updates; at 1700x601 that
+// ran 1.3x faster than the two blocks that 128 registers allowed.
 __global__ void __launch_bounds__(256, 4) k_grtm_fwd(const GCoop a) {
     if (ld_acquire_u32(reinterpret_cast<const unsigned *>(a.err))) return;   // an earlier run gave up
     const GRtm &g = a.g;
@@ -197,8 +141,8 @@ __global__ void __launch_bounds__(256, 4) k_grtm_fwd(const GCoop a) {
             const int ix = (int)(id / g.nnz), iz = (int)(id % g.nnz);
             if (!g_updated(g, ix, iz)) continue;
             const bool near = on && ((iz == a.izs && abs(ix - a.ixs) <= 4) || (ix == a.ixs && abs(iz - a.izs) <= 4));
-            if (near) vel_at<TTI, true>(a, a.S, a.tS, id, ix, iz, amp);
-            else vel_at<TTI, false>(a, a.S, a.tS, id, ix, iz, 0.0f);
+            if (near) tti_vel_at<true, true>(a.tg, a.tS, c_grtm, id, ix, iz, a.src, amp);
+            else tti_vel_at<true, false>(a.tg, a.tS, c_grtm, id, ix, iz);
         }
         if (!grid_barrier(a.bar, ++k * gridDim.x, a.err)) return;
         for (long id = first; id < n; id += stride) {
@@ -212,7 +156,7 @@ __global__ void __launch_bounds__(256, 4) k_grtm_fwd(const GCoop a) {
                 }
                 continue;
             }
-            const float2 pq = stress_at<TTI>(a, a.S, a.tS, id, ix, iz);
+            const float2 pq = tti_stress_at<true>(a.tg, a.tS, a.e2, a.d2, c_grtm, id, ix, iz);
             if (gz == 0 && inner) a.rec[(long)it * g.nx + gx] = pq.x;
             if (r >= 0) {
                 a.bp[(long)it * a.L + r] = pq.x;
@@ -254,7 +198,6 @@ __device__ __forceinline__ void restore_inject(const GCoop &a, long id, int ix, 
 // and the Poynting gathers (:718-766), then the restore and injection of
 // the next step at the same point, a grid barrier.  A ring or surface cell
 // is read by no other point of the phase that writes it.
-template <bool TTI>
 __global__ void __launch_bounds__(256, 4) k_grtm_bwd(const GCoop a) {
     if (ld_acquire_u32(reinterpret_cast<const unsigned *>(a.err))) return;
     const GRtm &g = a.g;
@@ -267,15 +210,15 @@ __global__ void __launch_bounds__(256, 4) k_grtm_bwd(const GCoop a) {
         for (long id = first; id < n; id += stride) {
             const int ix = (int)(id / g.nnz), iz = (int)(id % g.nnz);
             if (!g_updated(g, ix, iz)) continue;
-            vel_at<TTI, false>(a, a.S, a.tS, id, ix, iz, 0.0f);
-            vel_at<TTI, false>(a, a.R, a.tR, id, ix, iz, 0.0f);
+            tti_vel_at<true>(a.tg, a.tS, c_grtm, id, ix, iz);
+            tti_vel_at<true>(a.tg, a.tR, c_grtm, id, ix, iz);
         }
         if (!grid_barrier(a.bar, ++k * gridDim.x, a.err)) return;
         for (long id = first; id < n; id += stride) {
             const int ix = (int)(id / g.nnz), iz = (int)(id % g.nnz);
             if (g_updated(g, ix, iz)) {
-                const float2 s = stress_at<TTI>(a, a.S, a.tS, id, ix, iz);
-                const float2 r = stress_at<TTI>(a, a.R, a.tR, id, ix, iz);
+                const float2 s = tti_stress_at<true>(a.tg, a.tS, a.e2, a.d2, c_grtm, id, ix, iz);
+                const float2 r = tti_stress_at<true>(a.tg, a.tR, a.e2, a.d2, c_grtm, id, ix, iz);
                 const int gx = ix - g.npml, gz = iz - g.npml;
                 if (gx >= 0 && gx < g.nx && gz >= 0 && gz < g.nz) {
                     const long o = (long)gx * g.nz + gz;
@@ -379,11 +322,12 @@ int adcig_angle_tables(int nangle, int dangle, float *thr, float *cs, cudaStream
 
 __device__ float g_angle_stage[2 * kMaxAngles];
 
-static int gpu_adcig_tables(int nangle, int dangle, cudaStream_t s) {
+static int gpu_adcig_tables(int nangle, int dangle, bool tti, cudaStream_t s) {
     void *stage = nullptr;
     GEO_CUDA(cudaGetSymbolAddress(&stage, g_angle_stage));
     float *st = static_cast<float *>(stage);
     GEO_TRY(adcig_angle_tables(nangle, dangle, st, st + kMaxAngles, s));
+    if (!tti) return load_step2d_angles(st, st + kMaxAngles, s);
     GEO_CUDA(cudaMemcpyToSymbolAsync(c_gthr, st, kMaxAngles * 4, 0, cudaMemcpyDeviceToDevice, s));
     GEO_CUDA(cudaMemcpyToSymbolAsync(c_gcos, st + kMaxAngles, kMaxAngles * 4, 0, cudaMemcpyDeviceToDevice, s));
     return GEO_OK;
@@ -426,7 +370,9 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
     if (dcdp != 1 && !prog.tti) return fail(GEO_ERR_ARG, "the VTI program forms gathers at every CDP (dcdp 0 or 1)");
     if (mem != GEO_MEM_HOST && mem != GEO_MEM_DEVICE) return fail(GEO_ERR_ARG, "bad mem kind");
     const int nx = D.nx, nz = D.nz, npml = D.npml, nt = D.nt, nnx = nx + 2 * npml, nnz = nz + 2 * npml;
-    const size_t n0 = (size_t)nx * nz, n = (size_t)nnx * nnz;
+    // columns of the fused step's arrays are of a pitch that TMA takes
+    const int ldz = prog.tti ? nnz : (nnz + 3) / 4 * 4, mid = (int)((size_t)nnx * nnz / 2 / nnz);
+    const size_t n0 = (size_t)nx * nz, n = (size_t)nnx * ldz;
     cudaStream_t s = (cudaStream_t)stream;
     Raw2D raw;
     GEO_TRY(raw.open(nx, nz, v, e, d, prog.tti ? theta : nullptr, mem, s));
@@ -439,7 +385,7 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
         return raw_at(a, raw, std::min(std::max(ix - npml, 0), nx - 1), std::min(std::max(iz - npml, 0), nz - 1));
     };
     std::vector<unsigned long long> pick;
-    pick.push_back(at(0, (int)(n / 2 / nnz), (int)(n / 2 % nnz)));
+    pick.push_back(at(0, mid, (int)((size_t)nnx * nnz / 2 % nnz)));
     pick.push_back(at(0, 0, 1));
     pick.push_back(at(1, 0, 1));
     for (int is = 1; is <= D.ns; is++) {
@@ -459,11 +405,11 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
     // get_d0 and initial_coffe of the program (VTI :110-118; TTI :230-233, :289-320)
     const Variant sp = prog.tti ? V_TTIRTM : V_GPU;
     const float d0 = sponge_d0(sp, 2, 0.0f, rs.val[0], npml, D.dx, D.dx, D.dz);
-    std::vector<float> prof(4 * (size_t)(nnx + nnz));
+    std::vector<float> prof(4 * (size_t)(nnx + ldz), 1.0f);
     float *q = prof.data();
     sponge_profiles(sp, nx, npml, D.dt, d0, q, q + nnx, q + 2 * nnx, q + 3 * nnx);
     q += 4 * nnx;
-    sponge_profiles(sp, nz, npml, D.dt, d0, q, q + nnz, q + 2 * nnz, q + 3 * nnz);
+    sponge_profiles(sp, nz, npml, D.dt, d0, q, q + ldz, q + 2 * ldz, q + 3 * ldz);
     std::vector<float> amp;
     std::vector<uint8_t> on;
     source_amplitudes(V_GPU, nt, D.dt, D.favg, D.pfac, D.wtype, amp, on);
@@ -499,14 +445,15 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
     // one allocation; the state a shot starts from is cleared together
     Arena ar;
     float *fS = nullptr, *fR = nullptr, *rec = nullptr, *ring = nullptr, *mig = nullptr, *ill = nullptr, *ag = nullptr;
-    float *dvp = nullptr, *de2 = nullptr, *dd2 = nullptr, *dte2 = nullptr, *dtd2 = nullptr, *dct = nullptr, *dsn = nullptr;
+    float *dvp = nullptr, *dtvp = nullptr, *dct = nullptr, *dsn = nullptr;
     float *lap = nullptr, *stk = nullptr, *trs = nullptr;
     int *mlo = nullptr;
     unsigned *sync = nullptr;
     size_t shot_end = 0, clear_end = 0;
+    const int nf = prog.tti ? 8 : 12;   // arrays of a side
     for (int pass = 0; pass < 2; pass++) {
-        fS = ar.take<float>(8 * n);
-        fR = ar.take<float>(8 * n);
+        fS = ar.take<float>(nf * n);
+        fR = ar.take<float>(nf * n);
         rec = ar.take<float>((size_t)nt * nx);
         ring = ar.take<float>((size_t)2 * nt * L);
         shot_end = ar.off;
@@ -515,11 +462,8 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
         if (gathers) ag = ar.take<float>(nag);
         sync = ar.take<unsigned>(2);
         clear_end = ar.off;
-        dvp = ar.take<float>(n);
-        de2 = ar.take<float>(n);
-        dd2 = ar.take<float>(n);
-        dte2 = ar.take<float>(n);
-        dtd2 = ar.take<float>(n);
+        dvp = ar.take<float>(3 * n);    // vp, 1+2eps, sqrtf(1+2del)
+        dtvp = ar.take<float>(3 * n);   // the shot's, with the SV taper
         if (prog.tti) {
             dct = ar.take<float>(n);
             dsn = ar.take<float>(n);
@@ -530,9 +474,10 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
         mlo = ar.take<int>(2 * (size_t)nx);
         if (pass == 0) GEO_TRY(ar.alloc());
     }
+    float *de2 = dvp + n, *dd2 = de2 + n, *dte2 = dtvp + n, *dtd2 = dte2 + n;
     GEO_CUDA(cudaMemsetAsync(ar.buf.p, 0, clear_end, s));
     ModelJob job{};
-    job.nx = nx; job.nz = nz; job.npd = npml; job.ldz = nnz;
+    job.nx = nx; job.nz = nz; job.npd = npml; job.ldz = ldz;
     job.vp = dvp; job.e2 = de2; job.d2 = dd2; job.rad = dct;
     GEO_TRY(launch_model2d(raw, {job}, s));
     if (prog.tti) {
@@ -545,7 +490,7 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
         GEO_CUDA(cudaStreamSynchronize(s));
         mu_v = rs.val[1] * (1 + (sqrtf(1 + 2 * rs.val[2]) - 1) * c1);
     }
-    if (gathers) GEO_TRY(gpu_adcig_tables(D.nangle, D.dangle, s));
+    if (gathers) GEO_TRY(gpu_adcig_tables(D.nangle, D.dangle, prog.tti, s));
     GRtm g{};
     g.nnx = nnx; g.nnz = nnz; g.nx = nx; g.nz = nz; g.npml = npml; g.nangle = D.nangle; g.dcdp = dcdp;
     g.ct = dct;
@@ -555,7 +500,7 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
     const float *pp = small.at<float>(o_prof);
     g.cx1 = pp; g.cx2 = pp + nnx; g.ax1 = pp + 2 * nnx; g.ax2 = pp + 3 * nnx;
     pp += 4 * nnx;
-    g.cz1 = pp; g.cz2 = pp + nnz; g.az1 = pp + 2 * nnz; g.az2 = pp + 3 * nnz;
+    g.cz1 = pp; g.cz2 = pp + ldz; g.az1 = pp + 2 * ldz; g.az2 = pp + 3 * ldz;
     g.vp = dvp;
     auto fields = [&](float *p) {
         GField f;
@@ -588,10 +533,9 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
     a.err = reinterpret_cast<int *>(sync) + 1;
     // every block resident at once (the grid barrier needs it; the
     // cooperative launch checks it), threads striding over the points
-    const void *kf = prog.tti ? (const void *)k_grtm_fwd<true> : (const void *)k_grtm_fwd<false>;
-    const void *kb = prog.tti ? (const void *)k_grtm_bwd<true> : (const void *)k_grtm_bwd<false>;
+    const void *kf = (const void *)k_grtm_fwd, *kb = (const void *)k_grtm_bwd;
     int grid_f = 0, grid_b = 0;
-    {
+    if (prog.tti) {
         int dev = 0, sms = 0, occ_f = 0, occ_b = 0, coop = 0;
         GEO_CUDA(cudaGetDevice(&dev));
         GEO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -612,13 +556,36 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
         GEO_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(256), args, 0, s));
         return check_launch("grtm_pass");
     };
+    // VTI program: fused steps (step2d.cu)
+    SStep st{};
+    Fused2D fwd, bwd;
+    if (!prog.tti) {
+        SGrid &q2 = st.g;
+        q2.nnx = nnx; q2.nnz = nnz; q2.ldz = ldz; q2.npd = npml; q2.nx = nx; q2.nz = nz;
+        q2.dtx = g.dtx; q2.dtz = g.dtz;
+        q2.cx1 = g.cx1; q2.cx2 = g.cx2; q2.ax1 = g.ax1; q2.ax2 = g.ax2; q2.zp = g.cz1;
+        step2d_fields(fS, n, st.f[0]);
+        step2d_fields(fR, n, st.f[1]);
+        GEO_TRY(fwd.plan(SK_GFWD, q2));
+        GEO_TRY(fwd.maps(q2, st.f[0], 0));
+        GEO_TRY(fwd.model(q2, dtvp));
+        GEO_TRY(bwd.plan(SK_GBWD, q2));
+        for (int f = 0; f < 2; f++) GEO_TRY(bwd.maps(q2, st.f[f], f));
+        GEO_TRY(bwd.model(q2, dvp));
+        st.izs = npml + D.zs - 1;
+        st.amp = a.amp; st.on = a.on;
+        st.bar = a.bar;
+        st.rec = rec;
+        st.bp = bp; st.bq = bq; st.ill = ill; st.mig = mig; st.adcig = ag;
+        st.L = L; st.nangle = D.nangle;
+        st.err = a.err;
+    }
     Watchdog wd;
     GEO_TRY(wd.open());
     for (int is = 1; is <= D.ns; is++) {
         // the shot's tapered model: the untapered one with its box replaced
-        GEO_CUDA(cudaMemcpyAsync(dte2, de2, n * 4, cudaMemcpyDeviceToDevice, s));
-        GEO_CUDA(cudaMemcpyAsync(dtd2, dd2, n * 4, cudaMemcpyDeviceToDevice, s));
-        GEO_TRY(launch_box2d(dte2, dtd2, nnx, nnz, D.fs + (is - 1) * D.ds + npml - TR, D.zs + npml - TR, nb,
+        GEO_CUDA(cudaMemcpyAsync(dtvp, dvp, 3 * n * 4, cudaMemcpyDeviceToDevice, s));
+        GEO_TRY(launch_box2d(dte2, dtd2, nnx, ldz, D.fs + (is - 1) * D.ds + npml - TR, D.zs + npml - TR, nb,
                              small.at<float>(o_te2[is - 1]), small.at<float>(o_td2[is - 1]), s));
         if (is > 1) GEO_CUDA(cudaMemsetAsync(ar.buf.p, 0, shot_end, s));
         a.ixs = D.fs + (is - 1) * D.ds + npml - 1;
@@ -626,8 +593,21 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
         a.src = (long)a.ixs * nnz + a.izs;
         a.e2 = dte2;
         a.d2 = dtd2;
+        if (!prog.tti) {
+            st.ixs = a.ixs;
+            st.lev = 0;
+            for (st.it0 = 0; st.it0 < nt; st.it0 = st.it1) {
+                st.it1 = st.it0 + 1;
+                while (st.it1 < nt && !(wd.every > 0 && st.it1 % wd.every == 0)) st.it1++;
+                GEO_TRY(fwd.run(st, s));
+                st.lev = (st.lev + st.it1 - st.it0) & 1;
+                const int w = wd.check(st.f[0].P[st.lev], n, st.it1 - 1, st.it1 == nt, s);
+                if (w == GEO_ERR_NAN) break;
+                GEO_TRY(w);
+            }
+        }
         // runs of steps between the watchdog's scans, one launch each
-        for (int it0 = 0; it0 < nt;) {
+        for (int it0 = prog.tti ? 0 : nt; it0 < nt;) {
             int it1 = it0 + 1;
             while (it1 < nt && !(wd.every > 0 && it1 % wd.every == 0)) it1++;
             GEO_TRY(launch(kf, grid_f, it0, it1));
@@ -667,11 +647,23 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
             GEO_CUDA(cudaMemcpyAsync(trs, obs + (size_t)(is - 1) * nx * nt, (size_t)nx * nt * 4, kin, s));
             GEO_TRY(launch_transpose_records(trs, rec, nt, nx, s));
         }
+        if (!prog.tti) {
+            GEO_TRY(launch_step2d_restore(st, nt - 1, st.lev, s));
+            for (st.it0 = nt - 1; st.it0 >= 0; st.it0 = st.it1 - 1) {
+                st.it1 = st.it0;
+                while (st.it1 > 0 && !(wd.every > 0 && (nt - st.it1) % wd.every == 0)) st.it1--;
+                GEO_TRY(bwd.run(st, s));
+                st.lev = (st.lev + st.it0 - st.it1 + 1) & 1;
+                const int w = wd.check(st.f[1].P[st.lev], n, nt - 1 - st.it1, st.it1 == 0, s);
+                if (w == GEO_ERR_NAN) break;
+                GEO_TRY(w);
+            }
+        }
         a.e2 = de2;
         a.d2 = dd2;
         // runs of steps between the watchdog's scans (after backward step
         // it when (nt - it) is a multiple of the interval), one launch each
-        for (int hi = nt - 1; hi >= 0;) {
+        for (int hi = prog.tti ? nt - 1 : -1; hi >= 0;) {
             int lo = hi;
             while (lo > 0 && !(wd.every > 0 && (nt - lo) % wd.every == 0)) lo--;
             GEO_TRY(launch(kb, grid_b, hi, lo));

@@ -1,0 +1,594 @@
+// Fused 2D VTI time steps of one shot: the GUI programs' forward modelling
+// (CPU_vti2dfd_kernels.c:79-177, GPU_vti2dfd_kernels.cu:209-299) and the
+// passes of the 2D GPU RTM program (Toa_gpu2DvtiFdRtmAdcigsLaplace.cu:256-404).
+//
+// A run of steps is one cooperative launch.  A block owns the same tiles, 64
+// depths x TX columns, in every step; per tile P with seven columns, Q with
+// eight depths, u and w with four either side, the split stresses and the
+// model arrive as TMA boxes in shared memory, the next tile's while this one
+// is worked on.  The velocities are rebuilt on the tile and on the four-cell
+// halos the stresses read, in place in shared memory, then the stresses
+// follow and the new level is stored.  One grid barrier a step: half of what
+// two half-steps need, and a point costs about 110 B of L2 traffic against
+// 250 when each half-step reads its taps there.  A thread owns two
+// consecutive depths (one 8-byte vector), whose x taps share a sliding window
+// of shared-memory loads.  Every wait is bounded.
+//
+// The blocks stay for the run because of the two L2 halves: launched anew
+// each step, a tile lands on any SM, so on either half, and 93 MB of the
+// 1700x601 + 50 shot's 80 MB of state and model moved through DRAM every step;
+// with the same SM, 2 MB do (forward: 26 us a step launched per step, 17.6
+// here).  Odd steps walk the tiles backwards, so that what the step before
+// left in L2 is read first: nothing forward, where all of it fits, and 41.7
+// -> 39.1 us backward, where two sides (140 MB and the gathers) do not.
+//
+// Measured against the kernels this replaces (half-steps of one persistent
+// launch; tiles kept in shared memory with exchange copies where the grid
+// fits that way), us a step: 2401x601 + 50 39.5 -> 20.1; 1200x601 25.0 ->
+// 12.1; 600x601 10.9 -> 8.6; 401x401 7.4 -> 6.0; 101x121 + 20 5.4 -> 4.0; RTM
+// program 1700x601 forward 26.1 -> 17.6, backward with 70 angles 56.3 ->
+// 39.1.  Bound by instruction issue (55 % of the slots at 24 warps per SM;
+// 340 instructions a point, a quarter of them halo work) and, on small
+// grids, by the barrier and the TMA round trip.  Tried: four warps with two
+// columns each (18.3 forward, 51.5 backward), split stresses and model from
+// L2 into registers instead of TMA (18.6 and 45.8).
+//
+// The backward pass of the RTM program takes the source side and the
+// receiver side of a tile one after the other, the source side's new values
+// waiting in registers for the image; the ring and the record of the next
+// step go into the new level as it is stored.
+#include "step2d.cuh"
+#include "adcig.cuh"
+#include "gridsync.cuh"
+#include "tc_util.cuh"
+#include <algorithm>
+#include <cmath>
+#include <cudaTypedefs.h>
+
+namespace geo {
+
+__constant__ float cs_fd[4] = {1.196289f, -0.0797526f, 0.009570313f, -0.0006975447f};
+__constant__ double cs_gauss[49];   // exp(-x^2-z^2) on the 7x7 source window
+__constant__ float cs_thr[128];     // angle-bin thresholds (largest cosine of bins >= k)
+__constant__ float cs_cos[128];     // cosf(ia*pi/180) per bin
+
+namespace {
+
+constexpr int kTz = 64, kThreads = 256;
+constexpr int kQz = kTz + 16, kWz = kTz + 8;   // depths of a Q and a w box
+
+// Floats of a stage: boxes of P, Q, u, w, of the four split stresses and of
+// the three model arrays.
+__host__ __device__ constexpr int off_q(int tx) { return (tx + 14) * kTz; }
+__host__ __device__ constexpr int off_u(int tx) { return off_q(tx) + tx * kQz; }
+__host__ __device__ constexpr int off_w(int tx) { return off_u(tx) + (tx + 8) * kTz; }
+__host__ __device__ constexpr int off_s(int tx) { return off_w(tx) + tx * kWz; }
+__host__ __device__ constexpr int off_m(int tx) { return off_s(tx) + 4 * tx * kTz; }
+__host__ __device__ constexpr int stage_floats(int tx) { return off_m(tx) + 3 * tx * kTz; }
+constexpr size_t step_smem(int tx, int stages) { return (size_t)stages * stage_floats(tx) * 4; }
+
+__device__ __forceinline__ float2 lds2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
+__device__ __forceinline__ void sts2(float *p, float2 v) { *reinterpret_cast<float2 *>(p) = v; }
+__device__ __forceinline__ float2 ldg2(const float *p) { return __ldg(reinterpret_cast<const float2 *>(p)); }
+__device__ __forceinline__ float &at2(float2 &v, int j) { return j ? v.y : v.x; }
+
+// sum_m c_m (a_m - b_m), accumulated from 0 in the programs' order
+__device__ __forceinline__ float d8(float a0, float b0, float a1, float b1, float a2, float b2, float a3, float b3) {
+    float d = 0.0f;
+    d += cs_fd[0] * (a0 - b0);
+    d += cs_fd[1] * (a1 - b1);
+    d += cs_fd[2] * (a2 - b2);
+    d += cs_fd[3] * (a3 - b3);
+    return d;
+}
+// over eight vectors a(-3) .. a(+4) (or a(-4) .. a(+3))
+__device__ __forceinline__ float2 dx8(const float2 *q) {
+    return make_float2(d8(q[4].x, q[3].x, q[5].x, q[2].x, q[6].x, q[1].x, q[7].x, q[0].x),
+                       d8(q[4].y, q[3].y, q[5].y, q[2].y, q[6].y, q[1].y, q[7].y, q[0].y));
+}
+// along z at the pair p points to; SHIFT 1 forward, 0 backward stagger
+template <int SHIFT>
+__device__ __forceinline__ float2 dz8(const float *p) {
+    float e[10];
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        const float2 t = lds2(p - 4 + 2 * k);
+        e[2 * k] = t.x;
+        e[2 * k + 1] = t.y;
+    }
+    const float *a = e + 4 + SHIFT, *b = a + 1;
+    return make_float2(d8(a[0], a[-1], a[1], a[-2], a[2], a[-3], a[3], a[-4]),
+                       d8(b[0], b[-1], b[1], b[-2], b[2], b[-3], b[3], b[-4]));
+}
+
+__device__ __forceinline__ void tma3(float *dst, const CUtensorMap *map, int z, int x, uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::
+            "r"(tc::su32(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(z), "r"(x), "r"(0), "r"(tc::su32(bar))
+        : "memory");
+}
+
+// Wait for the boxes: 2 s at most, 1 ms once a step has given up.
+__device__ __forceinline__ bool boxes_here(uint64_t *bar, uint32_t parity, const int *err) {
+    if (tc::mbar_wait(bar, parity, 1000000ull)) return true;
+    return !*(const volatile int *)err && tc::mbar_wait(bar, parity);
+}
+
+// Position in the ring of wavefield_bndr (:532), -1 off it.
+__device__ __forceinline__ int ring_at(const SGrid &g, int ix, int iz) {
+    const int n = g.npd;
+    if (ix >= n && ix < n + g.nx) {
+        if (iz == n - 1) return ix - n;
+        if (iz == n + g.nz + 1) return g.nx + ix - n;
+    }
+    if (iz >= n && iz < n + g.nz) {
+        if (ix == n - 1) return 2 * g.nx + iz - n;
+        if (ix == n + g.nx + 1) return 2 * g.nx + g.nz + iz - n;
+    }
+    return -1;
+}
+
+struct Maps {
+    SMaps m[2][2];   // side, level
+    CUtensorMap model;
+};
+
+template <int KIND, int NC>
+__global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
+    k_step2d(const __grid_constant__ Maps tm, const __grid_constant__ SStep a, int ntiles, int stages) {
+    constexpr int W = kThreads / 32, TX = W * NC, SF = stage_floats(TX);
+    constexpr bool BWD = KIND == SK_GBWD;
+    extern __shared__ __align__(128) float sm[];
+    __shared__ __align__(8) uint64_t bar[2];
+    __shared__ int s_abort;
+    const SGrid &g = a.g;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int ntz = (g.nnz + kTz - 1) / kTz, zl = 2 * lane, c0 = warp * NC, ldz = g.ldz;
+    // this block's items of a step: its tiles, backward both sides of each,
+    // one after the other
+    const int nb = ((ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * (BWD ? 2 : 1);
+    unsigned base = 0;   // items of the steps before
+    const int step_z = (int)gridDim.x % ntz * kTz, step_x = (int)gridDim.x / ntz * TX;
+    auto fetch = [&](int k, int f, int z, int x, int lev) {
+        const int st = (base + k) & (stages - 1);
+        uint64_t *b = &bar[st];
+        float *s = sm + st * SF;
+        const SMaps &m = tm.m[f][lev];
+        tc::mbar_expect_tx(b, SF * 4);
+        tc::tma2(s, &m.P, z, x - 7, b);
+        tc::tma2(s + off_q(TX), &m.Q, z - 8, x, b);
+        tc::tma2(s + off_u(TX), &m.u, z, x - 4, b);
+        tc::tma2(s + off_w(TX), &m.w, z - 4, x, b);
+        tma3(s + off_s(TX), &m.S, z, x, b);
+        tma3(s + off_m(TX), &tm.model, z, x, b);
+    };
+    if (tid == 0) {
+        for (int k = 0; k < stages; k++) tc::mbar_init(&bar[k], 1);
+        s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (ld_acquire_u32(reinterpret_cast<const unsigned *>(a.err))) return;   // an earlier run gave up
+    __syncthreads();
+        float2 sv[NC][4];   // source side's new P, Q, u, w, for the image
+    const int steps = BWD ? a.it0 - a.it1 + 1 : a.it1 - a.it0;
+    for (int s = 0; s < steps; s++, base += nb) {
+        const int it = BWD ? a.it0 - s : a.it0 + s, lev = (a.lev + s) & 1, next = BWD ? it - 1 : -1;
+        const bool src_on = BWD ? false : a.on[it] != 0;
+        const float amp = BWD ? 0.0f : a.amp[it];
+        const bool rev = s & 1;
+        const int t_first = blockIdx.x + (rev ? (BWD ? nb / 2 - 1 : nb - 1) * gridDim.x : 0);
+        const int z_first = t_first % ntz * kTz, x_first = t_first / ntz * TX;
+        if (tid == 0) {
+            // other blocks' stores of the step before, then TMA reads of them
+            asm volatile("fence.proxy.async;" ::: "memory");
+            fetch(0, 0, z_first, x_first, lev);
+        }
+        int z0 = z_first, x0 = x_first, zn = z0, xn = x0;   // this item's tile, the next item's
+        for (int k = 0; k < nb; k++, z0 = zn, x0 = xn) {
+            const int side = BWD ? k & 1 : 0, zo = z0 + zl;
+            if (!BWD || side) {
+                zn += rev ? -step_z : step_z;
+                xn += rev ? -step_x : step_x;
+                if (zn >= ntz * kTz) {
+                    zn -= ntz * kTz;
+                    xn += TX;
+                }
+                if (zn < 0) {
+                    zn += ntz * kTz;
+                    xn -= TX;
+                }
+            }
+            if (k == 0 && stages > 1 && nb > 1 && tid == 0) fetch(1, BWD ? 1 : 0, zn, xn, lev);
+            const bool ring = !(KIND == SK_GFWD || KIND == SK_GBWD) ? false :
+                (z0 < g.npd && z0 + kTz >= g.npd) || (z0 <= g.npd + g.nz + 1 && z0 + kTz > g.npd + g.nz + 1) ||
+                (x0 < g.npd && x0 + TX >= g.npd) || (x0 <= g.npd + g.nx + 1 && x0 + TX > g.npd + g.nx + 1);
+            const int st = (base + k) & (stages - 1);
+            float *sP = sm + st * SF, *sQ = sP + off_q(TX), *sU = sP + off_u(TX), *sW = sP + off_w(TX);
+            const float *sS = sP + off_s(TX), *sM = sP + off_m(TX);
+            const bool z0u = zo >= 4 && zo < g.nnz - 4, z1u = zo + 1 >= 4 && zo + 1 < g.nnz - 4;
+            const int zc = min(zo, ldz - 2);   // profiles of the pair
+            const float2 cz1 = ldg2(g.zp + zc), cz2 = ldg2(g.zp + ldz + zc);
+            if (!boxes_here(&bar[st], ((base + k) >> (stages - 1)) & 1, a.err)) *(volatile int *)&s_abort = 1;
+            if ((KIND == SK_GPU || KIND == SK_GFWD) && src_on) {
+                // point source: P,Q += amp before the velocity update, on this
+                // block's copies of the source cell
+                const int px = a.ixs - (x0 - 7), pz = a.izs - z0, qx = a.ixs - x0, qz = a.izs - (z0 - 8);
+                const bool inP = px >= 0 && px < TX + 14 && pz >= 0 && pz < kTz, inQ = qx >= 0 && qx < TX && qz >= 0 && qz < kQz;
+                if (inP || inQ) {
+                    __syncthreads();
+                    if (tid == 0 && inP) sP[px * kTz + pz] += amp;
+                    if (tid == 0 && inQ) sQ[qx * kQz + qz] += amp;
+                    __syncthreads();
+                }
+            }
+            // u on the tile's columns and its halos: NU consecutive columns a
+            // warp, column uc at x = x0 - 4 + uc, taps P box columns uc .. uc+7
+            constexpr int NU = (TX + 7 + W - 1) / W;
+            {
+                const int u0 = warp * NU;
+                float2 q[8];
+    #pragma unroll
+                for (int j = 0; j < 7; j++) q[j + 1] = lds2(sP + min(u0 + j, TX + 13) * kTz + zl);
+    #pragma unroll
+                for (int j = 0; j < NU; j++) {
+                    const int uc = u0 + j, ix = x0 - 4 + uc;
+    #pragma unroll
+                    for (int m = 0; m < 7; m++) q[m] = q[m + 1];
+                    q[7] = lds2(sP + min(uc + 7, TX + 13) * kTz + zl);
+                    if (uc < TX + 7 && ix >= 4 && ix < g.nnx - 4) {
+                        const float c1 = __ldg(g.cx1 + ix) * g.dtx, c2 = __ldg(g.cx2 + ix);
+                        const float2 xx = dx8(q), uo = lds2(sU + uc * kTz + zl);
+                        sts2(sU + uc * kTz + zl,
+                             make_float2(z0u ? c2 * uo.x - c1 * xx.x : uo.x, z1u ? c2 * uo.y - c1 * xx.y : uo.y));
+                    }
+                }
+            }
+            // w of the own points, and of the four depths above and below
+            float2 wn[NC];
+    #pragma unroll
+            for (int c = 0; c < NC; c++) {
+                float *pw = sW + (c0 + c) * kWz + zl + 4;
+                const int ix = x0 + c0 + c;
+                const bool xu = ix >= 4 && ix < g.nnx - 4;
+                const float2 zz = dz8<1>(sQ + (c0 + c) * kQz + zl + 8), wo = lds2(pw);
+                wn[c] = make_float2(xu && z0u ? cz2.x * wo.x - cz1.x * g.dtz * zz.x : wo.x,
+                                    xu && z1u ? cz2.y * wo.y - cz1.y * g.dtz * zz.y : wo.y);
+                sts2(pw, wn[c]);
+            }
+            // (by the last warps, which have fewer columns of u)
+            if (tid >= 32 * W - 4 * TX) {
+                const int col = (tid - 32 * W + 4 * TX) >> 2, q = tid & 3, zr = q < 2 ? 2 * q - 4 : kTz + 2 * (q - 2), iz = z0 + zr, ix = x0 + col;
+                if (ix >= 4 && ix < g.nnx - 4) {
+                    float *pw = sW + col * kWz + zr + 4;
+                    const float2 zz = dz8<1>(sQ + col * kQz + zr + 8), wo = lds2(pw);
+                    const int i0 = min(max(iz, 0), ldz - 1), i1 = min(max(iz + 1, 0), ldz - 1);
+                    float2 r = wo;
+                    if (iz >= 4 && iz < g.nnz - 4) r.x = g.zp[ldz + i0] * wo.x - g.zp[i0] * g.dtz * zz.x;
+                    if (iz + 1 >= 4 && iz + 1 < g.nnz - 4) r.y = g.zp[ldz + i1] * wo.y - g.zp[i1] * g.dtz * zz.y;
+                    sts2(pw, r);
+                }
+            }
+            const float2 az1 = ldg2(g.zp + 2 * ldz + zc), az2 = ldg2(g.zp + 3 * ldz + zc);
+            const int gz = zo - g.npd;
+            bool in[NC][2];
+            float im[NC][2];   // illumination or image of the interior points
+            if (KIND == SK_GFWD || KIND == SK_GBWD) {
+    #pragma unroll
+                for (int c = 0; c < NC; c++)
+    #pragma unroll
+                    for (int j = 0; j < 2; j++) {
+                        const int gx = x0 + c0 + c - g.npd;
+                        in[c][j] = gx >= 0 && gx < g.nx && gz + j >= 0 && gz + j < g.nz;
+                        im[c][j] = in[c][j] && (!BWD || side) ? (BWD ? a.mig : a.ill)[(long)gx * g.nz + gz + j] : 0.0f;
+                    }
+            }
+            tc::fence_async_smem();
+            __syncthreads();
+            if (*(volatile int *)&s_abort) {   // boxes never came: report, let the copies end and leave
+                if (tid == 0) {
+                    atomicExch(a.err, 1);
+                    for (int j = 0; j < stages; j++) tc::mbar_wait(&bar[(base + k + j) & (stages - 1)], ((base + k + j) >> (stages - 1)) & 1, 1000000ull);
+                }
+                return;
+            }
+            // every thread is past the item before: its stage takes the next one
+            if (tid == 0 && stages > 1 && k >= 1 && k + 1 < nb) fetch(k + 1, BWD ? (k + 1) & 1 : 0, zn, xn, lev);
+            const int n = lev ^ 1;
+            const SField &F = a.f[side];
+            float2 q[8];
+    #pragma unroll
+            for (int j = 0; j < 7; j++) q[j + 1] = lds2(sU + (c0 + j) * kTz + zl);
+    #pragma unroll
+            for (int c = 0; c < NC; c++) {
+    #pragma unroll
+                for (int j = 0; j < 7; j++) q[j] = q[j + 1];
+                q[7] = lds2(sU + (c0 + c + 7) * kTz + zl);
+                const int ix = x0 + c0 + c, gx = ix - g.npd;
+                const long o = (long)ix * ldz + zo;
+                const bool xu = ix >= 4 && ix < g.nnx - 4, up[2] = {xu && z0u, xu && z1u};
+                if (KIND != SK_GFWD && KIND != SK_GBWD && !(up[0] || up[1])) continue;
+                // points off the updated band hold zeros in every array but P
+                // and Q on the ring, which is written below
+                float2 Pn = make_float2(0.0f, 0.0f), Qn = Pn;
+                if (up[0] || up[1]) {
+                    const float2 xx = dx8(q), zz = dz8<0>(sW + (c0 + c) * kWz + zl + 4);
+                    const float ax1 = __ldg(g.ax1 + ix), ax2 = __ldg(g.ax2 + ix);
+                    const int so = (c0 + c) * kTz + zl;
+                    float2 T[4], M[3];
+    #pragma unroll
+                    for (int j = 0; j < 4; j++) T[j] = lds2(sS + j * TX * kTz + so);
+    #pragma unroll
+                    for (int j = 0; j < 3; j++) M[j] = lds2(sM + j * TX * kTz + so);
+    #pragma unroll
+                    for (int j = 0; j < 2; j++) {
+                        const float v = at2(M[0], j), e = at2(M[1], j), d = at2(M[2], j);
+                        const float X = j ? xx.y : xx.x, Z = j ? zz.y : zz.x, z1 = j ? az1.y : az1.x, z2 = j ? az2.y : az2.x;
+                        const float px = ax2 * at2(T[0], j) - ax1 * v * v * e * g.dtx * X;
+                        const float pz = z2 * at2(T[1], j) - z1 * v * v * d * g.dtz * Z;
+                        const float qx = ax2 * at2(T[2], j) - ax1 * v * v * d * g.dtx * X;
+                        const float qz = z2 * at2(T[3], j) - z1 * v * v * g.dtz * Z;
+                        float P = px + pz, Q = qx + qz;
+                        if (KIND == SK_CPU) {
+                            // 7x7 Gaussian source window, added after the split sum
+                            float s = 0.0f;
+                            const int rx = ix - a.ixs, rz = zo + j - a.izs;
+                            if (src_on && rx >= -3 && rx <= 3 && rz >= -3 && rz <= 3)
+                                s = (float)((double)amp * cs_gauss[(rx + 3) * 7 + (rz + 3)]);
+                            P = P + s;
+                            Q = Q + s;
+                        }
+                        if (!up[j]) continue;
+                        at2(T[0], j) = px;
+                        at2(T[1], j) = pz;
+                        at2(T[2], j) = qx;
+                        at2(T[3], j) = qz;
+                        at2(Pn, j) = P;
+                        at2(Qn, j) = Q;
+                    }
+                    sts2(F.px + o, T[0]);
+                    sts2(F.pz + o, T[1]);
+                    sts2(F.qx + o, T[2]);
+                    sts2(F.qz + o, T[3]);
+                    sts2(F.u[n] + o, q[4]);
+                    sts2(F.w[n] + o, wn[c]);
+                }
+                if (KIND == SK_CPU || KIND == SK_GPU) {
+                    sts2(F.P[n] + o, Pn);
+                    sts2(F.Q[n] + o, Qn);
+                    const int j = a.rec_iz - zo;
+                    if ((j == 0 || j == 1) && gx >= 0 && gx < g.nx) {
+                        const float P = j ? Pn.y : Pn.x;
+                        a.rec[(long)it * g.nx + gx] = a.rec_scale == 2.0f ? P + P : P * a.rec_scale;
+                    }
+                    continue;
+                }
+                if (ix >= g.nnx) continue;
+                const int r[2] = {ring && zo < g.nnz ? ring_at(g, ix, zo) : -1, ring && zo + 1 < g.nnz ? ring_at(g, ix, zo + 1) : -1};
+                const long m = (long)gx * g.nz + gz;
+                if (KIND == SK_GFWD) {
+                    // record (shot_record :498), ring save (wavefield_bndr :532,
+                    // cells off the band with their unchanged zeros), illumination
+                    // (cal_illumination :654)
+    #pragma unroll
+                    for (int j = 0; j < 2; j++) {
+                        const float P = j ? Pn.y : Pn.x, Q = j ? Qn.y : Qn.x;
+                        if (r[j] >= 0) {
+                            a.bp[(long)it * a.L + r[j]] = P;
+                            a.bq[(long)it * a.L + r[j]] = Q;
+                        }
+                        if (in[c][j]) {
+                            if (gz + j == 0) a.rec[(long)it * g.nx + gx] = P;
+                            float v = im[c][j] + (P * P + Q * Q);
+                            if (v <= 0.0f) v = 1.0f;
+                            a.ill[m + j] = v;
+                        }
+                    }
+                    if (up[0] || up[1]) {
+                        sts2(F.P[n] + o, Pn);
+                        sts2(F.Q[n] + o, Qn);
+                    }
+                } else if (side == 0) {
+                    sv[c][0] = Pn;
+                    sv[c][1] = Qn;
+                    sv[c][2] = q[4];
+                    sv[c][3] = wn[c];
+                    // the next step's ring in place in the new level
+                    if (next >= 0) {
+    #pragma unroll
+                        for (int j = 0; j < 2; j++)
+                            if (r[j] >= 0) {
+                                at2(Pn, j) = a.bp[(long)next * a.L + r[j]];
+                                at2(Qn, j) = a.bq[(long)next * a.L + r[j]];
+                            }
+                    }
+                    if (up[0] || up[1] || r[0] >= 0 || r[1] >= 0) {
+                        sts2(F.P[n] + o, Pn);
+                        sts2(F.Q[n] + o, Qn);
+                    }
+                } else if (up[0] || up[1]) {
+                    // image (cal_migration :679) and Poynting gathers (:718-766)
+                    float *ag[2] = {nullptr, nullptr}, av[2], old[2];
+    #pragma unroll
+                    for (int j = 0; j < 2; j++) {
+                        if (!in[c][j]) continue;
+                        const float sP_ = at2(sv[c][0], j), gP = at2(Pn, j);
+                        if (!a.adcig) continue;
+                        const float Ssx = -sP_ * at2(sv[c][2], j), Ssz = -at2(sv[c][1], j) * at2(sv[c][3], j);
+                        const float Sgx = gP * at2(q[4], j), Sgz = at2(Qn, j) * at2(wn[c], j);
+                        const float b1 = Ssx * Ssx + Ssz * Ssz, b2 = Sgx * Sgx + Sgz * Sgz;
+                        const int ia = poynting_bin(Ssx * Sgx + Ssz * Sgz, b1, b2, cs_thr, a.nangle);
+                        if (ia < 0) continue;
+                        const float co = cs_cos[ia];
+                        av[j] = sP_ * gP * co * co * co;
+                        // sums start at +0 and never become -0, so a zero adds nothing
+                        if (av[j] == 0.0f) continue;
+                        ag[j] = a.adcig + gz + j + (long)g.nz * ia + (long)g.nz * a.nangle * gx;
+                        old[j] = __ldcs(ag[j]);
+                    }
+    #pragma unroll
+                    for (int j = 0; j < 2; j++)
+                        if (in[c][j]) a.mig[m + j] = im[c][j] + at2(sv[c][0], j) * at2(Pn, j);
+                    // the next step's record in place in the new level
+                    if (next >= 0 && gx >= 0 && gx < g.nx && (gz == 0 || gz == -1)) {
+                        const float v = a.rec[(long)next * g.nx + gx];
+                        at2(Pn, -gz) = v;
+                        at2(Qn, -gz) = v;
+                    }
+                    sts2(F.P[n] + o, Pn);
+                    sts2(F.Q[n] + o, Qn);
+    #pragma unroll
+                    for (int j = 0; j < 2; j++)
+                        if (ag[j]) __stcs(ag[j], old[j] + av[j]);
+                }
+            }
+        }
+        // this step's stores before the next step's TMA reads of them
+        asm volatile("fence.proxy.async;" ::: "memory");
+        if (s + 1 < steps && !grid_barrier(a.bar, (unsigned)(s + 1) * gridDim.x, a.err)) return;
+    }
+}
+
+__global__ void k_step2d_restore(const __grid_constant__ SStep a, int it, int lev) {
+    const SGrid &g = a.g;
+    const long n = (long)g.nnx * g.nnz;
+    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
+        const int ix = (int)(k / g.nnz), iz = (int)(k % g.nnz), r = ring_at(g, ix, iz), gx = ix - g.npd;
+        const long o = (long)ix * g.ldz + iz;
+        if (r >= 0) {
+            a.f[0].P[lev][o] = a.bp[(long)it * a.L + r];
+            a.f[0].Q[lev][o] = a.bq[(long)it * a.L + r];
+        }
+        if (iz == g.npd && gx >= 0 && gx < g.nx) a.f[1].P[lev][o] = a.f[1].Q[lev][o] = a.rec[(long)it * g.nx + gx];
+    }
+}
+
+const void *step_fn(StepKind k, int nc) {
+    switch (k) {
+        case SK_CPU: return nc == 1 ? (const void *)k_step2d<SK_CPU, 1> : (const void *)k_step2d<SK_CPU, 2>;
+        case SK_GPU: return nc == 1 ? (const void *)k_step2d<SK_GPU, 1> : (const void *)k_step2d<SK_GPU, 2>;
+        case SK_GFWD: return nc == 1 ? (const void *)k_step2d<SK_GFWD, 1> : (const void *)k_step2d<SK_GFWD, 2>;
+        default: return nc == 1 ? (const void *)k_step2d<SK_GBWD, 1> : (const void *)k_step2d<SK_GBWD, 2>;
+    }
+}
+
+PFN_cuTensorMapEncodeTiled_v12000 g_enc = nullptr;
+
+// Boxes of boxz x boxx of `arrays` arrays that lie one behind the other.
+int box_map(CUtensorMap *map, const float *base, const SGrid &g, int boxz, int boxx, int arrays) {
+    if (!g_enc) {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        GEO_CUDA(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q));
+        if (!fn || q != cudaDriverEntryPointSuccess) return fail(GEO_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
+        g_enc = (PFN_cuTensorMapEncodeTiled_v12000)fn;
+    }
+    cuuint64_t dims[3] = {(cuuint64_t)g.nnz, (cuuint64_t)g.nnx, (cuuint64_t)arrays};
+    cuuint64_t strides[2] = {(cuuint64_t)g.ldz * 4, (cuuint64_t)g.ldz * g.nnx * 4};
+    cuuint32_t box[3] = {(cuuint32_t)boxz, (cuuint32_t)boxx, (cuuint32_t)arrays}, es[3] = {1, 1, 1};
+    const CUresult r = g_enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, arrays > 1 ? 3 : 2, const_cast<float *>(base), dims,
+                             strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(GEO_ERR_CUDA, "cuTensorMapEncodeTiled (2D step) failed (%d)", (int)r);
+    return GEO_OK;
+}
+
+}  // namespace
+
+int Fused2D::maps(const SGrid &g, const SField &f, int side) {
+    SMaps *out = m[side];
+    for (int l = 0; l < 2; l++) {
+        GEO_TRY(box_map(&out[l].P, f.P[l], g, kTz, tx + 14, 1));
+        GEO_TRY(box_map(&out[l].Q, f.Q[l], g, kQz, tx, 1));
+        GEO_TRY(box_map(&out[l].u, f.u[l], g, kTz, tx + 8, 1));
+        GEO_TRY(box_map(&out[l].w, f.w[l], g, kWz, tx, 1));
+        GEO_TRY(box_map(&out[l].S, f.px, g, kTz, tx, 4));
+    }
+    return GEO_OK;
+}
+
+int Fused2D::model(const SGrid &g, const float *p) { return box_map(&mm, p, g, kTz, tx, 3); }
+
+// Tiles of 8 columns (three blocks per SM) or 16 (two; a quarter less halo
+// work): the fewer rounds of resident blocks weighted by what a round takes,
+// 2.5 and 3.1 us at 1700x601.  601 deep: 2401 columns 20.8 us a step with 8
+// and 20.1 with 16, 600 columns 8.7 and 8.6, 300 columns 6.9 and 6.1, the
+// RTM program's 1700 forward 17.6 and 18.1; 101x121 4.0 and 4.8.  One stage
+// where every tile has its own block, two where blocks walk several.
+int Fused2D::plan(StepKind k, const SGrid &g, int fixed) {
+    kind = k;
+    if (k == SK_CPU) GEO_TRY(load_step2d_gauss());
+    int dev = 0, sms = 0, coop = 0;
+    GEO_CUDA(cudaGetDevice(&dev));
+    GEO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    GEO_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    long best = 0;
+    for (int nc = 1; nc <= 2 && coop; nc++) {
+        const void *fn = step_fn(k, nc);
+        const int t = nc * kThreads / 32;
+        if (fixed && t != fixed) continue;
+        const int n = ((g.nnz + kTz - 1) / kTz) * ((g.nnx + t - 1) / t);
+        GEO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)step_smem(t, 2)));
+        for (int st = k == SK_GBWD ? 2 : 1; st <= 2; st++) {
+            int occ = 0;
+            GEO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kThreads, step_smem(t, st)));
+            if (occ < 1 || (st == 1 && n > occ * sms)) continue;
+            const long cost = (n + (long)occ * sms - 1) / ((long)occ * sms) * (nc == 1 ? 4 : 5);
+            if (!best || cost < best) {
+                best = cost;
+                tx = t;
+                tiles = n;
+                stages = st;
+                grid = std::min(n, occ * sms);
+            }
+            break;
+        }
+    }
+    if (!best) return fail(GEO_ERR_CUDA, "2D step: cooperative launch unavailable");
+    return GEO_OK;
+}
+
+void step2d_fields(float *p, size_t n, SField &f) {
+    float **q[12] = {&f.u[0], &f.u[1], &f.w[0], &f.w[1], &f.P[0], &f.P[1], &f.Q[0], &f.Q[1], &f.px, &f.pz, &f.qx, &f.qz};
+    for (int k = 0; k < 12; k++) *q[k] = p + k * n;
+}
+
+int load_step2d_angles(const float *thr, const float *cs, cudaStream_t s) {
+    GEO_CUDA(cudaMemcpyToSymbolAsync(cs_thr, thr, sizeof cs_thr, 0, cudaMemcpyDeviceToDevice, s));
+    GEO_CUDA(cudaMemcpyToSymbolAsync(cs_cos, cs, sizeof cs_cos, 0, cudaMemcpyDeviceToDevice, s));
+    return GEO_OK;
+}
+
+int load_step2d_gauss() {
+    static bool ready = false;
+    if (ready) return GEO_OK;
+    double g[49];
+    for (int x = -3; x <= 3; x++)
+        for (int z = -3; z <= 3; z++) g[(x + 3) * 7 + (z + 3)] = std::exp((double)(-z * z - x * x));
+    GEO_CUDA(cudaMemcpyToSymbol(cs_gauss, g, sizeof g));
+    ready = true;
+    return GEO_OK;
+}
+
+int Fused2D::run(const SStep &a, cudaStream_t s) const {
+    const long long steps = std::abs((long long)a.it1 - a.it0) + 1;
+    if (steps * grid >= 4000000000LL) return fail(GEO_ERR_ARG, "too many steps for one launch");
+    Maps tm;
+    for (int f = 0; f < 2; f++)
+        for (int l = 0; l < 2; l++) tm.m[f][l] = m[kind == SK_GBWD ? f : 0][l];
+    tm.model = mm;
+    GEO_CUDA(cudaMemsetAsync(a.bar, 0, 4, s));
+    int n = tiles, st = stages;
+    void *args[] = {(void *)&tm, (void *)&a, (void *)&n, (void *)&st};
+    GEO_CUDA(cudaLaunchCooperativeKernel(step_fn(kind, tx / (kThreads / 32)), dim3(grid), dim3(kThreads), args,
+                                         step_smem(tx, stages), s));
+    return check_launch("step2d");
+}
+
+int launch_step2d_restore(const SStep &a, int it, int lev, cudaStream_t s) {
+    const long n = (long)a.g.nnx * a.g.nnz;
+    k_step2d_restore<<<(int)std::min<long>((n + 255) / 256, 152 * 8), 256, 0, s>>>(a, it, lev);
+    return check_launch("step2d_restore");
+}
+
+}  // namespace geo

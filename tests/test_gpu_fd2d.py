@@ -135,3 +135,20 @@ def test_fd2d_bad_arguments(geo):
     with pytest.raises(geo.GeoError) as ei:
         geo.fd2d_shot(bad, e, d, **KW)
     assert ei.value.status == 4
+
+
+@pytest.mark.parametrize("tile", ["64x8", "64x16"])
+@pytest.mark.parametrize("nx,nz,npd", [(2, 2, 5), (6, 53, 5), (7, 54, 5), (5, 55, 5), (21, 108, 10), (22, 109, 10),
+                                       (1300, 46, 9)])
+def test_fd2d_fused_step_tile_edges(geo, orc, monkeypatch, tile, nx, nz, npd):
+    """Grids that end at, before and after a tile's last depth and column
+    (64 deep, 8 and 16 columns), a pitch beyond the depth, and one whose
+    tiles outnumber the resident blocks of a one-stage launch."""
+    monkeypatch.setenv("GEO_FD2D_TILE", tile)
+    v, e, d = layered_model(nx, nz, seed=3)
+    kw = dict(KW, npd=npd, fs=float(max(1, nx // 2)), zs=1.0, nt=60)
+    for variant, var in (("cpu", orc.V_CPU), ("gpu", orc.V_GPU)):
+        ref, rs = orc.fd2d(v, e, d, variant=var, snap_every=25, **kw)
+        out, os_ = geo.fd2d_shot(v, e, d, variant=variant, snap_every=25, **kw)
+        assert np.abs(ref).max() > 0
+        assert np.array_equal(out, ref) and np.array_equal(os_, rs), (variant, rel_l2(out, ref))

@@ -189,3 +189,18 @@ def test_rtm2d_gpu_program_stability_check(geo):
     with pytest.raises(geo.GeoError) as ei:
         geo.rtm2d_gpu(v, e, d, **dict(GKW, dt=np.float32(5e-3)))
     assert ei.value.status == 5
+
+
+# depths and columns that end at, before and after a tile of the fused steps
+# (64 deep, 8 or 16 columns), and the ring next to a tile's edge
+@pytest.mark.parametrize("nx,nz,npml", [(44, 44, 10), (45, 43, 10), (47, 53, 6), (60, 118, 5), (100, 46, 9)])
+def test_rtm2d_gpu_program_tile_edges(geo, orc, nx, nz, npml):
+    v, e, d = model(nx=nx, nz=nz)
+    kw = dict(GKW, npml=npml, ns=1, fs=nx // 2, zs=4, nt=220)
+    mig, ill, ag, shots = orc.rtm2d_gpu(v, e, d, **cuda_angle_tables(kw["dangle"]), **kw)
+    out = geo.rtm2d_gpu(v, e, d, **kw)
+    assert np.abs(ill).max() > 0
+    assert np.array_equal(out["shots"], shots)
+    assert np.array_equal(out["illum"], ill)
+    assert np.array_equal(out["mig_lap"], orc.laplace2d_adj(mig))
+    assert np.array_equal(out["adcigs"], ag)
