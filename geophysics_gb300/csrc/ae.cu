@@ -21,6 +21,7 @@
 // each, E1's weight gradient (k_ae_e1_bwd), Adam and the bf16 repack.
 #include "ae.cuh"
 #include "tc_gemm.cuh"
+#include "tc_util.cuh"
 #include "fd3d.cuh"
 #include <algorithm>
 #include <cmath>
@@ -80,10 +81,121 @@ static AeOffsets ae_offsets() {
 
 // Weights of the two CUDA-core levels, passed by value to the snapshot
 // kernels (the host keeps a copy of the current ones).
-struct AeSmallW {
-    float w1[128], b1[16];   // E1: W [16 x 8] (bf16 values), b [16]
-    float v1[128], c1[8];    // D1: W [8 x 16] (bf16 values), b [8]
+// Input by input, so that the weights of two neighbouring outputs are one
+// 8-byte operand of a packed multiply-add.
+struct __align__(8) AeSmallW {
+    float w1[128], b1[16];   // E1: W^T [8 x 16] (bf16 values), b [16]
+    float v1[128], c1[8];    // D1: W^T [16 x 8] (bf16 values), b [8]
 };
+
+// Two floats side by side and Blackwell's packed arithmetic on them: each
+// half rounds as its scalar instruction does.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 pair(const float *w) { return *reinterpret_cast<const f32x2 *>(w); }
+// the two values of a bf16x2 word, each twice
+__device__ __forceinline__ f32x2 twice_lo(uint32_t q) {
+    const float f = __uint_as_float(q << 16);
+    return pack2(f, f);
+}
+__device__ __forceinline__ f32x2 twice_hi(uint32_t q) {
+    const float f = __uint_as_float(q & 0xffff0000u);
+    return pack2(f, f);
+}
+
+// Where the value of Morton index m sits in a block's shared copy: bits 4 and
+// 2 take up bits 6 and 9 (the depth bits whose strides are multiples of the 32
+// banks: a warp's 16 depths of two rows land on 32 banks), and bit 2 takes up
+// bit 5 (eight neighbouring nodes' halves are 16-byte accesses to all banks).
+__device__ __forceinline__ int swz(int m) { return m ^ ((m >> 2) & 16) ^ ((m >> 3) & 4) ^ ((m >> 7) & 4); }
+// Thread (z, x)'s sixteen values, one per plane y: base[f] + off, f the parity of y's low bits.
+struct BlockCol {
+    int base[2];
+    __device__ __forceinline__ BlockCol(int z, int x) {
+        base[0] = swz(morton_of(z, x, 0));
+        base[1] = base[0] ^ 4;
+    }
+    __device__ __forceinline__ int at(int y) const {
+        return base[(y ^ (y >> 1)) & 1] + (morton_of(0, 0, y) & ~4);
+    }
+};
+
+// E1 of two nodes of a snapshot: x[r] the eight values of node r as bf16
+// pairs, out[r] 16 bf16.  Two nodes share every weight's load.
+__device__ __forceinline__ void e1_pairs(const AeSmallW &w, const uint32_t (&x)[2][4], uint4 (&out)[2][2]) {
+    f32x2 acc[2][8];
+#pragma unroll
+    for (int c = 0; c < 8; c++) acc[0][c] = acc[1][c] = 0;
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            const f32x2 k = pair(w.w1 + j * 16 + 2 * c);
+#pragma unroll
+            for (int r = 0; r < 2; r++) acc[r][c] = fma2(k, j & 1 ? twice_hi(x[r][j / 2]) : twice_lo(x[r][j / 2]), acc[r][c]);
+        }
+    const f32x2 leak = pack2(kLeak, kLeak);
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const f32x2 v = add2(acc[r][c], pair(w.b1 + 2 * c));
+            const float2 a = unpack2(v), b = unpack2(mul2(leak, v));
+            reinterpret_cast<__nv_bfloat162 *>(out[r])[c] = __floats2bfloat162_rn(fmaxf(a.x, b.x), fmaxf(a.y, b.y));
+        }
+}
+
+// D1 of two nodes of a snapshot times the block's scale s: in[r] their 16 bf16,
+// y[r] eight floats.
+__device__ __forceinline__ void d1_pairs(const AeSmallW &w, const uint4 (&in)[2][2], float s, float4 (&y)[2][2]) {
+    f32x2 acc[2][4];
+#pragma unroll
+    for (int c = 0; c < 4; c++) acc[0][c] = acc[1][c] = 0;
+#pragma unroll
+    for (int j = 0; j < 16; j++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const f32x2 k = pair(w.v1 + j * 8 + 2 * c);
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const uint32_t q = reinterpret_cast<const uint32_t *>(in[r])[j / 2];
+                acc[r][c] = fma2(k, j & 1 ? twice_hi(q) : twice_lo(q), acc[r][c]);
+            }
+        }
+    const f32x2 sc = pack2(s, s);
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+        float2 o[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) o[c] = unpack2(mul2(add2(acc[r][c], pair(w.c1 + 2 * c)), sc));
+        y[r][0] = make_float4(o[0].x, o[0].y, o[1].x, o[1].y);
+        y[r][1] = make_float4(o[2].x, o[2].y, o[3].x, o[3].y);
+    }
+}
 
 // E1 of one level-1 node: h = leaky(W1 x + b1) as 16 bf16 (32 bytes).
 __device__ __forceinline__ void e1_node(const float *w1, const float *b1, const float *x8, __nv_bfloat16 *out) {
@@ -206,7 +318,12 @@ __global__ void __launch_bounds__(256) k_ae_e1(const E1Args a) {
 // Interior-box gather of a snapshot, E1 with the weights passed by value
 // (each weight a constant-bank operand of its multiply-add, no load).
 // Thread t owns depth z = t & 15 of row x = t >> 4 of the block on all
-// sixteen planes y, so its Morton slot is fixed up to the y bits.
+// sixteen planes y, so its Morton slot is fixed up to the y bits, then nodes t
+// and t + 256; the block's 16 KB of bf16 leave by one bulk store.  Bound by
+// memory (16 KB in, 16 KB out a block) and instruction issue: a 512x512x384
+// snapshot takes 159 us, 5.1 TB/s; 207 us with one scalar multiply-add per
+// weight, four-way bank conflicts in the Morton exchange and half-sector
+// stores.  Five blocks per SM; at six it spills (162 us).
 struct E1Vol {
     AeVolume vol;
     int nb;
@@ -215,8 +332,8 @@ struct E1Vol {
     AeSmallW w;
 };
 
-__global__ void __launch_bounds__(256) k_ae_e1_vol(const E1Vol a) {
-    __shared__ float xs[kAePts];
+__global__ void __launch_bounds__(256, 5) k_ae_e1_vol(const E1Vol a) {
+    __shared__ __align__(128) float xs[kAePts];
     __shared__ float red[8];
     const int b = blockIdx.x, t = threadIdx.x;
     float mx = 0.0f;
@@ -225,15 +342,16 @@ __global__ void __launch_bounds__(256) k_ae_e1_vol(const E1Vol a) {
         const int bz = b % v.nbz, bx = (b / v.nbz) % v.nbx, by = b / (v.nbz * v.nbx);
         const int z = t & 15, x = t >> 4, iz = bz * 16 + z, ix = bx * 16 + x, iy0 = by * 16;
         const bool zx = iz < v.nz && ix < v.nx;
+        const int ylim = zx ? v.ny - iy0 : 0;
         const float *col = v.src + (long)(v.oz + iz) + v.ldz * (v.ox + ix) + v.sxy * (v.oy + iy0);
         // all sixteen loads in flight before the first use
         float vals[16];
 #pragma unroll
-        for (int y = 0; y < 16; y++) vals[y] = zx && iy0 + y < v.ny ? __ldg(col + v.sxy * y) : 0.0f;
-        const int m = morton_of(z, x, 0);
+        for (int y = 0; y < 16; y++, col += v.sxy) vals[y] = y < ylim ? __ldg(col) : 0.0f;
+        const BlockCol c(z, x);
 #pragma unroll
         for (int y = 0; y < 16; y++) {
-            xs[m + morton_of(0, 0, y)] = vals[y];
+            xs[c.at(y)] = vals[y];
             mx = fmaxf(mx, fabsf(vals[y]));
         }
     } else {
@@ -242,13 +360,36 @@ __global__ void __launch_bounds__(256) k_ae_e1_vol(const E1Vol a) {
     const float s = block_max(mx, red);
     const float inv = s >= kAeTiny ? 1.0f / s : 0.0f;
     if (t == 0) a.scale[b] = s >= kAeTiny ? s : 0.0f;
+    uint32_t x[2][4];
 #pragma unroll
     for (int r = 0; r < 2; r++) {
-        const int p = t + 256 * r;
-        float x8[8];
+        const int o = swz((t + 256 * r) * 8);
 #pragma unroll
-        for (int j = 0; j < 8; j++) x8[j] = bf16r(xs[p * 8 + j] * inv);
-        e1_node(a.w.w1, a.w.b1, x8, a.h1 + ((long)b * 512 + p) * 16);
+        for (int h = 0; h < 2; h++) {
+            const float4 q = *reinterpret_cast<const float4 *>(xs + (o ^ 4 * h));
+            const __nv_bfloat162 p0 = __floats2bfloat162_rn(q.x * inv, q.y * inv), p1 = __floats2bfloat162_rn(q.z * inv, q.w * inv);
+            x[r][2 * h] = *reinterpret_cast<const uint32_t *>(&p0);
+            x[r][2 * h + 1] = *reinterpret_cast<const uint32_t *>(&p1);
+        }
+    }
+    uint4 h[2][2];
+    e1_pairs(a.w, x, h);
+    __syncthreads();
+    // the 512 nodes' 32 bytes each, in order over the values: one bulk store
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+        uint4 *o = reinterpret_cast<uint4 *>(xs) + 2 * (t + 256 * r);
+        o[0] = h[r][0];
+        o[1] = h[r][1];
+    }
+    tc::fence_async_smem();
+    __syncthreads();
+    if (t == 0) {
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], 16384;" ::"l"(a.h1 + (long)b * 512 * 16),
+                     "r"(tc::su32(xs))
+                     : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     }
 }
 
@@ -419,9 +560,12 @@ __global__ void __launch_bounds__(256) k_ae_d1(const D1Args a) {
 // order) and its squared error and norm (the escape check).  Escaped blocks
 // (esc) add their residual in modes 0 and 1.  Thread t owns depth
 // z = t & 15 of row x = t >> 4 on all sixteen planes, as in k_ae_e1_vol.
+// Mode 0 of a 512x512x384 snapshot takes 118 us, at the copy bandwidth; 178 us
+// with scalar multiply-adds, bank conflicts in the Morton exchange and the
+// registers of the image mode (three blocks per SM; now six).
 struct D1Vol {
     AeVolume vol;
-    int nb, mode;
+    int nb;
     const __nv_bfloat16 *g1;      // [nbp*512 x 16]
     const float *scale;           // [nbp]
     float *dst;                   // mode 0
@@ -435,19 +579,27 @@ struct D1Vol {
     AeSmallW w;
 };
 
-__global__ void __launch_bounds__(256) k_ae_d1_vol(const D1Vol a) {
-    __shared__ float ys[kAePts];
+template <int MODE>
+__global__ void __launch_bounds__(256, MODE == 0 ? 6 : 4) k_ae_d1_vol(const D1Vol a) {
+    __shared__ __align__(16) float ys[kAePts];
     __shared__ float red2[2][8];
     const int b = blockIdx.x, t = threadIdx.x;
     if (b >= a.nb) return;
     const float s = a.scale[b];
+    uint4 g[2][2];
+    float4 yv[2][2];
 #pragma unroll
     for (int r = 0; r < 2; r++) {
-        const int p = t + 256 * r;
-        float g[16], y[8];
-        d1_node(a.w.v1, a.w.c1, a.g1 + ((long)b * 512 + p) * 16, g, y);
+        const uint4 *src = reinterpret_cast<const uint4 *>(a.g1 + ((long)b * 512 + t + 256 * r) * 16);
+        g[r][0] = src[0];
+        g[r][1] = src[1];
+    }
+    d1_pairs(a.w, g, s, yv);
 #pragma unroll
-        for (int c = 0; c < 8; c++) ys[p * 8 + c] = y[c] * s;
+    for (int r = 0; r < 2; r++) {
+        const int o = swz((t + 256 * r) * 8);
+        *reinterpret_cast<float4 *>(ys + o) = yv[r][0];
+        *reinterpret_cast<float4 *>(ys + (o ^ 4)) = yv[r][1];
     }
     __syncthreads();
     const AeVolume &v = a.vol;
@@ -455,8 +607,8 @@ __global__ void __launch_bounds__(256) k_ae_d1_vol(const D1Vol a) {
     const int z = t & 15, x = t >> 4, iz = bz * 16 + z, ix = bx * 16 + x, iy0 = by * 16;
     const bool zx = iz < v.nz && ix < v.nx;
     const long col = (long)(v.oz + iz) + v.ldz * (v.ox + ix) + v.sxy * (v.oy + iy0);
-    const int m = morton_of(z, x, 0);
-    if (a.mode == 3) {
+    const BlockCol c(z, x);
+    if (MODE == 3) {
         float e2 = 0.0f, x2 = 0.0f;
         __nv_bfloat16 *rb = a.resall + (long)b * kAePts;
         float vals[16];
@@ -464,7 +616,7 @@ __global__ void __launch_bounds__(256) k_ae_d1_vol(const D1Vol a) {
         for (int y = 0; y < 16; y++) vals[y] = zx && iy0 + y < v.ny ? __ldg(v.src + col + v.sxy * y) : 0.0f;
 #pragma unroll
         for (int y = 0; y < 16; y++) {
-            const float d = vals[y] - ys[m + morton_of(0, 0, y)];
+            const float d = vals[y] - ys[c.at(y)];
             rb[y * 256 + t] = __float2bfloat16_rn(d);
             e2 += d * d;
             x2 += vals[y] * vals[y];
@@ -493,11 +645,11 @@ __global__ void __launch_bounds__(256) k_ae_d1_vol(const D1Vol a) {
     if (!zx) return;
     const int slot = a.esc ? a.esc[b] : -1;
     const __nv_bfloat16 *res = slot >= 0 ? a.res + (long)slot * kAePts : nullptr;
-    if (a.mode == 0) {
+    if (MODE == 0) {
 #pragma unroll
         for (int y = 0; y < 16; y++) {
             if (iy0 + y >= v.ny) break;
-            float val = ys[m + morton_of(0, 0, y)];
+            float val = ys[c.at(y)];
             if (res) val += __bfloat162float(res[y * 256 + t]);   // escaped block: decoded + residual
             a.dst[col + v.sxy * y] = val;
         }
@@ -515,7 +667,7 @@ __global__ void __launch_bounds__(256) k_ae_d1_vol(const D1Vol a) {
 #pragma unroll
     for (int y = 0; y < 16; y++) {
         if (iy0 + y >= v.ny) break;
-        float val = ys[m + morton_of(0, 0, y)];
+        float val = ys[c.at(y)];
         if (res) val += __bfloat162float(res[y * 256 + t]);
         a.mig[o0 + so * y] = mg[y] + a.wimg * val * gp[y];
     }
@@ -916,11 +1068,16 @@ static int ae_mirror(geo_ae *ae, cudaStream_t s) {
     if (ae->hver == ae->wver) return GEO_OK;
     AeSmallW &h = ae->hw;
     const float *sm = ae->small.as<float>(), *pr = ae->params.as<float>();
-    GEO_CUDA(cudaMemcpyAsync(h.w1, sm, sizeof h.w1, cudaMemcpyDeviceToHost, s));
-    GEO_CUDA(cudaMemcpyAsync(h.v1, sm + 128, sizeof h.v1, cudaMemcpyDeviceToHost, s));
+    float w[256];
+    GEO_CUDA(cudaMemcpyAsync(w, sm, sizeof w, cudaMemcpyDeviceToHost, s));
     GEO_CUDA(cudaMemcpyAsync(h.b1, pr + ae->off.b[0], sizeof h.b1, cudaMemcpyDeviceToHost, s));
     GEO_CUDA(cudaMemcpyAsync(h.c1, pr + ae->off.b[7], sizeof h.c1, cudaMemcpyDeviceToHost, s));
     GEO_CUDA(cudaStreamSynchronize(s));
+    for (int c = 0; c < 16; c++)
+        for (int j = 0; j < 8; j++) {
+            h.w1[j * 16 + c] = w[c * 8 + j];
+            h.v1[c * 8 + j] = w[128 + j * 16 + c];
+        }
     ae->hver = ae->wver;
     return GEO_OK;
 }
@@ -988,14 +1145,13 @@ int ae_encode_volume(geo_ae *ae, const AeVolume &v, void *code, float *scale, in
     D1Vol c{};
     c.vol = v;
     c.nb = nb;
-    c.mode = 3;
     c.g1 = bf(ae->g1);
     c.scale = scale;
     c.resall = bf(ae->resall);
     c.err2 = ae->err2.as<float>();
     c.norm2 = ae->norm2.as<float>();
     c.w = ae->hw;
-    k_ae_d1_vol<<<rows, 256, 0, s>>>(c);
+    k_ae_d1_vol<3><<<rows, 256, 0, s>>>(c);
     GEO_TRY(check_launch("ae_check"));
     k_ae_select<<<1, 1024, 0, s>>>(ae->err2.as<float>(), ae->norm2.as<float>(), nb, ae->tau * ae->tau,
                                    ae_escape_cap(ae, v), esc, count);
@@ -1016,7 +1172,6 @@ int ae_decode_volume(geo_ae *ae, const AeVolume &v, const void *code, const floa
     D1Vol a{};
     a.vol = v;
     a.nb = nb;
-    a.mode = mode;
     a.g1 = bf(ae->g1);
     a.scale = scale;
     a.dst = dst;
@@ -1026,7 +1181,8 @@ int ae_decode_volume(geo_ae *ae, const AeVolume &v, const void *code, const floa
     a.esc = esc;
     a.res = static_cast<const __nv_bfloat16 *>(res);
     a.w = ae->hw;
-    k_ae_d1_vol<<<rows, 256, 0, s>>>(a);
+    if (mode == 0) k_ae_d1_vol<0><<<rows, 256, 0, s>>>(a);
+    else k_ae_d1_vol<1><<<rows, 256, 0, s>>>(a);
     return check_launch("ae_d1");
 }
 
@@ -1381,9 +1537,11 @@ extern "C" int geo_ae_roundtrip(geo_ae *ae, int nx, int ny, int nz, const float 
     cudaStream_t s = (cudaStream_t)stream;
     const AeVolume v = ae_volume(vol, nz, (long)nz * nx, 0, 0, 0, nz, nx, ny);
     const int rows = ae_code_rows(v), cap = ae_escape_cap(ae, v);
-    DevBuf code, scale, esc, res, cnt;
-    GEO_TRY(code.alloc((size_t)rows * kAeLat * 2));
-    GEO_TRY(scale.alloc((size_t)rows * 4));
+    DevBuf esc, res, cnt;
+    // the code and its scales stay in the codec's own scratch
+    GEO_TRY(ensure_rows(ae, rows));
+    void *code = ae->z.p;
+    float *scale = ae->scale.as<float>();
     if (escape) {
         GEO_TRY(esc.alloc((size_t)rows * 4));
         GEO_TRY(res.alloc((size_t)std::max(cap, 1) * kAePts * 2));
@@ -1391,8 +1549,8 @@ extern "C" int geo_ae_roundtrip(geo_ae *ae, int nx, int ny, int nz, const float 
         GEO_TRY(cnt.zero(s));
     }
     GEO_CUDA(cudaMemsetAsync(ae->err.p, 0, 4, s));
-    GEO_TRY(ae_encode_volume(ae, v, code.p, scale.as<float>(), esc.as<int>(), res.p, cnt.as<int>(), s));
-    GEO_TRY(ae_decode_volume(ae, v, code.p, scale.as<float>(), esc.as<int>(), res.p, 0, out, nullptr, nullptr, 0.0f,
+    GEO_TRY(ae_encode_volume(ae, v, code, scale, esc.as<int>(), res.p, cnt.as<int>(), s));
+    GEO_TRY(ae_decode_volume(ae, v, code, scale, esc.as<int>(), res.p, 0, out, nullptr, nullptr, 0.0f,
                              s));
     if (nesc) {
         *nesc = 0;

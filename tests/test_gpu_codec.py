@@ -176,3 +176,28 @@ def test_codec_roundtrip_escape_budget(geo, trained):
     assert ne == int(np.ceil(0.25 * nb))
     base = codec.roundtrip(vol)
     assert rel_l2(out.cpu().numpy(), vol.cpu().numpy()) < rel_l2(base.cpu().numpy(), vol.cpu().numpy())
+
+
+@pytest.mark.parametrize("nz,nx,ny", [(16, 16, 16), (17, 33, 15), (31, 16, 47), (160, 48, 100)])
+def test_snapshot_kernels_match_block_kernels(geo, nz, nx, ny):
+    """E1 and D1 of a snapshot (packed arithmetic, Morton exchange, bulk
+    store) against the block-wise evaluation's: the same bits, ragged edges
+    included."""
+    torch = pytest.importorskip("torch")
+    codec = geo.Codec(seed=3)
+    vol = torch.randn(ny, nx, nz, generator=torch.Generator().manual_seed(2)).cuda() * 1e-3
+    nb = [-(-n // 16) for n in (ny, nx, nz)]
+    pad = torch.zeros([16 * n for n in nb], device="cuda")
+    pad[:ny, :nx, :nz] = vol
+    blk = pad.reshape(nb[0], 16, nb[1], 16, nb[2], 16).permute(0, 2, 4, 5, 3, 1).reshape(-1, 16, 16, 16)   # [z][x][y]
+    z, x, y = np.meshgrid(*3 * [np.arange(16)], indexing="ij")
+    m = sum(((z >> b) & 1) << 3 * b | ((x >> b) & 1) << 3 * b + 1 | ((y >> b) & 1) << 3 * b + 2 for b in range(4))
+    m = torch.from_numpy(m.reshape(-1)).cuda()
+    rows = torch.zeros(-(-blk.shape[0] // 128) * 128, 4096, device="cuda")
+    rows[:blk.shape[0], m] = blk.reshape(-1, 4096)
+    rec, _, _ = codec.eval(rows, grad=False)
+    rec = (rec * rows.abs().amax(1, keepdim=True))[:blk.shape[0], m]
+    out = codec.roundtrip(vol)
+    ref = rec.reshape(nb[0], nb[1], nb[2], 16, 16, 16).permute(0, 5, 1, 4, 2, 3).reshape(pad.shape)[:ny, :nx, :nz]
+    assert float(out.abs().max()) > 0
+    assert torch.equal(out, ref)
