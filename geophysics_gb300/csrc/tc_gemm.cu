@@ -17,6 +17,7 @@
 #include "geo_internal.h"
 #include "tc_util.cuh"
 #include "tc_gemm.cuh"
+#include <algorithm>
 #include <cudaTypedefs.h>
 
 namespace geo {
@@ -199,6 +200,202 @@ __global__ void __launch_bounds__(128, 2)
     if (warp == 0) tmem_dealloc(tmem, S::kCols);
 }
 
+// ------------------------------------------------------------- many tiles
+// The same product with bf16 output, a bias and an activation, for GEMMs of
+// more tiles than SMs: one persistent CTA per SM walks 128 x BN tiles with ten
+// warps of fixed roles, so that loads, MMAs and epilogues of consecutive tiles
+// overlap:
+//   warp 8 lane 0  TMA producer over a ring of K slices that runs on across
+//                  tiles;
+//   warp 9 lane 0  MMA issuer into two TMEM accumulators in turn;
+//   warps 0-3, 4-7 epilogues of the even and of the odd tiles: warp w reads
+//                  lanes 32(w & 3).. of its accumulator 64 columns at a time,
+//                  adds the bias, applies the activation, and sends 32 x 64
+//                  bf16 boxes out by TMA stores from two buffers of its own.
+// RB: B (one tile wide, up to 32 KB) stays in shared memory for the run.
+// Bound by memory where K is small and by the ring's L2 reads (48 KB a slice)
+// where it is large.  A 512x512x384 snapshot's levels (24 576 blocks): the four
+// 256-wide ones 213 us against 357 with a CTA per tile, whose epilogue two
+// resident CTAs hid only in part; D2 101 against 128; E2 91 against 105 (6.6
+// TB/s).
+// Every wait is bounded; a role that gives up sets the error word and ends,
+// after which the others' waits run out too.
+template <int BN, bool RB>
+struct WalkShape {
+    static constexpr int kA = kGM * kGK * 2, kB = BN * kGK * 2;
+    static constexpr int kStage = kA + (RB ? 0 : kB);
+    static constexpr int kStages = RB ? 6 : 3;
+    static constexpr int kRes = RB ? 32768 : 0;          // resident B
+    static constexpr int kStg = 8 * 2 * 4096;            // two store buffers a warp
+    static constexpr int kMaxN = 2048;                   // bias floats
+    static constexpr size_t kData = (size_t)kRes + (size_t)kStages * kStage + kStg;
+    static constexpr size_t kSmem = kData + kMaxN * 4 + 256 + 1024;
+    static_assert(kSmem <= 232448, "one CTA per SM");
+    static_assert(2 * BN <= 512, "two accumulators fit in TMEM");
+};
+constexpr int kWalkThreads = 320;
+
+template <int BN, bool RB>
+__global__ void __launch_bounds__(kWalkThreads, 1)
+    k_tc_walk(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb,
+              const __grid_constant__ CUtensorMap to, const TcGemm g, int tiles) {
+    using S = WalkShape<BN, RB>;
+    constexpr int ST = S::kStages;
+    extern __shared__ unsigned char smem_raw[];
+    uint8_t *sm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t *ring = sm + S::kRes, *stg = ring + (size_t)ST * S::kStage;
+    float *sbias = reinterpret_cast<float *>(sm + S::kData);
+    uint64_t *full = reinterpret_cast<uint64_t *>(sbias + S::kMaxN), *empty = full + ST;
+    uint64_t *acc_full = empty + ST, *acc_empty = acc_full + 2, *b_full = acc_empty + 2;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(b_full + 1);
+    __shared__ int s_abort;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ntn = g.N / BN, nk = g.K / kGK;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < ST; s++) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int s = 0; s < 2; s++) {
+            mbar_init(&acc_full[s], 1);
+            mbar_init(&acc_empty[s], 4);
+        }
+        mbar_init(b_full, 1);
+        s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int n = threadIdx.x; n < g.N; n += kWalkThreads) sbias[n] = g.bias ? g.bias[n] : 0.0f;
+    __syncwarp();
+    if (warp == 9) tmem_alloc(tslot, 2 * BN < 32 ? 32 : 2 * BN);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tslot;
+
+    if (warp == 8 && lane == 0) {
+        bool ok = true;
+        unsigned it = 0;   // slices issued
+        if (RB) {
+            mbar_expect_tx(b_full, nk * S::kB);
+            for (int kb = 0; kb < nk; kb++) tma2(sm + kb * S::kB, &tb, kb * kGK, 0, b_full);
+        }
+        for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+            const int m0 = t / ntn * kGM, n0 = t % ntn * BN;
+            for (int kb = 0; kb < nk && ok; kb++, it++) {
+                const unsigned s = it % ST;
+                if (it >= ST && !mbar_wait(&empty[s], (it / ST - 1) & 1)) {
+                    s_abort = 1;
+                    ok = false;
+                    break;
+                }
+                uint8_t *st = ring + s * S::kStage;
+                mbar_expect_tx(&full[s], S::kStage);
+                tma2(st, &ta, kb * kGK, m0, &full[s]);
+                if (!RB) tma2(st + S::kA, &tb, kb * kGK, n0, &full[s]);
+            }
+        }
+        // after a failure, let the copies still in flight land (bounded)
+        if (!ok)
+            for (unsigned k = it > ST ? it - ST : 0; k < it; k++) mbar_wait(&full[k % ST], (k / ST) & 1);
+        if (RB && !ok) mbar_wait(b_full, 0);
+    } else if (warp == 9 && lane == 0) {
+        constexpr uint32_t idesc = idesc_bf16_f32(kGM, BN);
+        bool ok = true;
+        unsigned it = 0, i = 0;
+        if (RB && !mbar_wait(b_full, 0)) ok = false;
+        for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, i++) {
+            const unsigned ab = i & 1, use = i >> 1;
+            if (use && !mbar_wait(&acc_empty[ab], (use - 1) & 1)) {
+                ok = false;
+                break;
+            }
+            tc_fence_after();
+            for (int kb = 0; kb < nk; kb++, it++) {
+                const unsigned s = it % ST;
+                if (!mbar_wait(&full[s], (it / ST) & 1)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t a0 = su32(ring + s * S::kStage), b0 = RB ? su32(sm + kb * S::kB) : a0 + S::kA;
+#pragma unroll
+                for (int k = 0; k < kGK / 16; k++)
+                    mma_bf16(tmem + ab * BN, sdesc_k128(a0 + k * 32), sdesc_k128(b0 + k * 32), idesc, (kb | k) != 0);
+                mma_commit(&empty[s]);
+            }
+            mma_commit(&acc_full[ab]);
+        }
+        if (!ok) s_abort = 1;
+    } else if (warp < 8) {
+        const int grp = warp >> 2, quad = warp & 3;
+        uint8_t *buf = stg + warp * 8192;
+        unsigned i = 0, stores = 0;
+        for (int t = blockIdx.x; t < tiles; t += gridDim.x, i++) {
+            if ((int)(i & 1) != grp) continue;
+            const int m0 = t / ntn * kGM + quad * 32, n0 = t % ntn * BN;
+            if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[grp], (i >> 1) & 1))) {
+                s_abort = 1;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t ta0 = tmem + ((uint32_t)(quad * 32) << 16) + grp * BN;
+#pragma unroll 1
+            for (int c = 0; c < BN; c += 64, stores++) {
+                uint32_t r[64];
+                tmem_ld32(ta0 + c, r);
+                tmem_ld32(ta0 + c + 32, r + 32);
+                tmem_ld_wait();
+                if (c + 64 == BN) {   // the accumulator is in registers: the issuer may have it
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acc_empty[grp]);
+                }
+                uint8_t *b = buf + (stores & 1) * 4096;
+                // this buffer's store, two back, has left
+                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                __syncwarp();
+                const float4 *bp = reinterpret_cast<const float4 *>(sbias + n0 + c);
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    const float4 u = bp[2 * q], w = bp[2 * q + 1];
+                    const float bb[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
+                    uint4 o;
+                    __nv_bfloat162 *o2 = reinterpret_cast<__nv_bfloat162 *>(&o);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        float v0 = __uint_as_float(r[8 * q + 2 * j]), v1 = __uint_as_float(r[8 * q + 2 * j + 1]);
+                        if (g.bias) {
+                            v0 += bb[2 * j];
+                            v1 += bb[2 * j + 1];
+                        }
+                        if (g.act) {
+                            v0 = leaky(v0);
+                            v1 = leaky(v1);
+                        }
+                        o2[j] = __floats2bfloat162_rn(v0, v1);
+                    }
+                    *reinterpret_cast<uint4 *>(b + lane * 128 + ((q ^ (lane & 7)) << 4)) = o;
+                }
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
+                                     reinterpret_cast<uint64_t>(&to)),
+                                 "r"(su32(b)), "r"(n0 + c), "r"(m0)
+                                 : "memory");
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                }
+            }
+        }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    if (s_abort && threadIdx.x == 0) atomicExch(g.err, 2);
+    if (warp == 9) tmem_dealloc(tmem, 2 * BN < 32 ? 32 : 2 * BN);
+}
+
 static PFN_cuTensorMapEncodeTiled_v12000 g_enc2 = nullptr;
 
 // 2D bf16 map over a row-major [rows x cols] matrix, box box_rows x 64
@@ -238,14 +435,33 @@ static int launch_bn(const TcGemm &g, cudaStream_t s) {
     return check_launch("tc_gemm");
 }
 
+template <int BN, bool RB>
+static int launch_walk(const TcGemm &g, cudaStream_t s) {
+    using S = WalkShape<BN, RB>;
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
+        GEO_CUDA(cudaGetDevice(&dev));
+        GEO_CUDA(cudaFuncSetAttribute(k_tc_walk<BN, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem));
+        GEO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    }
+    CUtensorMap ta, tb, to;
+    GEO_TRY(encode_bf16_2d(&ta, g.A, g.M, g.K, kGM));
+    GEO_TRY(encode_bf16_2d(&tb, g.B, g.N, g.K, BN));
+    GEO_TRY(encode_bf16_2d(&to, g.out, g.M, g.N, 32));
+    const int tiles = (g.M / kGM) * (g.N / BN);
+    k_tc_walk<BN, RB><<<std::min(tiles, sms), kWalkThreads, S::kSmem, s>>>(ta, tb, to, g, tiles);
+    return check_launch("tc_walk");
+}
+
 // Tile width: the widest that divides N and leaves a tile for every SM,
 // else 64.  A training batch of 256 blocks has 4 to 32 tiles of width 256
 // (E4: 4 CTAs walking 32 K slices each behind a two-slot ring), so the chip
 // idles and a slice costs a full memory latency; with width 64 and, where
 // no more than one CTA lands on an SM anyway, an eight-slot ring, the ten
 // input and output GEMMs of such an evaluation take 80 us instead of
-// 145 us.  From 152 tiles on the wide tile's fewer operand reads win
-// (k_tc_gemm<256> at 24 576 blocks: 90 us a level).
+// 145 us.  From 152 tiles on the wide tile's fewer operand reads win, and
+// k_tc_walk takes what it handles (bf16 out, no gate).
 constexpr long kFewTiles = 152;
 
 // stages = K slices, up to the tile width's default
@@ -270,6 +486,11 @@ int tc_gemm(const TcGemm &g, cudaStream_t s) {
                          reinterpret_cast<uintptr_t>(g.out) | reinterpret_cast<uintptr_t>(g.gate);
     if (al & 15) return fail(GEO_ERR_ARG, "tc_gemm: operands must be 16-byte aligned");
     const long mt = g.M / kGM;
+    if (!g.gate && !g.out_f32 && g.N <= WalkShape<256, false>::kMaxN) {
+        if (g.N % 256 == 0 && mt * (g.N / 256) >= kFewTiles) return launch_walk<256, false>(g, s);
+        if (g.N == 128 && g.K <= 128 && mt >= kFewTiles) return launch_walk<128, true>(g, s);
+        if (g.N == 64 && g.K <= 256 && mt >= kFewTiles) return launch_walk<64, true>(g, s);
+    }
     if (g.N % 256 == 0 && mt * (g.N / 256) >= kFewTiles) return launch_bn_k<256>(g, s);
     if (g.N % 128 == 0 && mt * (g.N / 128) >= kFewTiles) return launch_bn_k<128>(g, s);
     return launch_bn_k<64>(g, s);

@@ -201,3 +201,24 @@ def test_snapshot_kernels_match_block_kernels(geo, nz, nx, ny):
     ref = rec.reshape(nb[0], nb[1], nb[2], 16, 16, 16).permute(0, 5, 1, 4, 2, 3).reshape(pad.shape)[:ny, :nx, :nz]
     assert float(out.abs().max()) > 0
     assert torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("M,N,K", [(19456, 256, 64), (19584, 256, 512), (40064, 256, 192), (4992, 1024, 320),
+                                   (2432, 2048, 64), (19456, 128, 64), (58496, 128, 128), (19456, 64, 64),
+                                   (39040, 64, 256), (19584, 64, 192)])
+def test_tc_gemm_many_tiles_bf16(geo, M, N, K):
+    """The persistent kernel of GEMMs with more tiles than SMs: one, two and
+    more tiles a block, even and odd, slices below and above the ring, B
+    resident or not.  Bound: half a bf16 ulp (2^-9, doubled) of the result
+    and the FP32 sums' 1e-5 of the largest, as the FP32-output test has it."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    A = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    B = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    bias = torch.randn(N, generator=g, device="cuda")
+    ref = A.double() @ B.double().T
+    for b, act in ((None, False), (bias, True), (bias, False)):
+        r = ref if b is None else ref + b
+        r = torch.where(r > 0, r, 0.1 * r) if act else r
+        out = geo.tc_gemm_bf16(A, B, bias=b, act=act, out_f32=False).double()
+        assert ((out - r).abs() <= 2.0 ** -8 * r.abs() + 1e-5 * ref.abs().max()).all()
