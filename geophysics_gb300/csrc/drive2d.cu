@@ -263,7 +263,7 @@ int FusedShot::build(const Raw2D &raw, float dx, float dz, float dt, const std::
     int tz = 0, tx = 0;
     if (const char *e = getenv("GEO_FD2D_TILE"))
         if (sscanf(e, "%dx%d", &tz, &tx) != 2 || tx < 4 || tx > 128) tx = 0;
-    GEO_TRY(plan.plan(X.var == V_CPU ? SK_CPU : SK_GPU, g, !tx ? 0 : tx < 16 ? 8 : 16));
+    GEO_TRY(plan.plan(X.var == V_CPU ? SK_CPU : SK_GPU, false, g, !tx ? 0 : tx < 16 ? 8 : 16));
     if (tx && tz >= 32 && tz <= 256 && !(tz & (tz - 1)) && plan.stages == 1 && 11L * tx * tz + 21L * (tx + tz) > 56320)
         return fail(GEO_ERR_ARG, "GEO_FD2D_TILE %dx%d: tile too large", tz, tx);
     GEO_TRY(plan.maps(g, st.f[0], 0));

@@ -19,8 +19,7 @@
 // adcigs_illum :768), the adjoint Laplacian of the image and of the angle
 // stack (stk_adcigs :799).  The image kernels of the program run over
 // nnx*nnz threads on nx*nz arrays (an overrun); here they cover nx*nz.
-// The VTI program's steps are those of step2d.cu; the TTI program's below
-// update single buffers in place (its u0 = u1 pointer assignment).
+// The steps are those of step2d.cu.
 //
 // The 2D TTI GPU RTM program (2D-tti-fd+rtm-cuda/
 // Toa_gpu_2dtti_rtm_adcigs_iorderfunciton.cu, main :500-800) has the same
@@ -37,8 +36,6 @@
 // here only the nx/dcdp gathers are divided.
 #include "geo_internal.h"
 #include "adcig.cuh"
-#include "tti2d.cuh"
-#include "gridsync.cuh"
 #include "model2d.cuh"
 #include "step2d.cuh"
 #include <cmath>
@@ -46,204 +43,6 @@
 #include <vector>
 
 namespace geo {
-
-__constant__ float c_grtm[4] = {1.196289f, -0.0797526f, 0.009570313f, -0.0006975447f};
-__constant__ float c_gthr[128];   // angle-bin thresholds (largest cosine of bins >= k)
-__constant__ float c_gcos[128];   // cosf(ia*pi/180) per bin
-
-struct GRtm {
-    int nnx, nnz, nx, nz, npml, nangle, dcdp;
-    float dtx, dtz;
-    const float *cx1, *cx2, *cz1, *cz2, *ax1, *ax2, *az1, *az2;
-    const float *vp;
-    const float *ct, *st;   // cos, sin of the tilt (TTI program)
-};
-
-struct GField {
-    float *u, *w, *P, *Q, *px, *pz, *qx, *qz;
-};
-
-static TtiGrid tti_grid(const GRtm &g) {
-    TtiGrid t;
-    t.nnx = g.nnx; t.nnz = g.nnz; t.dtx = g.dtx; t.dtz = g.dtz;
-    t.cx1 = g.cx1; t.cx2 = g.cx2; t.cz1 = g.cz1; t.cz2 = g.cz2;
-    t.ax1 = g.ax1; t.ax2 = g.ax2; t.az1 = g.az1; t.az2 = g.az2;
-    t.vp = g.vp; t.ct = g.ct; t.st = g.st;
-    return t;
-}
-
-static TtiField tti_field(const GField &f) {
-    TtiField t;
-    t.u = f.u; t.w = f.w; t.px = f.px; t.pz = f.pz; t.qx = f.qx; t.qz = f.qz; t.P = f.P; t.Q = f.Q;
-    return t;
-}
-
-// Everything one persistent launch of a TTI program's pass needs.
-struct GCoop {
-    GRtm g;
-    TtiGrid tg;
-    GField S, R;                 // source-side and receiver-side fields
-    TtiField tS, tR;
-    const float *e2, *d2;        // stress model of the pass (SV taper forward)
-    const float *amp;            // pfac*w(t) of every step
-    const unsigned char *on;     // source active at every step
-    long src;                    // source cell
-    int ixs, izs;
-    float *rec;                  // nt*nx, time-major
-    float *bp, *bq;              // ring of P and Q, nt*L each
-    float *ill, *mig, *adcig;
-    int L;
-    int it0, it1;                // forward: steps it0..it1-1; backward: it0 down to it1
-    unsigned *bar;               // grid-barrier arrival counter, zeroed before the launch
-    int *err;                    // set when a barrier wait gave up
-};
-
-// Position of (ix, iz) in the ring of wavefield_bndr (:532): rows npml-1
-// (top) and npml+nz+1 (bottom) over the nx interior columns, then columns
-// npml-1 (left) and npml+nx+1 (right) over the nz interior rows; -1 off it.
-__device__ __forceinline__ int ring_index(const GRtm &g, int ix, int iz) {
-    const int npml = g.npml, nx = g.nx, nz = g.nz;
-    if (ix >= npml && ix < npml + nx) {
-        if (iz == npml - 1) return ix - npml;
-        if (iz == npml + nz + 1) return nx + ix - npml;
-    }
-    if (iz >= npml && iz < npml + nz) {
-        if (ix == npml - 1) return 2 * nx + iz - npml;
-        if (ix == npml + nx + 1) return 2 * nx + nz + iz - npml;
-    }
-    return -1;
-}
-
-__device__ __forceinline__ bool g_updated(const GRtm &g, int ix, int iz) {
-    return ix >= 4 && ix < g.nnx - 4 && iz >= 4 && iz < g.nnz - 4;
-}
-
-// Forward pass, steps it0..it1-1, one cooperative launch: per step the
-// velocity half-step (source folded in), a grid barrier, the stress
-// half-step with the SV taper and, per point, the surface record
-// (shot_record :498), the ring save (wavefield_bndr :532) and the source
-// illumination (cal_illumination :654: ill += P*P + Q*Q, <= 0 -> 1), a grid
-// barrier.  The ring covers cells outside the updated band too (their
-// unchanged values).
-// Four blocks per SM (64 registers): the passes are bound by the latency of
-// their L2 round trips and the gathers' scattered updates; at 1700x601 that
-// ran 1.3x faster than the two blocks that 128 registers allowed.
-__global__ void __launch_bounds__(256, 4) k_grtm_fwd(const GCoop a) {
-    if (ld_acquire_u32(reinterpret_cast<const unsigned *>(a.err))) return;   // an earlier run gave up
-    const GRtm &g = a.g;
-    const long n = (long)g.nnx * g.nnz, stride = (long)gridDim.x * blockDim.x;
-    const long first = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    unsigned k = 0;
-    for (int it = a.it0; it < a.it1; it++) {
-        const bool on = a.on[it] != 0;
-        const float amp = a.amp[it];
-        for (long id = first; id < n; id += stride) {
-            const int ix = (int)(id / g.nnz), iz = (int)(id % g.nnz);
-            if (!g_updated(g, ix, iz)) continue;
-            const bool near = on && ((iz == a.izs && abs(ix - a.ixs) <= 4) || (ix == a.ixs && abs(iz - a.izs) <= 4));
-            if (near) tti_vel_at<true, true>(a.tg, a.tS, c_grtm, id, ix, iz, a.src, amp);
-            else tti_vel_at<true, false>(a.tg, a.tS, c_grtm, id, ix, iz);
-        }
-        if (!grid_barrier(a.bar, ++k * gridDim.x, a.err)) return;
-        for (long id = first; id < n; id += stride) {
-            const int ix = (int)(id / g.nnz), iz = (int)(id % g.nnz);
-            const int r = ring_index(g, ix, iz), gx = ix - g.npml, gz = iz - g.npml;
-            const bool inner = gx >= 0 && gx < g.nx && gz >= 0 && gz < g.nz;
-            if (!g_updated(g, ix, iz)) {
-                if (r >= 0) {
-                    a.bp[(long)it * a.L + r] = __ldcg(a.S.P + id);
-                    a.bq[(long)it * a.L + r] = __ldcg(a.S.Q + id);
-                }
-                continue;
-            }
-            const float2 pq = tti_stress_at<true>(a.tg, a.tS, a.e2, a.d2, c_grtm, id, ix, iz);
-            if (gz == 0 && inner) a.rec[(long)it * g.nx + gx] = pq.x;
-            if (r >= 0) {
-                a.bp[(long)it * a.L + r] = pq.x;
-                a.bq[(long)it * a.L + r] = pq.y;
-            }
-            if (inner) {
-                const long o = (long)gx * g.nz + gz;
-                float v = a.ill[o] + (pq.x * pq.x + pq.y * pq.y);
-                if (v <= 0.0f) v = 1.0f;
-                a.ill[o] = v;
-            }
-        }
-        if (it + 1 < a.it1 && !grid_barrier(a.bar, ++k * gridDim.x, a.err)) return;
-    }
-}
-
-// Before backward step it: the saved ring into the source-side P,Q and the
-// muted record into the receiver-side P,Q at row npml (shot_record with
-// record = false).
-__device__ __forceinline__ void restore_inject(const GCoop &a, long id, int ix, int iz, int it) {
-    const GRtm &g = a.g;
-    const int r = ring_index(g, ix, iz);
-    if (r >= 0) {
-        a.S.P[id] = a.bp[(long)it * a.L + r];
-        a.S.Q[id] = a.bq[(long)it * a.L + r];
-    }
-    const int gx = ix - g.npml;
-    if (iz == g.npml && gx >= 0 && gx < g.nx) {
-        const float v = a.rec[(long)it * g.nx + gx];
-        a.R.P[id] = v;
-        a.R.Q[id] = v;
-    }
-}
-
-// Backward pass, steps it0 down to it1, one cooperative launch: the ring
-// restore and record injection of step it0, a grid barrier, then per step
-// both fields' velocity half-steps, a grid barrier, both stress half-steps
-// with, per image point, the cross-correlation image (cal_migration :679)
-// and the Poynting gathers (:718-766), then the restore and injection of
-// the next step at the same point, a grid barrier.  A ring or surface cell
-// is read by no other point of the phase that writes it.
-__global__ void __launch_bounds__(256, 4) k_grtm_bwd(const GCoop a) {
-    if (ld_acquire_u32(reinterpret_cast<const unsigned *>(a.err))) return;
-    const GRtm &g = a.g;
-    const long n = (long)g.nnx * g.nnz, stride = (long)gridDim.x * blockDim.x;
-    const long first = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    unsigned k = 0;
-    for (long id = first; id < n; id += stride) restore_inject(a, id, (int)(id / g.nnz), (int)(id % g.nnz), a.it0);
-    if (!grid_barrier(a.bar, ++k * gridDim.x, a.err)) return;
-    for (int it = a.it0; it >= a.it1; it--) {
-        for (long id = first; id < n; id += stride) {
-            const int ix = (int)(id / g.nnz), iz = (int)(id % g.nnz);
-            if (!g_updated(g, ix, iz)) continue;
-            tti_vel_at<true>(a.tg, a.tS, c_grtm, id, ix, iz);
-            tti_vel_at<true>(a.tg, a.tR, c_grtm, id, ix, iz);
-        }
-        if (!grid_barrier(a.bar, ++k * gridDim.x, a.err)) return;
-        for (long id = first; id < n; id += stride) {
-            const int ix = (int)(id / g.nnz), iz = (int)(id % g.nnz);
-            if (g_updated(g, ix, iz)) {
-                const float2 s = tti_stress_at<true>(a.tg, a.tS, a.e2, a.d2, c_grtm, id, ix, iz);
-                const float2 r = tti_stress_at<true>(a.tg, a.tR, a.e2, a.d2, c_grtm, id, ix, iz);
-                const int gx = ix - g.npml, gz = iz - g.npml;
-                if (gx >= 0 && gx < g.nx && gz >= 0 && gz < g.nz) {
-                    const long o = (long)gx * g.nz + gz;
-                    const float sP = s.x, gP = r.x;
-                    a.mig[o] = a.mig[o] + sP * gP;
-                    // gathers at ix = 0, dcdp, ... below nx / dcdp * dcdp (Poynting_Adcigs
-                    // :473 runs id < nx/dcdp*nz; the array holds nx/dcdp gathers)
-                    if (a.adcig && gx % g.dcdp == 0 && gx / g.dcdp < g.nx / g.dcdp) {
-                        const float Ssx = -sP * __ldcg(a.S.u + id), Ssz = -s.y * __ldcg(a.S.w + id);
-                        const float Sgx = gP * __ldcg(a.R.u + id), Sgz = r.y * __ldcg(a.R.w + id);
-                        const float b1 = Ssx * Ssx + Ssz * Ssz, b2 = Sgx * Sgx + Sgz * Sgz;
-                        const int ia = poynting_bin(Ssx * Sgx + Ssz * Sgz, b1, b2, c_gthr, g.nangle);
-                        if (ia >= 0) {
-                            const float c = c_gcos[ia];
-                            float *ag = a.adcig + gz + (long)g.nz * ia + (long)g.nz * g.nangle * (gx / g.dcdp);
-                            *ag = *ag + sP * gP * c * c * c;
-                        }
-                    }
-                }
-            }
-            if (it > a.it1) restore_inject(a, id, ix, iz, it - 1);
-        }
-        if (it > a.it1 && !grid_barrier(a.bar, ++k * gridDim.x, a.err)) return;
-    }
-}
 
 // Zero samples lo <= it < hi of every trace, as flat positions ix*nt + it of
 // the trace-major record inside it (the record itself is time-major).
@@ -322,15 +121,12 @@ int adcig_angle_tables(int nangle, int dangle, float *thr, float *cs, cudaStream
 
 __device__ float g_angle_stage[2 * kMaxAngles];
 
-static int gpu_adcig_tables(int nangle, int dangle, bool tti, cudaStream_t s) {
+static int gpu_adcig_tables(int nangle, int dangle, cudaStream_t s) {
     void *stage = nullptr;
     GEO_CUDA(cudaGetSymbolAddress(&stage, g_angle_stage));
     float *st = static_cast<float *>(stage);
     GEO_TRY(adcig_angle_tables(nangle, dangle, st, st + kMaxAngles, s));
-    if (!tti) return load_step2d_angles(st, st + kMaxAngles, s);
-    GEO_CUDA(cudaMemcpyToSymbolAsync(c_gthr, st, kMaxAngles * 4, 0, cudaMemcpyDeviceToDevice, s));
-    GEO_CUDA(cudaMemcpyToSymbolAsync(c_gcos, st + kMaxAngles, kMaxAngles * 4, 0, cudaMemcpyDeviceToDevice, s));
-    return GEO_OK;
+    return load_step2d_angles(st, st + kMaxAngles, s);
 }
 
 // readFile's checks (:930-965): grid spacing for the frequency, dt, dispersion, stability.
@@ -371,7 +167,7 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
     if (mem != GEO_MEM_HOST && mem != GEO_MEM_DEVICE) return fail(GEO_ERR_ARG, "bad mem kind");
     const int nx = D.nx, nz = D.nz, npml = D.npml, nt = D.nt, nnx = nx + 2 * npml, nnz = nz + 2 * npml;
     // columns of the fused step's arrays are of a pitch that TMA takes
-    const int ldz = prog.tti ? nnz : (nnz + 3) / 4 * 4, mid = (int)((size_t)nnx * nnz / 2 / nnz);
+    const int ldz = (nnz + 3) / 4 * 4, mid = (int)((size_t)nnx * nnz / 2 / nnz);
     const size_t n0 = (size_t)nx * nz, n = (size_t)nnx * ldz;
     cudaStream_t s = (cudaStream_t)stream;
     Raw2D raw;
@@ -450,10 +246,9 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
     int *mlo = nullptr;
     unsigned *sync = nullptr;
     size_t shot_end = 0, clear_end = 0;
-    const int nf = prog.tti ? 8 : 12;   // arrays of a side
     for (int pass = 0; pass < 2; pass++) {
-        fS = ar.take<float>(nf * n);
-        fR = ar.take<float>(nf * n);
+        fS = ar.take<float>(12 * n);
+        fR = ar.take<float>(12 * n);
         rec = ar.take<float>((size_t)nt * nx);
         ring = ar.take<float>((size_t)2 * nt * L);
         shot_end = ar.off;
@@ -465,8 +260,8 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
         dvp = ar.take<float>(3 * n);    // vp, 1+2eps, sqrtf(1+2del)
         dtvp = ar.take<float>(3 * n);   // the shot's, with the SV taper
         if (prog.tti) {
-            dct = ar.take<float>(n);
-            dsn = ar.take<float>(n);
+            dct = ar.take<float>(2 * n);   // cos and sin of the tilt
+            dsn = dct + n;
         }
         lap = ar.take<float>(n0);
         if (stk_lap) stk = ar.take<float>(n0);
@@ -490,96 +285,36 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
         GEO_CUDA(cudaStreamSynchronize(s));
         mu_v = rs.val[1] * (1 + (sqrtf(1 + 2 * rs.val[2]) - 1) * c1);
     }
-    if (gathers) GEO_TRY(gpu_adcig_tables(D.nangle, D.dangle, prog.tti, s));
-    GRtm g{};
-    g.nnx = nnx; g.nnz = nnz; g.nx = nx; g.nz = nz; g.npml = npml; g.nangle = D.nangle; g.dcdp = dcdp;
-    g.ct = dct;
-    g.st = dsn;
+    if (gathers) GEO_TRY(gpu_adcig_tables(D.nangle, D.dangle, s));
+    SStep st{};
+    SGrid &g = st.g;
+    g.nnx = nnx; g.nnz = nnz; g.ldz = ldz; g.npd = npml; g.nx = nx; g.nz = nz;
     g.dtx = D.dt / D.dx;
     g.dtz = D.dt / D.dz;
     const float *pp = small.at<float>(o_prof);
     g.cx1 = pp; g.cx2 = pp + nnx; g.ax1 = pp + 2 * nnx; g.ax2 = pp + 3 * nnx;
-    pp += 4 * nnx;
-    g.cz1 = pp; g.cz2 = pp + ldz; g.az1 = pp + 2 * ldz; g.az2 = pp + 3 * ldz;
-    g.vp = dvp;
-    auto fields = [&](float *p) {
-        GField f;
-        f.u = p; f.w = p + n; f.P = p + 2 * n; f.Q = p + 3 * n;
-        f.px = p + 4 * n; f.pz = p + 5 * n; f.qx = p + 6 * n; f.qz = p + 7 * n;
-        return f;
-    };
-    const GField S = fields(fS), R = fields(fR);
+    g.zp = pp + 4 * nnx;
+    step2d_fields(fS, n, st.f[0]);
+    step2d_fields(fR, n, st.f[1]);
     float *bp = ring, *bq = bp + (size_t)nt * L;
     const int gi = grid_of_n((long)n0);
     const cudaMemcpyKind kout = mem == GEO_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
     const cudaMemcpyKind kin = mem == GEO_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    GCoop a{};
-    a.g = g;
-    a.tg = tti_grid(g);
-    a.S = S;
-    a.R = R;
-    a.tS = tti_field(S);
-    a.tR = tti_field(R);
-    a.amp = small.at<float>(o_amp);
-    a.on = small.at<unsigned char>(o_on);
-    a.rec = rec;
-    a.bp = bp;
-    a.bq = bq;
-    a.ill = ill;
-    a.mig = mig;
-    a.adcig = ag;
-    a.L = L;
-    a.bar = sync;
-    a.err = reinterpret_cast<int *>(sync) + 1;
-    // every block resident at once (the grid barrier needs it; the
-    // cooperative launch checks it), threads striding over the points
-    const void *kf = (const void *)k_grtm_fwd, *kb = (const void *)k_grtm_bwd;
-    int grid_f = 0, grid_b = 0;
-    if (prog.tti) {
-        int dev = 0, sms = 0, occ_f = 0, occ_b = 0, coop = 0;
-        GEO_CUDA(cudaGetDevice(&dev));
-        GEO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        GEO_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-        GEO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_f, kf, 256, 0));
-        GEO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_b, kb, 256, 0));
-        if (!coop || occ_f < 1 || occ_b < 1) return fail(GEO_ERR_CUDA, "cooperative launch unavailable");
-        grid_f = (int)std::min<size_t>((n + 255) / 256, (size_t)occ_f * sms);
-        grid_b = (int)std::min<size_t>((n + 255) / 256, (size_t)occ_b * sms);
-        if ((long long)std::max(grid_f, grid_b) * (2LL * nt + 2) >= 4000000000LL)
-            return fail(GEO_ERR_ARG, "too many steps for one launch");
-    }
-    auto launch = [&](const void *fn, int grid, int it0, int it1) -> int {
-        a.it0 = it0;
-        a.it1 = it1;
-        GEO_CUDA(cudaMemsetAsync(a.bar, 0, 4, s));
-        void *args[] = {(void *)&a};
-        GEO_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(256), args, 0, s));
-        return check_launch("grtm_pass");
-    };
-    // VTI program: fused steps (step2d.cu)
-    SStep st{};
+    st.amp = small.at<float>(o_amp);
+    st.on = small.at<unsigned char>(o_on);
+    st.izs = D.zs + npml - 1;
+    st.rec = rec;
+    st.bp = bp; st.bq = bq; st.ill = ill; st.mig = mig; st.adcig = ag;
+    st.L = L; st.nangle = D.nangle; st.dcdp = dcdp;
+    st.bar = sync;
+    st.err = reinterpret_cast<int *>(sync) + 1;
     Fused2D fwd, bwd;
-    if (!prog.tti) {
-        SGrid &q2 = st.g;
-        q2.nnx = nnx; q2.nnz = nnz; q2.ldz = ldz; q2.npd = npml; q2.nx = nx; q2.nz = nz;
-        q2.dtx = g.dtx; q2.dtz = g.dtz;
-        q2.cx1 = g.cx1; q2.cx2 = g.cx2; q2.ax1 = g.ax1; q2.ax2 = g.ax2; q2.zp = g.cz1;
-        step2d_fields(fS, n, st.f[0]);
-        step2d_fields(fR, n, st.f[1]);
-        GEO_TRY(fwd.plan(SK_GFWD, q2));
-        GEO_TRY(fwd.maps(q2, st.f[0], 0));
-        GEO_TRY(fwd.model(q2, dtvp));
-        GEO_TRY(bwd.plan(SK_GBWD, q2));
-        for (int f = 0; f < 2; f++) GEO_TRY(bwd.maps(q2, st.f[f], f));
-        GEO_TRY(bwd.model(q2, dvp));
-        st.izs = npml + D.zs - 1;
-        st.amp = a.amp; st.on = a.on;
-        st.bar = a.bar;
-        st.rec = rec;
-        st.bp = bp; st.bq = bq; st.ill = ill; st.mig = mig; st.adcig = ag;
-        st.L = L; st.nangle = D.nangle;
-        st.err = a.err;
-    }
+    GEO_TRY(fwd.plan(SK_GFWD, prog.tti, g));
+    GEO_TRY(fwd.maps(g, st.f[0], 0));
+    GEO_TRY(fwd.model(g, dtvp, dct));
+    GEO_TRY(bwd.plan(SK_GBWD, prog.tti, g));
+    for (int f = 0; f < 2; f++) GEO_TRY(bwd.maps(g, st.f[f], f));
+    GEO_TRY(bwd.model(g, dvp, dct));
     Watchdog wd;
     GEO_TRY(wd.open());
     for (int is = 1; is <= D.ns; is++) {
@@ -588,33 +323,17 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
         GEO_TRY(launch_box2d(dte2, dtd2, nnx, ldz, D.fs + (is - 1) * D.ds + npml - TR, D.zs + npml - TR, nb,
                              small.at<float>(o_te2[is - 1]), small.at<float>(o_td2[is - 1]), s));
         if (is > 1) GEO_CUDA(cudaMemsetAsync(ar.buf.p, 0, shot_end, s));
-        a.ixs = D.fs + (is - 1) * D.ds + npml - 1;
-        a.izs = D.zs + npml - 1;
-        a.src = (long)a.ixs * nnz + a.izs;
-        a.e2 = dte2;
-        a.d2 = dtd2;
-        if (!prog.tti) {
-            st.ixs = a.ixs;
-            st.lev = 0;
-            for (st.it0 = 0; st.it0 < nt; st.it0 = st.it1) {
-                st.it1 = st.it0 + 1;
-                while (st.it1 < nt && !(wd.every > 0 && st.it1 % wd.every == 0)) st.it1++;
-                GEO_TRY(fwd.run(st, s));
-                st.lev = (st.lev + st.it1 - st.it0) & 1;
-                const int w = wd.check(st.f[0].P[st.lev], n, st.it1 - 1, st.it1 == nt, s);
-                if (w == GEO_ERR_NAN) break;
-                GEO_TRY(w);
-            }
-        }
+        st.ixs = D.fs + (is - 1) * D.ds + npml - 1;
+        st.lev = 0;
         // runs of steps between the watchdog's scans, one launch each
-        for (int it0 = prog.tti ? 0 : nt; it0 < nt;) {
-            int it1 = it0 + 1;
-            while (it1 < nt && !(wd.every > 0 && it1 % wd.every == 0)) it1++;
-            GEO_TRY(launch(kf, grid_f, it0, it1));
-            const int w = wd.check(S.P, n, it1 - 1, it1 == nt, s);
+        for (st.it0 = 0; st.it0 < nt; st.it0 = st.it1) {
+            st.it1 = st.it0 + 1;
+            while (st.it1 < nt && !(wd.every > 0 && st.it1 % wd.every == 0)) st.it1++;
+            GEO_TRY(fwd.run(st, s));
+            st.lev = (st.lev + st.it1 - st.it0) & 1;
+            const int w = wd.check(st.f[0].P[st.lev], n, st.it1 - 1, st.it1 == nt, s);
             if (w == GEO_ERR_NAN) break;
             GEO_TRY(w);
-            it0 = it1;
         }
         GEO_TRY(wd.verdict(s, "2D RTM forward pass"));
         // direct-wave mute (GPU form, tt), exactly as the program's kernel
@@ -647,38 +366,25 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
             GEO_CUDA(cudaMemcpyAsync(trs, obs + (size_t)(is - 1) * nx * nt, (size_t)nx * nt * 4, kin, s));
             GEO_TRY(launch_transpose_records(trs, rec, nt, nx, s));
         }
-        if (!prog.tti) {
-            GEO_TRY(launch_step2d_restore(st, nt - 1, st.lev, s));
-            for (st.it0 = nt - 1; st.it0 >= 0; st.it0 = st.it1 - 1) {
-                st.it1 = st.it0;
-                while (st.it1 > 0 && !(wd.every > 0 && (nt - st.it1) % wd.every == 0)) st.it1--;
-                GEO_TRY(bwd.run(st, s));
-                st.lev = (st.lev + st.it0 - st.it1 + 1) & 1;
-                const int w = wd.check(st.f[1].P[st.lev], n, nt - 1 - st.it1, st.it1 == 0, s);
-                if (w == GEO_ERR_NAN) break;
-                GEO_TRY(w);
-            }
-        }
-        a.e2 = de2;
-        a.d2 = dd2;
-        // runs of steps between the watchdog's scans (after backward step
-        // it when (nt - it) is a multiple of the interval), one launch each
-        for (int hi = prog.tti ? nt - 1 : -1; hi >= 0;) {
-            int lo = hi;
-            while (lo > 0 && !(wd.every > 0 && (nt - lo) % wd.every == 0)) lo--;
-            GEO_TRY(launch(kb, grid_b, hi, lo));
-            const int w = wd.check(R.P, n, nt - 1 - lo, lo == 0, s);
+        // runs of steps between the watchdog's scans (after backward step it
+        // when (nt - it) is a multiple of the interval), one launch each
+        GEO_TRY(launch_step2d_restore(st, nt - 1, st.lev, s));
+        for (st.it0 = nt - 1; st.it0 >= 0; st.it0 = st.it1 - 1) {
+            st.it1 = st.it0;
+            while (st.it1 > 0 && !(wd.every > 0 && (nt - st.it1) % wd.every == 0)) st.it1--;
+            GEO_TRY(bwd.run(st, s));
+            st.lev = (st.lev + st.it0 - st.it1 + 1) & 1;
+            const int w = wd.check(st.f[1].P[st.lev], n, nt - 1 - st.it1, st.it1 == 0, s);
             if (w == GEO_ERR_NAN) break;
             GEO_TRY(w);
-            hi = lo - 1;
         }
         GEO_TRY(wd.verdict(s, "2D RTM backward pass"));
     }
     {
         int err = 0;
-        GEO_CUDA(cudaMemcpyAsync(&err, a.err, 4, cudaMemcpyDeviceToHost, s));
+        GEO_CUDA(cudaMemcpyAsync(&err, st.err, 4, cudaMemcpyDeviceToHost, s));
         GEO_CUDA(cudaStreamSynchronize(s));
-        if (err) return fail(GEO_ERR_CUDA, "2D RTM: a grid barrier wait timed out");
+        if (err) return fail(GEO_ERR_CUDA, "2D RTM: a device-side wait timed out");
     }
     GEO_TRY(launch_normalize_image(mig, ill, n0, s));
     GEO_TRY(launch_laplace2d(nx, nz, mig, lap, s));

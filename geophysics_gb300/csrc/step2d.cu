@@ -1,6 +1,9 @@
-// Fused 2D VTI time steps of one shot: the GUI programs' forward modelling
-// (CPU_vti2dfd_kernels.c:79-177, GPU_vti2dfd_kernels.cu:209-299) and the
-// passes of the 2D GPU RTM program (Toa_gpu2DvtiFdRtmAdcigsLaplace.cu:256-404).
+// Fused 2D time steps of one shot: the GUI programs' VTI forward modelling
+// (CPU_vti2dfd_kernels.c:79-177, GPU_vti2dfd_kernels.cu:209-299), the TTI
+// program's (2D-tti-fd+rtm-cuda/Toa_gpu_2dtti_fd_1orderfunction.cu:81-183) and
+// the passes of the 2D GPU RTM programs, VTI
+// (Toa_gpu2DvtiFdRtmAdcigsLaplace.cu:256-404) and TTI
+// (Toa_gpu_2dtti_rtm_adcigs_iorderfunciton.cu:126-228).
 //
 // A run of steps is one cooperative launch.  A block owns the same tiles, 64
 // depths x TX columns, in every step; per tile P with seven columns, Q with
@@ -27,7 +30,10 @@
 // fits that way), us a step: 2401x601 + 50 39.5 -> 20.1; 1200x601 25.0 ->
 // 12.1; 600x601 10.9 -> 8.6; 401x401 7.4 -> 6.0; 101x121 + 20 5.4 -> 4.0; RTM
 // program 1700x601 forward 26.1 -> 17.6, backward with 70 angles 56.3 ->
-// 39.1.  Bound by instruction issue (55 % of the slots at 24 warps per SM;
+// 39.1.  TTI, whose rotated derivatives need both halos of every field (twice
+// the velocity work of a tile of 8 columns, 1.6 times of 16): 600x300 11.5 ->
+// 8.4; RTM program 1700x601, 65 angles, forward 37.3 -> 25.7, backward 74.0
+// -> 56.2.  Bound by instruction issue (55 % of the slots at 24 warps per SM;
 // 340 instructions a point, a quarter of them halo work) and, on small
 // grids, by the barrier and the TMA round trip.  Tried: four warps with two
 // columns each (18.3 forward, 51.5 backward), split stresses and model from
@@ -43,6 +49,7 @@
 #include "tc_util.cuh"
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <cudaTypedefs.h>
 
 namespace geo {
@@ -57,15 +64,23 @@ namespace {
 constexpr int kTz = 64, kThreads = 256;
 constexpr int kQz = kTz + 16, kWz = kTz + 8;   // depths of a Q and a w box
 
-// Floats of a stage: boxes of P, Q, u, w, of the four split stresses and of
-// the three model arrays.
-__host__ __device__ constexpr int off_q(int tx) { return (tx + 14) * kTz; }
-__host__ __device__ constexpr int off_u(int tx) { return off_q(tx) + tx * kQz; }
-__host__ __device__ constexpr int off_w(int tx) { return off_u(tx) + (tx + 8) * kTz; }
-__host__ __device__ constexpr int off_s(int tx) { return off_w(tx) + tx * kWz; }
-__host__ __device__ constexpr int off_m(int tx) { return off_s(tx) + 4 * tx * kTz; }
-__host__ __device__ constexpr int stage_floats(int tx) { return off_m(tx) + 3 * tx * kTz; }
-constexpr size_t step_smem(int tx, int stages) { return (size_t)stages * stage_floats(tx) * 4; }
+// Boxes of a tile in a stage (floats): P, Q, u, w, the four split stresses,
+// the three model arrays and, TTI, cos and sin of the tilt.  The rotated
+// derivatives read every field along both axes, so TTI boxes have both halos.
+template <bool TTI, int TX>
+struct Box {
+    static constexpr int zp = TTI ? kQz : kTz, zu = TTI ? kWz : kTz;      // depths of a P and a u box
+    static constexpr int xq = TTI ? TX + 14 : TX, xw = TTI ? TX + 8 : TX; // columns of a Q and a w box
+    static constexpr int hz = TTI ? 8 : 0, hu = TTI ? 4 : 0;              // depths above the tile in P and u
+    static constexpr int hq = TTI ? 7 : 0, hw = TTI ? 4 : 0;              // columns left of it in Q and w
+    static constexpr int q = (TX + 14) * zp, u = q + xq * kQz, w = u + (TX + 8) * zu, s = w + xw * kWz,
+                         m = s + 4 * TX * kTz, t = m + 3 * TX * kTz, all = t + (TTI ? 2 * (TX + 8) * kWz : 0);
+    static_assert(q % 32 == 0 && u % 32 == 0 && w % 32 == 0 && s % 32 == 0 && t % 32 == 0 && all % 32 == 0, "128-byte boxes");
+};
+constexpr size_t step_smem(int tx, int stages, bool tti) {
+    return (size_t)stages * 4 *
+           (tti ? (tx == 8 ? Box<true, 8>::all : Box<true, 16>::all) : tx == 8 ? Box<false, 8>::all : Box<false, 16>::all);
+}
 
 __device__ __forceinline__ float2 lds2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
 __device__ __forceinline__ void sts2(float *p, float2 v) { *reinterpret_cast<float2 *>(p) = v; }
@@ -115,6 +130,26 @@ __device__ __forceinline__ bool boxes_here(uint64_t *bar, uint32_t parity, const
     return !*(const volatile int *)err && tc::mbar_wait(bar, parity);
 }
 
+// The TTI programs' velocity update (Toa_gpu_2dtti_fd_1orderfunction.cu:81-112)
+// of a pair of points, in place; on: which of them are on the updated grid.
+__device__ __forceinline__ void tti_vel(const SGrid &g, int ix, float2 cz1, float2 cz2, float2 ct, float2 sn, float2 Px, float2 Pz,
+                                        float2 Qx, float2 Qz, bool on0, bool on1, float *pu, float *pw) {
+    const float c1 = __ldg(g.cx1 + ix), c2 = __ldg(g.cx2 + ix);
+    float2 u = lds2(pu), w = lds2(pw);
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const float C = at2(ct, j), S = at2(sn, j), k2 = c2 * at2(cz2, j), k1 = c1 * at2(cz1, j);
+        const float un = k2 * at2(u, j) - k1 * (C * g.dtx * at2(Px, j) - S * g.dtz * at2(Pz, j));
+        const float wn = k2 * at2(w, j) - k1 * (S * g.dtx * at2(Qx, j) + C * g.dtz * at2(Qz, j));
+        if (j ? on1 : on0) {
+            at2(u, j) = un;
+            at2(w, j) = wn;
+        }
+    }
+    sts2(pu, u);
+    sts2(pw, w);
+}
+
 // Position in the ring of wavefield_bndr (:532), -1 off it.
 __device__ __forceinline__ int ring_at(const SGrid &g, int ix, int iz) {
     const int n = g.npd;
@@ -131,13 +166,15 @@ __device__ __forceinline__ int ring_at(const SGrid &g, int ix, int iz) {
 
 struct Maps {
     SMaps m[2][2];   // side, level
-    CUtensorMap model;
+    CUtensorMap model, trig;
 };
 
-template <int KIND, int NC>
+template <int KIND, bool TTI, int NC>
 __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
     k_step2d(const __grid_constant__ Maps tm, const __grid_constant__ SStep a, int ntiles, int stages) {
-    constexpr int W = kThreads / 32, TX = W * NC, SF = stage_floats(TX);
+    constexpr int W = kThreads / 32, TX = W * NC;
+    using B = Box<TTI, TX>;
+    constexpr int SF = B::all;
     constexpr bool BWD = KIND == SK_GBWD;
     extern __shared__ __align__(128) float sm[];
     __shared__ __align__(8) uint64_t bar[2];
@@ -156,12 +193,13 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
         float *s = sm + st * SF;
         const SMaps &m = tm.m[f][lev];
         tc::mbar_expect_tx(b, SF * 4);
-        tc::tma2(s, &m.P, z, x - 7, b);
-        tc::tma2(s + off_q(TX), &m.Q, z - 8, x, b);
-        tc::tma2(s + off_u(TX), &m.u, z, x - 4, b);
-        tc::tma2(s + off_w(TX), &m.w, z - 4, x, b);
-        tma3(s + off_s(TX), &m.S, z, x, b);
-        tma3(s + off_m(TX), &tm.model, z, x, b);
+        tc::tma2(s, &m.P, z - B::hz, x - 7, b);
+        tc::tma2(s + B::q, &m.Q, z - 8, x - B::hq, b);
+        tc::tma2(s + B::u, &m.u, z - B::hu, x - 4, b);
+        tc::tma2(s + B::w, &m.w, z - 4, x - B::hw, b);
+        tma3(s + B::s, &m.S, z, x, b);
+        tma3(s + B::m, &tm.model, z, x, b);
+        if (TTI) tma3(s + B::t, &tm.trig, z - 4, x - 4, b);
     };
     if (tid == 0) {
         for (int k = 0; k < stages; k++) tc::mbar_init(&bar[k], 1);
@@ -170,7 +208,7 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
     }
     if (ld_acquire_u32(reinterpret_cast<const unsigned *>(a.err))) return;   // an earlier run gave up
     __syncthreads();
-        float2 sv[NC][4];   // source side's new P, Q, u, w, for the image
+    float2 sv[NC][4];   // source side's new P, Q, u, w, for the image
     const int steps = BWD ? a.it0 - a.it1 + 1 : a.it1 - a.it0;
     for (int s = 0; s < steps; s++, base += nb) {
         const int it = BWD ? a.it0 - s : a.it0 + s, lev = (a.lev + s) & 1, next = BWD ? it - 1 : -1;
@@ -204,8 +242,8 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
                 (z0 < g.npd && z0 + kTz >= g.npd) || (z0 <= g.npd + g.nz + 1 && z0 + kTz > g.npd + g.nz + 1) ||
                 (x0 < g.npd && x0 + TX >= g.npd) || (x0 <= g.npd + g.nx + 1 && x0 + TX > g.npd + g.nx + 1);
             const int st = (base + k) & (stages - 1);
-            float *sP = sm + st * SF, *sQ = sP + off_q(TX), *sU = sP + off_u(TX), *sW = sP + off_w(TX);
-            const float *sS = sP + off_s(TX), *sM = sP + off_m(TX);
+            float *sP = sm + st * SF, *sQ = sP + B::q, *sU = sP + B::u, *sW = sP + B::w;
+            const float *sS = sP + B::s, *sM = sP + B::m, *sT = sP + B::t;
             const bool z0u = zo >= 4 && zo < g.nnz - 4, z1u = zo + 1 >= 4 && zo + 1 < g.nnz - 4;
             const int zc = min(zo, ldz - 2);   // profiles of the pair
             const float2 cz1 = ldg2(g.zp + zc), cz2 = ldg2(g.zp + ldz + zc);
@@ -213,60 +251,106 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
             if ((KIND == SK_GPU || KIND == SK_GFWD) && src_on) {
                 // point source: P,Q += amp before the velocity update, on this
                 // block's copies of the source cell
-                const int px = a.ixs - (x0 - 7), pz = a.izs - z0, qx = a.ixs - x0, qz = a.izs - (z0 - 8);
-                const bool inP = px >= 0 && px < TX + 14 && pz >= 0 && pz < kTz, inQ = qx >= 0 && qx < TX && qz >= 0 && qz < kQz;
+                const int px = a.ixs - (x0 - 7), pz = a.izs - (z0 - B::hz), qx = a.ixs - (x0 - B::hq), qz = a.izs - (z0 - 8);
+                const bool inP = px >= 0 && px < TX + 14 && pz >= 0 && pz < B::zp, inQ = qx >= 0 && qx < B::xq && qz >= 0 && qz < kQz;
                 if (inP || inQ) {
                     __syncthreads();
-                    if (tid == 0 && inP) sP[px * kTz + pz] += amp;
+                    if (tid == 0 && inP) sP[px * B::zp + pz] += amp;
                     if (tid == 0 && inQ) sQ[qx * kQz + qz] += amp;
                     __syncthreads();
                 }
             }
-            // u on the tile's columns and its halos: NU consecutive columns a
-            // warp, column uc at x = x0 - 4 + uc, taps P box columns uc .. uc+7
             constexpr int NU = (TX + 7 + W - 1) / W;
-            {
+            float2 wn[NC];
+            if constexpr (TTI) {
+                // u and w at once, on the columns of the tile and its halos
                 const int u0 = warp * NU;
-                float2 q[8];
-    #pragma unroll
-                for (int j = 0; j < 7; j++) q[j + 1] = lds2(sP + min(u0 + j, TX + 13) * kTz + zl);
-    #pragma unroll
+                const float *pP = sP + B::hz + zl, *pQ = sQ + 8 + zl;
+                float2 p[8], q[8];
+#pragma unroll
+                for (int j = 0; j < 7; j++) {
+                    p[j + 1] = lds2(pP + min(u0 + j, TX + 13) * kQz);
+                    q[j + 1] = lds2(pQ + min(u0 + j, TX + 13) * kQz);
+                }
+#pragma unroll
                 for (int j = 0; j < NU; j++) {
-                    const int uc = u0 + j, ix = x0 - 4 + uc;
-    #pragma unroll
-                    for (int m = 0; m < 7; m++) q[m] = q[m + 1];
-                    q[7] = lds2(sP + min(uc + 7, TX + 13) * kTz + zl);
+                    const int uc = u0 + j, ix = x0 - 4 + uc, n = min(uc + 7, TX + 13) * kQz;
+#pragma unroll
+                    for (int m = 0; m < 7; m++) {
+                        p[m] = p[m + 1];
+                        q[m] = q[m + 1];
+                    }
+                    p[7] = lds2(pP + n);
+                    q[7] = lds2(pQ + n);
                     if (uc < TX + 7 && ix >= 4 && ix < g.nnx - 4) {
-                        const float c1 = __ldg(g.cx1 + ix) * g.dtx, c2 = __ldg(g.cx2 + ix);
-                        const float2 xx = dx8(q), uo = lds2(sU + uc * kTz + zl);
-                        sts2(sU + uc * kTz + zl,
-                             make_float2(z0u ? c2 * uo.x - c1 * xx.x : uo.x, z1u ? c2 * uo.y - c1 * xx.y : uo.y));
+                        const float2 Pz = dz8<1>(pP + (uc + 3) * kQz), Qz = dz8<1>(pQ + (uc + 3) * kQz);
+                        tti_vel(g, ix, cz1, cz2, lds2(sT + uc * kWz + zl + 4), lds2(sT + (TX + 8 + uc) * kWz + zl + 4), dx8(p),
+                                Pz, dx8(q), Qz, z0u, z1u, sU + uc * kWz + zl + 4, sW + uc * kWz + zl + 4);
                     }
                 }
-            }
-            // w of the own points, and of the four depths above and below
-            float2 wn[NC];
-    #pragma unroll
-            for (int c = 0; c < NC; c++) {
-                float *pw = sW + (c0 + c) * kWz + zl + 4;
-                const int ix = x0 + c0 + c;
-                const bool xu = ix >= 4 && ix < g.nnx - 4;
-                const float2 zz = dz8<1>(sQ + (c0 + c) * kQz + zl + 8), wo = lds2(pw);
-                wn[c] = make_float2(xu && z0u ? cz2.x * wo.x - cz1.x * g.dtz * zz.x : wo.x,
-                                    xu && z1u ? cz2.y * wo.y - cz1.y * g.dtz * zz.y : wo.y);
-                sts2(pw, wn[c]);
-            }
-            // (by the last warps, which have fewer columns of u)
-            if (tid >= 32 * W - 4 * TX) {
-                const int col = (tid - 32 * W + 4 * TX) >> 2, q = tid & 3, zr = q < 2 ? 2 * q - 4 : kTz + 2 * (q - 2), iz = z0 + zr, ix = x0 + col;
-                if (ix >= 4 && ix < g.nnx - 4) {
-                    float *pw = sW + col * kWz + zr + 4;
-                    const float2 zz = dz8<1>(sQ + col * kQz + zr + 8), wo = lds2(pw);
-                    const int i0 = min(max(iz, 0), ldz - 1), i1 = min(max(iz + 1, 0), ldz - 1);
-                    float2 r = wo;
-                    if (iz >= 4 && iz < g.nnz - 4) r.x = g.zp[ldz + i0] * wo.x - g.zp[i0] * g.dtz * zz.x;
-                    if (iz + 1 >= 4 && iz + 1 < g.nnz - 4) r.y = g.zp[ldz + i1] * wo.y - g.zp[i1] * g.dtz * zz.y;
-                    sts2(pw, r);
+                // and on the four depths above and below the tile's columns
+                if (tid >= 32 * W - 4 * TX) {
+                    const int col = (tid - 32 * W + 4 * TX) >> 2, k4 = tid & 3, zr = k4 < 2 ? 2 * k4 - 4 : kTz + 2 * (k4 - 2);
+                    const int iz = z0 + zr, ix = x0 + col, i0 = min(max(iz, 0), ldz - 2);
+                    const bool h0 = iz >= 4 && iz < g.nnz - 4, h1 = iz + 1 >= 4 && iz + 1 < g.nnz - 4;
+                    if (ix >= 4 && ix < g.nnx - 4 && (h0 || h1)) {
+                        const float *hP = sP + (col + 7) * kQz + zr + 8, *hQ = sQ + (col + 7) * kQz + zr + 8;
+#pragma unroll
+                        for (int m = 0; m < 8; m++) {
+                            p[m] = lds2(hP + (m - 3) * kQz);
+                            q[m] = lds2(hQ + (m - 3) * kQz);
+                        }
+                        const int uc = col + 4, z4 = zr + 4;
+                        tti_vel(g, ix, ldg2(g.zp + i0), ldg2(g.zp + ldz + i0), lds2(sT + uc * kWz + z4),
+                                lds2(sT + (TX + 8 + uc) * kWz + z4), dx8(p), dz8<1>(hP), dx8(q), dz8<1>(hQ), h0, h1,
+                                sU + uc * kWz + z4, sW + uc * kWz + z4);
+                    }
+                }
+            } else {
+                // u on the tile's columns and its halos: NU consecutive columns a
+                // warp, column uc at x = x0 - 4 + uc, taps P box columns uc .. uc+7
+                                {
+                    const int u0 = warp * NU;
+                    float2 q[8];
+#pragma unroll
+                    for (int j = 0; j < 7; j++) q[j + 1] = lds2(sP + min(u0 + j, TX + 13) * kTz + zl);
+#pragma unroll
+                    for (int j = 0; j < NU; j++) {
+                        const int uc = u0 + j, ix = x0 - 4 + uc;
+#pragma unroll
+                        for (int m = 0; m < 7; m++) q[m] = q[m + 1];
+                        q[7] = lds2(sP + min(uc + 7, TX + 13) * kTz + zl);
+                        if (uc < TX + 7 && ix >= 4 && ix < g.nnx - 4) {
+                            const float c1 = __ldg(g.cx1 + ix) * g.dtx, c2 = __ldg(g.cx2 + ix);
+                            const float2 xx = dx8(q), uo = lds2(sU + uc * kTz + zl);
+                            sts2(sU + uc * kTz + zl,
+                                 make_float2(z0u ? c2 * uo.x - c1 * xx.x : uo.x, z1u ? c2 * uo.y - c1 * xx.y : uo.y));
+                        }
+                    }
+                }
+                // w of the own points, and of the four depths above and below
+#pragma unroll
+                for (int c = 0; c < NC; c++) {
+                    float *pw = sW + (c0 + c) * kWz + zl + 4;
+                    const int ix = x0 + c0 + c;
+                    const bool xu = ix >= 4 && ix < g.nnx - 4;
+                    const float2 zz = dz8<1>(sQ + (c0 + c) * kQz + zl + 8), wo = lds2(pw);
+                    wn[c] = make_float2(xu && z0u ? cz2.x * wo.x - cz1.x * g.dtz * zz.x : wo.x,
+                                        xu && z1u ? cz2.y * wo.y - cz1.y * g.dtz * zz.y : wo.y);
+                    sts2(pw, wn[c]);
+                }
+                // (by the last warps, which have fewer columns of u)
+                if (tid >= 32 * W - 4 * TX) {
+                    const int col = (tid - 32 * W + 4 * TX) >> 2, q = tid & 3, zr = q < 2 ? 2 * q - 4 : kTz + 2 * (q - 2), iz = z0 + zr, ix = x0 + col;
+                    if (ix >= 4 && ix < g.nnx - 4) {
+                        float *pw = sW + col * kWz + zr + 4;
+                        const float2 zz = dz8<1>(sQ + col * kQz + zr + 8), wo = lds2(pw);
+                        const int i0 = min(max(iz, 0), ldz - 1), i1 = min(max(iz + 1, 0), ldz - 1);
+                        float2 r = wo;
+                        if (iz >= 4 && iz < g.nnz - 4) r.x = g.zp[ldz + i0] * wo.x - g.zp[i0] * g.dtz * zz.x;
+                        if (iz + 1 >= 4 && iz + 1 < g.nnz - 4) r.y = g.zp[ldz + i1] * wo.y - g.zp[i1] * g.dtz * zz.y;
+                        sts2(pw, r);
+                    }
                 }
             }
             const float2 az1 = ldg2(g.zp + 2 * ldz + zc), az2 = ldg2(g.zp + 3 * ldz + zc);
@@ -274,9 +358,9 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
             bool in[NC][2];
             float im[NC][2];   // illumination or image of the interior points
             if (KIND == SK_GFWD || KIND == SK_GBWD) {
-    #pragma unroll
+#pragma unroll
                 for (int c = 0; c < NC; c++)
-    #pragma unroll
+#pragma unroll
                     for (int j = 0; j < 2; j++) {
                         const int gx = x0 + c0 + c - g.npd;
                         in[c][j] = gx >= 0 && gx < g.nx && gz + j >= 0 && gz + j < g.nz;
@@ -296,14 +380,25 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
             if (tid == 0 && stages > 1 && k >= 1 && k + 1 < nb) fetch(k + 1, BWD ? (k + 1) & 1 : 0, zn, xn, lev);
             const int n = lev ^ 1;
             const SField &F = a.f[side];
-            float2 q[8];
-    #pragma unroll
-            for (int j = 0; j < 7; j++) q[j + 1] = lds2(sU + (c0 + j) * kTz + zl);
-    #pragma unroll
+            float2 q[8], r8[8];   // u, and TTI w, of eight columns
+            const float *pU = sU + B::hu + zl, *pW = sW + 4 + zl;
+#pragma unroll
+            for (int j = 0; j < 7; j++) {
+                q[j + 1] = lds2(pU + (c0 + j) * B::zu);
+                if (TTI) r8[j + 1] = lds2(pW + (c0 + j) * kWz);
+            }
+#pragma unroll
             for (int c = 0; c < NC; c++) {
-    #pragma unroll
-                for (int j = 0; j < 7; j++) q[j] = q[j + 1];
-                q[7] = lds2(sU + (c0 + c + 7) * kTz + zl);
+#pragma unroll
+                for (int j = 0; j < 7; j++) {
+                    q[j] = q[j + 1];
+                    if (TTI) r8[j] = r8[j + 1];
+                }
+                q[7] = lds2(pU + (c0 + c + 7) * B::zu);
+                if (TTI) {
+                    r8[7] = lds2(pW + (c0 + c + 7) * kWz);
+                    wn[c] = r8[4];
+                }
                 const int ix = x0 + c0 + c, gx = ix - g.npd;
                 const long o = (long)ix * ldz + zo;
                 const bool xu = ix >= 4 && ix < g.nnx - 4, up[2] = {xu && z0u, xu && z1u};
@@ -312,22 +407,39 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
                 // and Q on the ring, which is written below
                 float2 Pn = make_float2(0.0f, 0.0f), Qn = Pn;
                 if (up[0] || up[1]) {
-                    const float2 xx = dx8(q), zz = dz8<0>(sW + (c0 + c) * kWz + zl + 4);
+                    const float2 xx = dx8(q), zz = dz8<0>(pW + (c0 + c + B::hw) * kWz);
+                    float2 uz, wx, ct, sn;
+                    if (TTI) {
+                        uz = dz8<0>(pU + (c0 + c + 4) * B::zu);
+                        wx = dx8(r8);
+                        ct = lds2(sT + (c0 + c + 4) * kWz + zl + 4);
+                        sn = lds2(sT + (TX + 12 + c0 + c) * kWz + zl + 4);
+                    }
                     const float ax1 = __ldg(g.ax1 + ix), ax2 = __ldg(g.ax2 + ix);
                     const int so = (c0 + c) * kTz + zl;
                     float2 T[4], M[3];
-    #pragma unroll
+#pragma unroll
                     for (int j = 0; j < 4; j++) T[j] = lds2(sS + j * TX * kTz + so);
-    #pragma unroll
+#pragma unroll
                     for (int j = 0; j < 3; j++) M[j] = lds2(sM + j * TX * kTz + so);
-    #pragma unroll
+#pragma unroll
                     for (int j = 0; j < 2; j++) {
                         const float v = at2(M[0], j), e = at2(M[1], j), d = at2(M[2], j);
                         const float X = j ? xx.y : xx.x, Z = j ? zz.y : zz.x, z1 = j ? az1.y : az1.x, z2 = j ? az2.y : az2.x;
-                        const float px = ax2 * at2(T[0], j) - ax1 * v * v * e * g.dtx * X;
-                        const float pz = z2 * at2(T[1], j) - z1 * v * v * d * g.dtz * Z;
-                        const float qx = ax2 * at2(T[2], j) - ax1 * v * v * d * g.dtx * X;
-                        const float qz = z2 * at2(T[3], j) - z1 * v * v * g.dtz * Z;
+                        float px, pz, qx, qz;
+                        if constexpr (TTI) {
+                            const float C = at2(ct, j), S = at2(sn, j), k2 = ax2 * z2, k1 = ax1 * z1;
+                            const float A = C * g.dtx * X - S * g.dtz * at2(uz, j), Bz = S * g.dtx * at2(wx, j) + C * g.dtz * Z;
+                            px = k2 * at2(T[0], j) - k1 * v * v * e * A;
+                            pz = k2 * at2(T[1], j) - k1 * v * v * d * Bz;
+                            qx = k2 * at2(T[2], j) - k1 * v * v * d * A;
+                            qz = k2 * at2(T[3], j) - k1 * v * v * Bz;
+                        } else {
+                            px = ax2 * at2(T[0], j) - ax1 * v * v * e * g.dtx * X;
+                            pz = z2 * at2(T[1], j) - z1 * v * v * d * g.dtz * Z;
+                            qx = ax2 * at2(T[2], j) - ax1 * v * v * d * g.dtx * X;
+                            qz = z2 * at2(T[3], j) - z1 * v * v * g.dtz * Z;
+                        }
                         float P = px + pz, Q = qx + qz;
                         if (KIND == SK_CPU) {
                             // 7x7 Gaussian source window, added after the split sum
@@ -357,9 +469,10 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
                     sts2(F.P[n] + o, Pn);
                     sts2(F.Q[n] + o, Qn);
                     const int j = a.rec_iz - zo;
-                    if ((j == 0 || j == 1) && gx >= 0 && gx < g.nx) {
+                    if ((j == 0 || j == 1) && gx >= 0 && gx < g.nx && (!TTI || up[j])) {
                         const float P = j ? Pn.y : Pn.x;
-                        a.rec[(long)it * g.nx + gx] = a.rec_scale == 2.0f ? P + P : P * a.rec_scale;
+                        if (TTI) a.rec[it + (long)a.nt * gx] = P;   // the TTI program's record is trace-major
+                        else a.rec[(long)it * g.nx + gx] = a.rec_scale == 2.0f ? P + P : P * a.rec_scale;
                     }
                     continue;
                 }
@@ -370,7 +483,7 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
                     // record (shot_record :498), ring save (wavefield_bndr :532,
                     // cells off the band with their unchanged zeros), illumination
                     // (cal_illumination :654)
-    #pragma unroll
+#pragma unroll
                     for (int j = 0; j < 2; j++) {
                         const float P = j ? Pn.y : Pn.x, Q = j ? Qn.y : Qn.x;
                         if (r[j] >= 0) {
@@ -395,7 +508,7 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
                     sv[c][3] = wn[c];
                     // the next step's ring in place in the new level
                     if (next >= 0) {
-    #pragma unroll
+#pragma unroll
                         for (int j = 0; j < 2; j++)
                             if (r[j] >= 0) {
                                 at2(Pn, j) = a.bp[(long)next * a.L + r[j]];
@@ -408,12 +521,14 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
                     }
                 } else if (up[0] || up[1]) {
                     // image (cal_migration :679) and Poynting gathers (:718-766)
+                    // (gathers at gx = 0, dcdp, ... below nx / dcdp * dcdp)
+                    const int ga = !a.adcig || gx < 0 ? -1 : a.dcdp == 1 ? gx : gx % a.dcdp || gx / a.dcdp >= g.nx / a.dcdp ? -1 : gx / a.dcdp;
                     float *ag[2] = {nullptr, nullptr}, av[2], old[2];
-    #pragma unroll
+#pragma unroll
                     for (int j = 0; j < 2; j++) {
                         if (!in[c][j]) continue;
                         const float sP_ = at2(sv[c][0], j), gP = at2(Pn, j);
-                        if (!a.adcig) continue;
+                        if (ga < 0) continue;
                         const float Ssx = -sP_ * at2(sv[c][2], j), Ssz = -at2(sv[c][1], j) * at2(sv[c][3], j);
                         const float Sgx = gP * at2(q[4], j), Sgz = at2(Qn, j) * at2(wn[c], j);
                         const float b1 = Ssx * Ssx + Ssz * Ssz, b2 = Sgx * Sgx + Sgz * Sgz;
@@ -423,10 +538,10 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
                         av[j] = sP_ * gP * co * co * co;
                         // sums start at +0 and never become -0, so a zero adds nothing
                         if (av[j] == 0.0f) continue;
-                        ag[j] = a.adcig + gz + j + (long)g.nz * ia + (long)g.nz * a.nangle * gx;
+                        ag[j] = a.adcig + gz + j + (long)g.nz * ia + (long)g.nz * a.nangle * ga;
                         old[j] = __ldcs(ag[j]);
                     }
-    #pragma unroll
+#pragma unroll
                     for (int j = 0; j < 2; j++)
                         if (in[c][j]) a.mig[m + j] = im[c][j] + at2(sv[c][0], j) * at2(Pn, j);
                     // the next step's record in place in the new level
@@ -437,10 +552,14 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
                     }
                     sts2(F.P[n] + o, Pn);
                     sts2(F.Q[n] + o, Qn);
-    #pragma unroll
+#pragma unroll
                     for (int j = 0; j < 2; j++)
                         if (ag[j]) __stcs(ag[j], old[j] + av[j]);
                 }
+            }
+            if (stages == 1 && k + 1 < nb) {   // one stage: the next item's boxes once all are done with this one's
+                __syncthreads();
+                if (tid == 0) fetch(k + 1, BWD ? (k + 1) & 1 : 0, zn, xn, lev);
             }
         }
         // this step's stores before the next step's TMA reads of them
@@ -463,13 +582,18 @@ __global__ void k_step2d_restore(const __grid_constant__ SStep a, int it, int le
     }
 }
 
-const void *step_fn(StepKind k, int nc) {
+template <bool TTI, int NC>
+const void *step_fn(StepKind k) {
     switch (k) {
-        case SK_CPU: return nc == 1 ? (const void *)k_step2d<SK_CPU, 1> : (const void *)k_step2d<SK_CPU, 2>;
-        case SK_GPU: return nc == 1 ? (const void *)k_step2d<SK_GPU, 1> : (const void *)k_step2d<SK_GPU, 2>;
-        case SK_GFWD: return nc == 1 ? (const void *)k_step2d<SK_GFWD, 1> : (const void *)k_step2d<SK_GFWD, 2>;
-        default: return nc == 1 ? (const void *)k_step2d<SK_GBWD, 1> : (const void *)k_step2d<SK_GBWD, 2>;
+        case SK_CPU: return TTI ? nullptr : (const void *)k_step2d<SK_CPU, false, NC>;
+        case SK_GPU: return (const void *)k_step2d<SK_GPU, TTI, NC>;
+        case SK_GFWD: return (const void *)k_step2d<SK_GFWD, TTI, NC>;
+        default: return (const void *)k_step2d<SK_GBWD, TTI, NC>;
     }
+}
+const void *step_fn(StepKind k, bool tti, int tx) {
+    if (tti) return tx == 8 ? step_fn<true, 1>(k) : step_fn<true, 2>(k);
+    return tx == 8 ? step_fn<false, 1>(k) : step_fn<false, 2>(k);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 g_enc = nullptr;
@@ -498,25 +622,34 @@ int box_map(CUtensorMap *map, const float *base, const SGrid &g, int boxz, int b
 int Fused2D::maps(const SGrid &g, const SField &f, int side) {
     SMaps *out = m[side];
     for (int l = 0; l < 2; l++) {
-        GEO_TRY(box_map(&out[l].P, f.P[l], g, kTz, tx + 14, 1));
-        GEO_TRY(box_map(&out[l].Q, f.Q[l], g, kQz, tx, 1));
-        GEO_TRY(box_map(&out[l].u, f.u[l], g, kTz, tx + 8, 1));
-        GEO_TRY(box_map(&out[l].w, f.w[l], g, kWz, tx, 1));
+        GEO_TRY(box_map(&out[l].P, f.P[l], g, tti ? kQz : kTz, tx + 14, 1));
+        GEO_TRY(box_map(&out[l].Q, f.Q[l], g, kQz, tti ? tx + 14 : tx, 1));
+        GEO_TRY(box_map(&out[l].u, f.u[l], g, tti ? kWz : kTz, tx + 8, 1));
+        GEO_TRY(box_map(&out[l].w, f.w[l], g, kWz, tti ? tx + 8 : tx, 1));
         GEO_TRY(box_map(&out[l].S, f.px, g, kTz, tx, 4));
     }
     return GEO_OK;
 }
 
-int Fused2D::model(const SGrid &g, const float *p) { return box_map(&mm, p, g, kTz, tx, 3); }
+int Fused2D::model(const SGrid &g, const float *p, const float *trig) {
+    if (tti) GEO_TRY(box_map(&mt, trig, g, kWz, tx + 8, 2));
+    else memset(&mt, 0, sizeof mt);
+    return box_map(&mm, p, g, kTz, tx, 3);
+}
 
 // Tiles of 8 columns (three blocks per SM) or 16 (two; a quarter less halo
 // work): the fewer rounds of resident blocks weighted by what a round takes,
 // 2.5 and 3.1 us at 1700x601.  601 deep: 2401 columns 20.8 us a step with 8
 // and 20.1 with 16, 600 columns 8.7 and 8.6, 300 columns 6.9 and 6.1, the
 // RTM program's 1700 forward 17.6 and 18.1; 101x121 4.0 and 4.8.  One stage
-// where every tile has its own block, two where blocks walk several.
-int Fused2D::plan(StepKind k, const SGrid &g, int fixed) {
+// where every tile has its own block, two where blocks walk several.  TTI
+// tiles are heavier and always take one stage (three blocks per SM instead of
+// two beat the prefetch); a TTI shot goes by the busiest SM's columns with
+// their halo: 600x300 9.0 us a step with 8 and 8.4 with 16, 1500x600 22.1 and
+// 20.2, 200x150 4.5 and 5.5.
+int Fused2D::plan(StepKind k, bool tti_, const SGrid &g, int fixed) {
     kind = k;
+    tti = tti_;
     if (k == SK_CPU) GEO_TRY(load_step2d_gauss());
     int dev = 0, sms = 0, coop = 0;
     GEO_CUDA(cudaGetDevice(&dev));
@@ -524,16 +657,17 @@ int Fused2D::plan(StepKind k, const SGrid &g, int fixed) {
     GEO_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     long best = 0;
     for (int nc = 1; nc <= 2 && coop; nc++) {
-        const void *fn = step_fn(k, nc);
         const int t = nc * kThreads / 32;
+        const void *fn = step_fn(k, tti, t);
         if (fixed && t != fixed) continue;
         const int n = ((g.nnz + kTz - 1) / kTz) * ((g.nnx + t - 1) / t);
-        GEO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)step_smem(t, 2)));
-        for (int st = k == SK_GBWD ? 2 : 1; st <= 2; st++) {
+        GEO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)step_smem(t, 2, tti)));
+        for (int st = k == SK_GBWD && !tti ? 2 : 1; st <= 2; st++) {
             int occ = 0;
-            GEO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kThreads, step_smem(t, st)));
-            if (occ < 1 || (st == 1 && n > occ * sms)) continue;
-            const long cost = (n + (long)occ * sms - 1) / ((long)occ * sms) * (nc == 1 ? 4 : 5);
+            GEO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kThreads, step_smem(t, st, tti)));
+            if (occ < 1 || (st == 1 && !tti && n > occ * sms)) continue;
+            const long slots = (long)occ * sms;
+            const long cost = tti && k == SK_GPU ? (n + sms - 1L) / sms * (t + 6) : (n + slots - 1) / slots * (nc == 1 ? 4 : 5);
             if (!best || cost < best) {
                 best = cost;
                 tx = t;
@@ -577,11 +711,12 @@ int Fused2D::run(const SStep &a, cudaStream_t s) const {
     for (int f = 0; f < 2; f++)
         for (int l = 0; l < 2; l++) tm.m[f][l] = m[kind == SK_GBWD ? f : 0][l];
     tm.model = mm;
+    tm.trig = mt;
     GEO_CUDA(cudaMemsetAsync(a.bar, 0, 4, s));
     int n = tiles, st = stages;
     void *args[] = {(void *)&tm, (void *)&a, (void *)&n, (void *)&st};
-    GEO_CUDA(cudaLaunchCooperativeKernel(step_fn(kind, tx / (kThreads / 32)), dim3(grid), dim3(kThreads), args,
-                                         step_smem(tx, stages), s));
+    GEO_CUDA(cudaLaunchCooperativeKernel(step_fn(kind, tti, tx), dim3(grid), dim3(kThreads), args,
+                                         step_smem(tx, stages, tti), s));
     return check_launch("step2d");
 }
 

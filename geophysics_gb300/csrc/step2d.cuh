@@ -37,10 +37,11 @@ struct SStep {
     float *rec;
     int rec_iz;
     float rec_scale;
+    int nt;                          // TTI: trace-major record, nt samples a trace
     // GPU RTM program: ring of P and Q (L entries a step), illumination,
     // image, angle gathers
     float *bp, *bq, *ill, *mig, *adcig;
-    int L, nangle;
+    int L, nangle, dcdp;             // gathers at every dcdp-th CDP
     unsigned *bar;                   // grid-barrier counter
     int *err;                        // set when a wait gave up
 };
@@ -50,13 +51,14 @@ struct SStep {
 // sqrtf(1+2del), one array behind the other), then run() any number of times.
 struct Fused2D {
     StepKind kind = SK_CPU;
+    bool tti = false;
     int tx = 0, tiles = 0, stages = 0, grid = 0;   // columns per tile
     SMaps m[2][2];                                 // side, level
-    CUtensorMap mm;
+    CUtensorMap mm, mt;
     // fixed: columns per tile (8 or 16) whatever the grid; 0: by the grid
-    int plan(StepKind k, const SGrid &g, int fixed = 0);
+    int plan(StepKind k, bool tti, const SGrid &g, int fixed = 0);
     int maps(const SGrid &g, const SField &f, int side);
-    int model(const SGrid &g, const float *p);
+    int model(const SGrid &g, const float *p, const float *trig = nullptr);
     int run(const SStep &a, cudaStream_t s) const;
 };
 // The 12 arrays of a side, n floats each, from p.

@@ -9,20 +9,17 @@
 // the record taken from P at the surface row after each step
 // (shot_record :273-283) and padded-P snapshots every snap_every steps from
 // snap_every on (:451-456).  The program swaps its old/new pointers without
-// keeping two buffers (u0 = u1 after the first step), so every field is
-// updated in place; this file does that directly.
+// keeping two buffers (u0 = u1 after the first step), so every field is in
+// effect updated in place.
 // cos and sin of the tilt are formed once on the device (cosf/sinf of the
 // angle in radians, theta * pi/180 as the program converts it).
 // The program launches four kernels per step; here the steps between two
-// host events (a snapshot, a watchdog scan) run as one cooperative launch
-// with grid barriers between the half-steps, the source folded into the
-// velocity taps that read its cell and the record written by the stress
-// phase.
+// host events (a snapshot, a watchdog scan) are one launch of the fused steps
+// of step2d.cu.
 #include "geo_internal.h"
 #include <algorithm>
-#include "tti2d.cuh"
 #include "model2d.cuh"
-#include "gridsync.cuh"
+#include "step2d.cuh"
 #include <cmath>
 #include <vector>
 
@@ -48,58 +45,6 @@ int launch_tilt_trig(float *th_cos, float *sn, size_t n, cudaStream_t s) {
     return check_launch("tilt_trig");
 }
 
-
-__constant__ float c_tti[4] = {1.196289f, -0.0797526f, 0.009570313f, -0.0006975447f};
-
-// A whole 2D TTI shot (or a run of its steps) in one cooperative launch:
-// per step the velocity half-step over every updated point (the step's
-// point source folded into the taps that read the source cell), a grid
-// barrier, the stress half-step with the surface record of P, a grid
-// barrier.  The per-point arithmetic is tti_vel_at / tti_stress_at's; field
-// values other blocks wrote are read through L2.
-struct TtiShot {
-    TtiGrid g;
-    TtiField f;
-    const float *e2, *d2;
-    const float *amp;            // pfac*w(t) of every step
-    const unsigned char *on;     // source active at every step
-    long src;                    // source cell
-    int ixs, izs;
-    float *rec;                  // nx*nt, trace-major
-    int nx, npd, rec_iz, nt;
-    int it0, it1;                // steps of this launch
-    unsigned *bar;               // grid-barrier arrival counter, zeroed before the launch
-    int *err;                    // set when a barrier wait gave up
-};
-
-__global__ void __launch_bounds__(256) k_tti_shot(const TtiShot a) {
-    if (ld_acquire_u32(reinterpret_cast<const unsigned *>(a.err))) return;   // an earlier run gave up
-    const TtiGrid &g = a.g;
-    const long n = (long)g.nnx * g.nnz, stride = (long)gridDim.x * blockDim.x;
-    const long first = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    unsigned k = 0;
-    for (int it = a.it0; it < a.it1; it++) {
-        const bool on = a.on[it] != 0;
-        const float amp = a.amp[it];
-        for (long id = first; id < n; id += stride) {
-            const int ix = (int)(id / g.nnz), iz = (int)(id % g.nnz);
-            if (ix < 4 || ix >= g.nnx - 4 || iz < 4 || iz >= g.nnz - 4) continue;
-            const bool near = on && ((iz == a.izs && abs(ix - a.ixs) <= 4) || (ix == a.ixs && abs(iz - a.izs) <= 4));
-            if (near) tti_vel_at<true, true>(g, a.f, c_tti, id, ix, iz, a.src, amp);
-            else tti_vel_at<true, false>(g, a.f, c_tti, id, ix, iz);
-        }
-        if (!grid_barrier(a.bar, ++k * gridDim.x, a.err)) return;
-        for (long id = first; id < n; id += stride) {
-            const int ix = (int)(id / g.nnz), iz = (int)(id % g.nnz);
-            if (ix < 4 || ix >= g.nnx - 4 || iz < 4 || iz >= g.nnz - 4) continue;
-            const float P = tti_stress_at<true>(g, a.f, a.e2, a.d2, c_tti, id, ix, iz).x;
-            // shot_record (:273-283): P at the receiver row, after the step
-            if (iz == a.rec_iz && ix >= a.npd && ix < a.npd + a.nx) a.rec[it + (long)a.nt * (ix - a.npd)] = P;
-        }
-        if (it + 1 < a.it1 && !grid_barrier(a.bar, ++k * gridDim.x, a.err)) return;
-    }
-}
-
 }  // namespace geo
 
 using namespace geo;
@@ -114,7 +59,8 @@ extern "C" int geo_tti2d_shot(const geo_fd2d_desc *desc, const float *v, const f
     if (snap && snap_every < 1) return fail(GEO_ERR_ARG, "snap_every must be >= 1");
     const int nx = D.nx, nz = D.nz, npd = D.npd, nt = D.nt;
     const int nnx = nx + 2 * npd, nnz = nz + 2 * npd;
-    const size_t n = (size_t)nnx * nnz;
+    const int ldz = (nnz + 3) / 4 * 4;   // columns of a pitch that TMA takes
+    const size_t n = (size_t)nnx * ldz, mid = (size_t)nnx * nnz / 2;
     if (D.rec_iz < 0 || D.rec_iz >= nnz) return fail(GEO_ERR_ARG, "receiver row outside the grid");
     cudaStream_t s = (cudaStream_t)stream;
     Raw2D raw;
@@ -128,7 +74,7 @@ extern "C" int geo_tti2d_shot(const geo_fd2d_desc *desc, const float *v, const f
     auto at = [&](int a, int ix, int iz) {   // padded position
         return raw_at(a, raw, std::min(std::max(ix - npd, 0), nx - 1), std::min(std::max(iz - npd, 0), nz - 1));
     };
-    pick.push_back(at(0, (int)(n / 2 / nnz), (int)(n / 2 % nnz)));
+    pick.push_back(at(0, (int)(mid / nnz), (int)(mid % nnz)));
     if (D.sv)
         for (int a = 1; a <= 2; a++)
             for (int b = 0; b < kTB * kTB; b++) pick.push_back(at(a, cx - kTB / 2 + b / kTB, cz - kTB / 2 + b % kTB));
@@ -138,11 +84,11 @@ extern "C" int geo_tti2d_shot(const geo_fd2d_desc *desc, const float *v, const f
     GEO_TRY(check_stability(V_GPU, 2, rs.vmin, rs.vmax, D.dt, D.dx, D.dx, D.dz, D.favg));
     // sponge (get_d0 :186-189 from the padded centre velocity; initial_coffe :227-271)
     const float d0 = sponge_d0(V_GPU, 2, 0.0f, rs.val[0], npd, D.dx, D.dx, D.dz);
-    std::vector<float> prof(4 * (size_t)(nnx + nnz));
+    std::vector<float> prof(4 * (size_t)(nnx + ldz), 1.0f);
     float *q = prof.data();
     sponge_profiles(V_GPU, nx, npd, D.dt, d0, q, q + nnx, q + 2 * nnx, q + 3 * nnx);
     q += 4 * nnx;
-    sponge_profiles(V_GPU, nz, npd, D.dt, d0, q, q + nnz, q + 2 * nnz, q + 3 * nnz);
+    sponge_profiles(V_GPU, nz, npd, D.dt, d0, q, q + ldz, q + 2 * ldz, q + 3 * ldz);
     std::vector<float> amp;
     std::vector<uint8_t> on;
     source_amplitudes(V_GPU, nt, D.dt, D.favg, D.pfac, D.wtype, amp, on);
@@ -170,7 +116,7 @@ extern "C" int geo_tti2d_shot(const geo_fd2d_desc *desc, const float *v, const f
     unsigned *sync = nullptr;
     size_t clear = 0;
     for (int pass = 0; pass < 2; pass++) {
-        fb = ar.take<float>(8 * n);
+        fb = ar.take<float>(12 * n);
         drec = ar.take<float>((size_t)nx * nt);
         sync = ar.take<unsigned>(2);
         clear = ar.off;
@@ -179,54 +125,36 @@ extern "C" int geo_tti2d_shot(const geo_fd2d_desc *desc, const float *v, const f
     }
     GEO_CUDA(cudaMemsetAsync(ar.buf.p, 0, clear, s));
     ModelJob job{};
-    job.nx = nx; job.nz = nz; job.npd = npd; job.ldz = nnz;
+    job.nx = nx; job.nz = nz; job.npd = npd; job.ldz = ldz;
     job.vp = model; job.e2 = model + n; job.d2 = model + 2 * n; job.rad = model + 3 * n;
     GEO_TRY(launch_model2d(raw, {job}, s));
     if (D.sv)
-        GEO_TRY(launch_box2d(job.e2, job.d2, nnx, nnz, tp.x0, tp.z0, kTB, small.at<float>(o_te2), small.at<float>(o_td2),
+        GEO_TRY(launch_box2d(job.e2, job.d2, nnx, ldz, tp.x0, tp.z0, kTB, small.at<float>(o_te2), small.at<float>(o_td2),
                              s));
     GEO_TRY(launch_tilt_trig(model + 3 * n, model + 4 * n, n, s));
-    TtiGrid g{};
-    g.nnx = nnx;
-    g.nnz = nnz;
+    SStep a{};
+    SGrid &g = a.g;
+    g.nnx = nnx; g.nnz = nnz; g.ldz = ldz; g.npd = npd; g.nx = nx; g.nz = nz;
     g.dtx = D.dt / D.dx;
     g.dtz = D.dt / D.dz;
     const float *pp = small.at<float>(o_prof);
     g.cx1 = pp; g.cx2 = pp + nnx; g.ax1 = pp + 2 * nnx; g.ax2 = pp + 3 * nnx;
-    pp += 4 * nnx;
-    g.cz1 = pp; g.cz2 = pp + nnz; g.az1 = pp + 2 * nnz; g.az2 = pp + 3 * nnz;
-    g.vp = model; g.ct = model + 3 * n; g.st = model + 4 * n;
-    const float *e2 = model + n, *d2 = model + 2 * n;
-    TtiField f;
-    f.u = fb; f.w = fb + n; f.px = fb + 2 * n; f.pz = fb + 3 * n; f.qx = fb + 4 * n; f.qz = fb + 5 * n;
-    f.P = fb + 6 * n; f.Q = fb + 7 * n;
-    const cudaMemcpyKind kout = mem == GEO_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    TtiShot a{};
-    a.g = g;
-    a.f = f;
-    a.e2 = e2;
-    a.d2 = d2;
+    g.zp = pp + 4 * nnx;
+    step2d_fields(fb, n, a.f[0]);
     a.amp = small.at<float>(o_amp);
     a.on = small.at<unsigned char>(o_on);
-    a.src = (long)ixs * nnz + izs;
     a.ixs = ixs;
     a.izs = izs;
     a.rec = drec;
-    a.nx = nx;
-    a.npd = npd;
     a.rec_iz = D.rec_iz;
     a.nt = nt;
     a.bar = sync;
     a.err = reinterpret_cast<int *>(sync) + 1;
-    // every block resident at once (the grid barrier needs it; the
-    // cooperative launch checks it), threads striding over the points
-    int dev = 0, sms = 0, occ = 0, coop = 0;
-    GEO_CUDA(cudaGetDevice(&dev));
-    GEO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    GEO_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    GEO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tti_shot, 256, 0));
-    if (!coop || occ < 1) return fail(GEO_ERR_CUDA, "cooperative launch unavailable");
-    const int grid = (int)std::min<size_t>((n + 255) / 256, (size_t)occ * sms);
+    const cudaMemcpyKind kout = mem == GEO_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
+    Fused2D plan;
+    GEO_TRY(plan.plan(SK_GPU, true, g));
+    GEO_TRY(plan.maps(g, a.f[0], 0));
+    GEO_TRY(plan.model(g, model, model + 3 * n));
     Watchdog wd;
     GEO_TRY(wd.open());
     // runs of steps between the host's work: a snapshot after step it
@@ -239,17 +167,17 @@ extern "C" int geo_tti2d_shot(const geo_fd2d_desc *desc, const float *v, const f
             const bool watch_due = wd.every > 0 && (it + 1) % wd.every == 0;
             if (snap_due || watch_due || it1 == nt) break;
         }
-        if ((long long)grid * 2 * (it1 - it0) >= 4000000000LL) it1 = it0 + (int)(1900000000LL / grid);
+        if ((long long)plan.grid * (it1 - it0 + 1) >= 4000000000LL) it1 = it0 + (int)(1900000000LL / plan.grid);
         a.it0 = it0;
         a.it1 = it1;
-        GEO_CUDA(cudaMemsetAsync(a.bar, 0, 4, s));
-        void *args[] = {(void *)&a};
-        GEO_CUDA(cudaLaunchCooperativeKernel((const void *)k_tti_shot, dim3(grid), dim3(256), args, 0, s));
-        GEO_TRY(check_launch("tti_shot"));
+        GEO_TRY(plan.run(a, s));
+        a.lev = (a.lev + it1 - it0) & 1;
+        const float *P = a.f[0].P[a.lev];
         const int it = it1 - 1;
         if (snap && it % snap_every == 0 && it != 0)
-            GEO_CUDA(cudaMemcpyAsync(snap + (size_t)(it / snap_every - 1) * n, f.P, n * 4, kout, s));
-        const int w = wd.check(f.P, n, it, it == nt - 1, s);
+            GEO_CUDA(cudaMemcpy2DAsync(snap + (size_t)(it / snap_every - 1) * nnx * nnz, (size_t)nnz * 4, P, (size_t)ldz * 4,
+                                       (size_t)nnz * 4, nnx, kout, s));
+        const int w = wd.check(P, n, it, it == nt - 1, s);
         if (w == GEO_ERR_NAN) break;
         GEO_TRY(w);
         it0 = it1;
@@ -257,7 +185,7 @@ extern "C" int geo_tti2d_shot(const geo_fd2d_desc *desc, const float *v, const f
     int err = 0;
     GEO_CUDA(cudaMemcpyAsync(&err, a.err, 4, cudaMemcpyDeviceToHost, s));
     GEO_CUDA(cudaStreamSynchronize(s));
-    if (err) return fail(GEO_ERR_CUDA, "2D TTI shot: a grid barrier wait timed out");
+    if (err) return fail(GEO_ERR_CUDA, "2D TTI shot: a device-side wait timed out");
     GEO_TRY(wd.verdict(s, "2D TTI shot"));
     GEO_CUDA(cudaMemcpyAsync(shot, drec, (size_t)nx * nt * 4, kout, s));
     GEO_CUDA(cudaStreamSynchronize(s));

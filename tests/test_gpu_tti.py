@@ -138,3 +138,28 @@ def test_rtm2d_tti_program_observed_shots_device(geo, orc):
     assert out["mig_lap"].is_cuda
     assert np.array_equal(out["mig_lap"].cpu().numpy(), orc.laplace2d_adj(mig))
     assert np.array_equal(out["adcigs"].cpu().numpy(), ag)
+
+
+# the fused steps' tiles (64 deep, 8 columns, 16 in the last): grids that end
+# at, before and after their edges
+@pytest.mark.parametrize("nx,nz,npd", [(2, 2, 5), (6, 54, 5), (7, 53, 5), (21, 108, 10), (22, 109, 10), (700, 390, 5)])
+def test_tti2d_tile_edges(geo, orc, nx, nz, npd):
+    v, e, d, th = _model(nx=nx, nz=nz, seed=7)
+    kw = dict(KW, npd=npd, nt=45, fs=max(1, nx // 2), zs=1)
+    ref, rs = orc.tti2d(v, e, d, th, sv=1, snap_every=15, trig=cuda_trig(th), **kw)
+    out, snaps = geo.tti2d_shot(v, e, d, th, sv=1, snap_every=15, **kw)
+    assert np.abs(rs).max() > 0
+    assert np.array_equal(out, ref) and np.array_equal(snaps, rs), rel_l2(snaps, rs)
+
+
+@pytest.mark.parametrize("nx,nz,npml", [(44, 44, 10), (47, 53, 6), (60, 118, 5)])
+def test_rtm2d_tti_program_tile_edges(geo, orc, nx, nz, npml):
+    v, e, d, th = _model(nx=nx, nz=nz, seed=8)
+    kw = dict(TKW, npml=npml, ns=1, fs=nx // 2, zs=4, nt=200)
+    mig, ill, ag, shots = orc.rtm2d_tti(v, e, d, th, dcdp=2, trig=cuda_trig(th),
+                                        **cuda_angle_tables(kw["dangle"]), **kw)
+    out = geo.rtm2d_tti(v, e, d, th, dcdp=2, **kw)
+    assert np.abs(ill).max() > 0
+    assert np.array_equal(out["shots"], shots) and np.array_equal(out["illum"], ill)
+    assert np.array_equal(out["mig_lap"], orc.laplace2d_adj(mig))
+    assert np.array_equal(out["adcigs"], ag)
