@@ -17,8 +17,8 @@
 // results are bit-identical to it.
 //
 // Two kernels per step, each marching along y over a 32(z) x 16(x) column
-// and a chunk of planes, two x columns per thread, every read through a
-// 3-stage TMA ring (one mbarrier per stage, waits bounded at 2 s like the
+// and a chunk of planes, two consecutive depths per thread (8-byte accesses
+// throughout), every read through a 3-stage TMA ring (one mbarrier per stage, waits bounded at 2 s like the
 // VTI step's), writes as plain coalesced stores:
 //
 //   velocity: x and z taps of P and Q from a halo box of the output plane
@@ -29,6 +29,13 @@
 //     plane, y taps from queues fed three planes ahead; P, Q of the old
 //     level, the model and the trig as own boxes; receivers and the RTM
 //     imaging epilogue.
+//
+// 300x300x200 + 40: velocity 357 -> 325 us, stress 500 -> 418 us a step
+// against two x columns per thread with 4-byte accesses (six derivatives of 16
+// shared-memory loads a point became five of 6.5) and four chunks whatever the
+// grid.  The velocity kernel runs at 6.0 TB/s of its 48 B a point; the stress
+// kernel (56 B a point, 283 instructions) is bound by issue at 16 warps per SM
+// as much as by memory.
 //
 // The point source is added to P,Q of the old level before the velocity
 // kernel (the cell's old values kept in `save` for the stress update), so
@@ -106,6 +113,51 @@ __device__ __forceinline__ float *align128(unsigned char *p) {
     return reinterpret_cast<float *>((reinterpret_cast<uintptr_t>(p) + 127) & ~uintptr_t(127));
 }
 
+// Two consecutive depths.
+__device__ __forceinline__ float2 lds2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
+__device__ __forceinline__ float &at2(float2 &v, int j) { return j ? v.y : v.x; }
+__device__ __forceinline__ void push(float2 *q, float2 v) {
+#pragma unroll
+    for (int k = 0; k < 7; k++) q[k] = q[k + 1];
+    q[7] = v;
+}
+// sum_m c_m (a_m - b_m), accumulated from 0 as the oracle does
+__device__ __forceinline__ float d8(float a0, float b0, float a1, float b1, float a2, float b2, float a3, float b3) {
+    float d = 0.0f;
+    d += c_tti3d[0] * (a0 - b0);
+    d += c_tti3d[1] * (a1 - b1);
+    d += c_tti3d[2] * (a2 - b2);
+    d += c_tti3d[3] * (a3 - b3);
+    return d;
+}
+// over eight pairs -3 .. +4 (forward stagger) or -4 .. +3 (backward)
+__device__ __forceinline__ float2 dq8(const float2 *q) {
+    return make_float2(d8(q[4].x, q[3].x, q[5].x, q[2].x, q[6].x, q[1].x, q[7].x, q[0].x),
+                       d8(q[4].y, q[3].y, q[5].y, q[2].y, q[6].y, q[1].y, q[7].y, q[0].y));
+}
+// along x at the pair p, columns `pitch` apart; SHIFT 1 forward, 0 backward
+template <int SHIFT>
+__device__ __forceinline__ float2 dx8(const float *p, int pitch) {
+    float2 q[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) q[k] = lds2(p + (k - 4 + SHIFT) * pitch);
+    return dq8(q);
+}
+// along z at the pair p
+template <int SHIFT>
+__device__ __forceinline__ float2 dz8(const float *p) {
+    float e[10];
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        const float2 t = lds2(p - 4 + 2 * k);
+        e[2 * k] = t.x;
+        e[2 * k + 1] = t.y;
+    }
+    const float *a = e + 4 + SHIFT, *b = a + 1;
+    return make_float2(d8(a[0], a[-1], a[1], a[-2], a[2], a[-3], a[3], a[-4]),
+                       d8(b[0], b[-1], b[1], b[-2], b[2], b[-3], b[3], b[-4]));
+}
+
 // Wait for stage s of iteration i; on a timeout report, let the copies in
 // flight land (bounded) and tell the caller to return.
 __device__ __forceinline__ bool stage_ready(uint64_t *bar, int s, uint32_t &phase, int *s_abort, int tid, int *err) {
@@ -175,65 +227,50 @@ __global__ void __launch_bounds__(TZ *NW, 2)
     if (lane == 0 && wy < 4)
         for (int i = 0; i < NST && i < NI; i++) issue(i);
 
-    const int ca = 2 * wy, xa = x0 + ca, zo = z0 + lane;
-    const bool z_upd = zo >= 4 && zo < g.nnz - 4;
-    const bool upd_a = z_upd && xa >= 4 && xa < g.nnx - 4, upd_b = z_upd && xa + 1 >= 4 && xa + 1 < g.nnx - 4;
-    const int xca = min(max(xa, 0), g.nnx - 1), xcb = min(max(xa + 1, 0), g.nnx - 1), zc = min(max(zo, 0), g.nnz - 1);
-    const float c1a = g.cx1[xca], c2a = g.cx2[xca], c1b = g.cx1[xcb], c2b = g.cx2[xcb];
-    const float c1z = g.cz1[zc], c2z = g.cz2[zc];
-    const int oa = ca * 32 + lane;          // own box index of column a (b: +32)
-    const int col_a = zo + g.ldz * xa;      // global index of column a at y = 0 (b: + ldz)
-    float pa[8], pb[8], qa[8], qb[8];
+    const int c = 2 * wy + (lane >> 4), zl = 2 * (lane & 15), xa = x0 + c, zo = z0 + zl;
+    const bool x_upd = xa >= 4 && xa < g.nnx - 4;
+    const bool upd[2] = {x_upd && zo >= 4 && zo < g.nnz - 4, x_upd && zo + 1 >= 4 && zo + 1 < g.nnz - 4};
+    const int xc = min(xa, g.nnx - 1), zc0 = min(zo, g.nnz - 1), zc1 = min(zo + 1, g.nnz - 1);
+    const float c1x = g.cx1[xc], c2x = g.cx2[xc], c1z[2] = {g.cz1[zc0], g.cz1[zc1]}, c2z[2] = {g.cz2[zc0], g.cz2[zc1]};
+    const int o = c * TZ + zl, h = (c + 4) * 40 + zl + 4;   // the pair in own and halo boxes
+    const int col = zo + g.ldz * xa;                        // global index of the pair at y = 0
+    float2 pq[8], qq[8];
 #pragma unroll
-    for (int k = 0; k < 8; k++) pa[k] = pb[k] = qa[k] = qb[k] = 0.0f;
+    for (int k = 0; k < 8; k++) pq[k] = qq[k] = make_float2(0.0f, 0.0f);
     uint32_t phase = 0;
     for (int i = 0; i < NI; i++) {
         const int s = i % NST;
         if (!stage_ready(bar, s, phase, &s_abort, tid, g.err)) return;
         if (lane == 0 && wy < 4 && i >= 1 && i - 1 + NST < NI) issue(i - 1 + NST);
         const float *sp = stages + s * VSTAGE;
-#pragma unroll
-        for (int k = 0; k < 7; k++) {
-            pa[k] = pa[k + 1]; pb[k] = pb[k + 1];
-            qa[k] = qa[k + 1]; qb[k] = qb[k + 1];
-        }
-        pa[7] = sp[V_PO + oa]; pb[7] = sp[V_PO + oa + 32];
-        qa[7] = sp[V_QO + oa]; qb[7] = sp[V_QO + oa + 32];
+        push(pq, lds2(sp + V_PO + o));
+        push(qq, lds2(sp + V_QO + o));
         if (i < 7) continue;
         const int y = ylo + i - 7;
         const float cy1 = __ldg(g.cy1 + y), cy2 = __ldg(g.cy2 + y);
+        float2 Px = dx8<1>(sp + V_PH + h, 40), Py = dq8(pq), Pz = dz8<1>(sp + V_PH + h);
+        float2 Qx = dx8<1>(sp + V_QH + h, 40), Qy = dq8(qq), Qz = dz8<1>(sp + V_QH + h);
+        float2 ct = lds2(sp + V_T + o), st = lds2(sp + V_T + OB + o), cp = lds2(sp + V_T + 2 * OB + o),
+               sn2 = lds2(sp + V_T + 3 * OB + o);
+        float2 u = lds2(sp + V_U + o), v = lds2(sp + V_U + OB + o), w = lds2(sp + V_U + 2 * OB + o);
 #pragma unroll
-        for (int cb = 0; cb < 2; cb++) {
-            const float *pq = cb ? pb : pa, *qq = cb ? qb : qa;
-            const float *PH = sp + V_PH + (ca + cb + 4) * 40 + lane + 4;   // the point in the P halo box
-            const float *QH = sp + V_QH + (ca + cb + 4) * 40 + lane + 4;
-            float Px = 0.0f, Py = 0.0f, Pz = 0.0f, Qx = 0.0f, Qy = 0.0f, Qz = 0.0f;
-#pragma unroll
-            for (int im = 0; im < 4; im++) {
-                const float c = c_tti3d[im];
-                Px += c * (PH[(im + 1) * 40] - PH[-im * 40]);
-                Py += c * (pq[im + 4] - pq[3 - im]);
-                Pz += c * (PH[im + 1] - PH[-im]);
-                Qx += c * (QH[(im + 1) * 40] - QH[-im * 40]);
-                Qy += c * (qq[im + 4] - qq[3 - im]);
-                Qz += c * (QH[im + 1] - QH[-im]);
-            }
-            const int o = oa + 32 * cb;
-            const float a = sp[V_T + o], b = sp[V_T + OB + o], cc = sp[V_T + 2 * OB + o], sn = sp[V_T + 3 * OB + o];
-            const float k2 = (cb ? c2b : c2a) * cy2 * c2z;
-            const float k1 = (cb ? c1b : c1a) * cy1 * c1z;
-            const float gx = a * cc * g.dtx * Px + a * sn * g.dty * Py - b * g.dtz * Pz;
-            const float gy = cc * g.dty * Py - sn * g.dtx * Px;
-            const float gz = b * cc * g.dtx * Qx + b * sn * g.dty * Qy + a * g.dtz * Qz;
-            const float un = k2 * sp[V_U + o] - k1 * gx;
-            const float vn = k2 * sp[V_U + OB + o] - k1 * gy;
-            const float wn = k2 * sp[V_U + 2 * OB + o] - k1 * gz;
-            if (cb ? upd_b : upd_a) {
-                const int id = col_a + cb * g.ldz + g.sxy * y;
-                u1[id] = un;
-                v1[id] = vn;
-                w1[id] = wn;
-            }
+        for (int j = 0; j < 2; j++) {
+            const float a = at2(ct, j), b = at2(st, j), cc = at2(cp, j), sn = at2(sn2, j);
+            const float k2 = c2x * cy2 * c2z[j];
+            const float k1 = c1x * cy1 * c1z[j];
+            const float gx = a * cc * g.dtx * at2(Px, j) + a * sn * g.dty * at2(Py, j) - b * g.dtz * at2(Pz, j);
+            const float gy = cc * g.dty * at2(Py, j) - sn * g.dtx * at2(Px, j);
+            const float gz = b * cc * g.dtx * at2(Qx, j) + b * sn * g.dty * at2(Qy, j) + a * g.dtz * at2(Qz, j);
+            // points off the updated grid keep their zeros
+            at2(u, j) = upd[j] ? k2 * at2(u, j) - k1 * gx : 0.0f;
+            at2(v, j) = upd[j] ? k2 * at2(v, j) - k1 * gy : 0.0f;
+            at2(w, j) = upd[j] ? k2 * at2(w, j) - k1 * gz : 0.0f;
+        }
+        if (upd[0] || upd[1]) {
+            const int id = col + g.sxy * y;
+            *reinterpret_cast<float2 *>(u1 + id) = u;
+            *reinterpret_cast<float2 *>(v1 + id) = v;
+            *reinterpret_cast<float2 *>(w1 + id) = w;
         }
     }
 }
@@ -290,105 +327,93 @@ __global__ void __launch_bounds__(TZ *NW, 2)
     if (lane == 0 && wy < 4)
         for (int i = 0; i < NST && i < NI; i++) issue(i);
 
-    const int ca = 2 * wy, xa = x0 + ca, zo = z0 + lane;
-    const bool z_upd = zo >= 4 && zo < g.nnz - 4;
-    const bool upd_a = z_upd && xa >= 4 && xa < g.nnx - 4, upd_b = z_upd && xa + 1 >= 4 && xa + 1 < g.nnx - 4;
-    const int xca = min(max(xa, 0), g.nnx - 1), xcb = min(max(xa + 1, 0), g.nnx - 1), zc = min(max(zo, 0), g.nnz - 1);
-    const float a1a = g.ax1[xca], a2a = g.ax2[xca], a1b = g.ax1[xcb], a2b = g.ax2[xcb];
-    const float a1z = g.az1[zc], a2z = g.az2[zc];
-    const bool z_in = zo >= g.npd && zo < g.npd + g.nz;
-    const bool in_a = z_in && xa >= g.npd && xa < g.npd + g.nx, in_b = z_in && xa + 1 >= g.npd && xa + 1 < g.npd + g.nx;
-    int rec_a = -1, rec_b = -1;
-    if (st.rec && zo == st.rec_iz) {
-        const int ra = xa - g.npd - st.rx0, rb = ra + 1;
-        if (ra >= 0 && ra % st.drx == 0 && ra / st.drx < st.nrx) rec_a = ra / st.drx;
-        if (rb >= 0 && rb % st.drx == 0 && rb / st.drx < st.nrx) rec_b = rb / st.drx;
+    const int c = 2 * wy + (lane >> 4), zl = 2 * (lane & 15), xa = x0 + c, zo = z0 + zl;
+    const bool x_upd = xa >= 4 && xa < g.nnx - 4;
+    const bool upd[2] = {x_upd && zo >= 4 && zo < g.nnz - 4, x_upd && zo + 1 >= 4 && zo + 1 < g.nnz - 4};
+    const int xc = min(xa, g.nnx - 1), zc0 = min(zo, g.nnz - 1), zc1 = min(zo + 1, g.nnz - 1);
+    const float a1x = g.ax1[xc], a2x = g.ax2[xc], a1z[2] = {g.az1[zc0], g.az1[zc1]}, a2z[2] = {g.az2[zc0], g.az2[zc1]};
+    const bool x_in = xa >= g.npd && xa < g.npd + g.nx;
+    const bool in[2] = {x_in && upd[0] && zo >= g.npd && zo < g.npd + g.nz,
+                        x_in && upd[1] && zo + 1 >= g.npd && zo + 1 < g.npd + g.nz};
+    int rec_x = -1;
+    const int rec_j = st.rec_iz - zo;
+    if (st.rec && (rec_j == 0 || rec_j == 1) && upd[rec_j]) {
+        const int r = xa - g.npd - st.rx0;
+        if (r >= 0 && r % st.drx == 0 && r / st.drx < st.nrx) rec_x = r / st.drx;
     }
-    const int oa = ca * 32 + lane;
-    const int col_a = zo + g.ldz * xa;
-    float ua[8], ub[8], va[8], vb[8], wa[8], wb[8];
+    const int o = c * TZ + zl, h = (c + 4) * 40 + zl + 4;
+    const int col = zo + g.ldz * xa;
+    float2 uq[8], vq[8], wq[8];
 #pragma unroll
-    for (int k = 0; k < 8; k++) ua[k] = ub[k] = va[k] = vb[k] = wa[k] = wb[k] = 0.0f;
+    for (int k = 0; k < 8; k++) uq[k] = vq[k] = wq[k] = make_float2(0.0f, 0.0f);
     uint32_t phase = 0;
     for (int i = 0; i < NI; i++) {
         const int s = i % NST;
         if (!stage_ready(bar, s, phase, &s_abort, tid, g.err)) return;
         if (lane == 0 && wy < 4 && i >= 1 && i - 1 + NST < NI) issue(i - 1 + NST);
         const float *sp = stages + s * SSTAGE;
-#pragma unroll
-        for (int k = 0; k < 7; k++) {
-            ua[k] = ua[k + 1]; ub[k] = ub[k + 1];
-            va[k] = va[k + 1]; vb[k] = vb[k + 1];
-            wa[k] = wa[k + 1]; wb[k] = wb[k + 1];
-        }
-        ua[7] = sp[S_UO + oa]; ub[7] = sp[S_UO + oa + 32];
-        va[7] = sp[S_UO + OB + oa]; vb[7] = sp[S_UO + OB + oa + 32];
-        wa[7] = sp[S_UO + 2 * OB + oa]; wb[7] = sp[S_UO + 2 * OB + oa + 32];
+        push(uq, lds2(sp + S_UO + o));
+        push(vq, lds2(sp + S_UO + OB + o));
+        push(wq, lds2(sp + S_UO + 2 * OB + o));
         if (i < 7) continue;
         const int y = ylo + i - 7;
         const float ay1 = __ldg(g.ay1 + y), ay2 = __ldg(g.ay2 + y);
         const bool y_in = y >= g.npd && y < g.npd + g.ny;
+        const int id = col + g.sxy * y;
         // RTM operands of this plane, loaded before the arithmetic
         float pre_ill[2] = {0.0f, 0.0f}, pre_mig[2] = {0.0f, 0.0f}, pre_oth[2] = {0.0f, 0.0f};
+        const long io = (long)(zo - g.npd) + (long)g.nz * ((xa - g.npd) + (long)g.nx * (y - g.npd));
         if ((st.ill || st.mig) && y_in) {
 #pragma unroll
-            for (int cb = 0; cb < 2; cb++) {
-                if (!(cb ? in_b : in_a)) continue;
-                const long o = (long)(zo - g.npd) + (long)g.nz * ((xa + cb - g.npd) + (long)g.nx * (y - g.npd));
-                if (st.ill) pre_ill[cb] = st.ill[o];
+            for (int j = 0; j < 2; j++) {
+                if (!in[j]) continue;
+                if (st.ill) pre_ill[j] = st.ill[io + j];
                 if (st.mig) {
-                    pre_mig[cb] = st.mig[o];
-                    pre_oth[cb] = st.other_P[col_a + cb * g.ldz + g.sxy * y];
+                    pre_mig[j] = st.mig[io + j];
+                    pre_oth[j] = st.other_P[id + j];
                 }
             }
         }
+        float2 ux = dx8<0>(sp + S_UH + h, 40), uy = dq8(uq), uz = dz8<0>(sp + S_UH + h);
+        float2 vx = dx8<0>(sp + S_VH + (c + 4) * 32 + zl, 32), vy = dq8(vq);
+        float2 wx = dx8<0>(sp + S_WH + h, 40), wy_ = dq8(wq), wz = dz8<0>(sp + S_WH + h);
+        float2 ct = lds2(sp + S_T + o), st_ = lds2(sp + S_T + OB + o), cp = lds2(sp + S_T + 2 * OB + o),
+               sn2 = lds2(sp + S_T + 3 * OB + o);
+        float2 p0 = lds2(sp + S_PQ + o), q0 = lds2(sp + S_PQ + OB + o);
+        float2 mA = lds2(sp + S_M + o), mB = lds2(sp + S_M + OB + o), mC = lds2(sp + S_M + 2 * OB + o);
+        if (st.src_on && (id == st.src || id + 1 == st.src)) {
+            at2(p0, (int)(st.src - id)) = save[0];
+            at2(q0, (int)(st.src - id)) = save[1];
+        }
+        float2 P, Q;
 #pragma unroll
-        for (int cb = 0; cb < 2; cb++) {
-            const float *uq = cb ? ub : ua, *vq = cb ? vb : va, *wq = cb ? wb : wa;
-            const float *UH = sp + S_UH + (ca + cb + 4) * 40 + lane + 4;
-            const float *VH = sp + S_VH + (ca + cb + 4) * 32 + lane;
-            const float *WH = sp + S_WH + (ca + cb + 4) * 40 + lane + 4;
-            float ux = 0.0f, uy = 0.0f, uz = 0.0f, vx = 0.0f, vy = 0.0f, wx = 0.0f, wy_ = 0.0f, wz = 0.0f;
+        for (int j = 0; j < 2; j++) {
+            const float a = at2(ct, j), b = at2(st_, j), cc = at2(cp, j), sn = at2(sn2, j);
+            const float ha = (a * cc * g.dtx * at2(ux, j) + a * sn * g.dty * at2(uy, j) - b * g.dtz * at2(uz, j)) +
+                             (cc * g.dty * at2(vy, j) - sn * g.dtx * at2(vx, j));
+            const float hb = b * cc * g.dtx * at2(wx, j) + b * sn * g.dty * at2(wy_, j) + a * g.dtz * at2(wz, j);
+            const float k2 = a2x * ay2 * a2z[j];
+            const float k1 = a1x * ay1 * a1z[j];
+            at2(P, j) = upd[j] ? k2 * at2(p0, j) - k1 * (at2(mA, j) * ha + at2(mB, j) * hb) : 0.0f;
+            at2(Q, j) = upd[j] ? k2 * at2(q0, j) - k1 * (at2(mB, j) * ha + at2(mC, j) * hb) : 0.0f;
+        }
+        if (!(upd[0] || upd[1])) continue;
+        *reinterpret_cast<float2 *>(P1 + id) = P;
+        *reinterpret_cast<float2 *>(Q1 + id) = Q;
+        if (rec_x >= 0) {
+            const int ry = y - g.npd - st.ry0;
+            if (ry >= 0 && ry % st.dry == 0 && ry / st.dry < st.nry) {
+                const float p = rec_j ? P.y : P.x, q = rec_j ? Q.y : Q.x;
+                st.rec[(long)st.it * st.nrx * st.nry + rec_x + (long)st.nrx * (ry / st.dry)] = st.rec_pq ? p + q : p;
+            }
+        }
+        if ((st.ill || st.mig) && y_in) {
 #pragma unroll
-            for (int im = 0; im < 4; im++) {
-                const float c = c_tti3d[im];
-                ux += c * (UH[im * 40] - UH[-(im + 1) * 40]);
-                uy += c * (uq[im + 4] - uq[3 - im]);
-                uz += c * (UH[im] - UH[-im - 1]);
-                vx += c * (VH[im * 32] - VH[-(im + 1) * 32]);
-                vy += c * (vq[im + 4] - vq[3 - im]);
-                wx += c * (WH[im * 40] - WH[-(im + 1) * 40]);
-                wy_ += c * (wq[im + 4] - wq[3 - im]);
-                wz += c * (WH[im] - WH[-im - 1]);
-            }
-            const int o = oa + 32 * cb;
-            const float a = sp[S_T + o], b = sp[S_T + OB + o], cc = sp[S_T + 2 * OB + o], sn = sp[S_T + 3 * OB + o];
-            const float ha = (a * cc * g.dtx * ux + a * sn * g.dty * uy - b * g.dtz * uz) + (cc * g.dty * vy - sn * g.dtx * vx);
-            const float hb = b * cc * g.dtx * wx + b * sn * g.dty * wy_ + a * g.dtz * wz;
-            const float k2 = (cb ? a2b : a2a) * ay2 * a2z;
-            const float k1 = (cb ? a1b : a1a) * ay1 * a1z;
-            const long id = (long)col_a + cb * g.ldz + (long)g.sxy * y;
-            float p0 = sp[S_PQ + o], q0 = sp[S_PQ + OB + o];
-            if (st.src_on && id == st.src) {
-                p0 = save[0];
-                q0 = save[1];
-            }
-            const float mA = sp[S_M + o], mB = sp[S_M + OB + o], mC = sp[S_M + 2 * OB + o];
-            const float P = k2 * p0 - k1 * (mA * ha + mB * hb);
-            const float Q = k2 * q0 - k1 * (mB * ha + mC * hb);
-            if (!(cb ? upd_b : upd_a)) continue;
-            P1[id] = P;
-            Q1[id] = Q;
-            const int rix = cb ? rec_b : rec_a;
-            if (rix >= 0) {
-                const int ry = y - g.npd - st.ry0;
-                if (ry >= 0 && ry % st.dry == 0 && ry / st.dry < st.nry)
-                    st.rec[(long)st.it * st.nrx * st.nry + rix + (long)st.nrx * (ry / st.dry)] = st.rec_pq ? P + Q : P;
-            }
-            if ((st.ill || st.mig) && (cb ? in_b : in_a) && y_in) {
-                const long o2 = (long)(zo - g.npd) + (long)g.nz * ((xa + cb - g.npd) + (long)g.nx * (y - g.npd));
-                if (st.ill) st.ill[o2] = pre_ill[cb] + (P * P + Q * Q);
-                if (st.mig) st.mig[o2] = pre_mig[cb] + pre_oth[cb] * P;
+            for (int j = 0; j < 2; j++) {
+                if (!in[j]) continue;
+                const float p = j ? P.y : P.x, q = j ? Q.y : Q.x;
+                if (st.ill) st.ill[io + j] = pre_ill[j] + (p * p + q * q);
+                if (st.mig) st.mig[io + j] = pre_mig[j] + pre_oth[j] * p;
             }
         }
     }
@@ -460,9 +485,30 @@ int tti_maps(const Tti3DStep &t, const MapPair **out) {
     return GEO_OK;
 }
 
-int tti_chunks() {
-    const char *e = getenv("GEO_TTI3D_CHUNKS");
-    return e ? std::max(1, atoi(e)) : 4;
+// y chunks of a tile column: the fewest rounds of resident blocks (two per
+// SM) times a chunk's planes, the seven that only fill the queues counted as
+// two.  300x300x200 + 40: 4 chunks (2.8 rounds of blocks) take 757 us a step, 7
+// (5.0) 743, 5 (3.6) 788, 1 (0.7) 1008.
+int tti_chunks(int tiles, int planes) {
+    static int sms = 0;
+    if (const char *e = getenv("GEO_TTI3D_CHUNKS")) return std::max(1, std::min(atoi(e), planes / 8));
+    if (!sms) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+            sms = 152;
+    }
+    int best = 1;
+    long cost = 0;
+    for (int n = 1; n <= 16 && n <= std::max(1, planes / 8); n++) {
+        const int chunk = (planes + n - 1) / n, blocks = tiles * ((planes + chunk - 1) / chunk);
+        const long c = (long)((blocks + 2 * sms - 1) / (2 * sms)) * (chunk + 2);
+        if (!cost || c < cost) {
+            cost = c;
+            best = n;
+        }
+    }
+    return best;
 }
 
 }  // namespace
@@ -493,7 +539,7 @@ int launch_tti3d(const Tti3DStep &t, const StepArgs3D &args, cudaStream_t s) {
     G.ntz = (g.nnz + TZ - 1) / TZ;
     G.ntiles = G.ntz * ((g.nnx + TX - 1) / TX);
     const int planes = g.nny - 8;
-    const int nch = std::max(1, std::min(tti_chunks(), planes / 8));
+    const int nch = std::max(1, tti_chunks(G.ntiles, planes));
     G.chunk = (planes + nch - 1) / nch;
     const int nchunks = (planes + G.chunk - 1) / G.chunk;
     G.err = t.err;

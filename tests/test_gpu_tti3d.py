@@ -91,3 +91,21 @@ def test_tti3d_rtm_bit_exact(geo, orc, method):
     assert np.array_equal(mig, mig_ref), rel_l2(mig, mig_ref)
     mig64, _, _ = orc.rtm3d(v, e, d, theta=th, phi=ph, snap_every=snap, prec=64, **kw)
     assert rel_l2(mig, mig64) < 1e-4   # measured 2.6e-6 - 3.4e-6
+
+
+# depths and columns that end at, before and after a tile (32 deep, 16 wide;
+# the last updated depth alone in its pair or not), chunks of few planes
+@pytest.mark.parametrize("ny,nx,nz,npd", [(7, 16, 16, 8), (9, 17, 17, 8), (24, 15, 15, 8), (40, 3, 47, 6), (6, 31, 20, 6)])
+def test_tti3d_vectors_and_tile_edges(geo, orc, ny, nx, nz, npd):
+    v, e, d = random_model_3d(nx, ny, nz, seed=9)
+    th, ph = smooth_angles(v.shape, seed=4)
+    kw = dict(KW, npd=npd, nt=50, fsx=max(1, nx // 2), fsy=max(1, ny // 2), fsz=2)
+    ref, rp, rq = orc.fd3d(v, e, d, theta=th, phi=ph, final=True, **kw)
+    plan = geo.FD3DPlan(nx=nx, ny=ny, nz=nz, mode="fast", **kw)
+    plan.set_model(v, e, d)
+    plan.set_tilt(th, ph)
+    out = plan.run_shot(0)
+    P, Q = plan.fields()
+    plan.close()
+    assert np.abs(rp).max() > 0
+    assert np.array_equal(out, ref) and np.array_equal(P, rp) and np.array_equal(Q, rq)
