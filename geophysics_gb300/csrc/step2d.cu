@@ -582,18 +582,22 @@ __global__ void k_step2d_restore(const __grid_constant__ SStep a, int it, int le
     }
 }
 
-template <bool TTI, int NC>
+template <int NC>
 const void *step_fn(StepKind k) {
     switch (k) {
-        case SK_CPU: return TTI ? nullptr : (const void *)k_step2d<SK_CPU, false, NC>;
-        case SK_GPU: return (const void *)k_step2d<SK_GPU, TTI, NC>;
-        case SK_GFWD: return (const void *)k_step2d<SK_GFWD, TTI, NC>;
-        default: return (const void *)k_step2d<SK_GBWD, TTI, NC>;
+        case SK_CPU: return (const void *)k_step2d<SK_CPU, false, NC>;
+        case SK_GPU: return (const void *)k_step2d<SK_GPU, false, NC>;
+        case SK_GFWD: return (const void *)k_step2d<SK_GFWD, false, NC>;
+        default: return (const void *)k_step2d<SK_GBWD, false, NC>;
     }
 }
 const void *step_fn(StepKind k, bool tti, int tx) {
-    if (tti) return tx == 8 ? step_fn<true, 1>(k) : step_fn<true, 2>(k);
-    return tx == 8 ? step_fn<false, 1>(k) : step_fn<false, 2>(k);
+    if (!tti) return tx == 8 ? step_fn<1>(k) : step_fn<2>(k);
+    switch (k) {
+        case SK_GFWD: return (const void *)k_step2d<SK_GFWD, true, 1>;
+        case SK_GBWD: return (const void *)k_step2d<SK_GBWD, true, 1>;
+        default: return tx == 8 ? (const void *)k_step2d<SK_GPU, true, 1> : (const void *)k_step2d<SK_GPU, true, 2>;
+    }
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 g_enc = nullptr;
@@ -637,16 +641,17 @@ int Fused2D::model(const SGrid &g, const float *p, const float *trig) {
     return box_map(&mm, p, g, kTz, tx, 3);
 }
 
-// Tiles of 8 columns (three blocks per SM) or 16 (two; a quarter less halo
-// work): the fewer rounds of resident blocks weighted by what a round takes,
-// 2.5 and 3.1 us at 1700x601.  601 deep: 2401 columns 20.8 us a step with 8
-// and 20.1 with 16, 600 columns 8.7 and 8.6, 300 columns 6.9 and 6.1, the
-// RTM program's 1700 forward 17.6 and 18.1; 101x121 4.0 and 4.8.  One stage
-// where every tile has its own block, two where blocks walk several.  TTI
-// tiles are heavier and always take one stage (three blocks per SM instead of
-// two beat the prefetch); a TTI shot goes by the busiest SM's columns with
-// their halo: 600x300 9.0 us a step with 8 and 8.4 with 16, 1500x600 22.1 and
-// 20.2, 200x150 4.5 and 5.5.
+// Tiles of 8 columns (three or four blocks per SM) or 16 (two; a quarter less
+// halo work): the fewer columns on the busiest SM, each tile's halo counted as
+// one (VTI) or six (TTI, whose halos cost both velocities).  us a step with 8
+// and with 16: VTI 601 deep 2401 wide 20.8 and 20.1, 600 8.7 and 8.6, 300 6.9
+// and 6.1, the RTM program's 1700 forward 17.6 and 18.1, 401x401 6.7 and 6.0,
+// 250x250 4.9 and 4.8, 101x121 4.0 and 4.8; TTI 600x300 9.0 and 8.4, 1500x600
+// 22.1 and 20.2, 200x150 4.5 and 5.5.  The TTI RTM passes take 8: 1100x450
+// 15.2 and 16.4 forward, 31.3 and 37.8 backward.  VTI takes one stage where
+// every tile has its own block, two where blocks walk several; TTI tiles are
+// heavier and always take one (three blocks per SM instead of two beat the
+// prefetch).
 int Fused2D::plan(StepKind k, bool tti_, const SGrid &g, int fixed) {
     kind = k;
     tti = tti_;
@@ -659,15 +664,14 @@ int Fused2D::plan(StepKind k, bool tti_, const SGrid &g, int fixed) {
     for (int nc = 1; nc <= 2 && coop; nc++) {
         const int t = nc * kThreads / 32;
         const void *fn = step_fn(k, tti, t);
-        if (fixed && t != fixed) continue;
+        if (fixed ? t != fixed : tti && k != SK_GPU && t != 8) continue;
         const int n = ((g.nnz + kTz - 1) / kTz) * ((g.nnx + t - 1) / t);
         GEO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)step_smem(t, 2, tti)));
         for (int st = k == SK_GBWD && !tti ? 2 : 1; st <= 2; st++) {
             int occ = 0;
             GEO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kThreads, step_smem(t, st, tti)));
             if (occ < 1 || (st == 1 && !tti && n > occ * sms)) continue;
-            const long slots = (long)occ * sms;
-            const long cost = tti && k == SK_GPU ? (n + sms - 1L) / sms * (t + 6) : (n + slots - 1) / slots * (nc == 1 ? 4 : 5);
+            const long cost = (n + sms - 1L) / sms * (t + (tti ? 6 : 1));
             if (!best || cost < best) {
                 best = cost;
                 tx = t;
