@@ -30,7 +30,7 @@
 //     level, the model and the trig as own boxes; receivers and the RTM
 //     imaging epilogue.
 //
-// 300x300x200 + 40: velocity 357 -> 325 us, stress 500 -> 418 us a step
+// 300x300x200 + 40: velocity 357 -> 321 us, stress 500 -> 408 us a step
 // against two x columns per thread with 4-byte accesses (six derivatives of 16
 // shared-memory loads a point became five of 6.5) and four chunks whatever the
 // grid.  The velocity kernel runs at 6.0 TB/s of its 48 B a point; the stress
@@ -123,8 +123,7 @@ __device__ __forceinline__ void push(float2 *q, float2 v) {
 }
 // sum_m c_m (a_m - b_m), accumulated from 0 as the oracle does
 __device__ __forceinline__ float d8(float a0, float b0, float a1, float b1, float a2, float b2, float a3, float b3) {
-    float d = 0.0f;
-    d += c_tti3d[0] * (a0 - b0);
+    float d = __fmaf_rn(c_tti3d[0], a0 - b0, 0.0f);   // 0 + c s in one instruction: the same value
     d += c_tti3d[1] * (a1 - b1);
     d += c_tti3d[2] * (a2 - b2);
     d += c_tti3d[3] * (a3 - b3);
@@ -487,8 +486,8 @@ int tti_maps(const Tti3DStep &t, const MapPair **out) {
 
 // y chunks of a tile column: the fewest rounds of resident blocks (two per
 // SM) times a chunk's planes, the seven that only fill the queues counted as
-// two.  300x300x200 + 40: 4 chunks (2.8 rounds of blocks) take 757 us a step, 7
-// (5.0) 743, 5 (3.6) 788, 1 (0.7) 1008.
+// two.  300x300x200 + 40: 4 chunks (2.8 rounds of blocks) take 745 us a step, 7
+// (5.0) 731, 5 (3.6) 776, 1 (0.7) 996.
 int tti_chunks(int tiles, int planes) {
     static int sms = 0;
     if (const char *e = getenv("GEO_TTI3D_CHUNKS")) return std::max(1, std::min(atoi(e), planes / 8));
