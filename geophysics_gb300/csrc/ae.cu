@@ -2,14 +2,16 @@
 //
 // Inference (snapshot encode in the forward pass of RTM, decode + imaging in
 // the backward pass):
-//   k_ae_e1_vol  gather one 16^3 block of the wavefield into Morton order,
-//                scale by its max |value|, level E1 (8 -> 16) on CUDA cores;
-//   tc_gemm x3   E2, E3, E4 on tcgen05 (the last one writes the bf16 code);
-//   tc_gemm x3   D4, D3, D2 on tcgen05;
-//   k_ae_d1_vol  level D1 (16 -> 8), unscale, scatter back to the field order
-//                and either store the snapshot or add its product with the
-//                receiver wavefield to the image (or, for the escape check,
-//                compare it with the field).
+//   k_ae_e12     gather the cells of 16^3 blocks of the wavefield, scale by the
+//                block's max |value|, level E1 (8 -> 16) on CUDA cores, E2 on
+//                tcgen05;
+//   tc_gemm x2   E3, E4 on tcgen05 (the last one writes the bf16 code);
+//   tc_gemm x2   D4, D3 on tcgen05;
+//   k_ae_d21     D2 on tcgen05, D1 (16 -> 8) on CUDA cores, unscale, store the
+//                snapshot; or
+//   tc_gemm, k_ae_d1_vol  D2, then D1 with the product with the receiver
+//                wavefield added to the image (or, for the escape check, the
+//                comparison with the field).
 // The snapshot kernels take E1's and D1's weights by value (a host copy kept
 // per weight version), so every weight is an operand of its multiply-add.
 // Training (one CUDA graph per iteration): the same forward on blocks drawn
@@ -315,82 +317,382 @@ __global__ void __launch_bounds__(256) k_ae_e1(const E1Args a) {
     }
 }
 
-// Interior-box gather of a snapshot, E1 with the weights passed by value
-// (each weight a constant-bank operand of its multiply-add, no load).
-// Thread t owns depth z = t & 15 of row x = t >> 4 of the block on all
-// sixteen planes y, so its Morton slot is fixed up to the y bits, then nodes t
-// and t + 256; the block's 16 KB of bf16 leave by one bulk store.  Bound by
-// memory (16 KB in, 16 KB out a block) and instruction issue: a 512x512x384
-// snapshot takes 159 us, 5.1 TB/s; 207 us with one scalar multiply-add per
-// weight, four-way bank conflicts in the Morton exchange and half-sector
-// stores.  Five blocks per SM; at six it spills (162 us).
-struct E1Vol {
+// A thread's place in a snapshot: row r of a tile of two blocks (128 rows) is
+// one 4x4x4 cell of block 2 tile + r / 64.  Consecutive rows are Morton
+// neighbours, so a warp's 16-byte accesses at one (x, y) of its cells are whole
+// 64-byte runs of the field's lines.
+struct CellAt {
+    int b, iz, ix, iy;            // block, first point of the cell
+    __device__ __forceinline__ CellAt(const AeVolume &v, int tile, int r) {
+        b = 2 * tile + (r >> 6);
+        const int bz = b % v.nbz, bx = (b / v.nbz) % v.nbx, by = b / (v.nbz * v.nbx);
+        iz = bz * 16 + 4 * ((r & 1) | ((r >> 2) & 2));
+        ix = bx * 16 + 4 * (((r >> 1) & 1) | ((r >> 3) & 2));
+        iy = by * 16 + 4 * (((r >> 2) & 1) | ((r >> 4) & 2));
+    }
+};
+// Whether four consecutive depths of every line are one aligned vector.
+__device__ __forceinline__ bool lines_aligned(const AeVolume &v, const float *p) {
+    return !((reinterpret_cast<uintptr_t>(p + v.oz) & 15) || (v.ldz & 3) || (v.sxy & 3));
+}
+
+// E1 and E2 of a snapshot in one launch: a group of 128 threads takes a tile
+// of two blocks, a thread one cell -- 64 points, eight E1 nodes, one row of
+// E2's operand.  It loads its points, scales them by the block's max, forms E1
+// (packed FP32 multiply-adds, weights by value) and writes the row's 256 bytes
+// as the swizzled shared-memory operand tcgen05 reads; one thread multiplies
+// by E2's weights (resident), and the same threads finish E2 from TMEM and
+// send 32 x 64 boxes out by TMA.  E1's output, 16 KB a block, never leaves the
+// SM.  Persistent, two CTAs of two groups per SM.  Waits are bounded.
+// A 512x512x384 snapshot takes 164 us; E1 and E2 one after the other took 250
+// (159 + 91), E1's output costing 800 MB of traffic.  Bound by instruction
+// issue and the latency of the constant loads at 16 warps per SM (2000
+// instructions a cell, half of them E1's products); the next tile's points are
+// loaded during this one's arithmetic (172 us without).  Weights from shared
+// memory instead, 16 bytes a load: 225 us.
+struct E12Args {
     AeVolume vol;
-    int nb;
-    __nv_bfloat16 *h1;            // [nbp*512 x 16]
+    int nb, tiles;                // blocks of the volume; tiles of two, padding included
     float *scale;                 // [nbp]
+    const float *bias;            // E2's
+    int *err;
     AeSmallW w;
 };
+constexpr int kE12Group = 32768;                             // bytes of a group's operand
+constexpr size_t kE12Smem = 16384 + 2 * kE12Group + 1024;
 
-__global__ void __launch_bounds__(256, 5) k_ae_e1_vol(const E1Vol a) {
-    __shared__ __align__(128) float xs[kAePts];
-    __shared__ float red[8];
-    const int b = blockIdx.x, t = threadIdx.x;
-    float mx = 0.0f;
-    if (b < a.nb) {
+__global__ void __launch_bounds__(256, 2) k_ae_e12(const __grid_constant__ CUtensorMap tw, const __grid_constant__ CUtensorMap to,
+                                                   const __grid_constant__ E12Args a) {
+    extern __shared__ unsigned char smem_raw[];
+    uint8_t *sm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const int grp = threadIdx.x >> 7, r = threadIdx.x & 127, warp = r >> 5, lane = r & 31;
+    uint8_t *A = sm + 16384 + grp * kE12Group;
+    __shared__ __align__(8) float sbias[64];
+    __shared__ float red[2][4];
+    __shared__ __align__(8) uint64_t wbar, done[2];
+    __shared__ uint32_t tslot;
+    __shared__ int s_abort[2];   // of each group: set by its warps, read by all of them after a barrier
+    if (threadIdx.x == 0) {
+        tc::mbar_init(&wbar, 1);
+        tc::mbar_init(&done[0], 1);
+        tc::mbar_init(&done[1], 1);
+        s_abort[0] = s_abort[1] = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        // E2's weights, two slices of 64 inputs
+        tc::mbar_expect_tx(&wbar, 16384);
+        tc::tma2(sm, &tw, 0, 0, &wbar);
+        tc::tma2(sm + 8192, &tw, 64, 0, &wbar);
+    }
+    if (threadIdx.x < 64) sbias[threadIdx.x] = a.bias[threadIdx.x];
+    __syncwarp();
+    if (threadIdx.x < 32) tc::tmem_alloc(&tslot, 128);
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tmem = tslot + grp * 64;
+    if (!tc::mbar_wait(&wbar, 0)) s_abort[0] = s_abort[1] = 1;
+    __syncthreads();
+    const AeVolume &v = a.vol;
+    const bool vec = lines_aligned(v, v.src);
+    float4 f[16];   // line x + 4 y of the thread's cell of tile t
+    auto load = [&](int t) {
+        const CellAt c(v, t, r);
+        const float *p = v.src + (long)(v.oz + c.iz) + v.ldz * (v.ox + c.ix) + v.sxy * (v.oy + c.iy);
+        const bool in = c.b < a.nb;
+        if (vec && in && c.iz + 4 <= v.nz && c.ix + 4 <= v.nx && c.iy + 4 <= v.ny) {
+#pragma unroll
+            for (int q = 0; q < 16; q++) f[q] = __ldg(reinterpret_cast<const float4 *>(p + v.ldz * (q & 3) + v.sxy * (q >> 2)));
+        } else {
+#pragma unroll
+            for (int q = 0; q < 16; q++) {
+                const bool l = in && c.ix + (q & 3) < v.nx && c.iy + (q >> 2) < v.ny;
+                const float *s = p + v.ldz * (q & 3) + v.sxy * (q >> 2);
+                f[q].x = l && c.iz < v.nz ? __ldg(s) : 0.0f;
+                f[q].y = l && c.iz + 1 < v.nz ? __ldg(s + 1) : 0.0f;
+                f[q].z = l && c.iz + 2 < v.nz ? __ldg(s + 2) : 0.0f;
+                f[q].w = l && c.iz + 3 < v.nz ? __ldg(s + 3) : 0.0f;
+            }
+        }
+    };
+    unsigned k = 0;
+    if ((int)blockIdx.x * 2 + grp < a.tiles) load(blockIdx.x * 2 + grp);
+    for (int t = blockIdx.x * 2 + grp; t < a.tiles; t += gridDim.x * 2, k++) {
+        float mx = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 16; q++) mx = fmaxf(mx, fmaxf(fmaxf(fabsf(f[q].x), fabsf(f[q].y)), fmaxf(fabsf(f[q].z), fabsf(f[q].w))));
+#pragma unroll
+        for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        // the last tile's boxes have left this warp's part of the operand
+        if (lane == 0) {
+            red[grp][warp] = mx;
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        }
+        asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory");
+        if (*(volatile int *)&s_abort[grp]) break;
+        const float s = fmaxf(red[grp][warp & 2], red[grp][warp | 1]);
+        const float inv = s >= kAeTiny ? 1.0f / s : 0.0f;
+        if ((r & 63) == 0) a.scale[2 * t + (r >> 6)] = s >= kAeTiny ? s : 0.0f;
+        // the scaled points wait as bf16 in the row's second half: the two
+        // nodes along z at (x1, y1) = (m & 1, m >> 1) in its chunks 2m, 2m + 1
+        uint8_t *row = A + r * 128;
+        const int sw = (r & 7) << 4;
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            uint32_t x[2][4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {   // line (x0, y0) = (q & 1, q >> 1) of the nodes
+                const float4 l = f[2 * (m & 1) + (q & 1) + 4 * (2 * (m >> 1) + (q >> 1))];
+                const __nv_bfloat162 lo = __floats2bfloat162_rn(l.x * inv, l.y * inv), hi = __floats2bfloat162_rn(l.z * inv, l.w * inv);
+                x[0][q] = *reinterpret_cast<const uint32_t *>(&lo);
+                x[1][q] = *reinterpret_cast<const uint32_t *>(&hi);
+            }
+#pragma unroll
+            for (int n = 0; n < 2; n++)
+                *reinterpret_cast<uint4 *>(row + 16384 + (((2 * m + n) << 4) ^ sw)) = make_uint4(x[n][0], x[n][1], x[n][2], x[n][3]);
+        }
+        // the next tile's points, on their way during this one's arithmetic
+        if (t + (int)gridDim.x * 2 < a.tiles) load(t + gridDim.x * 2);
+        // E1 of two nodes at a time; nodes 4-7 overwrite the points of pairs
+        // already done
+#pragma unroll 1
+        for (int m = 0; m < 4; m++) {
+            uint32_t x[2][4];
+#pragma unroll
+            for (int n = 0; n < 2; n++) {
+                const uint4 q = *reinterpret_cast<const uint4 *>(row + 16384 + (((2 * m + n) << 4) ^ sw));
+                x[n][0] = q.x; x[n][1] = q.y; x[n][2] = q.z; x[n][3] = q.w;
+            }
+            uint4 h[2][2];
+            e1_pairs(a.w, x, h);
+            uint8_t *half = row + (m >> 1) * 16384;
+#pragma unroll
+            for (int n = 0; n < 2; n++)
+#pragma unroll
+                for (int e = 0; e < 2; e++)
+                    *reinterpret_cast<uint4 *>(half + ((((m & 1) * 4 + n * 2 + e) << 4) ^ sw)) = h[n][e];
+        }
+        tc::fence_async_smem();
+        tc::tc_fence_before();
+        asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory");
+        if (r == 0) {
+            tc::tc_fence_after();
+            constexpr uint32_t idesc = tc::idesc_bf16_f32(128, 64);
+            const uint32_t a0 = tc::su32(A), b0 = tc::su32(sm);
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+                tc::mma_bf16(tmem, tc::sdesc_k128(a0 + (q >> 2) * 16384 + (q & 3) * 32),
+                             tc::sdesc_k128(b0 + (q >> 2) * 8192 + (q & 3) * 32), idesc, q != 0);
+            tc::mma_commit(&done[grp]);
+        }
+        __syncwarp();
+        if (!__all_sync(0xffffffffu, tc::mbar_wait(&done[grp], k & 1))) {
+            s_abort[grp] = 1;
+            continue;   // the group leaves together, after its next barrier
+        }
+        tc::tc_fence_after();
+        const uint32_t ta = tmem + ((uint32_t)(warp * 32) << 16);
+        uint8_t *o = A + warp * 4096;   // this warp's rows of the first slice, read by the MMAs and free
+#pragma unroll 1
+        for (int e = 0; e < 2; e++) {
+            uint32_t d[32];
+            tc::tmem_ld32(ta + 32 * e, d);
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                uint4 w4;
+                __nv_bfloat162 *w2 = reinterpret_cast<__nv_bfloat162 *>(&w4);
+#pragma unroll
+                for (int n = 0; n < 4; n++) {
+                    const float2 bb = *reinterpret_cast<const float2 *>(sbias + 32 * e + 8 * q + 2 * n);
+                    w2[n] = __floats2bfloat162_rn(leaky_d(__uint_as_float(d[8 * q + 2 * n]) + bb.x),
+                                                  leaky_d(__uint_as_float(d[8 * q + 2 * n + 1]) + bb.y));
+                }
+                *reinterpret_cast<uint4 *>(o + lane * 128 + (((4 * e + q) ^ (lane & 7)) << 4)) = w4;
+            }
+        }
+        tc::fence_async_smem();
+        tc::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
+                             reinterpret_cast<uint64_t>(&to)),
+                         "r"(tc::su32(o)), "r"(0), "r"(t * 128 + warp * 32)
+                         : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+    }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    __syncwarp();
+    tc::tc_fence_before();
+    __syncthreads();
+    if ((s_abort[0] || s_abort[1]) && threadIdx.x == 0) atomicExch(a.err, 2);
+    if (threadIdx.x < 32) tc::tmem_dealloc(tslot, 128);
+}
+
+// D2 and D1 of a snapshot in one launch, unscaled and stored to the interior
+// box (dst, the box's strides) with the escaped blocks' residuals added: the
+// walk of tc_gemm.cu (persistent, TMA producer, MMA issuer, two epilogue groups
+// on two accumulators) over D2 with its weights resident, where an epilogue
+// thread finishes a cell: D2's bias and activation, bf16, D1 of its eight
+// nodes (packed FP32 multiply-adds) and 16 four-depth stores.  D2's output, 16
+// KB a block, never leaves the SM.  Two CTAs per SM.  Waits are bounded.
+// A 512x512x384 snapshot takes 116 us, 5.1 TB/s; D2 and D1 one after the other
+// took 221 (101 + 120).
+struct D21Args {
+    AeVolume vol;
+    int nb, tiles;
+    const float *scale;           // [nbp]
+    const float *bias;            // D2's
+    float *dst;
+    const int *esc;               // escaped-block slot per row (-1: none), or null
+    const __nv_bfloat16 *res;     // residual pool (4096 per slot, natural order)
+    int *err;
+    AeSmallW w;
+};
+constexpr int kD21Stages = 4, kD21Threads = 320;
+constexpr size_t kD21Smem = 16384 + kD21Stages * 16384 + 1024;
+
+__global__ void __launch_bounds__(kD21Threads, 2)
+    k_ae_d21(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tw, const __grid_constant__ D21Args a) {
+    extern __shared__ unsigned char smem_raw[];
+    uint8_t *sm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t *ring = sm + 16384;
+    __shared__ __align__(16) float sbias[128];
+    __shared__ __align__(8) uint64_t wbar, full[kD21Stages], empty[kD21Stages], acc_full[2], acc_empty[2];
+    __shared__ uint32_t tslot;
+    __shared__ int s_abort;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        tc::mbar_init(&wbar, 1);
+        for (int s = 0; s < kD21Stages; s++) {
+            tc::mbar_init(&full[s], 1);
+            tc::mbar_init(&empty[s], 1);
+        }
+        for (int s = 0; s < 2; s++) {
+            tc::mbar_init(&acc_full[s], 1);
+            tc::mbar_init(&acc_empty[s], 4);
+        }
+        s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (threadIdx.x < 128) sbias[threadIdx.x] = a.bias[threadIdx.x];
+    __syncwarp();
+    if (warp == 9) tc::tmem_alloc(&tslot, 256);
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tmem = tslot;
+
+    if (warp == 8 && lane == 0) {
+        unsigned it = 0;
+        bool ok = true;
+        tc::mbar_expect_tx(&wbar, 16384);
+        tc::tma2(sm, &tw, 0, 0, &wbar);
+        for (int t = blockIdx.x; t < a.tiles; t += gridDim.x, it++) {
+            const unsigned s = it % kD21Stages;
+            if (it >= kD21Stages && !tc::mbar_wait(&empty[s], (it / kD21Stages - 1) & 1)) {
+                s_abort = 1;
+                ok = false;
+                break;
+            }
+            tc::mbar_expect_tx(&full[s], 16384);
+            tc::tma2(ring + s * 16384, &ta, 0, t * 128, &full[s]);
+        }
+        if (!ok) {   // let the copies still in flight land (bounded)
+            for (unsigned k = it > kD21Stages ? it - kD21Stages : 0; k < it; k++)
+                tc::mbar_wait(&full[k % kD21Stages], (k / kD21Stages) & 1);
+            tc::mbar_wait(&wbar, 0);
+        }
+    } else if (warp == 9 && lane == 0) {
+        constexpr uint32_t idesc = tc::idesc_bf16_f32(128, 128);
+        bool ok = tc::mbar_wait(&wbar, 0);
+        unsigned i = 0;
+        for (int t = blockIdx.x; t < a.tiles && ok; t += gridDim.x, i++) {
+            const unsigned ab = i & 1, s = i % kD21Stages;
+            if ((i >= 2 && !tc::mbar_wait(&acc_empty[ab], ((i >> 1) - 1) & 1)) ||
+                !tc::mbar_wait(&full[s], (i / kD21Stages) & 1)) {
+                ok = false;
+                break;
+            }
+            tc::tc_fence_after();
+            const uint32_t a0 = tc::su32(ring + s * 16384), b0 = tc::su32(sm);
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                tc::mma_bf16(tmem + ab * 128, tc::sdesc_k128(a0 + k * 32), tc::sdesc_k128(b0 + k * 32), idesc, k != 0);
+            tc::mma_commit(&empty[s]);
+            tc::mma_commit(&acc_full[ab]);
+        }
+        if (!ok) s_abort = 1;
+    } else if (warp < 8) {
+        const int grp = warp >> 2, quad = warp & 3;
         const AeVolume &v = a.vol;
-        const int bz = b % v.nbz, bx = (b / v.nbz) % v.nbx, by = b / (v.nbz * v.nbx);
-        const int z = t & 15, x = t >> 4, iz = bz * 16 + z, ix = bx * 16 + x, iy0 = by * 16;
-        const bool zx = iz < v.nz && ix < v.nx;
-        const int ylim = zx ? v.ny - iy0 : 0;
-        const float *col = v.src + (long)(v.oz + iz) + v.ldz * (v.ox + ix) + v.sxy * (v.oy + iy0);
-        // all sixteen loads in flight before the first use
-        float vals[16];
+        const bool vec = lines_aligned(v, a.dst);
+        unsigned i = 0;
+        for (int t = blockIdx.x; t < a.tiles; t += gridDim.x, i++) {
+            if ((int)(i & 1) != grp) continue;
+            const CellAt c(v, t, quad * 32 + lane);
+            const bool in = c.b < a.nb;
+            const float s = in ? a.scale[c.b] : 0.0f;
+            const int slot = in && a.esc ? a.esc[c.b] : -1;
+            if (!__all_sync(0xffffffffu, tc::mbar_wait(&acc_full[grp], (i >> 1) & 1))) {
+                s_abort = 1;
+                break;
+            }
+            tc::tc_fence_after();
+            const uint32_t ta0 = tmem + ((uint32_t)(quad * 32) << 16) + grp * 128;
+            float *p = a.dst + (long)(v.oz + c.iz) + v.ldz * (v.ox + c.ix) + v.sxy * (v.oy + c.iy);
+            const bool whole = vec && in && c.iz + 4 <= v.nz && c.ix + 4 <= v.nx && c.iy + 4 <= v.ny;
+#pragma unroll 1
+            for (int m = 0; m < 4; m++) {   // the two nodes along z at (x1, y1) = (m & 1, m >> 1)
+                uint32_t d[32];
+                tc::tmem_ld32(ta0 + m * 32, d);
+                tc::tmem_ld_wait();
+                if (m == 3) {
+                    tc::tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(&acc_empty[grp]);
+                }
+                uint4 g[2][2];
 #pragma unroll
-        for (int y = 0; y < 16; y++, col += v.sxy) vals[y] = y < ylim ? __ldg(col) : 0.0f;
-        const BlockCol c(z, x);
+                for (int q = 0; q < 16; q++) {
+                    const float2 bb = *reinterpret_cast<const float2 *>(sbias + m * 32 + 2 * q);
+                    reinterpret_cast<__nv_bfloat162 *>(g)[q] = __floats2bfloat162_rn(
+                        leaky_d(__uint_as_float(d[2 * q]) + bb.x), leaky_d(__uint_as_float(d[2 * q + 1]) + bb.y));
+                }
+                float4 y[2][2];
+                d1_pairs(a.w, g, s, y);
+                if (!in) continue;
+                const float *y0 = reinterpret_cast<const float *>(y[0]), *y1 = reinterpret_cast<const float *>(y[1]);
 #pragma unroll
-        for (int y = 0; y < 16; y++) {
-            xs[c.at(y)] = vals[y];
-            mx = fmaxf(mx, fabsf(vals[y]));
+                for (int q = 0; q < 4; q++) {
+                    const int dx = 2 * (m & 1) + (q & 1), dy = 2 * (m >> 1) + (q >> 1);
+                    float4 o = make_float4(y0[2 * q], y0[2 * q + 1], y1[2 * q], y1[2 * q + 1]);
+                    if (slot >= 0) {   // escaped block: decoded + residual
+                        const uint2 e = *reinterpret_cast<const uint2 *>(
+                            a.res + (long)slot * kAePts + ((c.iy + dy) & 15) * 256 + ((c.ix + dx) & 15) * 16 + (c.iz & 15));
+                        o.x += __uint_as_float(e.x << 16);
+                        o.y += __uint_as_float(e.x & 0xffff0000u);
+                        o.z += __uint_as_float(e.y << 16);
+                        o.w += __uint_as_float(e.y & 0xffff0000u);
+                    }
+                    float *l = p + v.ldz * dx + v.sxy * dy;
+                    if (whole) {
+                        *reinterpret_cast<float4 *>(l) = o;
+                    } else if (c.ix + dx < v.nx && c.iy + dy < v.ny) {
+                        if (c.iz < v.nz) l[0] = o.x;
+                        if (c.iz + 1 < v.nz) l[1] = o.y;
+                        if (c.iz + 2 < v.nz) l[2] = o.z;
+                        if (c.iz + 3 < v.nz) l[3] = o.w;
+                    }
+                }
+            }
         }
-    } else {
-        for (int p = 0; p < 16; p++) xs[p * 256 + t] = 0.0f;
     }
-    const float s = block_max(mx, red);
-    const float inv = s >= kAeTiny ? 1.0f / s : 0.0f;
-    if (t == 0) a.scale[b] = s >= kAeTiny ? s : 0.0f;
-    uint32_t x[2][4];
-#pragma unroll
-    for (int r = 0; r < 2; r++) {
-        const int o = swz((t + 256 * r) * 8);
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const float4 q = *reinterpret_cast<const float4 *>(xs + (o ^ 4 * h));
-            const __nv_bfloat162 p0 = __floats2bfloat162_rn(q.x * inv, q.y * inv), p1 = __floats2bfloat162_rn(q.z * inv, q.w * inv);
-            x[r][2 * h] = *reinterpret_cast<const uint32_t *>(&p0);
-            x[r][2 * h + 1] = *reinterpret_cast<const uint32_t *>(&p1);
-        }
-    }
-    uint4 h[2][2];
-    e1_pairs(a.w, x, h);
+    __syncwarp();
+    tc::tc_fence_before();
     __syncthreads();
-    // the 512 nodes' 32 bytes each, in order over the values: one bulk store
-#pragma unroll
-    for (int r = 0; r < 2; r++) {
-        uint4 *o = reinterpret_cast<uint4 *>(xs) + 2 * (t + 256 * r);
-        o[0] = h[r][0];
-        o[1] = h[r][1];
-    }
-    tc::fence_async_smem();
-    __syncthreads();
-    if (t == 0) {
-        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], 16384;" ::"l"(a.h1 + (long)b * 512 * 16),
-                     "r"(tc::su32(xs))
-                     : "memory");
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-    }
+    if (s_abort && threadIdx.x == 0) atomicExch(a.err, 2);
+    if (warp == 9) tc::tmem_dealloc(tmem, 256);
 }
 
 // out[(c * SC + j * SJ)] += sum over the block's 512 nodes of a[c] b[j], and
@@ -553,34 +855,30 @@ __global__ void __launch_bounds__(256) k_ae_d1(const D1Args a) {
     if (a.gd1) block_outer<true, 16, 1>(sm, a.gd1, a.gd1 + 128);
 }
 
-// D1 of a snapshot's blocks with the weights passed by value, unscaled and
-// scattered to the interior box: mode 0 stores the snapshot (dst, the box's
-// strides), mode 1 adds wimg * snapshot * gP to the image, mode 3 compares
-// with the field vol.src and keeps every block's residual (bf16, natural
-// order) and its squared error and norm (the escape check).  Escaped blocks
-// (esc) add their residual in modes 0 and 1.  Thread t owns depth
-// z = t & 15 of row x = t >> 4 on all sixteen planes, as in k_ae_e1_vol.
-// Mode 0 of a 512x512x384 snapshot takes 118 us, at the copy bandwidth; 178 us
-// with scalar multiply-adds, bank conflicts in the Morton exchange and the
-// registers of the image mode (three blocks per SM; now six).
+// D1 of a snapshot's blocks with the weights passed by value, unscaled: mode 1
+// adds wimg * snapshot * gP to the image (escaped blocks with their residual),
+// mode 3 compares with the field vol.src and keeps every block's residual
+// (bf16, natural order) and its squared error and norm (the escape check).
+// Thread t owns nodes t and t + 256, then depth z = t & 15 of row x = t >> 4 on
+// all sixteen planes; the values change hands in shared memory without bank
+// conflicts (swz).
 struct D1Vol {
     AeVolume vol;
     int nb;
     const __nv_bfloat16 *g1;      // [nbp*512 x 16]
     const float *scale;           // [nbp]
-    float *dst;                   // mode 0
     const float *gP;              // mode 1: receiver field (vol's strides)
     float *mig;                   // mode 1: image, iz + nz*(ix + nx*iy)
     float wimg;                   // mode 1: weight of this snapshot
-    const int *esc;               // modes 0/1: escaped-block slot per row (-1: none), or null
-    const __nv_bfloat16 *res;     // modes 0/1: residual pool (4096 per slot, natural order)
+    const int *esc;               // mode 1: escaped-block slot per row (-1: none), or null
+    const __nv_bfloat16 *res;     // mode 1: residual pool (4096 per slot, natural order)
     __nv_bfloat16 *resall;        // mode 3: residual of every row (natural order)
     float *err2, *norm2;          // mode 3: per-row squared error and squared norm
     AeSmallW w;
 };
 
 template <int MODE>
-__global__ void __launch_bounds__(256, MODE == 0 ? 6 : 4) k_ae_d1_vol(const D1Vol a) {
+__global__ void __launch_bounds__(256, 4) k_ae_d1_vol(const D1Vol a) {
     __shared__ __align__(16) float ys[kAePts];
     __shared__ float red2[2][8];
     const int b = blockIdx.x, t = threadIdx.x;
@@ -645,16 +943,6 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 6 : 4) k_ae_d1_vol(const D1Vo
     if (!zx) return;
     const int slot = a.esc ? a.esc[b] : -1;
     const __nv_bfloat16 *res = slot >= 0 ? a.res + (long)slot * kAePts : nullptr;
-    if (MODE == 0) {
-#pragma unroll
-        for (int y = 0; y < 16; y++) {
-            if (iy0 + y >= v.ny) break;
-            float val = ys[c.at(y)];
-            if (res) val += __bfloat162float(res[y * 256 + t]);   // escaped block: decoded + residual
-            a.dst[col + v.sxy * y] = val;
-        }
-        return;
-    }
     // mode 1: all image and receiver-field loads in flight first
     const long o0 = iz + (long)v.nz * (ix + (long)v.nx * iy0), so = (long)v.nz * v.nx;
     float gp[16], mg[16];
@@ -1112,6 +1400,24 @@ int ae_escape_cap(geo_ae *ae, const AeVolume &v) {
     return std::min(nb, (int)std::ceil(ae->frac * nb));
 }
 
+static int ae_sms() {
+    static int n = 0;
+    if (!n) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 152;
+    }
+    return n;
+}
+static int ae_smem() {
+    static bool set = false;
+    if (set) return GEO_OK;
+    GEO_CUDA(cudaFuncSetAttribute(k_ae_e12, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kE12Smem));
+    GEO_CUDA(cudaFuncSetAttribute(k_ae_d21, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kD21Smem));
+    set = true;
+    return GEO_OK;
+}
+
 // Encode the interior box v into code[rows x 512] (bf16) and scale[rows];
 // with esc != null also decode, and keep the residuals of the blocks the
 // code misses (esc[rows], res[cap x 4096] bf16, *count escaped blocks).
@@ -1120,15 +1426,22 @@ int ae_encode_volume(geo_ae *ae, const AeVolume &v, void *code, float *scale, in
     const int nb = blocks_of(v), rows = pad128(nb);
     GEO_TRY(ensure_rows(ae, rows));
     GEO_TRY(ae_mirror(ae, s));
-    E1Vol a{};
+    E12Args a{};
     a.vol = v;
     a.nb = nb;
-    a.h1 = bf(ae->h1);
+    a.tiles = rows / 2;
     a.scale = scale;
+    a.bias = ae->params.as<float>() + ae->off.b[1];
+    a.err = ae->err.as<int>();
     a.w = ae->hw;
-    k_ae_e1_vol<<<rows, 256, 0, s>>>(a);
-    GEO_TRY(check_launch("ae_e1"));
-    GEO_TRY(encode_rows(ae, rows, static_cast<__nv_bfloat16 *>(code), s));
+    CUtensorMap tw, to;
+    GEO_TRY(tc_map_bf16(&tw, bf(ae->wb) + ae->off.wb[1], 64, 128, 64));
+    GEO_TRY(tc_map_bf16(&to, ae->h2.p, rows * 64, 64, 32));
+    GEO_TRY(ae_smem());
+    k_ae_e12<<<std::min((a.tiles + 1) / 2, 2 * ae_sms()), 256, kE12Smem, s>>>(tw, to, a);
+    GEO_TRY(check_launch("ae_e12"));
+    GEO_TRY(level(ae, 2, rows, bf(ae->h2), bf(ae->h3), s));
+    GEO_TRY(level(ae, 3, rows, bf(ae->h3), static_cast<__nv_bfloat16 *>(code), s));
     if (!esc) return GEO_OK;
     if (ae_escape_cap(ae, v) == 0) {   // no escape budget: no re-decode
         GEO_CUDA(cudaMemsetAsync(esc, 0xff, (size_t)rows * 4, s));
@@ -1167,22 +1480,41 @@ int ae_decode_volume(geo_ae *ae, const AeVolume &v, const void *code, const floa
                      const void *res, int mode, float *dst, const float *gP, float *mig, float w, cudaStream_t s) {
     const int nb = blocks_of(v), rows = pad128(nb);
     GEO_TRY(ensure_rows(ae, rows));
-    GEO_TRY(decode_rows(ae, rows, static_cast<const __nv_bfloat16 *>(code), s));
     GEO_TRY(ae_mirror(ae, s));
+    if (mode == 0) {
+        GEO_TRY(level(ae, 4, rows, static_cast<const __nv_bfloat16 *>(code), bf(ae->g3), s));
+        GEO_TRY(level(ae, 5, rows, bf(ae->g3), bf(ae->g2), s));
+        D21Args a{};
+        a.vol = v;
+        a.nb = nb;
+        a.tiles = (nb + 1) / 2;
+        a.scale = scale;
+        a.bias = ae->params.as<float>() + ae->off.b[6];
+        a.dst = dst;
+        a.esc = esc;
+        a.res = static_cast<const __nv_bfloat16 *>(res);
+        a.err = ae->err.as<int>();
+        a.w = ae->hw;
+        CUtensorMap ta, tw;
+        GEO_TRY(tc_map_bf16(&ta, ae->g2.p, rows * 64, 64, 128));
+        GEO_TRY(tc_map_bf16(&tw, bf(ae->wb) + ae->off.wb[6], 128, 64, 128));
+        GEO_TRY(ae_smem());
+        k_ae_d21<<<std::min(a.tiles, 2 * ae_sms()), kD21Threads, kD21Smem, s>>>(ta, tw, a);
+        return check_launch("ae_d21");
+    }
+    GEO_TRY(decode_rows(ae, rows, static_cast<const __nv_bfloat16 *>(code), s));
     D1Vol a{};
     a.vol = v;
     a.nb = nb;
     a.g1 = bf(ae->g1);
     a.scale = scale;
-    a.dst = dst;
     a.gP = gP;
     a.mig = mig;
     a.wimg = w;
     a.esc = esc;
     a.res = static_cast<const __nv_bfloat16 *>(res);
     a.w = ae->hw;
-    if (mode == 0) k_ae_d1_vol<0><<<rows, 256, 0, s>>>(a);
-    else k_ae_d1_vol<1><<<rows, 256, 0, s>>>(a);
+    k_ae_d1_vol<1><<<rows, 256, 0, s>>>(a);
     return check_launch("ae_d1");
 }
 

@@ -398,9 +398,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1)
 
 static PFN_cuTensorMapEncodeTiled_v12000 g_enc2 = nullptr;
 
-// 2D bf16 map over a row-major [rows x cols] matrix, box box_rows x 64
-// columns (128 bytes), 128-byte swizzle.
-static int encode_bf16_2d(CUtensorMap *map, const void *base, int rows, int cols, int box_rows) {
+int tc_map_bf16(CUtensorMap *map, const void *base, int rows, int cols, int box_rows) {
     if (!g_enc2) {
         void *fn = nullptr;
         cudaDriverEntryPointQueryResult q;
@@ -428,8 +426,8 @@ static int launch_bn(const TcGemm &g, cudaStream_t s) {
         attr = true;
     }
     CUtensorMap ta, tb;
-    GEO_TRY(encode_bf16_2d(&ta, g.A, g.M, g.K, kGM));
-    GEO_TRY(encode_bf16_2d(&tb, g.B, g.N, g.K, BN));
+    GEO_TRY(tc_map_bf16(&ta, g.A, g.M, g.K, kGM));
+    GEO_TRY(tc_map_bf16(&tb, g.B, g.N, g.K, BN));
     const dim3 grid((unsigned)(g.M / kGM) * (unsigned)(g.N / BN));
     k_tc_gemm<BN, ST><<<grid, 128, S::kSmem, s>>>(ta, tb, g);
     return check_launch("tc_gemm");
@@ -446,9 +444,9 @@ static int launch_walk(const TcGemm &g, cudaStream_t s) {
         GEO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     }
     CUtensorMap ta, tb, to;
-    GEO_TRY(encode_bf16_2d(&ta, g.A, g.M, g.K, kGM));
-    GEO_TRY(encode_bf16_2d(&tb, g.B, g.N, g.K, BN));
-    GEO_TRY(encode_bf16_2d(&to, g.out, g.M, g.N, 32));
+    GEO_TRY(tc_map_bf16(&ta, g.A, g.M, g.K, kGM));
+    GEO_TRY(tc_map_bf16(&tb, g.B, g.N, g.K, BN));
+    GEO_TRY(tc_map_bf16(&to, g.out, g.M, g.N, 32));
     const int tiles = (g.M / kGM) * (g.N / BN);
     k_tc_walk<BN, RB><<<std::min(tiles, sms), kWalkThreads, S::kSmem, s>>>(ta, tb, to, g, tiles);
     return check_launch("tc_walk");
@@ -640,8 +638,8 @@ int tc_wgrad(const TcWgradLevel *lv, int n, int *err, cudaStream_t s) {
         if ((reinterpret_cast<uintptr_t>(L.A) | reinterpret_cast<uintptr_t>(L.B) |
              reinterpret_cast<uintptr_t>(L.out)) & 15)
             return fail(GEO_ERR_ARG, "tc_wgrad: operands must be 16-byte aligned");
-        GEO_TRY(encode_bf16_2d(&g.ta[l], L.A, L.M, L.wa, 64));
-        GEO_TRY(encode_bf16_2d(&g.tb[l], L.B, L.M, L.wb, 64));
+        GEO_TRY(tc_map_bf16(&g.ta[l], L.A, L.M, L.wa, 64));
+        GEO_TRY(tc_map_bf16(&g.tb[l], L.B, L.M, L.wb, 64));
         WgradItem &w = g.it[l];
         w.out = L.out;
         w.sa = L.sa;

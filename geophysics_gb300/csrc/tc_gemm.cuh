@@ -1,6 +1,7 @@
 // BF16 tensor-core GEMM (tcgen05, TMEM accumulator, TMA-fed) used by the
 // snapshot codec: C[M x N] = A[M x K] * B[N x K]^T with a fused epilogue.
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 
@@ -22,6 +23,10 @@ struct TcGemm {
 constexpr float kLeak = 0.1f;
 
 int tc_gemm(const TcGemm &g, cudaStream_t s);
+
+// TMA map over a row-major [rows x cols] bf16 matrix, boxes of box_rows x 64
+// columns (128 bytes), 128-byte swizzle.
+int tc_map_bf16(CUtensorMap *map, const void *base, int rows, int cols, int box_rows);
 
 // Weight gradients of up to kWgradMax levels in one launch: for each,
 // out[a*sa + b*sb] += sum over m < M of A[m*wa + a] * B[m*wb + b].

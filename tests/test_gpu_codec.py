@@ -222,3 +222,26 @@ def test_tc_gemm_many_tiles_bf16(geo, M, N, K):
         r = torch.where(r > 0, r, 0.1 * r) if act else r
         out = geo.tc_gemm_bf16(A, B, bias=b, act=act, out_f32=False).double()
         assert ((out - r).abs() <= 2.0 ** -8 * r.abs() + 1e-5 * ref.abs().max()).all()
+
+
+@pytest.mark.parametrize("nz,nx,ny,off", [(16, 16, 16, 0), (33, 17, 16, 0), (48, 31, 49, 0), (64, 64, 288, 0), (64, 16, 16, 1),
+                                          (30, 20, 18, 1)])
+def test_snapshot_kernels_vector_and_scalar_lines(geo, nz, nx, ny, off):
+    """E1+E2 and D2+D1 of a snapshot over cells that leave the volume, an odd
+    number of blocks, more tiles than blocks in flight, and lines that are not
+    16-byte aligned (a volume `off` floats into its buffer, odd depths): the
+    aligned volume of the same values, padded to whole blocks, gives the same
+    reconstruction."""
+    torch = pytest.importorskip("torch")
+    codec = geo.Codec(seed=5)
+    g = torch.Generator().manual_seed(4)
+    buf = torch.empty(ny * nx * nz + off, device="cuda")
+    vol = buf[off:].view(ny, nx, nz)
+    vol.copy_(torch.randn(ny, nx, nz, generator=g))
+    pad = torch.zeros([-(-n // 16) * 16 for n in (ny, nx, nz)], device="cuda")
+    pad[:ny, :nx, :nz] = vol
+    out, ref = codec.roundtrip(vol), codec.roundtrip(pad)
+    assert float(out.abs().max()) > 0
+    assert torch.equal(out, ref[:ny, :nx, :nz])
+    eout, ne = codec.roundtrip(vol, escape=True)
+    assert ne > 0 and (eout - vol).norm() < (out - vol).norm()
