@@ -14,29 +14,34 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
 }
 
 // One arrival per block on a counter that only grows (barrier k completes at
-// k*gridDim.x arrivals).  The fence before the arrival publishes the block's
-// writes; the wait is bounded (2 s) and a timeout sets the error word and
-// ends the block, after which every other block's next wait times out too.
-// Values other blocks wrote before the barrier are read through L2
-// (__ldcg): L1 is not coherent with them.
+// k*gridDim.x arrivals).  grid_arrive, by one thread after a __syncthreads,
+// publishes the block's writes (release, cumulative over the block's barrier);
+// grid_wait, by one thread, waits for the target (acquire), 2 s at most, and
+// sets the error word when it gives up, after which every other block's next
+// wait runs out too.  Values other blocks wrote before the barrier are read
+// through L2 (__ldcg) or by TMA: L1 is not coherent with them.
+// A release reduction instead of a fence and an atomic, and no fence after
+// the acquire: a step of a 101x121 2D shot 4.0 -> 3.6 us, of 401x401 6.0 -> 5.6.
+__device__ __forceinline__ void grid_arrive(unsigned *bar) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+}
+__device__ __forceinline__ bool grid_wait(const unsigned *bar, unsigned target, int *err) {
+    if (ld_acquire_u32(bar) >= target) return true;
+    const uint64_t t0 = tc::gtimer();
+    while (ld_acquire_u32(bar) < target)
+        if (tc::gtimer() - t0 > 2000000000ull) {
+            atomicExch(err, 1);
+            return false;
+        }
+    return true;
+}
+// Both, for the whole block.
 __device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned target, int *err) {
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0 && threadIdx.y == 0) {
-        int ok = 1;
-        __threadfence();
-        atomicAdd(bar, 1u);
-        if (ld_acquire_u32(bar) < target) {
-            const uint64_t t0 = tc::gtimer();
-            while (ld_acquire_u32(bar) < target)
-                if (tc::gtimer() - t0 > 2000000000ull) {
-                    atomicExch(err, 1);
-                    ok = 0;
-                    break;
-                }
-        }
-        __threadfence();
-        s_ok = ok;
+        grid_arrive(bar);
+        s_ok = grid_wait(bar, target, err);
     }
     __syncthreads();
     return s_ok != 0;

@@ -25,19 +25,27 @@
 // left in L2 is read first: nothing forward, where all of it fits, and 41.7
 // -> 39.1 us backward, where two sides (140 MB and the gathers) do not.
 //
+// Between two steps only one thread waits: it brings the first tile's own boxes
+// (split stresses, model) before the barrier completes and the shared ones
+// after, while the others load the profiles their tile needs and wait for the
+// boxes (a barrier of the whole block, and profiles loaded where they are used
+// -- an L2 round trip, since the acquire empties L1 -- cost a 101x121 shot 0.7 us
+// a step and a 401x401 one 0.9).
+//
 // Measured against the kernels this replaces (half-steps of one persistent
 // launch; tiles kept in shared memory with exchange copies where the grid
-// fits that way), us a step: 2401x601 + 50 39.5 -> 20.1; 1200x601 25.0 ->
-// 12.1; 600x601 10.9 -> 8.6; 401x401 7.4 -> 6.0; 101x121 + 20 5.4 -> 4.0; RTM
-// program 1700x601 forward 26.1 -> 17.6, backward with 70 angles 56.3 ->
-// 39.1.  TTI, whose rotated derivatives need both halos of every field (twice
-// the velocity work of a tile of 8 columns, 1.6 times of 16): 600x300 11.5 ->
-// 8.4; RTM program 1700x601, 65 angles, forward 37.3 -> 25.7, backward 74.0
-// -> 56.2.  Bound by instruction issue (55 % of the slots at 24 warps per SM;
-// 340 instructions a point, a quarter of them halo work) and, on small
-// grids, by the barrier and the TMA round trip.  Tried: four warps with two
-// columns each (18.3 forward, 51.5 backward), split stresses and model from
-// L2 into registers instead of TMA (18.6 and 45.8).
+// fits that way), us a step: 2401x601 + 50 39.5 -> 18.0; 1200x601 25.0 -> 10.1;
+// 600x601 10.9 -> 7.4; 401x401 7.4 -> 5.1; 101x121 + 20 5.4 -> 3.3; RTM program
+// 1700x601 forward 26.1 -> 17.1, backward with 70 angles 56.3 -> 38.9.  TTI,
+// whose rotated derivatives need both halos of every field (twice the velocity
+// work of a tile of 8 columns, 1.6 times of 16): 600x300 11.5 -> 7.5; RTM
+// program 1700x601, 65 angles, forward 37.3 -> 24.9, backward 74.0 -> 56.3.
+// Large grids are bound by instruction issue (55 % of the slots at 24 warps per
+// SM; 340 instructions a point, a quarter of them halo work), small ones by the
+// barrier and the TMA round trip.  Tried: four warps with two columns each
+// (1.04 times forward, 1.3 backward), split stresses and model from L2 into
+// registers instead of TMA (1.05 and 1.15), flags of the neighbours' blocks
+// instead of the barrier (0.95 where a block has one tile, 1.3 where several).
 //
 // The backward pass of the RTM program takes the source side and the
 // receiver side of a tile one after the other, the source side's new values
@@ -132,9 +140,8 @@ __device__ __forceinline__ bool boxes_here(uint64_t *bar, uint32_t parity, const
 
 // The TTI programs' velocity update (Toa_gpu_2dtti_fd_1orderfunction.cu:81-112)
 // of a pair of points, in place; on: which of them are on the updated grid.
-__device__ __forceinline__ void tti_vel(const SGrid &g, int ix, float2 cz1, float2 cz2, float2 ct, float2 sn, float2 Px, float2 Pz,
+__device__ __forceinline__ void tti_vel(const SGrid &g, float c1, float c2, float2 cz1, float2 cz2, float2 ct, float2 sn, float2 Px, float2 Pz,
                                         float2 Qx, float2 Qz, bool on0, bool on1, float *pu, float *pw) {
-    const float c1 = __ldg(g.cx1 + ix), c2 = __ldg(g.cx2 + ix);
     float2 u = lds2(pu), w = lds2(pw);
 #pragma unroll
     for (int j = 0; j < 2; j++) {
@@ -187,19 +194,29 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
     const int nb = ((ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * (BWD ? 2 : 1);
     unsigned base = 0;   // items of the steps before
     const int step_z = (int)gridDim.x % ntz * kTz, step_x = (int)gridDim.x / ntz * TX;
-    auto fetch = [&](int k, int f, int z, int x, int lev) {
+    // boxes of item k: what other blocks do not write, and what they do
+    auto fetch_own = [&](int k, int f, int z, int x) {
+        const int st = (base + k) & (stages - 1);
+        uint64_t *b = &bar[st];
+        float *s = sm + st * SF;
+        tc::mbar_expect_tx(b, SF * 4);
+        tma3(s + B::s, &tm.m[f][0].S, z, x, b);
+        tma3(s + B::m, &tm.model, z, x, b);
+        if (TTI) tma3(s + B::t, &tm.trig, z - 4, x - 4, b);
+    };
+    auto fetch_shared = [&](int k, int f, int z, int x, int lev) {
         const int st = (base + k) & (stages - 1);
         uint64_t *b = &bar[st];
         float *s = sm + st * SF;
         const SMaps &m = tm.m[f][lev];
-        tc::mbar_expect_tx(b, SF * 4);
         tc::tma2(s, &m.P, z - B::hz, x - 7, b);
         tc::tma2(s + B::q, &m.Q, z - 8, x - B::hq, b);
         tc::tma2(s + B::u, &m.u, z - B::hu, x - 4, b);
         tc::tma2(s + B::w, &m.w, z - 4, x - B::hw, b);
-        tma3(s + B::s, &m.S, z, x, b);
-        tma3(s + B::m, &tm.model, z, x, b);
-        if (TTI) tma3(s + B::t, &tm.trig, z - 4, x - 4, b);
+    };
+    auto fetch = [&](int k, int f, int z, int x, int lev) {
+        fetch_own(k, f, z, x);
+        fetch_shared(k, f, z, x, lev);
     };
     if (tid == 0) {
         for (int k = 0; k < stages; k++) tc::mbar_init(&bar[k], 1);
@@ -217,10 +234,15 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
         const bool rev = s & 1;
         const int t_first = blockIdx.x + (rev ? (BWD ? nb / 2 - 1 : nb - 1) * gridDim.x : 0);
         const int z_first = t_first % ntz * kTz, x_first = t_first / ntz * TX;
-        if (tid == 0) {
-            // other blocks' stores of the step before, then TMA reads of them
-            asm volatile("fence.proxy.async;" ::: "memory");
-            fetch(0, 0, z_first, x_first, lev);
+        if (tid == 0) {   // the others wait for the boxes
+            fetch_own(0, 0, z_first, x_first);
+            if (s && !grid_wait(a.bar, (unsigned)s * gridDim.x, a.err)) {
+                s_abort = 1;
+            } else {
+                // other blocks' stores of the step before, then TMA reads of them
+                asm volatile("fence.proxy.async;" ::: "memory");
+                fetch_shared(0, 0, z_first, x_first, lev);
+            }
         }
         int z0 = z_first, x0 = x_first, zn = z0, xn = x0;   // this item's tile, the next item's
         for (int k = 0; k < nb; k++, z0 = zn, x0 = xn) {
@@ -246,7 +268,22 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
             const float *sS = sP + B::s, *sM = sP + B::m, *sT = sP + B::t;
             const bool z0u = zo >= 4 && zo < g.nnz - 4, z1u = zo + 1 >= 4 && zo + 1 < g.nnz - 4;
             const int zc = min(zo, ldz - 2);   // profiles of the pair
-            const float2 cz1 = ldg2(g.zp + zc), cz2 = ldg2(g.zp + ldz + zc);
+            const float2 cz1 = ldg2(g.zp + zc), cz2 = ldg2(g.zp + ldz + zc), az1 = ldg2(g.zp + 2 * ldz + zc),
+                         az2 = ldg2(g.zp + 3 * ldz + zc);
+            constexpr int NU = (TX + 7 + W - 1) / W;   // columns of u a warp
+            float cu1[NU], cu2[NU], ca1[NC], ca2[NC];
+#pragma unroll
+            for (int j = 0; j < NU; j++) {
+                const int ix = min(max(x0 - 4 + warp * NU + j, 0), g.nnx - 1);
+                cu1[j] = __ldg(g.cx1 + ix);
+                cu2[j] = __ldg(g.cx2 + ix);
+            }
+#pragma unroll
+            for (int c = 0; c < NC; c++) {
+                const int ix = min(x0 + c0 + c, g.nnx - 1);
+                ca1[c] = __ldg(g.ax1 + ix);
+                ca2[c] = __ldg(g.ax2 + ix);
+            }
             if (!boxes_here(&bar[st], ((base + k) >> (stages - 1)) & 1, a.err)) *(volatile int *)&s_abort = 1;
             if ((KIND == SK_GPU || KIND == SK_GFWD) && src_on) {
                 // point source: P,Q += amp before the velocity update, on this
@@ -260,7 +297,6 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
                     __syncthreads();
                 }
             }
-            constexpr int NU = (TX + 7 + W - 1) / W;
             float2 wn[NC];
             if constexpr (TTI) {
                 // u and w at once, on the columns of the tile and its halos
@@ -284,7 +320,7 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
                     q[7] = lds2(pQ + n);
                     if (uc < TX + 7 && ix >= 4 && ix < g.nnx - 4) {
                         const float2 Pz = dz8<1>(pP + (uc + 3) * kQz), Qz = dz8<1>(pQ + (uc + 3) * kQz);
-                        tti_vel(g, ix, cz1, cz2, lds2(sT + uc * kWz + zl + 4), lds2(sT + (TX + 8 + uc) * kWz + zl + 4), dx8(p),
+                        tti_vel(g, cu1[j], cu2[j], cz1, cz2, lds2(sT + uc * kWz + zl + 4), lds2(sT + (TX + 8 + uc) * kWz + zl + 4), dx8(p),
                                 Pz, dx8(q), Qz, z0u, z1u, sU + uc * kWz + zl + 4, sW + uc * kWz + zl + 4);
                     }
                 }
@@ -301,7 +337,7 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
                             q[m] = lds2(hQ + (m - 3) * kQz);
                         }
                         const int uc = col + 4, z4 = zr + 4;
-                        tti_vel(g, ix, ldg2(g.zp + i0), ldg2(g.zp + ldz + i0), lds2(sT + uc * kWz + z4),
+                        tti_vel(g, __ldg(g.cx1 + ix), __ldg(g.cx2 + ix), ldg2(g.zp + i0), ldg2(g.zp + ldz + i0), lds2(sT + uc * kWz + z4),
                                 lds2(sT + (TX + 8 + uc) * kWz + z4), dx8(p), dz8<1>(hP), dx8(q), dz8<1>(hQ), h0, h1,
                                 sU + uc * kWz + z4, sW + uc * kWz + z4);
                     }
@@ -321,7 +357,7 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
                         for (int m = 0; m < 7; m++) q[m] = q[m + 1];
                         q[7] = lds2(sP + min(uc + 7, TX + 13) * kTz + zl);
                         if (uc < TX + 7 && ix >= 4 && ix < g.nnx - 4) {
-                            const float c1 = __ldg(g.cx1 + ix) * g.dtx, c2 = __ldg(g.cx2 + ix);
+                            const float c1 = cu1[j] * g.dtx, c2 = cu2[j];
                             const float2 xx = dx8(q), uo = lds2(sU + uc * kTz + zl);
                             sts2(sU + uc * kTz + zl,
                                  make_float2(z0u ? c2 * uo.x - c1 * xx.x : uo.x, z1u ? c2 * uo.y - c1 * xx.y : uo.y));
@@ -353,7 +389,6 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
                     }
                 }
             }
-            const float2 az1 = ldg2(g.zp + 2 * ldz + zc), az2 = ldg2(g.zp + 3 * ldz + zc);
             const int gz = zo - g.npd;
             bool in[NC][2];
             float im[NC][2];   // illumination or image of the interior points
@@ -415,7 +450,7 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
                         ct = lds2(sT + (c0 + c + 4) * kWz + zl + 4);
                         sn = lds2(sT + (TX + 12 + c0 + c) * kWz + zl + 4);
                     }
-                    const float ax1 = __ldg(g.ax1 + ix), ax2 = __ldg(g.ax2 + ix);
+                    const float ax1 = ca1[c], ax2 = ca2[c];
                     const int so = (c0 + c) * kTz + zl;
                     float2 T[4], M[3];
 #pragma unroll
@@ -564,7 +599,8 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
         }
         // this step's stores before the next step's TMA reads of them
         asm volatile("fence.proxy.async;" ::: "memory");
-        if (s + 1 < steps && !grid_barrier(a.bar, (unsigned)(s + 1) * gridDim.x, a.err)) return;
+        __syncthreads();
+        if (tid == 0) grid_arrive(a.bar);
     }
 }
 
@@ -644,14 +680,13 @@ int Fused2D::model(const SGrid &g, const float *p, const float *trig) {
 // Tiles of 8 columns (three or four blocks per SM) or 16 (two; a quarter less
 // halo work): the fewer columns on the busiest SM, each tile's halo counted as
 // one (VTI) or six (TTI, whose halos cost both velocities).  us a step with 8
-// and with 16: VTI 601 deep 2401 wide 20.8 and 20.1, 600 8.7 and 8.6, 300 6.9
-// and 6.1, the RTM program's 1700 forward 17.6 and 18.1, 401x401 6.7 and 6.0,
-// 250x250 4.9 and 4.8, 101x121 4.0 and 4.8; TTI 600x300 9.0 and 8.4, 1500x600
-// 22.1 and 20.2, 200x150 4.5 and 5.5.  The TTI RTM passes take 8: 1100x450
-// 15.2 and 16.4 forward, 31.3 and 37.8 backward.  VTI takes one stage where
-// every tile has its own block, two where blocks walk several; TTI tiles are
-// heavier and always take one (three blocks per SM instead of two beat the
-// prefetch).
+// and with 16: VTI 601 deep 2401 wide 19.7 and 18.0, 600 8.5 and 7.4, 300 6.3
+// and 4.9, the RTM program's 1700 forward 17.1 and 17.6, 401x401 6.5 and 5.0,
+// 250x250 4.1 and 4.1, 101x121 3.3 and 3.9; TTI 600x300 8.1 and 7.5, 1500x600
+// 21 and 19.2, 200x150 3.8 and 4.8.  The TTI RTM passes take 8: 1100x450 15.2
+// and 16.4 forward, 31.3 and 37.8 backward.  VTI takes one stage where every
+// tile has its own block, two where blocks walk several; TTI tiles are heavier
+// and always take one (three blocks per SM instead of two beat the prefetch).
 int Fused2D::plan(StepKind k, bool tti_, const SGrid &g, int fixed) {
     kind = k;
     tti = tti_;
