@@ -189,7 +189,6 @@ struct geo_fd3d_plan {
     DevBuf raw;                        // unpadded vp, eps, del (3 x nx*ny*nz), kept for the SV taper
     float vp1 = 0, eps1 = 0;           // padded model at linear index 1 (mute)
     bool model_set = false;
-    bool tuned = false;
     // 3D TTI medium (geo_fd3d_set_tilt): cos/sin of tilt and azimuth, 4 x nalloc
     DevBuf tilt, save;
     bool tti = false;
@@ -270,11 +269,37 @@ static int alloc_fields(geo_fd3d_plan *p, int f) {
 }
 
 // y chunking: a block marches over one chunk of y planes after filling its
-// queues (14 planes of P, 7 of v), so more chunks mean more blocks in flight
-// and shorter tails at the price of the fill.  The best count varies with
-// the grid (measured on GB300: 8-12 for 480^3, 6-12 for 216x200x184, 12-16
-// for 161x133x147), so set_model times the candidates (autotune_chunks);
-// this is the starting guess.
+// queues, so more chunks mean more blocks in flight and shorter tails at the
+// price of the fill.  The count is the one with the fewest rounds of resident
+// blocks (two per SM) times a chunk's planes, the fill counted as one; of those
+// within 1.5 % of it the largest, whose tail is shorter.  us a step of the
+// exact / fast form with it and with the best of 1 to 24: 121x93x107 + 20 (11
+// chunks) 65 / 60 against 64 / 60; 176x160x144 + 20 (7) 137 / 121, the best; 250x200x150 + 20 (8)
+// 219 / 189, the best; 400^3 + 40 (8) 1706 / 1379 against 1702 / 1374;
+// 500x120x260 + 30 (6) 499 / 419, the best.  (Timing seven counts on the device
+// at the first set_model, which this replaces, took 24 to 28 steps and did not
+// try 7.)
+int march_chunks(int tiles, int planes) {
+    static int slots = 0;
+    if (!slots) {
+        int dev = 0, sms = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+            sms = 152;
+        slots = 2 * sms;
+    }
+    long best = 0;
+    int n = 1;
+    for (int pass = 0; pass < 2; pass++)   // the least cost, then the largest count near it
+        for (int c = 1; c <= 16 && c <= std::max(1, planes / 8); c++) {
+            const int chunk = (planes + c - 1) / c, blocks = tiles * ((planes + chunk - 1) / chunk);
+            const long cost = (long)((blocks + slots - 1) / slots) * (chunk + 1);
+            if (pass == 0) best = best ? std::min(best, cost) : cost;
+            else if (1000 * cost <= 1015 * best) n = c;
+        }
+    return n;
+}
+
 static void set_chunks(geo_fd3d_plan *p, int c) {
     const int planes = p->nny - 8, ntiles = p->ntz * p->ntx;
     c = std::max(1, std::min(c, planes / 8));
@@ -282,12 +307,9 @@ static void set_chunks(geo_fd3d_plan *p, int c) {
     p->nitems = ntiles * ((planes + p->chunk - 1) / p->chunk);
 }
 
-static bool g_chunks_fixed() { return getenv("GEO_FD3D_CHUNKS") != nullptr; }
-
 static void choose_chunks(geo_fd3d_plan *p) {
-    int c = 4;
-    if (const char *e = getenv("GEO_FD3D_CHUNKS")) c = std::max(1, atoi(e));
-    set_chunks(p, c);
+    const char *e = getenv("GEO_FD3D_CHUNKS");
+    set_chunks(p, e ? std::max(1, atoi(e)) : march_chunks(p->ntz * p->ntx, p->nny - 8));
 }
 
 // One time step of field set f: the fused kernel reads level cur and writes
@@ -334,46 +356,6 @@ static int check_err(geo_fd3d_plan *p, cudaStream_t s) {
     GEO_CUDA(cudaStreamSynchronize(s));
     if (e) return fail(GEO_ERR_CUDA, "3D step: a TMA pipeline stage timed out");
     return GEO_OK;
-}
-
-// Autotuner for the y chunking: bare steps of the zeroed field set 0 (which
-// stays zero) timed with events for each candidate chunk count.
-static int autotune_chunks(geo_fd3d_plan *p, cudaStream_t s) {
-    if (g_chunks_fixed()) return GEO_OK;
-    GEO_TRY(zero_state(p, 0, s));
-    GEO_TRY(p->err.zero(s));
-    cudaEvent_t a, b;
-    GEO_CUDA(cudaEventCreate(&a));
-    GEO_CUDA(cudaEventCreate(&b));
-    StepArgs3D st{};
-    float best = 1e30f;
-    int best_c = 4;
-    const int planes = p->nny - 8;
-    for (int c : {2, 4, 6, 8, 10, 12, 16}) {
-        if (planes / c < 8) break;
-        set_chunks(p, c);
-        int rc = step3d(p, 0, st, s);
-        if (rc == GEO_OK && cudaEventRecord(a, s) != cudaSuccess) rc = fail(GEO_ERR_CUDA, "event record");
-        for (int k = 0; k < 3 && rc == GEO_OK; k++) rc = step3d(p, 0, st, s);
-        float ms = 0;
-        if (rc == GEO_OK && (cudaEventRecord(b, s) != cudaSuccess || cudaEventSynchronize(b) != cudaSuccess ||
-                             cudaEventElapsedTime(&ms, a, b) != cudaSuccess))
-            rc = fail(GEO_ERR_CUDA, "chunk autotune timing");
-        if (rc != GEO_OK) {
-            cudaEventDestroy(a);
-            cudaEventDestroy(b);
-            return rc;
-        }
-        if (ms < best) {
-            best = ms;
-            best_c = c;
-        }
-    }
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    set_chunks(p, best_c);
-    p->fs[0].cur = 0;
-    return check_err(p, s);
 }
 
 // SV taper box for shot `is` (GPU_vti3dfd_kernels.cu:155-174: R=15, r=4,
@@ -704,9 +686,9 @@ extern "C" int geo_fd3d_set_model(geo_fd3d_plan *p, const float *v, const float 
     sponge_profiles(V_GPU, D.nz, D.npd, D.dt, d0, q, q + p->nnz, q + 2 * p->nnz, q + 3 * p->nnz);
     GEO_CUDA(cudaMemcpyAsync(p->prof.p, prof.data(), prof.size() * 4, cudaMemcpyHostToDevice, s));
     GEO_CUDA(cudaStreamSynchronize(s));
-    if (!p->tuned) {
-        GEO_TRY(autotune_chunks(p, s));
-        p->tuned = true;
+    if (!p->model_set) {   // the first model: fields start from zero
+        GEO_TRY(zero_state(p, 0, s));
+        p->fs[0].cur = 0;
     }
     p->model_set = true;
     return GEO_OK;

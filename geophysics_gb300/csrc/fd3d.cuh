@@ -51,4 +51,8 @@ int run_shot_3d(geo_fd3d_plan *p, int is, cudaStream_t s, int (*on_step)(void *,
 int fetch_shot_3d(geo_fd3d_plan *p, float *shot, int mem, cudaStream_t s);
 int plan3d_dims(const geo_fd3d_plan *p, int *nnx, int *nny, int *nnz);
 
+// y chunks of a tile column for a kernel that marches along y with two blocks
+// per SM (fd3d.cu).
+int march_chunks(int tiles, int planes);
+
 }  // namespace geo

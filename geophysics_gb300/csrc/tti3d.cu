@@ -484,32 +484,6 @@ int tti_maps(const Tti3DStep &t, const MapPair **out) {
     return GEO_OK;
 }
 
-// y chunks of a tile column: the fewest rounds of resident blocks (two per
-// SM) times a chunk's planes, the seven that only fill the queues counted as
-// two.  300x300x200 + 40: 4 chunks (2.8 rounds of blocks) take 745 us a step, 7
-// (5.0) 731, 5 (3.6) 776, 1 (0.7) 996.
-int tti_chunks(int tiles, int planes) {
-    static int sms = 0;
-    if (const char *e = getenv("GEO_TTI3D_CHUNKS")) return std::max(1, std::min(atoi(e), planes / 8));
-    if (!sms) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
-            sms = 152;
-    }
-    int best = 1;
-    long cost = 0;
-    for (int n = 1; n <= 16 && n <= std::max(1, planes / 8); n++) {
-        const int chunk = (planes + n - 1) / n, blocks = tiles * ((planes + chunk - 1) / chunk);
-        const long c = (long)((blocks + 2 * sms - 1) / (2 * sms)) * (chunk + 2);
-        if (!cost || c < cost) {
-            cost = c;
-            best = n;
-        }
-    }
-    return best;
-}
-
 }  // namespace
 
 int launch_tti3d(const Tti3DStep &t, const StepArgs3D &args, cudaStream_t s) {
@@ -538,7 +512,10 @@ int launch_tti3d(const Tti3DStep &t, const StepArgs3D &args, cudaStream_t s) {
     G.ntz = (g.nnz + TZ - 1) / TZ;
     G.ntiles = G.ntz * ((g.nnx + TX - 1) / TX);
     const int planes = g.nny - 8;
-    const int nch = std::max(1, tti_chunks(G.ntiles, planes));
+    // 300x300x200 + 40: 4 chunks (2.8 rounds of blocks) take 745 us a step, 7
+    // (5.0, the rule's) 731, 5 (3.6) 776, 1 (0.7) 996
+    const char *e = getenv("GEO_TTI3D_CHUNKS");
+    const int nch = std::max(1, e ? std::min(std::max(1, atoi(e)), planes / 8) : march_chunks(G.ntiles, planes));
     G.chunk = (planes + nch - 1) / nch;
     const int nchunks = (planes + G.chunk - 1) / G.chunk;
     G.err = t.err;
