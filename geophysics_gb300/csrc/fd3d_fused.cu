@@ -223,6 +223,11 @@ __global__ void __launch_bounds__(kFusedThreads, kFusedBlocks)
         zprof[3 * kTZ + tid] = g.az2[z];
     }
     __syncthreads();
+    // Launched while the step before still runs (the profiles above are fixed
+    // for the run); from here on that step's results are read.  The next step's
+    // blocks may start once all of this one's have.
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     // Boxes of plane ylo + i into stage s, spread over the warps'
     // first lanes.  The expected byte count may be posted after a copy
@@ -637,7 +642,17 @@ int launch_fused3d(const StepMaps &maps, const Fused3D &g, int mode, const StepA
         attr_set[fast][rtm] = true;
     }
     void *a[] = {(void *)&maps, (void *)&g, (void *)&st};
-    GEO_CUDA(cudaLaunchKernel(fn, dim3(g.nitems), dim3(kFusedThreads), a, kFusedSmem, s));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(g.nitems);
+    cfg.blockDim = dim3(kFusedThreads);
+    cfg.dynamicSmemBytes = kFusedSmem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    GEO_CUDA(cudaLaunchKernelExC(&cfg, fn, a));
     return check_launch("fused3d");
 }
 
