@@ -275,6 +275,7 @@ __device__ __forceinline__ float block_max(float v, float *red) {
 __global__ void __launch_bounds__(256) k_ae_e1(const E1Args a) {
     __shared__ float xs[kAePts];
     __shared__ float red[8];
+    tc::after_predecessor();
     const int b = blockIdx.x, t = threadIdx.x;
     float mx = 0.0f;
     if (b < a.nb) {
@@ -390,6 +391,7 @@ __global__ void __launch_bounds__(256, 2) k_ae_e12(const __grid_constant__ CUten
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = tslot + grp * 64;
+    tc::after_predecessor();
     if (!tc::mbar_wait(&wbar, 0)) s_abort[0] = s_abort[1] = 1;
     __syncthreads();
     const AeVolume &v = a.vol;
@@ -582,6 +584,7 @@ __global__ void __launch_bounds__(kD21Threads, 2)
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = tslot;
+    tc::after_predecessor();
 
     if (warp == 8 && lane == 0) {
         unsigned it = 0;
@@ -787,6 +790,7 @@ struct D1Args {
 __global__ void __launch_bounds__(256) k_ae_d1(const D1Args a) {
     extern __shared__ float sm[];
     __shared__ float red[8];
+    tc::after_predecessor();
     const int b = blockIdx.x, t = threadIdx.x;
     if (b >= a.nb) return;
     float *A = sm, *B = sm + 512 * kOutA;
@@ -1014,6 +1018,7 @@ __global__ void __launch_bounds__(256) k_ae_escape_copy(const int *esc, const __
 // gradient at E1's output.
 __global__ void __launch_bounds__(256) k_ae_e1_bwd(const float *xn, const __nv_bfloat16 *dh1, float *ge1, int nb) {
     extern __shared__ float sm[];
+    tc::after_predecessor();
     const int b = blockIdx.x, t = threadIdx.x;
     if (b >= nb) return;
     float *A = sm, *B = sm + 512 * kOutA;
@@ -1054,6 +1059,7 @@ struct ColsumArgs {
 
 __global__ void __launch_bounds__(256) k_ae_colsum(const ColsumArgs g) {
     __shared__ float red[256 * 8];
+    tc::after_predecessor();
     int l = 0;
     while (l < 5 && (int)blockIdx.x >= g.it[l + 1].base) l++;
     const ColsumLevel &w = g.it[l];
@@ -1311,7 +1317,7 @@ static int wgrads(geo_ae *ae, int rows, const __nv_bfloat16 *const *dout, const 
         base += k.ctas;
     }
     GEO_TRY(tc_wgrad(lv, 6, ae->err.as<int>(), s));
-    k_ae_colsum<<<base, 256, 0, s>>>(c);
+    GEO_CUDA(launch_early(k_ae_colsum, base, 256, 0, s, c));
     return check_launch("ae_colsum");
 }
 
@@ -1438,7 +1444,7 @@ int ae_encode_volume(geo_ae *ae, const AeVolume &v, void *code, float *scale, in
     GEO_TRY(tc_map_bf16(&tw, bf(ae->wb) + ae->off.wb[1], 64, 128, 64));
     GEO_TRY(tc_map_bf16(&to, ae->h2.p, rows * 64, 64, 32));
     GEO_TRY(ae_smem());
-    k_ae_e12<<<std::min((a.tiles + 1) / 2, 2 * ae_sms()), 256, kE12Smem, s>>>(tw, to, a);
+    GEO_CUDA(launch_early(k_ae_e12, std::min((a.tiles + 1) / 2, 2 * ae_sms()), 256, kE12Smem, s, tw, to, a));
     GEO_TRY(check_launch("ae_e12"));
     GEO_TRY(level(ae, 2, rows, bf(ae->h2), bf(ae->h3), s));
     GEO_TRY(level(ae, 3, rows, bf(ae->h3), static_cast<__nv_bfloat16 *>(code), s));
@@ -1499,7 +1505,7 @@ int ae_decode_volume(geo_ae *ae, const AeVolume &v, const void *code, const floa
         GEO_TRY(tc_map_bf16(&ta, ae->g2.p, rows * 64, 64, 128));
         GEO_TRY(tc_map_bf16(&tw, bf(ae->wb) + ae->off.wb[6], 128, 64, 128));
         GEO_TRY(ae_smem());
-        k_ae_d21<<<std::min(a.tiles, 2 * ae_sms()), kD21Threads, kD21Smem, s>>>(ta, tw, a);
+        GEO_CUDA(launch_early(k_ae_d21, std::min(a.tiles, 2 * ae_sms()), kD21Threads, kD21Smem, s, ta, tw, a));
         return check_launch("ae_d21");
     }
     GEO_TRY(decode_rows(ae, rows, static_cast<const __nv_bfloat16 *>(code), s));
@@ -1548,7 +1554,7 @@ static int train_pass(geo_ae *ae, int rows, double *loss, const float *wsum, con
     a.wrow = wsum ? ae->wrow.as<float>() : nullptr;
     a.wsum = wsum;
     GEO_TRY(outer_smem());
-    k_ae_d1<<<rows, 256, kOutFloats * 4, s>>>(a);
+    GEO_CUDA(launch_early(k_ae_d1, rows, 256, kOutFloats * 4, s, a));
     GEO_TRY(check_launch("ae_d1_train"));
     if (!backward) return GEO_OK;
     GEO_TRY(level_bwd(ae, 6, rows, bf(ae->dg1), bf(ae->dg2), bf(ae->g2), s));   // D2
@@ -1560,7 +1566,8 @@ static int train_pass(geo_ae *ae, int rows, double *loss, const float *wsum, con
     const __nv_bfloat16 *dout[7] = {nullptr, bf(ae->dh2), bf(ae->dh3), bf(ae->dz), bf(ae->dg3), bf(ae->dg2), bf(ae->dg1)};
     const __nv_bfloat16 *in[7] = {nullptr, bf(ae->h1), bf(ae->h2), bf(ae->h3), bf(ae->z), bf(ae->g3), bf(ae->g2)};
     GEO_TRY(wgrads(ae, rows, dout, in, s));
-    k_ae_e1_bwd<<<rows, 256, kOutFloats * 4, s>>>(ae->xn.as<float>(), bf(ae->dh1), ae->grad.as<float>() + ae->off.w[0], rows);
+    GEO_CUDA(launch_early(k_ae_e1_bwd, rows, 256, kOutFloats * 4, s, ae->xn.as<float>(), bf(ae->dh1),
+                          ae->grad.as<float>() + ae->off.w[0], rows));
     return check_launch("ae_e1_bwd");
 }
 

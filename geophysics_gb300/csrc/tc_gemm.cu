@@ -95,6 +95,7 @@ __global__ void __launch_bounds__(128, 2)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
+    after_predecessor();
 
     if (warp == 0 && lane == 0) {
         // producer
@@ -264,13 +265,15 @@ __global__ void __launch_bounds__(kWalkThreads, 1)
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int n = threadIdx.x; n < g.N; n += kWalkThreads) sbias[n] = g.bias ? g.bias[n] : 0.0f;
     __syncwarp();
     if (warp == 9) tmem_alloc(tslot, 2 * BN < 32 ? 32 : 2 * BN);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
+    after_predecessor();
+    for (int n = threadIdx.x; n < g.N; n += kWalkThreads) sbias[n] = g.bias ? g.bias[n] : 0.0f;
+    __syncthreads();
 
     if (warp == 8 && lane == 0) {
         bool ok = true;
@@ -429,7 +432,7 @@ static int launch_bn(const TcGemm &g, cudaStream_t s) {
     GEO_TRY(tc_map_bf16(&ta, g.A, g.M, g.K, kGM));
     GEO_TRY(tc_map_bf16(&tb, g.B, g.N, g.K, BN));
     const dim3 grid((unsigned)(g.M / kGM) * (unsigned)(g.N / BN));
-    k_tc_gemm<BN, ST><<<grid, 128, S::kSmem, s>>>(ta, tb, g);
+    GEO_CUDA(launch_early(k_tc_gemm<BN, ST>, grid.x, 128, S::kSmem, s, ta, tb, g));
     return check_launch("tc_gemm");
 }
 
@@ -448,7 +451,7 @@ static int launch_walk(const TcGemm &g, cudaStream_t s) {
     GEO_TRY(tc_map_bf16(&tb, g.B, g.N, g.K, BN));
     GEO_TRY(tc_map_bf16(&to, g.out, g.M, g.N, 32));
     const int tiles = (g.M / kGM) * (g.N / BN);
-    k_tc_walk<BN, RB><<<std::min(tiles, sms), kWalkThreads, S::kSmem, s>>>(ta, tb, to, g, tiles);
+    GEO_CUDA(launch_early(k_tc_walk<BN, RB>, std::min(tiles, sms), kWalkThreads, S::kSmem, s, ta, tb, to, g, tiles));
     return check_launch("tc_walk");
 }
 
@@ -560,6 +563,7 @@ __global__ void __launch_bounds__(128, 2) k_tc_wgrad(const __grid_constant__ Wgr
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
+    after_predecessor();
     const int nbox = w.bn / 64;
 
     if (warp == 0 && lane == 0) {
@@ -660,7 +664,7 @@ int tc_wgrad(const TcWgradLevel *lv, int n, int *err, cudaStream_t s) {
         GEO_CUDA(cudaFuncSetAttribute(k_tc_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgSmem));
         attr = true;
     }
-    k_tc_wgrad<<<base, 128, kWgSmem, s>>>(g);
+    GEO_CUDA(launch_early(k_tc_wgrad, base, 128, kWgSmem, s, g));
     return check_launch("tc_wgrad");
 }
 

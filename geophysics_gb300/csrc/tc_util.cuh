@@ -5,6 +5,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <utility>
 
 namespace geo {
 namespace tc {
@@ -33,6 +34,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
         : "r"(su32(bar)), "r"(parity)
         : "memory");
     return ok != 0;
+}
+
+// First thing of a kernel that launch_early starts while its predecessor in the
+// stream still runs: wait for that one's results, then let the successor come.
+// (What kernels before the predecessor wrote is complete by then.)
+__device__ __forceinline__ void after_predecessor() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 __device__ __forceinline__ uint64_t gtimer() {
@@ -164,4 +173,22 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t *r) {
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 }  // namespace tc
+
+// Launch a kernel that calls tc::after_predecessor: its blocks come up while
+// the kernel before it in the stream ends.
+template <class... P, class... A>
+cudaError_t launch_early(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A &&...args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
+}
+
 }  // namespace geo
