@@ -226,8 +226,7 @@ __global__ void __launch_bounds__(kFusedThreads, kFusedBlocks)
     // Launched while the step before still runs (the profiles above are fixed
     // for the run); from here on that step's results are read.  The next step's
     // blocks may start once all of this one's have.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    tc::after_predecessor();
 
     // Boxes of plane ylo + i into stage s, spread over the warps'
     // first lanes.  The expected byte count may be posted after a copy
@@ -641,18 +640,8 @@ int launch_fused3d(const StepMaps &maps, const Fused3D &g, int mode, const StepA
         GEO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFusedSmem));
         attr_set[fast][rtm] = true;
     }
-    void *a[] = {(void *)&maps, (void *)&g, (void *)&st};
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(g.nitems);
-    cfg.blockDim = dim3(kFusedThreads);
-    cfg.dynamicSmemBytes = kFusedSmem;
-    cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    GEO_CUDA(cudaLaunchKernelExC(&cfg, fn, a));
+    using Fn = void (*)(const StepMaps, const Fused3D, const StepArgs3D);
+    GEO_CUDA(launch_early(reinterpret_cast<Fn>(const_cast<void *>(fn)), (unsigned)g.nitems, dim3(kFusedThreads), kFusedSmem, s, maps, g, st));
     return check_launch("fused3d");
 }
 

@@ -177,10 +177,10 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 // Launch a kernel that calls tc::after_predecessor: its blocks come up while
 // the kernel before it in the stream ends.
 template <class... P, class... A>
-cudaError_t launch_early(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A &&...args) {
+cudaError_t launch_early(void (*k)(P...), unsigned grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
+    cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at{};

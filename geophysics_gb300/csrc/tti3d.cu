@@ -196,6 +196,7 @@ __global__ void __launch_bounds__(TZ *NW, 2)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    tc::after_predecessor();
     auto issue = [&](int i) {
         const int s = i % NST, q = ylo - 3 + i, y = ylo + i - 7;
         const bool out = i >= 7;
@@ -294,6 +295,7 @@ __global__ void __launch_bounds__(TZ *NW, 2)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    tc::after_predecessor();
     auto issue = [&](int i) {
         const int s = i % NST, q = ylo - 4 + i, y = ylo + i - 7;
         const bool out = i >= 7;
@@ -520,9 +522,9 @@ int launch_tti3d(const Tti3DStep &t, const StepArgs3D &args, cudaStream_t s) {
     const int nchunks = (planes + G.chunk - 1) / G.chunk;
     G.err = t.err;
     const dim3 block(TZ, NW), grid(G.ntiles * nchunks);
-    k_tti3d_vel<<<grid, block, VEL_SMEM, s>>>(m->v, G, t.u1, t.v1, t.w1);
+    GEO_CUDA(launch_early(k_tti3d_vel, grid.x, block, VEL_SMEM, s, m->v, G, t.u1, t.v1, t.w1));
     GEO_TRY(check_launch("tti3d_vel"));
-    k_tti3d_stress<<<grid, block, STR_SMEM, s>>>(m->s, G, t.P1, t.Q1, t.save, st);
+    GEO_CUDA(launch_early(k_tti3d_stress, grid.x, block, STR_SMEM, s, m->s, G, t.P1, t.Q1, t.save, st));
     return check_launch("tti3d_stress");
 }
 
