@@ -43,7 +43,7 @@ CFG = {"workload": "3D VTI FD shot 400^3 (+40 sponge), 2500 steps, dt=0.8 ms, 10
 # from ncu on the 200^3 + 20 case (same sponge fraction, 240^3 padded, a
 # few GB on the device) scaled by the updated points (472/232)^3; command and
 # figures in profiles/fd3d_fused_200cube_traffic.md.
-TRAFFIC_BYTES_PER_STEP = 8665488602
+TRAFFIC_BYTES_PER_STEP = 8237399441
 
 
 def updates_per_step():

@@ -20,8 +20,8 @@
 // The blocks stay for the run because of the two L2 halves: launched anew
 // each step, a tile lands on any SM, so on either half, and 93 MB of the
 // 1700x601 + 50 shot's 80 MB of state and model moved through DRAM every step;
-// with the same SM, 2 MB do (forward: 26 us a step launched per step, 17.6
-// here).  Odd steps walk the tiles backwards, so that what the step before
+// with the same SM, 12 MB do (forward: 22.7 to 26 us a step launched per step,
+// 17.1 here).  Odd steps walk the tiles backwards, so that what the step before
 // left in L2 is read first: nothing forward, where all of it fits, and 41.7
 // -> 39.1 us backward, where two sides (140 MB and the gathers) do not.
 //
@@ -40,8 +40,8 @@
 // whose rotated derivatives need both halos of every field (twice the velocity
 // work of a tile of 8 columns, 1.6 times of 16): 600x300 11.5 -> 7.5; RTM
 // program 1700x601, 65 angles, forward 37.3 -> 24.9, backward 74.0 -> 56.3.
-// Large grids are bound by instruction issue (55 % of the slots at 24 warps per
-// SM; 340 instructions a point, a quarter of them halo work), small ones by the
+// Large grids are bound by instruction issue (60 % of the slots at 24 warps per
+// SM; 325 instructions a point with 8 columns, 200 with 16), small ones by the
 // barrier and the TMA round trip.  Tried: four warps with two columns each
 // (1.04 times forward, 1.3 backward), split stresses and model from L2 into
 // registers instead of TMA (1.05 and 1.15), flags of the neighbours' blocks

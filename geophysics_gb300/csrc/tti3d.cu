@@ -34,7 +34,7 @@
 // against two x columns per thread with 4-byte accesses (six derivatives of 16
 // shared-memory loads a point became five of 6.5) and four chunks whatever the
 // grid.  The velocity kernel runs at 6.0 TB/s of its 48 B a point; the stress
-// kernel (56 B a point, 283 instructions) is bound by issue at 16 warps per SM
+// kernel (56 B a point, 290 instructions) is bound by issue at 16 warps per SM
 // as much as by memory.
 //
 // The point source is added to P,Q of the old level before the velocity
