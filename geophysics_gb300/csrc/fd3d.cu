@@ -751,22 +751,66 @@ extern "C" int geo_fd3d_shot(const geo_fd3d_desc *desc, int is, const float *v, 
 // ---------------------------------------------------------------- RTM 3D
 namespace geo {
 
-// Source P of the interior box into a dense snapshot (iz + nz*(ix + nx*iy)).
-__global__ void k_snap_store(Grid3D g, const float *P, float *snap) {
-    const long n = (long)g.nx * g.ny * g.nz;
-    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
-        const int iz = (int)(k % g.nz), ix = (int)((k / g.nz) % g.nx), iy = (int)(k / ((long)g.nz * g.nx));
-        snap[k] = P[(g.npd + iz) + (long)g.ldz * (g.npd + ix) + g.sxy * (g.npd + iy)];
+// Interior column k = ix + nx iy of a padded field: its first depth.
+__device__ __forceinline__ long interior_col(const Grid3D &g, int k) {
+    return g.npd + (long)g.ldz * (g.npd + k % g.nx) + g.sxy * (g.npd + k / g.nx);
+}
+
+// Source P of the interior box into a dense snapshot (iz + nz*(ix + nx*iy)),
+// and mig += w * snap * gP on the interior box (the codec's imaging, same
+// order).  A warp copies a column, V depths a lane (four where npd and nz are
+// multiples of four, so that every column starts on a vector); bound by
+// memory.  176x160x144: 19.4 -> 8.9 and 21.7 -> 14.9 us against an element per
+// thread and step of a grid-stride loop with three divisions each.
+template <int V>
+__global__ void __launch_bounds__(256) k_snap_store(Grid3D g, const float *__restrict__ P, float *__restrict__ snap) {
+    const int k = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (k >= g.nx * g.ny) return;
+    const float *src = P + interior_col(g, k);
+    float *dst = snap + (long)k * g.nz;
+    for (int z = (threadIdx.x & 31) * V; z < g.nz; z += 32 * V) {
+        if constexpr (V == 4) *reinterpret_cast<float4 *>(dst + z) = *reinterpret_cast<const float4 *>(src + z);
+        else dst[z] = src[z];
     }
 }
 
-// mig += w * snap * gP on the interior box (the codec's imaging, same order).
-__global__ void k_snap_image(Grid3D g, const float *snap, const float *gP, float *mig, float w) {
-    const long n = (long)g.nx * g.ny * g.nz;
-    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
-        const int iz = (int)(k % g.nz), ix = (int)((k / g.nz) % g.nx), iy = (int)(k / ((long)g.nz * g.nx));
-        mig[k] = mig[k] + w * snap[k] * gP[(g.npd + iz) + (long)g.ldz * (g.npd + ix) + g.sxy * (g.npd + iy)];
+template <int V>
+__global__ void __launch_bounds__(256) k_snap_image(Grid3D g, const float *__restrict__ snap, const float *__restrict__ gP,
+                                                    float *__restrict__ mig, float w) {
+    const int k = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (k >= g.nx * g.ny) return;
+    const float *p = gP + interior_col(g, k);
+    const long o = (long)k * g.nz;
+    for (int z = (threadIdx.x & 31) * V; z < g.nz; z += 32 * V) {
+        if constexpr (V == 4) {
+            const float4 a = *reinterpret_cast<const float4 *>(snap + o + z), b = *reinterpret_cast<const float4 *>(p + z);
+            float4 m = *reinterpret_cast<float4 *>(mig + o + z);
+            m.x = m.x + w * a.x * b.x;
+            m.y = m.y + w * a.y * b.y;
+            m.z = m.z + w * a.z * b.z;
+            m.w = m.w + w * a.w * b.w;
+            *reinterpret_cast<float4 *>(mig + o + z) = m;
+        } else {
+            mig[o + z] = mig[o + z] + w * snap[o + z] * p[z];
+        }
     }
+}
+
+static bool snap_vectors(const Grid3D &g, const float *a, const float *b, const float *c) {
+    return g.npd % 4 == 0 && g.nz % 4 == 0 && g.ldz % 4 == 0 && g.sxy % 4 == 0 &&
+           ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
+}
+static int snap_store(const Grid3D &g, const float *P, float *snap, cudaStream_t s) {
+    const unsigned n = (unsigned)(((long)g.nx * g.ny + 7) / 8);
+    if (snap_vectors(g, P, snap, nullptr)) k_snap_store<4><<<n, 256, 0, s>>>(g, P, snap);
+    else k_snap_store<1><<<n, 256, 0, s>>>(g, P, snap);
+    return check_launch("snap_store");
+}
+static int snap_image(const Grid3D &g, const float *snap, const float *gP, float *mig, float w, cudaStream_t s) {
+    const unsigned n = (unsigned)(((long)g.nx * g.ny + 7) / 8);
+    if (snap_vectors(g, snap, gP, mig)) k_snap_image<4><<<n, 256, 0, s>>>(g, snap, gP, mig, w);
+    else k_snap_image<1><<<n, 256, 0, s>>>(g, snap, gP, mig, w);
+    return check_launch("snap_image");
 }
 
 // Poynting angle gathers after a backward step (Poynting_Adcigs :618-661):
@@ -960,8 +1004,7 @@ extern "C" int geo_rtm3d_adcig(const geo_rtm3d_desc *desc, const float *v, const
                 const Grid3D g = grid_of(p, 0);
                 const int j = it / k;
                 if (method == GEO_RTM_SNAPSHOT) {
-                    k_snap_store<<<grid_blocks(nimg), 256, 0, s>>>(g, g.P, snaps.as<float>() + (size_t)j * nimg);
-                    GEO_TRY(check_launch("snap_store"));
+                    GEO_TRY(snap_store(g, g.P, snaps.as<float>() + (size_t)j * nimg, s));
                 } else {
                     AeVolume vb = box;
                     vb.src = g.P;
@@ -1019,9 +1062,7 @@ extern "C" int geo_rtm3d_adcig(const geo_rtm3d_desc *desc, const float *v, const
                     GEO_TRY(step3d(p, 0, sr, s));
                     if (is_snap(j)) {
                         const Grid3D g = grid_of(p, 0);
-                        k_snap_store<<<grid_blocks(nimg), 256, 0, s>>>(
-                            g, g.P, snaps.as<float>() + (size_t)((j - c * K) / k) * nimg);
-                        GEO_TRY(check_launch("snap_store"));
+                        GEO_TRY(snap_store(g, g.P, snaps.as<float>() + (size_t)((j - c * K) / k) * nimg, s));
                     }
                 }
             }
@@ -1043,9 +1084,7 @@ extern "C" int geo_rtm3d_adcig(const geo_rtm3d_desc *desc, const float *v, const
                 const int j = it / k;
                 if (method == GEO_RTM_SNAPSHOT || method == GEO_RTM_CHECKPOINT) {
                     const size_t slot = method == GEO_RTM_SNAPSHOT ? (size_t)j : (size_t)((it % K) / k);
-                    k_snap_image<<<grid_blocks(nimg), 256, 0, s>>>(g, snaps.as<float>() + slot * nimg, g.P,
-                                                                    mig.as<float>(), (float)k);
-                    GEO_TRY(check_launch("snap_image"));
+                    GEO_TRY(snap_image(g, snaps.as<float>() + slot * nimg, g.P, mig.as<float>(), (float)k, s));
                 } else {
                     GEO_TRY(ae_decode_volume(R.ae, box, codes.as<__nv_bfloat16>() + (size_t)j * crow * kAeLat,
                                              scales.as<float>() + (size_t)j * crow, escs.as<int>() + (size_t)j * crow,

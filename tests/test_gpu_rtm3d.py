@@ -130,3 +130,16 @@ def test_fused_step_vectors_and_tile_edges(geo, orc, monkeypatch, nx, ny, nz, np
         a, b = plan.fields()
         plan.close()
         assert np.array_equal(a, P) and np.array_equal(b, Q)
+
+
+# snapshots stored and imaged four depths at a time (npd and nz multiples of
+# four) and one by one, columns longer than a warp's 128 depths
+@pytest.mark.parametrize("nx,ny,nz,npd", [(6, 5, 132, 8), (7, 6, 24, 8), (6, 5, 131, 8), (7, 5, 24, 6), (9, 4, 10, 7)])
+def test_rtm3d_snapshot_columns(geo, orc, nx, ny, nz, npd):
+    v, e, d = random_model_3d(nx, ny, nz, seed=16)
+    kw = dict(npd=npd, nt=60, dx=10.0, dy=10.0, dz=10.0, dt=np.float32(1e-3), favg=25.0, pfac=10.0, fsx=nx // 2,
+              fsy=ny // 2, fsz=2, dsx=1, ns=1, mute_tt=5)
+    mo, io, _ = orc.rtm3d(v, e, d, mode=1, snap_every=3, **kw)
+    mg, ig = geo.rtm3d(v, e, d, mode=1, laplace=False, illum=True, method="snapshot", snap_every=3, **kw)
+    assert np.abs(mo).max() > 0
+    assert np.array_equal(ig, io) and np.array_equal(mg, mo)
