@@ -833,6 +833,7 @@ __global__ void k_adcig3d(Grid3D s, Grid3D r, float *adcig, const float *tab, in
         const int ix = (int)(c % nxa), iy = (int)(c / nxa);
         const long id = (s.npd + iz) + s.ldz * (long)(s.npd + ix * dcdp) + s.sxy * (long)(s.npd + iy * dcdp);
         const float sP = s.P[id], gP = r.P[id];
+        if (sP * gP == 0.0f) continue;   // adds nothing: the sums start at +0 and never become -0
         const float Ssx = -sP * s.u[id], Ssy = -sP * s.v[id], Ssz = -s.Q[id] * s.w[id];
         const float Sgx = gP * r.u[id], Sgy = gP * r.v[id], Sgz = r.Q[id] * r.w[id];
         const float b1 = Ssx * Ssx + Ssy * Ssy + Ssz * Ssz, b2 = Sgx * Sgx + Sgy * Sgy + Sgz * Sgz;

@@ -25,10 +25,10 @@
 //
 // Measured per step against one depth and two columns per thread with every
 // array in the TMA stages and two barriers a plane: 400^3 + 40 fast 1.557 ->
-// 1.395 ms (8.4 GB of DRAM traffic: 6.0 TB/s), exact 1.780 -> 1.736 ms;
+// 1.395 ms (8.2 GB of DRAM traffic: 5.9 TB/s), exact 1.780 -> 1.736 ms;
 // 176x160x144 + 20 with imaging 0.184 -> 0.137 ms; 121x93x107 + 20 exact 83
 // -> 62 us.  The fast form is bound by DRAM at the large size (halos miss L2:
-// 1.24x the algorithmic bytes), by issue and latency at the small ones (240^3:
+// 1.21x the algorithmic bytes), by issue and latency at the small ones (240^3:
 // 333 thread instructions a point, issue 58%, DRAM 64% busy).  Four depths
 // per thread (128 threads, 168 registers, 12 warps an SM) took 1.53 ms, 190
 // and 100 us: half the instructions' latency is exposed; capped at 128

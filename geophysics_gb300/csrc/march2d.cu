@@ -445,6 +445,8 @@ __global__ void __launch_bounds__(kMarchThreads, march_blocks(MODE))
 #pragma unroll
                         for (int j = 0; j < 4; j++) {
                             if (gz0 + j < 0 || gz0 + j >= nz) continue;
+                            // a zero product adds nothing: the sums start at +0 and never become -0
+                            if (Pn.v[j] * sP[j] == 0.0f) continue;
                             const float sx = -sP[j] * su[j], sz = -sQ[j] * sw[j];
                             const float rx = Pn.v[j] * q[4].v[j], rz = Qn.v[j] * wn.v[j];
                             const float b1 = sx * sx + sz * sz, b2 = rx * rx + rz * rz, a = sx * rx + sz * rz;

@@ -36,10 +36,10 @@
 // launch; tiles kept in shared memory with exchange copies where the grid
 // fits that way), us a step: 2401x601 + 50 39.5 -> 18.0; 1200x601 25.0 -> 10.1;
 // 600x601 10.9 -> 7.4; 401x401 7.4 -> 5.1; 101x121 + 20 5.4 -> 3.3; RTM program
-// 1700x601 forward 26.1 -> 17.1, backward with 70 angles 56.3 -> 38.9.  TTI,
+// 1700x601 forward 26.1 -> 17.1, backward with 70 angles 56.3 -> 36.4.  TTI,
 // whose rotated derivatives need both halos of every field (twice the velocity
 // work of a tile of 8 columns, 1.6 times of 16): 600x300 11.5 -> 7.5; RTM
-// program 1700x601, 65 angles, forward 37.3 -> 24.9, backward 74.0 -> 56.3.
+// program 1700x601, 65 angles, forward 37.3 -> 24.4, backward 74.0 -> 52.9.
 // Large grids are bound by instruction issue (60 % of the slots at 24 warps per
 // SM; 325 instructions a point with 8 columns, 200 with 16), small ones by the
 // barrier and the TMA round trip.  Tried: four warps with two columns each
@@ -563,16 +563,18 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
                     for (int j = 0; j < 2; j++) {
                         if (!in[c][j]) continue;
                         const float sP_ = at2(sv[c][0], j), gP = at2(Pn, j);
-                        if (ga < 0) continue;
+                        // a zero product adds nothing to any bin (the sums start at +0
+                        // and never become -0): most points ahead of the wavefronts
+                        // (1700x601 backward 38.9 -> 36.4 us a step)
+                        const float sg = sP_ * gP;
+                        if (ga < 0 || sg == 0.0f) continue;
                         const float Ssx = -sP_ * at2(sv[c][2], j), Ssz = -at2(sv[c][1], j) * at2(sv[c][3], j);
                         const float Sgx = gP * at2(q[4], j), Sgz = at2(Qn, j) * at2(wn[c], j);
                         const float b1 = Ssx * Ssx + Ssz * Ssz, b2 = Sgx * Sgx + Sgz * Sgz;
                         const int ia = poynting_bin(Ssx * Sgx + Ssz * Sgz, b1, b2, cs_thr, a.nangle);
                         if (ia < 0) continue;
                         const float co = cs_cos[ia];
-                        av[j] = sP_ * gP * co * co * co;
-                        // sums start at +0 and never become -0, so a zero adds nothing
-                        if (av[j] == 0.0f) continue;
+                        av[j] = sg * co * co * co;
                         ag[j] = a.adcig + gz + j + (long)g.nz * ia + (long)g.nz * a.nangle * ga;
                         old[j] = __ldcs(ag[j]);
                     }
