@@ -14,6 +14,7 @@
 // Layout: id = iz + nnz*(ix + nnx*iy), z fastest, as the reference.
 #include "geo_internal.h"
 #include "fd3d.cuh"
+#include "tc_util.cuh"
 #include "fd3d_fused.cuh"
 #include "ae.cuh"
 #include "adcig.cuh"
@@ -71,6 +72,7 @@ __global__ void k_ring3d(Grid3D g, float *P, float *Q, float *bp, float *bq, lon
 // time-major record back at depth npml-1.
 __global__ void k_inject3d(Grid3D g, float *P, float *Q, const float *rec_tm, int it, int rx0, int drx, int nrx,
                            int ry0, int dry, int nry) {
+    tc::after_predecessor();
     const int npd = g.npd;
     const long n = (long)nrx * nry;
     for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
@@ -764,6 +766,7 @@ __device__ __forceinline__ long interior_col(const Grid3D &g, int k) {
 // thread and step of a grid-stride loop with three divisions each.
 template <int V>
 __global__ void __launch_bounds__(256) k_snap_store(Grid3D g, const float *__restrict__ P, float *__restrict__ snap) {
+    tc::after_predecessor();
     const int k = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (k >= g.nx * g.ny) return;
     const float *src = P + interior_col(g, k);
@@ -777,6 +780,7 @@ __global__ void __launch_bounds__(256) k_snap_store(Grid3D g, const float *__res
 template <int V>
 __global__ void __launch_bounds__(256) k_snap_image(Grid3D g, const float *__restrict__ snap, const float *__restrict__ gP,
                                                     float *__restrict__ mig, float w) {
+    tc::after_predecessor();
     const int k = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (k >= g.nx * g.ny) return;
     const float *p = gP + interior_col(g, k);
@@ -802,14 +806,12 @@ static bool snap_vectors(const Grid3D &g, const float *a, const float *b, const 
 }
 static int snap_store(const Grid3D &g, const float *P, float *snap, cudaStream_t s) {
     const unsigned n = (unsigned)(((long)g.nx * g.ny + 7) / 8);
-    if (snap_vectors(g, P, snap, nullptr)) k_snap_store<4><<<n, 256, 0, s>>>(g, P, snap);
-    else k_snap_store<1><<<n, 256, 0, s>>>(g, P, snap);
+    GEO_CUDA(launch_early(snap_vectors(g, P, snap, nullptr) ? k_snap_store<4> : k_snap_store<1>, n, 256, 0, s, g, P, snap));
     return check_launch("snap_store");
 }
 static int snap_image(const Grid3D &g, const float *snap, const float *gP, float *mig, float w, cudaStream_t s) {
     const unsigned n = (unsigned)(((long)g.nx * g.ny + 7) / 8);
-    if (snap_vectors(g, snap, gP, mig)) k_snap_image<4><<<n, 256, 0, s>>>(g, snap, gP, mig, w);
-    else k_snap_image<1><<<n, 256, 0, s>>>(g, snap, gP, mig, w);
+    GEO_CUDA(launch_early(snap_vectors(g, snap, gP, mig) ? k_snap_image<4> : k_snap_image<1>, n, 256, 0, s, g, snap, gP, mig, w));
     return check_launch("snap_image");
 }
 
@@ -1069,8 +1071,8 @@ extern "C" int geo_rtm3d_adcig(const geo_rtm3d_desc *desc, const float *v, const
             }
             {
                 Grid3D gg = grid_of(p, 1);
-                k_inject3d<<<grid_blocks(ntr), 256, 0, s>>>(gg, gg.P, gg.Q, p->rec_tm.as<float>(), it, D.rx0, D.drx,
-                                                             D.nrx, D.ry0, D.dry, D.nry);
+                GEO_CUDA(launch_early(k_inject3d, grid_blocks(ntr), 256, 0, s, gg, gg.P, gg.Q, p->rec_tm.as<float>(), it, D.rx0,
+                                      D.drx, D.nrx, D.ry0, D.dry, D.nry));
                 GEO_TRY(check_launch("inject3d"));
             }
             if (method == GEO_RTM_BOUNDARY) gb.other_P = grid_of(p, 0).P;  // the source side's new level
