@@ -396,23 +396,25 @@ __global__ void __launch_bounds__(256, 2) k_ae_e12(const __grid_constant__ CUten
     __syncthreads();
     const AeVolume &v = a.vol;
     const bool vec = lines_aligned(v, v.src);
-    float4 f[16];   // line x + 4 y of the thread's cell of tile t
+    // line x + 4 y of the thread's cell of tile t: plain loads, the step that
+    // wrote the field may still run when this kernel starts
+    float4 f[16];
     auto load = [&](int t) {
         const CellAt c(v, t, r);
         const float *p = v.src + (long)(v.oz + c.iz) + v.ldz * (v.ox + c.ix) + v.sxy * (v.oy + c.iy);
         const bool in = c.b < a.nb;
         if (vec && in && c.iz + 4 <= v.nz && c.ix + 4 <= v.nx && c.iy + 4 <= v.ny) {
 #pragma unroll
-            for (int q = 0; q < 16; q++) f[q] = __ldg(reinterpret_cast<const float4 *>(p + v.ldz * (q & 3) + v.sxy * (q >> 2)));
+            for (int q = 0; q < 16; q++) f[q] = *reinterpret_cast<const float4 *>(p + v.ldz * (q & 3) + v.sxy * (q >> 2));
         } else {
 #pragma unroll
             for (int q = 0; q < 16; q++) {
                 const bool l = in && c.ix + (q & 3) < v.nx && c.iy + (q >> 2) < v.ny;
                 const float *s = p + v.ldz * (q & 3) + v.sxy * (q >> 2);
-                f[q].x = l && c.iz < v.nz ? __ldg(s) : 0.0f;
-                f[q].y = l && c.iz + 1 < v.nz ? __ldg(s + 1) : 0.0f;
-                f[q].z = l && c.iz + 2 < v.nz ? __ldg(s + 2) : 0.0f;
-                f[q].w = l && c.iz + 3 < v.nz ? __ldg(s + 3) : 0.0f;
+                f[q].x = l && c.iz < v.nz ? *s : 0.0f;
+                f[q].y = l && c.iz + 1 < v.nz ? s[1] : 0.0f;
+                f[q].z = l && c.iz + 2 < v.nz ? s[2] : 0.0f;
+                f[q].w = l && c.iz + 3 < v.nz ? s[3] : 0.0f;
             }
         }
     };

@@ -763,9 +763,11 @@ __device__ __forceinline__ long interior_col(const Grid3D &g, int k) {
 // order).  A warp copies a column, V depths a lane (four where npd and nz are
 // multiples of four, so that every column starts on a vector); bound by
 // memory.  176x160x144: 19.4 -> 8.9 and 21.7 -> 14.9 us against an element per
-// thread and step of a grid-stride loop with three divisions each.
+// thread and step of a grid-stride loop with three divisions each.  Not
+// __restrict__: the kernel that wrote the fields may still run when these
+// start, so their loads must not become read-only ones.
 template <int V>
-__global__ void __launch_bounds__(256) k_snap_store(Grid3D g, const float *__restrict__ P, float *__restrict__ snap) {
+__global__ void __launch_bounds__(256) k_snap_store(Grid3D g, const float *P, float *snap) {
     tc::after_predecessor();
     const int k = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (k >= g.nx * g.ny) return;
@@ -778,8 +780,7 @@ __global__ void __launch_bounds__(256) k_snap_store(Grid3D g, const float *__res
 }
 
 template <int V>
-__global__ void __launch_bounds__(256) k_snap_image(Grid3D g, const float *__restrict__ snap, const float *__restrict__ gP,
-                                                    float *__restrict__ mig, float w) {
+__global__ void __launch_bounds__(256) k_snap_image(Grid3D g, const float *snap, const float *gP, float *mig, float w) {
     tc::after_predecessor();
     const int k = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (k >= g.nx * g.ny) return;

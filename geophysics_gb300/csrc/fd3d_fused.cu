@@ -97,13 +97,16 @@ __device__ __forceinline__ FV unpack(const T &t) {
     return r;
 }
 __device__ __forceinline__ FV ld_s(const float *p) { return unpack(*reinterpret_cast<const VecT *>(p)); }
+// Plain loads throughout, also of arrays that this launch only reads: its
+// blocks come up while the kernel before, which wrote them, still runs, and
+// ld.global.nc (__ldg) is defined only for what nobody writes while a kernel
+// lives and may be moved ahead of the wait for that kernel.
+__device__ __forceinline__ FV ld_g(const float *p) { return unpack(*reinterpret_cast<const VecT *>(p)); }
 __device__ __forceinline__ FV ld_g(const float *p, bool on) {
     VecT t{};
-    if (on) t = __ldg(reinterpret_cast<const VecT *>(p));
+    if (on) t = *reinterpret_cast<const VecT *>(p);
     return unpack(t);
 }
-// data this launch also writes (own points only): a plain load
-__device__ __forceinline__ FV ld_rw(const float *p) { return unpack(*reinterpret_cast<const VecT *>(p)); }
 template <class T = VecT>
 __device__ __forceinline__ void st_v(float *p, const FV &a) {
     T t;
@@ -378,8 +381,8 @@ __global__ void __launch_bounds__(kFusedThreads, kFusedBlocks)
         }
         FV S[6];
         if (split && own_split) {
-            S[0] = ld_rw(g.px + off); S[1] = ld_rw(g.py + off); S[2] = ld_rw(g.pz + off);
-            S[3] = ld_rw(g.qx + off); S[4] = ld_rw(g.qy + off); S[5] = ld_rw(g.qz + off);
+            S[0] = ld_g(g.px + off); S[1] = ld_g(g.py + off); S[2] = ld_g(g.pz + off);
+            S[3] = ld_g(g.qx + off); S[4] = ld_g(g.qy + off); S[5] = ld_g(g.qz + off);
         }
         // illumination / image inputs (RTM), loaded here so that their latency
         // hides behind the plane's arithmetic
@@ -390,8 +393,8 @@ __global__ void __launch_bounds__(kFusedThreads, kFusedBlocks)
         if (RTM && im) {
             io = (long)(zo - g.npd) + (long)g.nz * ((xa - g.npd) + (long)g.nx * (y - g.npd));
             if (imv) {
-                if (st.ill) ill = ld_rw(st.ill + io);
-                if (st.mig) mig = ld_rw(st.mig + io);
+                if (st.ill) ill = ld_g(st.ill + io);
+                if (st.mig) mig = ld_g(st.mig + io);
             } else {
 #pragma unroll
                 for (int j = 0; j < kW; j++)
@@ -400,7 +403,7 @@ __global__ void __launch_bounds__(kFusedThreads, kFusedBlocks)
                         if (st.mig) mig.v[j] = st.mig[io + j];
                     }
             }
-            if (st.mig) oth = ld_g(st.other_P + off, true);
+            if (st.mig) oth = ld_g(st.other_P + off);
         }
 
         add_source(pc, y + 7);

@@ -38,7 +38,11 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
 
 // First thing of a kernel that launch_early starts while its predecessor in the
 // stream still runs: wait for that one's results, then let the successor come.
-// (What kernels before the predecessor wrote is complete by then.)
+// (What kernels before the predecessor wrote is complete by then.)  A kernel
+// that calls it reads what other kernels write by plain loads or TMA, never by
+// read-only ones (__ldg, const __restrict__): those are defined only for
+// memory that nobody writes while the kernel lives, and its life begins before
+// the wait.
 __device__ __forceinline__ void after_predecessor() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

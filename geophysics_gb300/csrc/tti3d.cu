@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(TZ *NW, 2)
 
 __global__ void __launch_bounds__(TZ *NW, 2)
     k_tti3d_stress(const __grid_constant__ StrMaps M, const TtiGeom g, float *__restrict__ P1, float *__restrict__ Q1,
-                   const float *__restrict__ save, const StepArgs3D st) {
+                   const float *save, const StepArgs3D st) {
     extern __shared__ unsigned char smem_raw[];
     float *stages = align128(smem_raw);
     uint64_t *bar = reinterpret_cast<uint64_t *>(stages + NST * SSTAGE);
