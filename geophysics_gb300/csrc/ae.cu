@@ -379,19 +379,22 @@ __global__ void __launch_bounds__(256, 2) k_ae_e12(const __grid_constant__ CUten
         tc::mbar_init(&done[1], 1);
         s_abort[0] = s_abort[1] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        // E2's weights, two slices of 64 inputs
-        tc::mbar_expect_tx(&wbar, 16384);
-        tc::tma2(sm, &tw, 0, 0, &wbar);
-        tc::tma2(sm + 8192, &tw, 64, 0, &wbar);
     }
-    if (threadIdx.x < 64) sbias[threadIdx.x] = a.bias[threadIdx.x];
     __syncwarp();
     if (threadIdx.x < 32) tc::tmem_alloc(&tslot, 128);
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = tslot + grp * 64;
+    // the weights too: the kernel before may be the one that packs them
     tc::after_predecessor();
+    if (threadIdx.x == 0) {
+        // E2's weights, two slices of 64 inputs
+        tc::mbar_expect_tx(&wbar, 16384);
+        tc::tma2(sm, &tw, 0, 0, &wbar);
+        tc::tma2(sm + 8192, &tw, 64, 0, &wbar);
+    }
+    if (threadIdx.x < 64) sbias[threadIdx.x] = a.bias[threadIdx.x];
     if (!tc::mbar_wait(&wbar, 0)) s_abort[0] = s_abort[1] = 1;
     __syncthreads();
     const AeVolume &v = a.vol;
@@ -579,7 +582,6 @@ __global__ void __launch_bounds__(kD21Threads, 2)
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (threadIdx.x < 128) sbias[threadIdx.x] = a.bias[threadIdx.x];
     __syncwarp();
     if (warp == 9) tc::tmem_alloc(&tslot, 256);
     tc::tc_fence_before();
@@ -587,6 +589,8 @@ __global__ void __launch_bounds__(kD21Threads, 2)
     tc::tc_fence_after();
     const uint32_t tmem = tslot;
     tc::after_predecessor();
+    if (threadIdx.x < 128) sbias[threadIdx.x] = a.bias[threadIdx.x];
+    __syncthreads();
 
     if (warp == 8 && lane == 0) {
         unsigned it = 0;

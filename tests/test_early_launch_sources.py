@@ -1,5 +1,6 @@
 """Kernels that come up while their predecessor in the stream still runs
-(tc::after_predecessor) must not use read-only loads (__ldg, a const
+(tc::after_predecessor) read nothing but a run's fixed profiles before they
+have waited for it, and must not use read-only loads (__ldg, a const
 __restrict__ parameter) for what that predecessor writes: such loads are
 defined only for memory nobody writes while the kernel lives, and the
 compiler may move them ahead of the wait.  No device run can show that they
@@ -10,6 +11,8 @@ import re
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "geophysics_gb300", "csrc")
 # written once, by the host, before the first launch of a run
 PROFILES = re.compile(r"\s*g\.[ca][xyz][12]\b")
+# an array inside the kernel's parameters
+PARAMS = ("g.it[",)
 
 
 def functions():
@@ -76,4 +79,13 @@ def test_no_read_only_loads_in_early_kernels():
             bad += [(key, k[1], "ld.global.nc")] if "ld.global.nc" in body else []
             bad += [(key, k[1], body[m.start():m.end() + 40]) for m in re.finditer(r"__ldg\(", body)
                     if not PROFILES.match(body[m.end():])]
+    assert not bad, bad
+
+
+def test_nothing_is_read_before_the_wait():
+    bad = []
+    for key in EARLY:
+        head = FUNCS[key][1].split("after_predecessor()")[0]
+        bad += [(key, m.group(0)) for m in re.finditer(r"\b(?:tma[23]\s*\(|row_copy\s*\(|[a-z]\.\w+\[)", head)
+                if not PROFILES.match(m.group(0)) and m.group(0) not in PARAMS]
     assert not bad, bad
