@@ -1412,22 +1412,10 @@ int ae_escape_cap(geo_ae *ae, const AeVolume &v) {
     return std::min(nb, (int)std::ceil(ae->frac * nb));
 }
 
-static int ae_sms() {
-    static int n = 0;
-    if (!n) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 152;
-    }
-    return n;
-}
 static int ae_smem() {
-    static bool set = false;
-    if (set) return GEO_OK;
-    GEO_CUDA(cudaFuncSetAttribute(k_ae_e12, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kE12Smem));
-    GEO_CUDA(cudaFuncSetAttribute(k_ae_d21, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kD21Smem));
-    set = true;
-    return GEO_OK;
+    static OncePerDevice e12, d21;
+    GEO_TRY(allow_smem(e12, (const void *)k_ae_e12, kE12Smem));
+    return allow_smem(d21, (const void *)k_ae_d21, kD21Smem);
 }
 
 // Encode the interior box v into code[rows x 512] (bf16) and scale[rows];
@@ -1450,7 +1438,7 @@ int ae_encode_volume(geo_ae *ae, const AeVolume &v, void *code, float *scale, in
     GEO_TRY(tc_map_bf16(&tw, bf(ae->wb) + ae->off.wb[1], 64, 128, 64));
     GEO_TRY(tc_map_bf16(&to, ae->h2.p, rows * 64, 64, 32));
     GEO_TRY(ae_smem());
-    GEO_CUDA(launch_early(k_ae_e12, std::min((a.tiles + 1) / 2, 2 * ae_sms()), 256, kE12Smem, s, tw, to, a));
+    GEO_CUDA(launch_early(k_ae_e12, std::min((a.tiles + 1) / 2, 2 * sm_count()), 256, kE12Smem, s, tw, to, a));
     GEO_TRY(check_launch("ae_e12"));
     GEO_TRY(level(ae, 2, rows, bf(ae->h2), bf(ae->h3), s));
     GEO_TRY(level(ae, 3, rows, bf(ae->h3), static_cast<__nv_bfloat16 *>(code), s));
@@ -1511,7 +1499,7 @@ int ae_decode_volume(geo_ae *ae, const AeVolume &v, const void *code, const floa
         GEO_TRY(tc_map_bf16(&ta, ae->g2.p, rows * 64, 64, 128));
         GEO_TRY(tc_map_bf16(&tw, bf(ae->wb) + ae->off.wb[6], 128, 64, 128));
         GEO_TRY(ae_smem());
-        GEO_CUDA(launch_early(k_ae_d21, std::min(a.tiles, 2 * ae_sms()), kD21Threads, kD21Smem, s, ta, tw, a));
+        GEO_CUDA(launch_early(k_ae_d21, std::min(a.tiles, 2 * sm_count()), kD21Threads, kD21Smem, s, ta, tw, a));
         return check_launch("ae_d21");
     }
     GEO_TRY(decode_rows(ae, rows, static_cast<const __nv_bfloat16 *>(code), s));
@@ -1532,12 +1520,9 @@ int ae_decode_volume(geo_ae *ae, const AeVolume &v, const void *code, const floa
 
 // Dynamic shared memory of the kernels that end in block_outer (64 KB).
 static int outer_smem() {
-    static bool set = false;
-    if (set) return GEO_OK;
-    GEO_CUDA(cudaFuncSetAttribute(k_ae_d1, cudaFuncAttributeMaxDynamicSharedMemorySize, kOutFloats * 4));
-    GEO_CUDA(cudaFuncSetAttribute(k_ae_e1_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, kOutFloats * 4));
-    set = true;
-    return GEO_OK;
+    static OncePerDevice d1, e1;
+    GEO_TRY(allow_smem(d1, (const void *)k_ae_d1, kOutFloats * 4));
+    return allow_smem(e1, (const void *)k_ae_e1_bwd, kOutFloats * 4);
 }
 
 // Forward (+ backward when grads are wanted) over `rows` blocks already

@@ -14,17 +14,6 @@
 
 namespace geo {
 
-static int sm_count() {
-    static int n = 0;
-    if (!n) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 1;
-    }
-    return n;
-}
-
 // One shot's window of the model and its source.
 struct ShotGeom {
     int nx, col0;        // window width, model column of window column 0

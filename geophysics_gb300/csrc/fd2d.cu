@@ -27,15 +27,15 @@ __constant__ float c_fd[4] = {1.196289f, -0.0797526f, 0.009570313f, -0.000697544
 // CPU_vti2dfd_kernels.c:72); filled from the host's exp() at load.
 __constant__ double c_gauss[49];
 
-static bool g_gauss_ready = false;
 static int ensure_gauss() {
-    if (g_gauss_ready) return GEO_OK;
-    double g[49];
-    for (int x = -3; x <= 3; x++)
-        for (int z = -3; z <= 3; z++) g[(x + 3) * 7 + (z + 3)] = std::exp((double)(-z * z - x * x));
-    GEO_CUDA(cudaMemcpyToSymbol(c_gauss, g, sizeof g));
-    g_gauss_ready = true;
-    return GEO_OK;
+    static OncePerDevice once;
+    return once.run([]() -> int {
+        double g[49];
+        for (int x = -3; x <= 3; x++)
+            for (int z = -3; z <= 3; z++) g[(x + 3) * 7 + (z + 3)] = std::exp((double)(-z * z - x * x));
+        GEO_CUDA(cudaMemcpyToSymbol(c_gauss, g, sizeof g));
+        return GEO_OK;
+    });
 }
 
 struct Tile2D {

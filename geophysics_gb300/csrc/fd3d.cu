@@ -282,14 +282,7 @@ static int alloc_fields(geo_fd3d_plan *p, int f) {
 // at the first set_model, which this replaces, took 24 to 28 steps and did not
 // try 7.)
 int march_chunks(int tiles, int planes) {
-    static int slots = 0;
-    if (!slots) {
-        int dev = 0, sms = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
-            sms = 152;
-        slots = 2 * sms;
-    }
+    const int slots = 2 * sm_count();
     long best = 0;
     int n = 1;
     for (int pass = 0; pass < 2; pass++)   // the least cost, then the largest count near it

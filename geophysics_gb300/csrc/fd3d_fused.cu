@@ -631,7 +631,7 @@ int encode_map(CUtensorMap *map, const float *base, int nnz, int ldz, int nnx, i
 }
 
 int launch_fused3d(const StepMaps &maps, const Fused3D &g, int mode, const StepArgs3D &args, cudaStream_t s) {
-    static bool attr_set[2][2];
+    static OncePerDevice once[2][2];
     StepArgs3D st = args;
     const bool rtm = st.ill || st.mig, fast = mode == GEO_MODE_FAST;
     // 16-byte image accesses need aligned rows whose first depth sits on a vector
@@ -639,10 +639,7 @@ int launch_fused3d(const StepMaps &maps, const Fused3D &g, int mode, const StepA
                  ((reinterpret_cast<uintptr_t>(st.ill) | reinterpret_cast<uintptr_t>(st.mig)) & (4 * kW - 1)) == 0;
     const void *fn = fast ? (rtm ? (const void *)k_fused3d<GEO_MODE_FAST, true> : (const void *)k_fused3d<GEO_MODE_FAST, false>)
                           : (rtm ? (const void *)k_fused3d<GEO_MODE_EXACT, true> : (const void *)k_fused3d<GEO_MODE_EXACT, false>);
-    if (!attr_set[fast][rtm]) {
-        GEO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFusedSmem));
-        attr_set[fast][rtm] = true;
-    }
+    GEO_TRY(allow_smem(once[fast][rtm], fn, kFusedSmem));
     using Fn = void (*)(const StepMaps, const Fused3D, const StepArgs3D);
     GEO_CUDA(launch_early(reinterpret_cast<Fn>(const_cast<void *>(fn)), (unsigned)g.nitems, dim3(kFusedThreads), kFusedSmem, s, maps, g, st));
     return check_launch("fused3d");

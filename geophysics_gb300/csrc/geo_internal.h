@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <cstdio>
 #include <cstdint>
+#include <mutex>
 #include <vector>
 #include <string>
 #include "../../include/geofd.h"
@@ -44,6 +45,36 @@ struct DevBuf {
     void release();
     template <class T> T *as() const { return static_cast<T *>(p); }
 };
+
+// Set-up of what belongs to a device and not to the process (constant memory,
+// kernel attributes): f once per device, under a lock so that host threads
+// find it done, and again after a failure.  No heap use.
+class OncePerDevice {
+    static constexpr int kDevices = 64;   // set up on every call beyond
+    std::mutex mu;
+    bool done[kDevices] = {};
+
+public:
+    template <class F>
+    int run(F &&f) {
+        int dev = 0;
+        GEO_CUDA(cudaGetDevice(&dev));
+        std::lock_guard<std::mutex> lock(mu);
+        if (dev < kDevices && done[dev]) return GEO_OK;
+        GEO_TRY(f());
+        if (dev < kDevices) done[dev] = true;
+        return GEO_OK;
+    }
+};
+// Allow a kernel `bytes` of dynamic shared memory on the current device.
+inline int allow_smem(OncePerDevice &once, const void *fn, size_t bytes) {
+    return once.run([&]() -> int {
+        GEO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        return GEO_OK;
+    });
+}
+// SMs of the current device.
+int sm_count();
 
 // ------------------------------------------------------------ host setup
 // Reference program whose arithmetic a run follows.

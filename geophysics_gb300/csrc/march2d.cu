@@ -590,12 +590,8 @@ const void *march_fn(int mode, bool fast, bool wide) {
 }
 
 int march_attr(int mode, bool fast, bool wide) {
-    static bool set[3][2][2];
-    if (set[mode][fast][wide]) return GEO_OK;
-    GEO_CUDA(cudaFuncSetAttribute(march_fn(mode, fast, wide), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)march_smem(mode)));
-    set[mode][fast][wide] = true;
-    return GEO_OK;
+    static OncePerDevice once[3][2][2];
+    return allow_smem(once[mode][fast][wide], march_fn(mode, fast, wide), march_smem(mode));
 }
 
 int march_mode(bool backward, bool adcig) { return !backward ? MM_FWD : adcig ? MM_ADCIG : MM_BWD; }
@@ -668,8 +664,8 @@ int load_march_tables(bool adcig, cudaStream_t s) {
     if (!adcig) return GEO_OK;
     static float thr[kAdcigAngles];
     static double w[kAdcigAngles];
-    static bool built = false;
-    if (!built) {
+    static std::once_flag built;
+    std::call_once(built, [] {
         const uint32_t lo = order_key(-1.0f), hi = order_key(1.0f);
         for (int k = 1; k <= kAdcigAngles; k++) {
             if (ref_adcig_bin(-1.0f) < k) {
@@ -685,8 +681,7 @@ int load_march_tables(bool adcig, cudaStream_t s) {
             thr[k - 1] = key_float(a);
         }
         for (int ia = 0; ia < kAdcigAngles; ia++) w[ia] = std::pow(std::cos(ia * kPiMpi / 180.0), 3);
-        built = true;
-    }
+    });
     GEO_CUDA(cudaMemcpyToSymbolAsync(cm_adthr, thr, sizeof thr, 0, cudaMemcpyHostToDevice, s));
     GEO_CUDA(cudaMemcpyToSymbolAsync(cm_adw, w, sizeof w, 0, cudaMemcpyHostToDevice, s));
     return GEO_OK;

@@ -51,6 +51,14 @@ int DevBuf::zero(cudaStream_t s) {
     return GEO_OK;
 }
 
+int sm_count() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1)
+        n = 152;
+    return n;
+}
+
 void DevBuf::release() {
     if (p) cudaFree(p);
     p = nullptr;

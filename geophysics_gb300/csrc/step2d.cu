@@ -735,14 +735,14 @@ int load_step2d_angles(const float *thr, const float *cs, cudaStream_t s) {
 }
 
 int load_step2d_gauss() {
-    static bool ready = false;
-    if (ready) return GEO_OK;
-    double g[49];
-    for (int x = -3; x <= 3; x++)
-        for (int z = -3; z <= 3; z++) g[(x + 3) * 7 + (z + 3)] = std::exp((double)(-z * z - x * x));
-    GEO_CUDA(cudaMemcpyToSymbol(cs_gauss, g, sizeof g));
-    ready = true;
-    return GEO_OK;
+    static OncePerDevice once;
+    return once.run([]() -> int {
+        double g[49];
+        for (int x = -3; x <= 3; x++)
+            for (int z = -3; z <= 3; z++) g[(x + 3) * 7 + (z + 3)] = std::exp((double)(-z * z - x * x));
+        GEO_CUDA(cudaMemcpyToSymbol(cs_gauss, g, sizeof g));
+        return GEO_OK;
+    });
 }
 
 int Fused2D::run(const SStep &a, cudaStream_t s) const {

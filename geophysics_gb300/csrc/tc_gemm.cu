@@ -423,11 +423,8 @@ int tc_map_bf16(CUtensorMap *map, const void *base, int rows, int cols, int box_
 template <int BN, int ST>
 static int launch_bn(const TcGemm &g, cudaStream_t s) {
     using S = GemmShape<BN, ST>;
-    static bool attr = false;
-    if (!attr) {
-        GEO_CUDA(cudaFuncSetAttribute(k_tc_gemm<BN, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem));
-        attr = true;
-    }
+    static OncePerDevice once;
+    GEO_TRY(allow_smem(once, (const void *)k_tc_gemm<BN, ST>, S::kSmem));
     CUtensorMap ta, tb;
     GEO_TRY(tc_map_bf16(&ta, g.A, g.M, g.K, kGM));
     GEO_TRY(tc_map_bf16(&tb, g.B, g.N, g.K, BN));
@@ -439,19 +436,14 @@ static int launch_bn(const TcGemm &g, cudaStream_t s) {
 template <int BN, bool RB>
 static int launch_walk(const TcGemm &g, cudaStream_t s) {
     using S = WalkShape<BN, RB>;
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        GEO_CUDA(cudaGetDevice(&dev));
-        GEO_CUDA(cudaFuncSetAttribute(k_tc_walk<BN, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem));
-        GEO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    }
+    static OncePerDevice once;
+    GEO_TRY(allow_smem(once, (const void *)k_tc_walk<BN, RB>, S::kSmem));
     CUtensorMap ta, tb, to;
     GEO_TRY(tc_map_bf16(&ta, g.A, g.M, g.K, kGM));
     GEO_TRY(tc_map_bf16(&tb, g.B, g.N, g.K, BN));
     GEO_TRY(tc_map_bf16(&to, g.out, g.M, g.N, 32));
     const int tiles = (g.M / kGM) * (g.N / BN);
-    GEO_CUDA(launch_early(k_tc_walk<BN, RB>, std::min(tiles, sms), kWalkThreads, S::kSmem, s, ta, tb, to, g, tiles));
+    GEO_CUDA(launch_early(k_tc_walk<BN, RB>, std::min(tiles, sm_count()), kWalkThreads, S::kSmem, s, ta, tb, to, g, tiles));
     return check_launch("tc_walk");
 }
 
@@ -659,11 +651,8 @@ int tc_wgrad(const TcWgradLevel *lv, int n, int *err, cudaStream_t s) {
     }
     g.n = n;
     g.err = err;
-    static bool attr = false;
-    if (!attr) {
-        GEO_CUDA(cudaFuncSetAttribute(k_tc_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgSmem));
-        attr = true;
-    }
+    static OncePerDevice once;
+    GEO_TRY(allow_smem(once, (const void *)k_tc_wgrad, kWgSmem));
     GEO_CUDA(launch_early(k_tc_wgrad, base, 128, kWgSmem, s, g));
     return check_launch("tc_wgrad");
 }

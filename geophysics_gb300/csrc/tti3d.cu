@@ -489,7 +489,7 @@ int tti_maps(const Tti3DStep &t, const MapPair **out) {
 }  // namespace
 
 int launch_tti3d(const Tti3DStep &t, const StepArgs3D &args, cudaStream_t s) {
-    static bool attr = false;
+    static OncePerDevice vel, stress;
     StepArgs3D st = args;
     const Grid3D &g = t.g;
     st.src = st.izs + (long)g.ldz * (st.ixs + (long)g.nnx * st.iys);
@@ -499,11 +499,8 @@ int launch_tti3d(const Tti3DStep &t, const StepArgs3D &args, cudaStream_t s) {
     }
     const MapPair *m = nullptr;
     GEO_TRY(tti_maps(t, &m));
-    if (!attr) {
-        GEO_CUDA(cudaFuncSetAttribute(k_tti3d_vel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VEL_SMEM));
-        GEO_CUDA(cudaFuncSetAttribute(k_tti3d_stress, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STR_SMEM));
-        attr = true;
-    }
+    GEO_TRY(allow_smem(vel, (const void *)k_tti3d_vel, VEL_SMEM));
+    GEO_TRY(allow_smem(stress, (const void *)k_tti3d_stress, STR_SMEM));
     if ((long)g.sxy * g.nny >= (1L << 31)) return fail(GEO_ERR_ARG, "grid too large for 32-bit plane offsets");
     TtiGeom G;
     G.nnx = g.nnx; G.nny = g.nny; G.nnz = g.nnz; G.ldz = g.ldz; G.npd = g.npd;

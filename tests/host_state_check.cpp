@@ -1,0 +1,113 @@
+// Host-side state of libgeofd against a CUDA runtime without a device
+// (fake_cuda.h).  Usage: host_state_check <check>; prints what fails.
+#include "fake_cuda.h"
+#include "geofd.h"
+#include <cmath>
+#include <vector>
+
+extern "C" const char *geo_strerror(int);
+static int failures = 0;
+#define OK(call)                                                                              \
+    do {                                                                                      \
+        const int s_ = (call);                                                                \
+        if (s_ != GEO_OK) {                                                                   \
+            printf("device %d: %s: %s\n", fake::device, #call, geo_strerror(s_));             \
+            failures++;                                                                       \
+        }                                                                                     \
+    } while (0)
+
+static std::vector<float> filled(size_t n, float v) { return std::vector<float>(n, v); }
+
+static geo_fd2d_desc fd2d_desc(int variant) {
+    geo_fd2d_desc d{};
+    d.nx = 40; d.nz = 30; d.npd = 8; d.nt = 3;
+    d.dx = d.dz = 10; d.dt = 1e-3f; d.favg = 20; d.pfac = 10; d.wtype = 1;
+    d.fs = 20; d.zs = 5; d.is = 1; d.variant = variant; d.rec_iz = 12; d.rec_scale = 1;
+    return d;
+}
+
+// One call of every entry point that owns kernels or tables.
+static void every_entry_point() {
+    const int nx = 40, nz = 30, n2 = nx * nz;
+    auto v = filled(n2, 2000), e = filled(n2, 0.1f), d = filled(n2, 0.05f), th = filled(n2, 10);
+    std::vector<float> out(200 * n2);
+    for (int var : {GEO_VARIANT_CPU, GEO_VARIANT_GPU, GEO_VARIANT_MPI}) {
+        geo_fd2d_desc D = fd2d_desc(var);
+        OK(geo_fd2d_shot(&D, v.data(), e.data(), d.data(), out.data(), nullptr, 0, GEO_MEM_HOST, nullptr));
+    }
+    geo_fd2d_desc D = fd2d_desc(GEO_VARIANT_GPU);
+    OK(geo_tti2d_shot(&D, v.data(), e.data(), d.data(), th.data(), out.data(), nullptr, 0, GEO_MEM_HOST, nullptr));
+    geo_rtm2d_gpu_desc G{};
+    G.nx = nx; G.nz = nz; G.npml = 8; G.nt = 3; G.dx = G.dz = 10; G.dt = 1e-3f; G.favg = 20; G.pfac = 10; G.wtype = 1;
+    G.ns = 1; G.fs = 20; G.zs = 1; G.mute_tt = 20; G.nangle = 60; G.dangle = 1;
+    std::vector<float> ill(n2), ag((size_t)60 * n2);
+    OK(geo_rtm2d_gpu(&G, v.data(), e.data(), d.data(), nullptr, out.data(), ill.data(), ag.data(), nullptr, nullptr, GEO_MEM_HOST, nullptr));
+    OK(geo_rtm2d_tti(&G, v.data(), e.data(), d.data(), th.data(), nullptr, out.data(), ill.data(), ag.data(), nullptr, GEO_MEM_HOST, nullptr));
+    const int xs[2] = {18, 20}, ws[2] = {9, 11};
+    for (int mode : {GEO_MODE_EXACT, GEO_MODE_FAST})
+        for (int gathers = 0; gathers < 2; gathers++) {
+            geo_rtm2d_desc B{};
+            B.nx = nx; B.nz = nz; B.npd = 8; B.nt = 3; B.dx = B.dz = 10; B.dt_ms = 1; B.favg = 20; B.pfac = 10; B.zs = 2;
+            B.ns = 2; B.shot_x = xs; B.shot_nxs = ws; B.mode = mode;
+            OK(geo_rtm2d_batch_adcig(&B, v.data(), e.data(), d.data(), ill.data(), nullptr, gathers ? out.data() : nullptr, GEO_MEM_HOST, nullptr));
+        }
+    const int m = 20, n3 = m * m * m;
+    auto v3 = filled(n3, 2000), e3 = filled(n3, 0.1f), d3 = filled(n3, 0.05f), t3 = filled(n3, 10);
+    std::vector<float> o3(4 * n3);
+    geo_ae *ae = nullptr;
+    OK(geo_ae_create(&ae, 1));
+    for (int mode : {GEO_MODE_EXACT, GEO_MODE_FAST}) {
+        geo_fd3d_desc F{};
+        F.nx = F.ny = F.nz = m; F.npd = 8; F.nt = 8; F.dx = F.dy = F.dz = 10; F.dt = 1e-3f; F.favg = 20; F.pfac = 10; F.wtype = 1;
+        F.mode = mode; F.fsx = F.fsy = 10; F.fsz = 2; F.rec_iz = 8; F.drx = F.dry = 1; F.nrx = F.nry = m;
+        OK(geo_fd3d_shot(&F, 0, v3.data(), e3.data(), d3.data(), std::vector<float>(8 * m * m).data(), GEO_MEM_HOST, nullptr));
+        for (int method = 0; method < 4; method++) {
+            geo_rtm3d_desc R{};
+            R.fd = F; R.ns = 1; R.mute_tt = 5; R.method = method; R.snap_every = 2; R.ae = ae;
+            OK(geo_rtm3d(&R, v3.data(), e3.data(), d3.data(), o3.data(), nullptr, nullptr, GEO_MEM_HOST, nullptr));
+            if (mode == GEO_MODE_EXACT || method != GEO_RTM_SNAPSHOT) continue;
+            R.theta = R.phi = t3.data();
+            OK(geo_rtm3d(&R, v3.data(), e3.data(), d3.data(), o3.data(), nullptr, nullptr, GEO_MEM_HOST, nullptr));
+        }
+    }
+    std::vector<float> blk((size_t)128 * 4096, 1.0f), rec(blk), grad(geo_ae_num_params());
+    double loss;
+    OK(geo_ae_eval(ae, blk.data(), 128, rec.data(), &loss, grad.data(), GEO_MEM_HOST, nullptr));
+    for (int side : {32, 512}) {   // few and many tiles
+        std::vector<float> a((size_t)side * side * 128), b(a.size());
+        OK(geo_ae_roundtrip(ae, side, side, 128, a.data(), b.data(), 1, nullptr, nullptr));
+    }
+    for (int w : {64, 128, 256})   // every kernel of the GEMM rule
+        for (int rows : {128, 512, 152 * 128})
+            for (int K : {64, 128, 192, 256, 320}) {
+                std::vector<unsigned short> A((size_t)rows * K), B((size_t)w * K);
+                std::vector<float> o((size_t)rows * w);
+                for (int f32 = 0; f32 < 2; f32++)
+                    OK(geo_tc_gemm_bf16(rows, w, K, A.data(), B.data(), nullptr, 0, o.data(), f32, nullptr));
+            }
+    OK(geo_ae_destroy(ae));
+}
+
+// Constant tables and kernel attributes belong to a device: a second device
+// gets what the first did, and none of its launches is refused.
+static void check_devices() {
+    for (int dev : {0, 1}) {
+        fake::device = dev;
+        every_entry_point();
+    }
+    for (const auto &s : fake::st().symbols[0])
+        if (!fake::st().symbols[1].count(s)) { printf("constant %s not set on device 1\n", s.c_str()); failures++; }
+    for (const auto &s : fake::st().attributes[0])
+        if (!fake::st().attributes[1].count(s)) { printf("attribute of %s not set on device 1\n", s.c_str()); failures++; }
+    printf("%s", fake::st().refused.c_str());
+    if (!fake::st().refused.empty()) failures++;
+    if (fake::st().symbols[0].size() < 5 || fake::st().attributes[0].size() < 20) { printf("too few calls seen\n"); failures++; }
+    printf("%zu constants, %zu kernels with attributes\n", fake::st().symbols[0].size(), fake::st().attributes[0].size());
+}
+
+int main(int argc, char **argv) {
+    const std::string check = argc > 1 ? argv[1] : "";
+    if (check == "devices") check_devices();
+    else return 2;
+    return failures ? 1 : 0;
+}

@@ -1,0 +1,37 @@
+"""Host-side state of libgeofd, run against a CUDA runtime without a device
+(fake_cuda.h): what belongs to a device is set up on every device."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+PKG = os.path.join(ROOT, "geophysics_gb300")
+
+
+@pytest.fixture(scope="module")
+def check(tmp_path_factory):
+    cxx = shutil.which("g++") or shutil.which("c++")
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    inc = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
+    lib = os.path.join(PKG, "libgeofd.so")
+    if not cxx or not os.path.exists(os.path.join(inc, "cuda_runtime.h")) or not os.path.exists(lib):
+        pytest.skip("needs a C++ compiler, the CUDA headers and the built library")
+    exe = str(tmp_path_factory.mktemp("host_state") / "host_state_check")
+    subprocess.run([cxx, "-O1", "-std=c++17", "-I" + os.path.join(ROOT, "include"), "-I" + inc,
+                    os.path.join(ROOT, "tests", "host_state_check.cpp"), "-o", exe, lib, "-rdynamic",
+                    "-Wl,-rpath," + PKG, "-Wl,--allow-shlib-undefined", "-lpthread"], check=True)
+
+    def run(name):
+        r = subprocess.run([exe, name], capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-1000:]
+        return r.stdout
+
+    return run
+
+
+def test_second_device_gets_tables_and_kernel_attributes(check):
+    """Every entry point on one device, then on another: the same constant
+    tables are copied to both, the same kernels' shared-memory limits set."""
+    check("devices")
