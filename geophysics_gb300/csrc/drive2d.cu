@@ -259,13 +259,18 @@ int FusedShot::build(const Raw2D &raw, float dx, float dz, float dt, const std::
     return plan.model(g, model);
 }
 
-// The shots of a batched RTM on the device for the fused steps.
+// A group of consecutive shots of a batched RTM on the device for the fused
+// steps: M[k] is shot first + k of the set.
 struct MarchBatch {
-    ShotSet X;
+    ShotSet &X;
+    const int first, ns;
     std::vector<March2D> M;
     DevBuf d_M, d_items[2];
     std::vector<int4> items[2];   // forward, backward
-    bool fast = false, wide = false, adcig = false;
+    const bool fast, adcig;
+    bool wide = false;
+    MarchBatch(ShotSet &set, int first_, int ns_, bool fast_, bool adcig_)
+        : X(set), first(first_), ns(ns_), fast(fast_), adcig(adcig_) {}
     int build(const Raw2D &raw, float dx, float dz, float dt, int nt, cudaStream_t s);
     int clear_side(int k, int slots, cudaStream_t s) {
         GEO_CUDA(cudaMemsetAsync(M[k].f, 0, (size_t)slots * M[k].n * 4, s));
@@ -285,7 +290,7 @@ struct MarchBatch {
 // take 182 us a forward and 328 us a backward step with chunks of about 12,
 // 200 and 376 us with one wave (35 and 70 columns).
 int MarchBatch::work(bool backward) {
-    const int nnz = X.nnz, depths = nnz - 8, ns = (int)M.size();
+    const int nnz = X.nnz, depths = nnz - 8;
     const int strips = (depths + 119) / 120, len = ((depths + strips - 1) / strips + 3) / 4 * 4;
     long cols = 0;
     for (int k = 0; k < ns; k++) cols += (long)strips * (M[k].nnx - 8);
@@ -304,13 +309,17 @@ int MarchBatch::work(bool backward) {
 }
 
 int MarchBatch::build(const Raw2D &raw, float dx, float dz, float dt, int nt, cudaStream_t s) {
-    const int ns = (int)X.G.size(), npd = X.npd, nz = X.nz, nnz = X.nnz, ldz = (nnz + 3) / 4 * 4;
+    const int npd = X.npd, nz = X.nz, nnz = X.nnz, ldz = (nnz + 3) / 4 * 4;
+    const ShotGeom *const G = X.G.data() + first;
+    X.small.h.clear();
+    X.mem.buf.release();   // the last group's
+    X.mem.off = 0;
     DevBuf d_pw;
     if (!fast) GEO_TRY(upload_pow_half(raw, d_pw, s));
     std::vector<ShotSet::Off> off(ns);
     std::vector<size_t> o_tpw2(ns), o_tpw(ns);
     for (int k = 0; k < ns; k++) {
-        X.tables(k, dx, dz, dt, ldz, off[k]);
+        X.tables(first + k, dx, dz, dt, ldz, off[k]);
         if (fast) continue;
         std::vector<double> pw(kTB * kTB);
         std::vector<float> p2(2 * kTB * kTB);
@@ -327,7 +336,7 @@ int MarchBatch::build(const Raw2D &raw, float dx, float dz, float dt, int nt, cu
     std::vector<ModelJob> jobs(ns, ModelJob{});
     for (int pass = 0; pass < 2; pass++) {   // sizes, then addresses
         for (int k = 0; k < ns; k++) {
-            const int nx = X.G[k].nx, nnx = nx + 2 * npd;
+            const int nx = G[k].nx, nnx = nx + 2 * npd;
             const size_t n = (size_t)nnx * ldz, L = 2 * (size_t)nx + 2 * (size_t)nz;
             March2D &m = M[k];
             m.n = (unsigned)n;
@@ -345,7 +354,7 @@ int MarchBatch::build(const Raw2D &raw, float dx, float dz, float dt, int nt, cu
     }
     for (int k = 0; k < ns; k++) {
         March2D &m = M[k];
-        const int nx = X.G[k].nx;
+        const int nx = G[k].nx;
         m.nnx = nx + 2 * npd; m.nnz = nnz; m.ldz = ldz; m.npd = npd; m.nx = nx; m.nz = nz;
         m.dtx = dt / dx; m.dtz = dt / dz;
         const float *xp = X.small.at<float>(off[k].xprof);
@@ -359,10 +368,10 @@ int MarchBatch::build(const Raw2D &raw, float dx, float dz, float dt, int nt, cu
             m.tpw = X.small.at<double>(o_tpw[k]);
             m.tpw2 = X.small.at<float2>(o_tpw2[k]);
         }
-        X.source(k, m.ixs, m.izs);
+        X.source(first + k, m.ixs, m.izs);
         ModelJob &j = jobs[k];
         const size_t n = m.n;
-        j.nx = nx; j.nz = nz; j.npd = npd; j.ldz = ldz; j.col0 = X.G[k].col0;
+        j.nx = nx; j.nz = nz; j.npd = npd; j.ldz = ldz; j.col0 = G[k].col0;
         j.vp2 = 1;   // vp <- rho*vp^2 with rho == 1 (Toa_rtm_vti_adcig_cdp.c:641)
         j.vp = m.f + MS_VP * n;
         j.e2 = m.f + MS_E2 * n;
@@ -426,13 +435,20 @@ struct Batch2D {
     }
 };
 
+// GEO_ERR_NOMEM where the device has no room for a graph.
+static int no_memory(cudaError_t e, const char *what) {
+    if (e == cudaSuccess) return GEO_OK;
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+    return fail(e == cudaErrorMemoryAllocation ? GEO_ERR_NOMEM : GEO_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+}
+
 // Graph of a range of steps; capture on a private stream.
 struct Graph {
     cudaGraph_t g = nullptr;
     cudaGraphExec_t x = nullptr;
     long long kernels = 0;     // kernel nodes, counted once per replay
     int launch(cudaStream_t s) {
-        GEO_CUDA(cudaGraphLaunch(x, s));
+        GEO_TRY(no_memory(cudaGraphLaunch(x, s), "graph launch"));
         count_launch(kernels);
         return GEO_OK;
     }
@@ -457,8 +473,7 @@ static int capture(Graph &G, cudaStream_t cs, F &&body) {
     }
     if (e != cudaSuccess) return fail(GEO_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
     G.g = g;
-    GEO_CUDA(cudaGraphInstantiate(&G.x, g, 0));
-    return GEO_OK;
+    return no_memory(cudaGraphInstantiate(&G.x, g, 0), "graph instantiation");
 }
 
 // Event-ordered hand-off between the caller's stream and a private one.
@@ -654,37 +669,36 @@ extern "C" int geo_rtm2d_batch_adcig(const geo_rtm2d_desc *desc, const float *v,
     GEO_TRY(raw.open(D.nx, D.nz, v, e, d, nullptr, mem, ss.cs));
     const float dt = D.dt_ms / 1000;
     const int nt = D.nt, nz = D.nz, npd = D.npd;
-    MarchBatch B;
-    B.fast = fast != 0;
-    B.adcig = adcig != nullptr;
-    ShotSet &X = B.X;
+    ShotSet X;
     X.var = V_MPI;
     X.nz = nz; X.npd = npd; X.nnz = nz + 2 * npd;
     X.taper = true;
-    int maxline = 0;
     for (int k = 0; k < D.ns; k++) {
         const int nxs = D.shot_nxs[k], kk = D.shot_x[k];
         // window column c <- model column c + k - nxs/2, clamped into the pad;
         // shot position inside its window: fs = nxs/2+1, ds = 0
         X.G.push_back(ShotGeom{nxs, kk - nxs / 2, (float)(nxs / 2 + 1), (float)D.zs});
-        maxline = std::max(maxline, 2 * nxs + 2 * nz);
     }
     GEO_TRY(X.read(raw, ss.cs));
     GEO_TRY(check_stability(V_MPI, 2, X.st.vmin, X.st.vmax, dt, D.dx, D.dx, D.dz, D.favg));
     std::vector<float> amp;
     std::vector<uint8_t> on;
     source_amplitudes(V_MPI, nt, dt, D.favg, D.pfac, 1, amp, on);
-    GEO_TRY(B.build(raw, D.dx, D.dz, dt, nt, ss.cs));
     GEO_TRY(load_march_tables(adcig != nullptr, ss.cs));
-    const March2D *d_M = B.d_M.as<March2D>();
-    // non-finite detector: every wd.every steps (and the last) the graphs
-    // scan every shot's P; the verdict follows each pass
     Watchdog wd;
     GEO_TRY(wd.open());
-    auto watch = [&](int k, bool last, int nf, int lev) -> int {
-        if (wd.every <= 0 || ((k + 1) % wd.every && !last)) return GEO_OK;
-        return launch_march_watch(d_M, D.ns, nf, lev, wd.d, k + 1, ss.cs);
-    };
+    const size_t nimg = (size_t)D.nx * nz;
+    const cudaMemcpyKind kout = mem == GEO_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
+    DevBuf stack, lap, gathers;
+    GEO_TRY(stack.alloc(nimg * 4));
+    GEO_TRY(stack.zero(ss.cs));
+    if (D.laplace) GEO_TRY(lap.alloc(nimg * 4));
+    if (adcig) {
+        GEO_TRY(gathers.alloc((size_t)kAdcigAngles * nimg * 4));
+        GEO_TRY(gathers.zero(ss.cs));
+    }
+    std::vector<size_t> shot_off(D.ns + 1, 0);   // of the per-shot images
+    for (int k = 0; k < D.ns; k++) shot_off[k + 1] = shot_off[k] + (size_t)D.shot_nxs[k] * nz;
     DevBuf d_err;
     GEO_TRY(d_err.alloc(4));
     GEO_TRY(d_err.zero(ss.cs));
@@ -700,124 +714,139 @@ extern "C" int geo_rtm2d_batch_adcig(const geo_rtm2d_desc *desc, const float *v,
         st.dhz = (float)st.ddtz; st.dlz = (float)(st.ddtz - (double)st.dhz);
         return st;
     };
-    // forward: source side only, with records and edge lines
-    {
-        Graph G;
-        GEO_TRY(capture(G, ss.cs, [&]() -> int {
-            for (int it = 0; it < nt; it++) {
-                MarchStep st = step(it, it);
-                st.amp = amp[it];
-                st.src_on = on[it];
-                GEO_TRY(B.step(false, st, ss.cs));
-                GEO_TRY(watch(it, it == nt - 1, 1, st.lev ^ 1));
-            }
-            return GEO_OK;
-        }));
-        GEO_TRY(G.launch(ss.cs));
-    }
-    GEO_TRY(wd.verdict(ss.cs, "batched 2D RTM forward pass"));
-    // mute both records (tt = 285) and restart the source side from zero
-    std::vector<int> mute;
-    for (int k = 0; k < D.ns; k++) {
-        const int nxs = D.shot_nxs[k];
-        std::vector<int> lo, hi;
-        mute_window_mpi(nxs, nt, D.dt_ms, D.favg, D.dx, D.dz, nxs / 2 + 1, 0, D.zs, k + 1, X.mu_v[k], 285, lo, hi);
-        mute.insert(mute.end(), hi.begin(), hi.end());
-    }
-    DevBuf d_mute;
-    GEO_TRY(d_mute.alloc(mute.size() * 4));
-    GEO_CUDA(cudaMemcpyAsync(d_mute.p, mute.data(), mute.size() * 4, cudaMemcpyHostToDevice, ss.cs));
-    for (int k = 0, o = 0; k < D.ns; o += D.shot_nxs[k++]) {
-        const int *hi = d_mute.as<int>() + o;
-        GEO_TRY(launch_mute_records(B.M[k].rec_p, D.shot_nxs[k], nt, nullptr, hi, ss.cs));
-        GEO_TRY(launch_mute_records(B.M[k].rec_q, D.shot_nxs[k], nt, nullptr, hi, ss.cs));
-        GEO_TRY(B.clear_side(k, MS_SIDE, ss.cs));
-    }
-    // backward: both propagations with fused imaging; each step's lines and
-    // records go into the level it reads, the first by a launch of its own,
-    // the others as the step before stores that level
-    {
-        Graph G;
-        GEO_TRY(capture(G, ss.cs, [&]() -> int {
-            GEO_TRY(launch_march_inject(d_M, D.ns, maxline, nt - 1, 0, ss.cs));
-            for (int it = nt - 1; it >= 0; it--) {
-                MarchStep st = step(it, nt - 1 - it);
-                st.inject = it - 1;
-                GEO_TRY(B.step(true, st, ss.cs));
-                GEO_TRY(watch(nt - 1 - it, it == 0, 2, st.lev ^ 1));
-            }
-            return GEO_OK;
-        }));
-        GEO_TRY(G.launch(ss.cs));
-    }
-    int gave_up = 0;
-    GEO_CUDA(cudaMemcpyAsync(&gave_up, d_err.p, 4, cudaMemcpyDeviceToHost, ss.cs));
-    GEO_TRY(wd.verdict(ss.cs, "batched 2D RTM backward pass"));
-    GEO_CUDA(cudaStreamSynchronize(ss.cs));
-    if (gave_up) return fail(GEO_ERR_CUDA, "batched 2D RTM: a pipeline wait timed out");
-    // normalise per shot, stack in shot order, Laplacian
-    std::vector<float *> imgs(2 * (size_t)D.ns);   // images, then illuminations
-    std::vector<int> offs(D.ns), wid(D.ns);
-    Arena out;
-    for (int pass = 0; pass < 2; pass++) {
-        for (int k = 0; k < D.ns; k++) {
-            const size_t m = (size_t)D.shot_nxs[k] * nz;
-            imgs[k] = out.take<float>(m);
-            imgs[D.ns + k] = out.take<float>(m);
-            offs[k] = D.shot_x[k] - D.shot_nxs[k] / 2 - 1;
-            wid[k] = D.shot_nxs[k];
+    // Shots first .. first + n - 1, both passes, their images and gathers added
+    // to the stacks.  Memory is taken before anything is added.
+    auto group = [&](int first, int n) -> int {
+        MarchBatch B(X, first, n, fast != 0, adcig != nullptr);
+        GEO_TRY(B.build(raw, D.dx, D.dz, dt, nt, ss.cs));
+        const int *nxs = D.shot_nxs + first;
+        const March2D *d_M = B.d_M.as<March2D>();
+        int maxline = 0, traces = 0;
+        // after the backward pass the source side's fields are done with: image
+        // and illumination of a shot lie there without the sponge
+        std::vector<float *> imgs(2 * (size_t)n);   // images, then illuminations
+        std::vector<int> offs(n);
+        std::vector<const float *> ap(adcig ? (size_t)kAdcigAngles * n : 0);   // gathers, an angle after the other
+        for (int k = 0; k < n; k++) {
+            maxline = std::max(maxline, 2 * nxs[k] + 2 * nz);
+            traces += nxs[k];
+            imgs[k] = B.M[k].f + (size_t)MS_P * B.M[k].n;
+            imgs[n + k] = B.M[k].f + (size_t)MS_Q * B.M[k].n;
+            offs[k] = D.shot_x[first + k] - nxs[k] / 2 - 1;
+            for (size_t ia = 0; ia < ap.size() / n; ia++) ap[ia * n + k] = B.M[k].adcig + ia * nxs[k] * nz;
         }
-        if (pass == 0) GEO_TRY(out.alloc());
+        DevBuf d_mute, d_imgs, d_offs, d_wid, d_aptr;
+        GEO_TRY(d_mute.alloc((size_t)traces * 4));
+        GEO_TRY(d_imgs.alloc(imgs.size() * sizeof(float *)));
+        GEO_TRY(d_offs.alloc(n * 4));
+        GEO_TRY(d_wid.alloc(n * 4));
+        if (adcig) GEO_TRY(d_aptr.alloc(ap.size() * sizeof(float *)));
+        // non-finite detector: every wd.every steps (and the last) the graphs
+        // scan every shot's P; the verdict follows each pass
+        auto watch = [&](int k, bool last, int nf, int lev) -> int {
+            if (wd.every <= 0 || ((k + 1) % wd.every && !last)) return GEO_OK;
+            return launch_march_watch(d_M, n, nf, lev, wd.d, k + 1, ss.cs);
+        };
+        // forward: source side only, with records and edge lines
+        {
+            Graph G;
+            GEO_TRY(capture(G, ss.cs, [&]() -> int {
+                for (int it = 0; it < nt; it++) {
+                    MarchStep st = step(it, it);
+                    st.amp = amp[it];
+                    st.src_on = on[it];
+                    GEO_TRY(B.step(false, st, ss.cs));
+                    GEO_TRY(watch(it, it == nt - 1, 1, st.lev ^ 1));
+                }
+                return GEO_OK;
+            }));
+            GEO_TRY(G.launch(ss.cs));
+        }
+        GEO_TRY(wd.verdict(ss.cs, "batched 2D RTM forward pass"));
+        // mute both records (tt = 285) and restart the source side from zero
+        std::vector<int> mute;
+        for (int k = 0; k < n; k++) {
+            std::vector<int> lo, hi;
+            mute_window_mpi(nxs[k], nt, D.dt_ms, D.favg, D.dx, D.dz, nxs[k] / 2 + 1, 0, D.zs, first + k + 1,
+                            X.mu_v[first + k], 285, lo, hi);
+            mute.insert(mute.end(), hi.begin(), hi.end());
+        }
+        GEO_CUDA(cudaMemcpyAsync(d_mute.p, mute.data(), mute.size() * 4, cudaMemcpyHostToDevice, ss.cs));
+        for (int k = 0, o = 0; k < n; o += nxs[k++]) {
+            const int *hi = d_mute.as<int>() + o;
+            GEO_TRY(launch_mute_records(B.M[k].rec_p, nxs[k], nt, nullptr, hi, ss.cs));
+            GEO_TRY(launch_mute_records(B.M[k].rec_q, nxs[k], nt, nullptr, hi, ss.cs));
+            GEO_TRY(B.clear_side(k, MS_SIDE, ss.cs));
+        }
+        // backward: both propagations with fused imaging; each step's lines and
+        // records go into the level it reads, the first by a launch of its own,
+        // the others as the step before stores that level
+        {
+            Graph G;
+            GEO_TRY(capture(G, ss.cs, [&]() -> int {
+                GEO_TRY(launch_march_inject(d_M, n, maxline, nt - 1, 0, ss.cs));
+                for (int it = nt - 1; it >= 0; it--) {
+                    MarchStep st = step(it, nt - 1 - it);
+                    st.inject = it - 1;
+                    GEO_TRY(B.step(true, st, ss.cs));
+                    GEO_TRY(watch(nt - 1 - it, it == 0, 2, st.lev ^ 1));
+                }
+                return GEO_OK;
+            }));
+            GEO_TRY(G.launch(ss.cs));
+        }
+        int gave_up = 0;
+        GEO_CUDA(cudaMemcpyAsync(&gave_up, d_err.p, 4, cudaMemcpyDeviceToHost, ss.cs));
+        GEO_TRY(wd.verdict(ss.cs, "batched 2D RTM backward pass"));
+        GEO_CUDA(cudaStreamSynchronize(ss.cs));
+        if (gave_up) return fail(GEO_ERR_CUDA, "batched 2D RTM: a pipeline wait timed out");
+        // normalise per shot, stack in shot order
+        GEO_CUDA(cudaMemcpyAsync(d_imgs.p, imgs.data(), imgs.size() * sizeof(float *), cudaMemcpyHostToDevice, ss.cs));
+        GEO_CUDA(cudaMemcpyAsync(d_offs.p, offs.data(), n * 4, cudaMemcpyHostToDevice, ss.cs));
+        GEO_CUDA(cudaMemcpyAsync(d_wid.p, nxs, n * 4, cudaMemcpyHostToDevice, ss.cs));
+        GEO_TRY(launch_march_image(d_M, n, d_imgs.as<float *>(), d_imgs.as<float *>() + n, ss.cs));
+        GEO_TRY(launch_stack_image(stack.as<float>(), nz, d_imgs.as<const float *const>(), d_offs.as<int>(),
+                                   d_wid.as<int>(), n, D.nx, ss.cs));
+        if (adcig) {
+            // per shot: divide by the source illumination (Toa_rtm_vti_adcig_cdp.c:1083-1090), then stack
+            // every angle plane in shot order into [90][nx][nz] (adcig_ns0)
+            for (int q = 0; q < n; q++)
+                GEO_TRY(launch_normalize_planes(B.M[q].adcig, imgs[n + q], (size_t)nxs[q] * nz, kAdcigAngles, ss.cs));
+            GEO_CUDA(cudaMemcpyAsync(d_aptr.p, ap.data(), ap.size() * sizeof(float *), cudaMemcpyHostToDevice, ss.cs));
+            for (int ia = 0; ia < kAdcigAngles; ia++)
+                GEO_TRY(launch_stack_image(gathers.as<float>() + ia * nimg, nz,
+                                           d_aptr.as<const float *const>() + (size_t)ia * n, d_offs.as<int>(),
+                                           d_wid.as<int>(), n, D.nx, ss.cs));
+        }
+        for (int k = 0; k < n && per_shot; k++)
+            GEO_CUDA(cudaMemcpyAsync(per_shot + shot_off[first + k], imgs[k], (size_t)nxs[k] * nz * 4, kout, ss.cs));
+        GEO_CUDA(cudaStreamSynchronize(ss.cs));
+        return GEO_OK;
+    };
+    // All shots together where they fit (a shot takes 128 B a padded point in
+    // the exact form, 116 in the fast one, and its records and edge lines), else
+    // in the largest of halved groups that do: the stacks add in shot order
+    // either way, so the images are the same.
+    int n = D.ns;
+    if (const char *e = getenv("GEO_RTM2D_GROUP"))
+        if (const int k = atoi(e); k > 0) n = std::min(n, k);
+    for (int first = 0; first < D.ns;) {
+        n = std::min(n, D.ns - first);
+        const int rc = group(first, n);
+        if (rc == GEO_ERR_NOMEM && n > 1) {
+            n = (n + 1) / 2;
+            continue;
+        }
+        GEO_TRY(rc);
+        first += n;
     }
-    DevBuf d_imgs, d_offs, d_wid, stack, lap;
-    GEO_TRY(d_imgs.alloc(2 * D.ns * sizeof(float *)));
-    GEO_TRY(d_offs.alloc(D.ns * 4));
-    GEO_TRY(d_wid.alloc(D.ns * 4));
-    GEO_CUDA(cudaMemcpyAsync(d_imgs.p, imgs.data(), 2 * D.ns * sizeof(float *), cudaMemcpyHostToDevice, ss.cs));
-    GEO_CUDA(cudaMemcpyAsync(d_offs.p, offs.data(), D.ns * 4, cudaMemcpyHostToDevice, ss.cs));
-    GEO_CUDA(cudaMemcpyAsync(d_wid.p, wid.data(), D.ns * 4, cudaMemcpyHostToDevice, ss.cs));
-    GEO_TRY(launch_march_image(d_M, D.ns, d_imgs.as<float *>(), d_imgs.as<float *>() + D.ns, ss.cs));
-    const size_t nimg = (size_t)D.nx * nz;
-    GEO_TRY(stack.alloc(nimg * 4));
-    GEO_TRY(stack.zero(ss.cs));
-    GEO_TRY(launch_stack_image(stack.as<float>(), nz, d_imgs.as<const float *const>(), d_offs.as<int>(),
-                               d_wid.as<int>(), D.ns, D.nx, ss.cs));
     const float *result = stack.as<float>();
     if (D.laplace) {
-        GEO_TRY(lap.alloc(nimg * 4));
         GEO_TRY(launch_laplace2d(D.nx, nz, stack.as<float>(), lap.as<float>(), ss.cs));
         result = lap.as<float>();
     }
-    const cudaMemcpyKind k = mem == GEO_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    GEO_CUDA(cudaMemcpyAsync(image, result, nimg * 4, k, ss.cs));
-    DevBuf gathers, d_aptr;
-    if (adcig) {
-        // per shot: divide by the source illumination (Toa_rtm_vti_adcig_cdp.c:1083-1090), then stack
-        // every angle plane in shot order into [90][nx][nz] (adcig_ns0)
-        std::vector<const float *> ap((size_t)kAdcigAngles * D.ns);
-        for (int q = 0; q < D.ns; q++) {
-            const size_t m = (size_t)D.shot_nxs[q] * nz;
-            GEO_TRY(launch_normalize_planes(B.M[q].adcig, imgs[D.ns + q], m, kAdcigAngles, ss.cs));
-            for (int ia = 0; ia < kAdcigAngles; ia++) ap[(size_t)ia * D.ns + q] = B.M[q].adcig + ia * m;
-        }
-        GEO_TRY(d_aptr.alloc(ap.size() * sizeof(float *)));
-        GEO_CUDA(cudaMemcpyAsync(d_aptr.p, ap.data(), ap.size() * sizeof(float *), cudaMemcpyHostToDevice, ss.cs));
-        GEO_TRY(gathers.alloc((size_t)kAdcigAngles * nimg * 4));
-        GEO_TRY(gathers.zero(ss.cs));
-        for (int ia = 0; ia < kAdcigAngles; ia++)
-            GEO_TRY(launch_stack_image(gathers.as<float>() + ia * nimg, nz,
-                                       d_aptr.as<const float *const>() + (size_t)ia * D.ns, d_offs.as<int>(),
-                                       d_wid.as<int>(), D.ns, D.nx, ss.cs));
-        GEO_CUDA(cudaMemcpyAsync(adcig, gathers.p, (size_t)kAdcigAngles * nimg * 4, k, ss.cs));
-    }
-    if (per_shot) {
-        size_t o = 0;
-        for (int q = 0; q < D.ns; q++) {
-            const size_t m = (size_t)D.shot_nxs[q] * nz;
-            GEO_CUDA(cudaMemcpyAsync(per_shot + o, imgs[q], m * 4, k, ss.cs));
-            o += m;
-        }
-    }
+    GEO_CUDA(cudaMemcpyAsync(image, result, nimg * 4, kout, ss.cs));
+    if (adcig) GEO_CUDA(cudaMemcpyAsync(adcig, gathers.p, (size_t)kAdcigAngles * nimg * 4, kout, ss.cs));
     GEO_CUDA(cudaStreamSynchronize(ss.cs));
     return GEO_OK;
 }

@@ -39,6 +39,7 @@ int DevBuf::alloc(size_t n) {
     cudaError_t e = cudaMalloc(&p, n);
     if (e != cudaSuccess) {
         p = nullptr;
+        cudaGetLastError();   // or the next launch check would report it
         return fail(GEO_ERR_NOMEM, "cudaMalloc(%zu): %s", n, cudaGetErrorString(e));
     }
     bytes = n;

@@ -257,7 +257,9 @@ int geo_rtm3d_adcig(const geo_rtm3d_desc *desc, const float *v, const float *e, 
  * (2D-vti-fd+rtm-mpi/Toa_rtm_vti_adcig_cdp.c:295-392 with
  * model_vti_get_boundry :483 and RTM_corr_adcig :739).  All shots run
  * together: each time step is one launch over every shot, and the time
- * loop is replayed from a CUDA graph.  The stacked image
+ * loop is replayed from a CUDA graph.  Where their memory (128 B a padded
+ * point of every window in GEO_MODE_EXACT, 116 in GEO_MODE_FAST, and the
+ * records) does not fit, they run in groups.  The stacked image
  * is formed in shot order and optionally passed through the adjoint
  * Laplacian (laplac2_lop adj=1). */
 typedef struct geo_rtm2d_desc {

@@ -105,9 +105,39 @@ static void check_devices() {
     printf("%zu constants, %zu kernels with attributes\n", fake::st().symbols[0].size(), fake::st().attributes[0].size());
 }
 
+// A batch that does not fit at once runs in groups of shots: it succeeds where
+// only half of its shots' memory is left, and one that cannot run at all says
+// so and leaves no error behind for the next call.
+static void check_batch_memory() {
+    const int nx = 600, nz = 150, npd = 20, n2 = nx * nz, ns = 9;
+    auto v = filled(n2, 2000), e = filled(n2, 0.1f), d = filled(n2, 0.05f);
+    std::vector<int> xs(ns), ws(ns, 201);
+    for (int k = 0; k < ns; k++) xs[k] = 200 + 20 * k;
+    std::vector<float> img(n2), ag((size_t)90 * n2), per((size_t)ns * 201 * nz);
+    for (int mode : {GEO_MODE_EXACT, GEO_MODE_FAST})
+        for (int gathers = 0; gathers < 2; gathers++) {
+            geo_rtm2d_desc B{};
+            B.nx = nx; B.nz = nz; B.npd = npd; B.nt = 4; B.dx = B.dz = 10; B.dt_ms = 1; B.favg = 20; B.pfac = 10; B.zs = 2;
+            B.ns = ns; B.shot_x = xs.data(); B.shot_nxs = ws.data(); B.mode = mode;
+            auto run = [&](size_t limit) {
+                fake::st().limit = limit;
+                fake::st().peak = fake::st().in_use;
+                return geo_rtm2d_batch_adcig(&B, v.data(), e.data(), d.data(), img.data(), per.data(),
+                                             gathers ? ag.data() : nullptr, GEO_MEM_HOST, nullptr);
+            };
+            OK(run(~size_t(0)));
+            const size_t all = fake::st().peak, fixed = gathers ? (size_t)90 * n2 * 4 : 0;
+            for (double share : {0.99, 0.8, 0.5, 0.25}) OK(run(fixed + (size_t)(share * (all - fixed))));
+            if (run(1 << 20) != GEO_ERR_NOMEM) { printf("1 MiB was enough\n"); failures++; }
+            OK(run(~size_t(0)));
+            if (fake::st().in_use) { printf("%zu bytes left allocated\n", fake::st().in_use); failures++; }
+        }
+}
+
 int main(int argc, char **argv) {
     const std::string check = argc > 1 ? argv[1] : "";
     if (check == "devices") check_devices();
+    else if (check == "batch_memory") check_batch_memory();
     else return 2;
     return failures ? 1 : 0;
 }

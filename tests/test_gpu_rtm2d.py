@@ -204,3 +204,20 @@ def test_rtm2d_gpu_program_tile_edges(geo, orc, nx, nz, npml):
     assert np.array_equal(out["illum"], ill)
     assert np.array_equal(out["mig_lap"], orc.laplace2d_adj(mig))
     assert np.array_equal(out["adcigs"], ag)
+
+
+# shots run a group at a time (as they do where memory holds no more): images,
+# per-shot images and gathers stacked in the same order, so the same bits
+@pytest.mark.parametrize("mode", ["exact", "fast"])
+@pytest.mark.parametrize("n", [1, 2, 4])
+def test_rtm2d_batch_groups_of_shots(geo, monkeypatch, mode, n):
+    v, e, d = model(103, 107)
+    kw = dict(npd=10, nt=420, dx=10.0, dz=10.0, dt_ms=1.0, favg=25.0, pfac=1000.0, zs=2, shot_x=[40, 52, 45, 60, 52],
+              shot_nxs=[31, 41, 33, 25, 61], per_shot=True, adcig=True, laplace=False, mode=mode)
+    ref = geo.rtm2d_batch(v, e, d, **kw)
+    monkeypatch.setenv("GEO_RTM2D_GROUP", str(n))
+    out = geo.rtm2d_batch(v, e, d, **kw)
+    flat = lambda r: [a for x in r for a in (x if isinstance(x, (list, tuple)) else [x])]
+    assert len(flat(ref)) == len(flat(out)) == 7
+    for a, b in zip(flat(ref), flat(out)):
+        assert np.abs(a).max() > 0 and np.array_equal(a, b)

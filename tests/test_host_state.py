@@ -1,5 +1,6 @@
 """Host-side state of libgeofd, run against a CUDA runtime without a device
-(fake_cuda.h): what belongs to a device is set up on every device."""
+(fake_cuda.h): what belongs to a device is set up on every device, and runs
+that do not fit in memory at once."""
 import os
 import shutil
 import subprocess
@@ -35,3 +36,7 @@ def test_second_device_gets_tables_and_kernel_attributes(check):
     """Every entry point on one device, then on another: the same constant
     tables are copied to both, the same kernels' shared-memory limits set."""
     check("devices")
+
+
+def test_batched_rtm_beyond_memory_runs_in_groups(check):
+    check("batch_memory")
