@@ -701,7 +701,8 @@ int Fused2D::plan(StepKind k, bool tti_, const SGrid &g, int fixed) {
     for (int nc = 1; nc <= 2 && coop; nc++) {
         const int t = nc * kThreads / 32;
         const void *fn = step_fn(k, tti, t);
-        if (fixed ? t != fixed : tti && k != SK_GPU && t != 8) continue;
+        if (fixed && t != fixed) continue;
+        if (tti && k != SK_GPU && t != 8) continue;   // no such kernel (step_fn)
         const int n = ((g.nnz + kTz - 1) / kTz) * ((g.nnx + t - 1) / t);
         GEO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)step_smem(t, 2, tti)));
         for (int st = k == SK_GBWD && !tti ? 2 : 1; st <= 2; st++) {
@@ -719,6 +720,7 @@ int Fused2D::plan(StepKind k, bool tti_, const SGrid &g, int fixed) {
             break;
         }
     }
+    if (!best && coop && fixed) return fail(GEO_ERR_ARG, "2D step: no tiles of %d columns", fixed);
     if (!best) return fail(GEO_ERR_CUDA, "2D step: cooperative launch unavailable");
     return GEO_OK;
 }

@@ -2,6 +2,7 @@
 // (fake_cuda.h).  Usage: host_state_check <check>; prints what fails.
 #include "fake_cuda.h"
 #include "geofd.h"
+#include "step2d.cuh"
 #include <cmath>
 #include <vector>
 
@@ -134,10 +135,34 @@ static void check_batch_memory() {
         }
 }
 
+// Tile widths of the 2D RTM programs' passes: the grids of
+// test_rtm2d_gpu_program_wide_tiles take 16 columns on 152 SMs, with a tile a
+// block and with several, and a width without a kernel is refused.
+static void check_plans() {
+    const int grids[][4] = {{143, 443, 5, 1}, {150, 450, 5, 1}, {1665, 200, 7, 0}};   // nx, nz, sponge, a tile a block
+    for (const auto &q : grids)
+        for (geo::StepKind k : {geo::SK_GFWD, geo::SK_GBWD}) {
+            geo::SGrid g{};
+            g.nx = q[0]; g.nz = q[1]; g.npd = q[2];
+            g.nnx = q[0] + 2 * q[2]; g.nnz = q[1] + 2 * q[2]; g.ldz = (g.nnz + 3) / 4 * 4;
+            geo::Fused2D p;
+            OK(p.plan(k, false, g));
+            if (p.tx != 16 || (p.tiles == p.grid) != (q[3] == 1)) {
+                printf("%dx%d kind %d: %d columns, %d tiles on %d blocks\n", q[0], q[1], k, p.tx, p.tiles, p.grid);
+                failures++;
+            }
+            OK(p.plan(k, true, g, 8));
+            if (p.plan(k, true, g, 16) == GEO_OK) { printf("kind %d: 16 columns of the tilted medium accepted\n", k); failures++; }
+            OK(p.plan(k, true, g));
+            if (p.tx != 8) { printf("kind %d: tilted medium, %d columns\n", k, p.tx); failures++; }
+        }
+}
+
 int main(int argc, char **argv) {
     const std::string check = argc > 1 ? argv[1] : "";
     if (check == "devices") check_devices();
     else if (check == "batch_memory") check_batch_memory();
+    else if (check == "plans") check_plans();
     else return 2;
     return failures ? 1 : 0;
 }

@@ -221,3 +221,19 @@ def test_rtm2d_batch_groups_of_shots(geo, monkeypatch, mode, n):
     assert len(flat(ref)) == len(flat(out)) == 7
     for a, b in zip(flat(ref), flat(out)):
         assert np.abs(a).max() > 0 and np.array_equal(a, b)
+
+
+# grids on which both passes take tiles of 16 columns (152 SMs; checked without
+# a GPU in test_host_state.py): columns and depths that end inside a tile and
+# at its edge, a tile a block, and blocks that walk several tiles
+@pytest.mark.parametrize("nx,nz,npml,nt", [(143, 443, 5, 220), (150, 450, 5, 400), (1665, 200, 7, 220)])
+def test_rtm2d_gpu_program_wide_tiles(geo, orc, nx, nz, npml, nt):
+    v, e, d = model(nx=nx, nz=nz)
+    kw = dict(GKW, npml=npml, ns=1, fs=nx // 2, zs=4, nt=nt)
+    mig, ill, ag, shots = orc.rtm2d_gpu(v, e, d, **cuda_angle_tables(kw["dangle"]), **kw)
+    out = geo.rtm2d_gpu(v, e, d, **kw)
+    assert np.abs(mig).max() > 0 and np.abs(ag).max() > 0
+    assert np.array_equal(out["shots"], shots)
+    assert np.array_equal(out["illum"], ill)
+    assert np.array_equal(out["mig_lap"], orc.laplace2d_adj(mig))
+    assert np.array_equal(out["adcigs"], ag)

@@ -20,7 +20,8 @@ def check(tmp_path_factory):
     if not cxx or not os.path.exists(os.path.join(inc, "cuda_runtime.h")) or not os.path.exists(lib):
         pytest.skip("needs a C++ compiler, the CUDA headers and the built library")
     exe = str(tmp_path_factory.mktemp("host_state") / "host_state_check")
-    subprocess.run([cxx, "-O1", "-std=c++17", "-I" + os.path.join(ROOT, "include"), "-I" + inc,
+    subprocess.run([cxx, "-O1", "-std=c++17", "-I" + os.path.join(ROOT, "include"),
+                    "-I" + os.path.join(PKG, "csrc"), "-I" + inc,
                     os.path.join(ROOT, "tests", "host_state_check.cpp"), "-o", exe, lib, "-rdynamic",
                     "-Wl,-rpath," + PKG, "-Wl,--allow-shlib-undefined", "-lpthread"], check=True)
 
@@ -40,3 +41,7 @@ def test_second_device_gets_tables_and_kernel_attributes(check):
 
 def test_batched_rtm_beyond_memory_runs_in_groups(check):
     check("batch_memory")
+
+
+def test_2d_rtm_tile_widths(check):
+    check("plans")
