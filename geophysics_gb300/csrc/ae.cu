@@ -1190,16 +1190,13 @@ struct geo_ae {
     DevBuf store, wstore, count, snapmax;
     long cap = 0;
     // forward scratch (rows = padded blocks)
-    int rows = 0;
     DevBuf h1, h2, h3, z, g3, g2, g1, scale;
     // training scratch
-    int trows = 0;
     DevBuf xn, dg1, dg2, dg3, dz, dh3, dh2, dh1, wrow;
     DevBuf ev;                                 // evaluation: loss (double), zero step counter
     // escape settings
     float tau = 0.05f, frac = 0.03f;
     DevBuf resall, err2, norm2;
-    int erows = 0;
     long long st_blocks = 0, st_escaped = 0;   // totals over RTM shots
     // host copy of the CUDA-core levels' weights for the snapshot kernels:
     // wver counts weight updates (packs), hver the version copied
@@ -1230,36 +1227,34 @@ static int ae_pack(geo_ae *ae, int inc, cudaStream_t s) {
     return check_launch("ae_pack");
 }
 
+// A scratch buffer of at least n bytes.  A buffer that could not grow is empty
+// and is asked for again by the next call.
+static int at_least(DevBuf &b, size_t n) { return b.bytes >= n ? GEO_OK : b.alloc(n); }
+
 static int ensure_rows(geo_ae *ae, int rows) {
-    if (rows <= ae->rows) return GEO_OK;
     const size_t r = (size_t)rows;
-    GEO_TRY(ae->h1.alloc(r * 512 * 16 * 2));
-    GEO_TRY(ae->h2.alloc(r * 64 * 64 * 2));
-    GEO_TRY(ae->h3.alloc(r * 8 * 256 * 2));
-    GEO_TRY(ae->z.alloc(r * 512 * 2));
-    GEO_TRY(ae->g3.alloc(r * 2048 * 2));
-    GEO_TRY(ae->g2.alloc(r * 8 * 512 * 2));
-    GEO_TRY(ae->g1.alloc(r * 64 * 128 * 2));
-    GEO_TRY(ae->scale.alloc(r * 4));
-    ae->rows = rows;
-    return GEO_OK;
+    GEO_TRY(at_least(ae->h1, r * 512 * 16 * 2));
+    GEO_TRY(at_least(ae->h2, r * 64 * 64 * 2));
+    GEO_TRY(at_least(ae->h3, r * 8 * 256 * 2));
+    GEO_TRY(at_least(ae->z, r * 512 * 2));
+    GEO_TRY(at_least(ae->g3, r * 2048 * 2));
+    GEO_TRY(at_least(ae->g2, r * 8 * 512 * 2));
+    GEO_TRY(at_least(ae->g1, r * 64 * 128 * 2));
+    return at_least(ae->scale, r * 4);
 }
 
 static int ensure_train(geo_ae *ae, int rows) {
     GEO_TRY(ensure_rows(ae, rows));
-    if (rows <= ae->trows) return GEO_OK;
     const size_t r = (size_t)rows;
-    GEO_TRY(ae->xn.alloc(r * kAePts * 4));
-    GEO_TRY(ae->dg1.alloc(r * 8192 * 2));
-    GEO_TRY(ae->dg2.alloc(r * 4096 * 2));
-    GEO_TRY(ae->dg3.alloc(r * 2048 * 2));
-    GEO_TRY(ae->dz.alloc(r * 512 * 2));
-    GEO_TRY(ae->dh3.alloc(r * 2048 * 2));
-    GEO_TRY(ae->dh2.alloc(r * 4096 * 2));
-    GEO_TRY(ae->dh1.alloc(r * 8192 * 2));
-    GEO_TRY(ae->wrow.alloc(r * 4));
-    ae->trows = rows;
-    return GEO_OK;
+    GEO_TRY(at_least(ae->xn, r * kAePts * 4));
+    GEO_TRY(at_least(ae->dg1, r * 8192 * 2));
+    GEO_TRY(at_least(ae->dg2, r * 4096 * 2));
+    GEO_TRY(at_least(ae->dg3, r * 2048 * 2));
+    GEO_TRY(at_least(ae->dz, r * 512 * 2));
+    GEO_TRY(at_least(ae->dh3, r * 2048 * 2));
+    GEO_TRY(at_least(ae->dh2, r * 4096 * 2));
+    GEO_TRY(at_least(ae->dh1, r * 8192 * 2));
+    return at_least(ae->wrow, r * 4);
 }
 
 static __nv_bfloat16 *bf(const DevBuf &b) { return b.as<__nv_bfloat16>(); }
@@ -1448,12 +1443,9 @@ int ae_encode_volume(geo_ae *ae, const AeVolume &v, void *code, float *scale, in
         if (count) GEO_CUDA(cudaMemsetAsync(count, 0, 4, s));
         return GEO_OK;
     }
-    if (rows > ae->erows) {
-        GEO_TRY(ae->resall.alloc((size_t)rows * kAePts * 2));
-        GEO_TRY(ae->err2.alloc((size_t)rows * 4));
-        GEO_TRY(ae->norm2.alloc((size_t)rows * 4));
-        ae->erows = rows;
-    }
+    GEO_TRY(at_least(ae->resall, (size_t)rows * kAePts * 2));
+    GEO_TRY(at_least(ae->err2, (size_t)rows * 4));
+    GEO_TRY(at_least(ae->norm2, (size_t)rows * 4));
     GEO_TRY(decode_rows(ae, rows, static_cast<const __nv_bfloat16 *>(code), s));
     D1Vol c{};
     c.vol = v;
@@ -1653,6 +1645,7 @@ extern "C" long long geo_ae_num_blocks(geo_ae *ae) {
 
 extern "C" int geo_ae_reserve(geo_ae *ae, long long max_blocks) {
     if (!ae || max_blocks < 1) return fail(GEO_ERR_ARG, "bad argument");
+    ae->cap = 0;   // no store until both buffers stand
     GEO_TRY(ae->store.alloc((size_t)max_blocks * kAePts * 4));
     GEO_TRY(ae->wstore.alloc((size_t)max_blocks * 4));
     ae->cap = max_blocks;

@@ -190,10 +190,11 @@ FAKE cudaError_t cudaGetLastError() {
     fake::last = cudaSuccess;
     return e;
 }
-inline CUresult fake_encode(CUtensorMap *m, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+inline CUresult fake_encode(CUtensorMap *m, CUtensorMapDataType, cuuint32_t, void *base, const cuuint64_t *, const cuuint64_t *,
                             const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                             CUtensorMapL2promotion, CUtensorMapFloatOOBfill) {
     memset(m, 0, sizeof *m);
+    if (!base) fake::st().refused += "tensor map of a null buffer\n";
     return CUDA_SUCCESS;
 }
 FAKE cudaError_t cudaGetDriverEntryPointByVersion(const char *, void **f, unsigned, unsigned long long,

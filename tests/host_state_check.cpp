@@ -135,6 +135,33 @@ static void check_batch_memory() {
         }
 }
 
+// Scratch of the codec that could not grow: the calls after it, of any size,
+// find buffers again.
+static void check_codec_growth() {
+    geo_ae *ae = nullptr;
+    OK(geo_ae_create(&ae, 1));
+    std::vector<float> a((size_t)256 * 256 * 64), b(a.size()), blk((size_t)512 * 4096, 1.0f), grad(geo_ae_num_params());
+    double loss;
+    auto trip = [&](int n, int escape) { return geo_ae_roundtrip(ae, n, n, 64, a.data(), b.data(), escape, nullptr, nullptr); };
+    auto eval = [&](int n) { return geo_ae_eval(ae, blk.data(), n, nullptr, &loss, grad.data(), GEO_MEM_DEVICE, nullptr); };
+    OK(trip(64, 1));
+    OK(eval(128));
+    const size_t base = fake::st().in_use;
+    // stop the growth at each of its buffers in turn
+    for (int mib = 2; mib < 64; mib += 3) {
+        fake::st().limit = base + ((size_t)mib << 20);
+        const int st[2] = {trip(256, 1), eval(512)};
+        for (int s : st)
+            if (s != GEO_OK && s != GEO_ERR_NOMEM) { printf("limit %d MiB: %s\n", mib, geo_strerror(s)); failures++; }
+        fake::st().limit = ~size_t(0);
+        OK(trip(64, 1));
+        OK(eval(128));
+    }
+    OK(geo_ae_destroy(ae));
+    printf("%s", fake::st().refused.c_str());
+    if (!fake::st().refused.empty()) failures++;
+}
+
 // Tile widths of the 2D RTM programs' passes: the grids of
 // test_rtm2d_gpu_program_wide_tiles take 16 columns on 152 SMs, with a tile a
 // block and with several, and a width without a kernel is refused.
@@ -163,6 +190,7 @@ int main(int argc, char **argv) {
     if (check == "devices") check_devices();
     else if (check == "batch_memory") check_batch_memory();
     else if (check == "plans") check_plans();
+    else if (check == "codec_growth") check_codec_growth();
     else return 2;
     return failures ? 1 : 0;
 }

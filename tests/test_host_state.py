@@ -45,3 +45,7 @@ def test_batched_rtm_beyond_memory_runs_in_groups(check):
 
 def test_2d_rtm_tile_widths(check):
     check("plans")
+
+
+def test_codec_scratch_that_failed_to_grow(check):
+    check("codec_growth")
