@@ -1233,18 +1233,22 @@ static int at_least(DevBuf &b, size_t n) { return b.bytes >= n ? GEO_OK : b.allo
 
 static int ensure_rows(geo_ae *ae, int rows) {
     const size_t r = (size_t)rows;
-    GEO_TRY(at_least(ae->h1, r * 512 * 16 * 2));
     GEO_TRY(at_least(ae->h2, r * 64 * 64 * 2));
     GEO_TRY(at_least(ae->h3, r * 8 * 256 * 2));
     GEO_TRY(at_least(ae->z, r * 512 * 2));
     GEO_TRY(at_least(ae->g3, r * 2048 * 2));
     GEO_TRY(at_least(ae->g2, r * 8 * 512 * 2));
-    GEO_TRY(at_least(ae->g1, r * 64 * 128 * 2));
     return at_least(ae->scale, r * 4);
 }
+// E1's output: training only (snapshots have E1 and E2 in one kernel).
+static int ensure_h1(geo_ae *ae, int rows) { return at_least(ae->h1, (size_t)rows * 512 * 16 * 2); }
+// D2's output: training, imaging and the escape check (a plain decode has D2 and D1 in one kernel).
+static int ensure_g1(geo_ae *ae, int rows) { return at_least(ae->g1, (size_t)rows * 64 * 128 * 2); }
 
 static int ensure_train(geo_ae *ae, int rows) {
     GEO_TRY(ensure_rows(ae, rows));
+    GEO_TRY(ensure_h1(ae, rows));
+    GEO_TRY(ensure_g1(ae, rows));
     const size_t r = (size_t)rows;
     GEO_TRY(at_least(ae->xn, r * kAePts * 4));
     GEO_TRY(at_least(ae->dg1, r * 8192 * 2));
@@ -1420,6 +1424,7 @@ int ae_encode_volume(geo_ae *ae, const AeVolume &v, void *code, float *scale, in
                      cudaStream_t s) {
     const int nb = blocks_of(v), rows = pad128(nb);
     GEO_TRY(ensure_rows(ae, rows));
+    if (esc) GEO_TRY(ensure_g1(ae, rows));   // before a run, not at its first decode
     GEO_TRY(ae_mirror(ae, s));
     E12Args a{};
     a.vol = v;
@@ -1494,6 +1499,7 @@ int ae_decode_volume(geo_ae *ae, const AeVolume &v, const void *code, const floa
         GEO_CUDA(launch_early(k_ae_d21, std::min(a.tiles, 2 * sm_count()), kD21Threads, kD21Smem, s, ta, tw, a));
         return check_launch("ae_d21");
     }
+    GEO_TRY(ensure_g1(ae, rows));
     GEO_TRY(decode_rows(ae, rows, static_cast<const __nv_bfloat16 *>(code), s));
     D1Vol a{};
     a.vol = v;

@@ -162,6 +162,19 @@ static void check_codec_growth() {
     if (!fake::st().refused.empty()) failures++;
 }
 
+// A plain round trip takes the scratch that its kernels use: 25604 B a block
+// (E2 to E4's, D4's and D3's outputs and the scale), blocks padded to 128.
+static void check_codec_memory() {
+    geo_ae *ae = nullptr;
+    OK(geo_ae_create(&ae, 1));
+    std::vector<float> a((size_t)256 * 256 * 64), b(a.size());
+    const size_t before = fake::st().in_use, blocks = a.size() / 4096;
+    OK(geo_ae_roundtrip(ae, 256, 256, 64, a.data(), b.data(), 0, nullptr, nullptr));
+    const size_t used = fake::st().in_use - before, want = blocks * 25604;
+    if (used > want + 65536) { printf("%zu bytes of scratch, %zu used by the kernels\n", used, want); failures++; }
+    OK(geo_ae_destroy(ae));
+}
+
 // Tile widths of the 2D RTM programs' passes: the grids of
 // test_rtm2d_gpu_program_wide_tiles take 16 columns on 152 SMs, with a tile a
 // block and with several, and a width without a kernel is refused.
@@ -191,6 +204,7 @@ int main(int argc, char **argv) {
     else if (check == "batch_memory") check_batch_memory();
     else if (check == "plans") check_plans();
     else if (check == "codec_growth") check_codec_growth();
+    else if (check == "codec_memory") check_codec_memory();
     else return 2;
     return failures ? 1 : 0;
 }

@@ -49,3 +49,7 @@ def test_2d_rtm_tile_widths(check):
 
 def test_codec_scratch_that_failed_to_grow(check):
     check("codec_growth")
+
+
+def test_codec_scratch_is_what_its_kernels_use(check):
+    check("codec_memory")
