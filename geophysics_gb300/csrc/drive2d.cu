@@ -285,22 +285,44 @@ struct MarchBatch {
 
 // Strips of at most 120 depths and chunks of columns.  A chunk repeats 14
 // columns' worth of P and 7 of u, so long chunks save work; short ones
-// balance it, since warps on a wavefront's rim take longer (ziv.cuh).  Four
-// waves of warps, within 8 and 48 columns: 16 shots of 401-1199 columns x 601
-// take 182 us a forward and 328 us a backward step with chunks of about 12,
-// 200 and 376 us with one wave (35 and 70 columns).
+// balance it, since warps on a wavefront's rim take longer (ziv.cuh).
+//
+// Work for several waves of warps: four waves, within 8 and 48 columns.  16
+// shots of 401-1199 columns x 601 take 182 us a forward and 328 us a backward
+// step with chunks of about 12, 200 and 376 us with one wave (35 and 70
+// columns).
+//
+// Work that one wave takes in chunks of 8 or fewer: the shortest chunks that
+// leave it one wave.  There a step lasts as long as a warp's march, about 8 us
+// and 3 a column (2 in the fast form, 9 backward with gathers on full
+// wavefields), and half the warps idle.  us a forward and a backward step
+// together, chunks of 8 and by the rule: one shot 61x101 + 30 54.9 and 18.4,
+// 201x301 64.8 and 22.7, four of 201x301 69.0 and 40.4, eight 78.5 and 62,
+// three of 401x401 76.9 and 55.4.
 int MarchBatch::work(bool backward) {
     const int nnz = X.nnz, depths = nnz - 8;
     const int strips = (depths + 119) / 120, len = ((depths + strips - 1) / strips + 3) / 4 * 4;
-    long cols = 0;
-    for (int k = 0; k < ns; k++) cols += (long)strips * (M[k].nnx - 8);
     int res = 0;
     GEO_TRY(march2d_resident(backward, fast, adcig, &res));
-    const int chunk = (int)std::min(48L, std::max(8L, cols / (4L * res)));
+    auto chunks = [&](int k, int chunk) { return (M[k].nnx - 8 + chunk - 1) / chunk; };
+    int chunk = 0;
+    for (int c = 1; c <= 8 && !chunk; c++) {
+        long n = 0;
+        for (int k = 0; k < ns; k++) n += (long)strips * chunks(k, c);
+        if (n <= res) chunk = c;
+    }
+    const bool one_wave = chunk != 0;
+    if (!one_wave) {
+        long cols = 0;
+        for (int k = 0; k < ns; k++) cols += (long)strips * (M[k].nnx - 8);
+        chunk = (int)std::min(48L, std::max(8L, cols / (4L * res)));
+    }
+    if (const char *e = getenv("GEO_RTM2D_CHUNK"))
+        if (const int c = atoi(e); c > 0) chunk = c;
     std::vector<int4> &v = items[backward];
     v.clear();
     for (int k = 0; k < ns; k++) {
-        const int w = M[k].nnx - 8, nc = std::max(1, (w + chunk / 2) / chunk);
+        const int w = M[k].nnx - 8, nc = one_wave ? chunks(k, chunk) : std::max(1, (w + chunk / 2) / chunk);
         for (int t = 0; t < strips; t++)
             for (int c = 0; c < nc; c++)
                 v.push_back(make_int4(k | (len / 4) << 24, t * len, 4 + (int)((long)w * c / nc), 4 + (int)((long)w * (c + 1) / nc)));

@@ -25,7 +25,7 @@ struct State {
     std::map<std::pair<int, const void *>, size_t> smem_limit;
     std::map<void *, size_t> blocks;
     size_t in_use = 0, peak = 0, limit = ~size_t(0);
-    std::map<std::string, long> launches;
+    std::map<std::string, long> launches, blocks_max;
     std::string refused;   // launches that a device would refuse
 };
 inline State &st() {
@@ -40,10 +40,11 @@ inline cudaError_t err(cudaError_t e) {
     return e;
 }
 
-inline cudaError_t launch(const void *f, void **args, size_t smem) {
+inline cudaError_t launch(const void *f, dim3 grid, void **args, size_t smem) {
     std::lock_guard<std::recursive_mutex> g(st().mu);
     const std::string &n = st().kernel_name[f];
     st().launches[n]++;
+    if (grid.x > st().blocks_max[n]) st().blocks_max[n] = grid.x;
     const auto it = st().smem_limit.find({device, f});
     if (smem > 49152 && (it == st().smem_limit.end() || it->second < smem)) {
         st().refused += n + " on device " + std::to_string(device) + "\n";
@@ -91,15 +92,17 @@ FAKE cudaError_t __cudaPopCallConfiguration(dim3 *g, dim3 *b, size_t *smem, void
     return cudaSuccess;
 }
 FAKE cudaError_t __cudaGetKernel(cudaKernel_t *k, const void *f) { *k = (cudaKernel_t)f; return cudaSuccess; }
-FAKE cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void **args, size_t smem, cudaStream_t) {
-    return fake::launch((const void *)k, args, smem);
+FAKE cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 g, dim3, void **args, size_t smem, cudaStream_t) {
+    return fake::launch((const void *)k, g, args, smem);
 }
-FAKE cudaError_t cudaLaunchKernel(const void *f, dim3, dim3, void **args, size_t smem, cudaStream_t) { return fake::launch(f, args, smem); }
-FAKE cudaError_t cudaLaunchCooperativeKernel(const void *f, dim3, dim3, void **args, size_t smem, cudaStream_t) {
-    return fake::launch(f, args, smem);
+FAKE cudaError_t cudaLaunchKernel(const void *f, dim3 g, dim3, void **args, size_t smem, cudaStream_t) {
+    return fake::launch(f, g, args, smem);
+}
+FAKE cudaError_t cudaLaunchCooperativeKernel(const void *f, dim3 g, dim3, void **args, size_t smem, cudaStream_t) {
+    return fake::launch(f, g, args, smem);
 }
 FAKE cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **args) {
-    return fake::launch(f, args, c->dynamicSmemBytes);
+    return fake::launch(f, c->gridDim, args, c->dynamicSmemBytes);
 }
 FAKE cudaError_t cudaFuncSetAttribute(const void *f, enum cudaFuncAttribute, int v) {
     std::lock_guard<std::recursive_mutex> g(fake::st().mu);

@@ -3,6 +3,7 @@
 #include "fake_cuda.h"
 #include "geofd.h"
 #include "step2d.cuh"
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -135,6 +136,35 @@ static void check_batch_memory() {
         }
 }
 
+// A batch of little work spreads over the warps that it has columns for: four
+// of them a block forward, two pairs a block backward.
+static void check_batch_spread() {
+    struct Case { int ns, w, nz; } cases[] = {{1, 61, 101}, {1, 201, 301}, {4, 201, 301}, {3, 401, 401}, {2, 3, 20}};
+    for (const Case &q : cases)
+        for (int gathers = 0; gathers < 2; gathers++) {
+            const int nx = q.w + 40, npd = 30, n2 = nx * q.nz;
+            auto v = filled(n2, 2000), e = filled(n2, 0.1f), d = filled(n2, 0.05f);
+            std::vector<float> img(n2), ag((size_t)90 * n2);
+            std::vector<int> xs(q.ns, q.w / 2 + 1), ws(q.ns, q.w);
+            geo_rtm2d_desc B{};
+            B.nx = nx; B.nz = q.nz; B.npd = npd; B.nt = 2; B.dx = B.dz = 10; B.dt_ms = 1; B.favg = 20; B.pfac = 10; B.zs = 2;
+            B.ns = q.ns; B.shot_x = xs.data(); B.shot_nxs = ws.data();
+            fake::st().blocks_max.clear();
+            OK(geo_rtm2d_batch_adcig(&B, v.data(), e.data(), d.data(), img.data(), nullptr, gathers ? ag.data() : nullptr, GEO_MEM_HOST, nullptr));
+            // columns of all strips, at most 8 a warp, at least half of the resident warps (pairs) busy
+            const long cols = (long)q.ns * (q.w + 2 * npd - 8) * ((q.nz + 2 * npd - 8 + 119) / 120);
+            for (const auto &kv : fake::st().blocks_max) {
+                if (kv.first.find("k_march2d") == std::string::npos) continue;
+                const bool fwd = kv.first.find("k_march2dILi0E") != std::string::npos;
+                const long res = 152 * 2 * (fwd ? 4 : 2), per = (fwd ? 4 : 2);   // two blocks an SM (fake occupancy)
+                if (kv.second * per < std::min(cols, res / 2)) {
+                    printf("%d shots %dx%d: %ld blocks of %s for %ld columns\n", q.ns, q.w, q.nz, kv.second, kv.first.c_str(), cols);
+                    failures++;
+                }
+            }
+        }
+}
+
 // Scratch of the codec that could not grow: the calls after it, of any size,
 // find buffers again.
 static void check_codec_growth() {
@@ -205,6 +235,7 @@ int main(int argc, char **argv) {
     else if (check == "plans") check_plans();
     else if (check == "codec_growth") check_codec_growth();
     else if (check == "codec_memory") check_codec_memory();
+    else if (check == "batch_spread") check_batch_spread();
     else return 2;
     return failures ? 1 : 0;
 }

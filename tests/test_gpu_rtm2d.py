@@ -237,3 +237,24 @@ def test_rtm2d_gpu_program_wide_tiles(geo, orc, nx, nz, npml, nt):
     assert np.array_equal(out["illum"], ill)
     assert np.array_equal(out["mig_lap"], orc.laplace2d_adj(mig))
     assert np.array_equal(out["adcigs"], ag)
+
+
+# chunks of 1 to 48 columns (and longer than a window) whatever the batch:
+# windows that end inside a chunk and at its edge, one and two strips
+@pytest.mark.parametrize("mode,chunk", [("exact", c) for c in (1, 2, 3, 5, 8, 12, 48, 200)] + [("fast", 2), ("fast", 8)])
+def test_rtm2d_batch_chunk_lengths(geo, orc, monkeypatch, mode, chunk):
+    v, e, d = model(103, 113)
+    xs, widths = [52, 40, 60], [61, 33, 41]
+    kw = dict(npd=10, nt=420, dx=10.0, dz=10.0, dt_ms=1.0, favg=25.0, pfac=1000.0)
+    run = lambda: geo.rtm2d_batch(v, e, d, zs=2, shot_x=xs, shot_nxs=widths, per_shot=True, adcig=True, laplace=False,
+                                  mode=mode, **kw)
+    base = run()
+    monkeypatch.setenv("GEO_RTM2D_CHUNK", str(chunk))
+    img, per, ag = run()
+    assert np.abs(img).max() > 0 and np.abs(ag).max() > 0
+    assert np.array_equal(img, base[0]) and np.array_equal(ag, base[2])
+    for k, (x, w) in enumerate(zip(xs, widths)):
+        assert np.array_equal(per[k], base[1][k])
+        if mode == "exact":
+            mo, _, _ = orc.rtm2d_mpi_shot(v, e, d, fs_sxd=x, ds_sxd=0, zs_sxd=2, is_=k + 1, nxs=w, **kw)
+            assert np.array_equal(per[k], mo)

@@ -53,3 +53,7 @@ def test_codec_scratch_that_failed_to_grow(check):
 
 def test_codec_scratch_is_what_its_kernels_use(check):
     check("codec_memory")
+
+
+def test_small_batch_spreads_over_the_warps(check):
+    check("batch_spread")
