@@ -763,11 +763,11 @@ extern "C" int geo_rtm2d_batch_adcig(const geo_rtm2d_desc *desc, const float *v,
         GEO_TRY(d_offs.alloc(n * 4));
         GEO_TRY(d_wid.alloc(n * 4));
         if (adcig) GEO_TRY(d_aptr.alloc(ap.size() * sizeof(float *)));
-        // non-finite detector: every wd.every steps (and the last) the graphs
-        // scan every shot's P; the verdict follows each pass
-        auto watch = [&](int k, bool last, int nf, int lev) -> int {
-            if (wd.every <= 0 || ((k + 1) % wd.every && !last)) return GEO_OK;
-            return launch_march_watch(d_M, n, nf, lev, wd.d, k + 1, ss.cs);
+        // non-finite detector: after every wd.every steps (and the last) the
+        // graphs scan every shot's P; the verdict follows each pass
+        auto watched = [&](int k) { return wd.every > 0 && ((k + 1) % wd.every == 0 || k == nt - 1); };
+        auto watch = [&](int k, int nf, int lev) {
+            return watched(k) ? launch_march_watch(d_M, n, nf, lev, wd.d, k + 1, ss.cs) : (int)GEO_OK;
         };
         // forward: source side only, with records and edge lines
         {
@@ -778,7 +778,7 @@ extern "C" int geo_rtm2d_batch_adcig(const geo_rtm2d_desc *desc, const float *v,
                     st.amp = amp[it];
                     st.src_on = on[it];
                     GEO_TRY(B.step(false, st, ss.cs));
-                    GEO_TRY(watch(it, it == nt - 1, 1, st.lev ^ 1));
+                    GEO_TRY(watch(it, 1, st.lev ^ 1));
                 }
                 return GEO_OK;
             }));
@@ -801,17 +801,20 @@ extern "C" int geo_rtm2d_batch_adcig(const geo_rtm2d_desc *desc, const float *v,
             GEO_TRY(B.clear_side(k, MS_SIDE, ss.cs));
         }
         // backward: both propagations with fused imaging; each step's lines and
-        // records go into the level it reads, the first by a launch of its own,
-        // the others as the step before stores that level
+        // records go into the level it reads, as the step before stores that
+        // level, or by a launch of their own before the first step and after a
+        // scan, which is to see the step's own values
         {
             Graph G;
             GEO_TRY(capture(G, ss.cs, [&]() -> int {
                 GEO_TRY(launch_march_inject(d_M, n, maxline, nt - 1, 0, ss.cs));
                 for (int it = nt - 1; it >= 0; it--) {
-                    MarchStep st = step(it, nt - 1 - it);
-                    st.inject = it - 1;
+                    const int k = nt - 1 - it;
+                    MarchStep st = step(it, k);
+                    st.inject = watched(k) ? -1 : it - 1;
                     GEO_TRY(B.step(true, st, ss.cs));
-                    GEO_TRY(watch(nt - 1 - it, it == 0, 2, st.lev ^ 1));
+                    GEO_TRY(watch(k, 2, st.lev ^ 1));
+                    if (watched(k) && it > 0) GEO_TRY(launch_march_inject(d_M, n, maxline, it - 1, st.lev ^ 1, ss.cs));
                 }
                 return GEO_OK;
             }));

@@ -42,7 +42,8 @@ enum MarchSlot {
 struct MarchStep {
     int it, lev;       // step, level read (lev ^ 1 is written)
     float amp;
-    int src_on, inject;   // forward source; backward: step whose lines go into the new level (-1: none)
+    int src_on, inject;   // forward source; backward: step whose lines go into the new level (-1: none, also
+                          // ahead of a scan of that level)
     float dhx, dlx, dhz, dlz;   // two-float (double)(dt/dx), (double)(dt/dz)
     double ddtx, ddtz;
     int *err;             // set when a pipeline wait gave up

@@ -368,10 +368,10 @@ static int gpu_rtm_run(const GpuRtmProgram &prog, const geo_rtm2d_gpu_desc &D, c
         }
         // runs of steps between the watchdog's scans (after backward step it
         // when (nt - it) is a multiple of the interval), one launch each
-        GEO_TRY(launch_step2d_restore(st, nt - 1, st.lev, s));
         for (st.it0 = nt - 1; st.it0 >= 0; st.it0 = st.it1 - 1) {
             st.it1 = st.it0;
             while (st.it1 > 0 && !(wd.every > 0 && (nt - st.it1) % wd.every == 0)) st.it1--;
+            GEO_TRY(launch_step2d_restore(st, st.it0, st.lev, s));   // after the scan, which sees a step's own values
             GEO_TRY(bwd.run(st, s));
             st.lev = (st.lev + st.it0 - st.it1 + 1) & 1;
             const int w = wd.check(st.f[1].P[st.lev], n, nt - 1 - st.it1, st.it1 == 0, s);

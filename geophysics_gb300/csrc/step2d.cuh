@@ -63,7 +63,7 @@ struct Fused2D {
 };
 // The 12 arrays of a side, n floats each, from p.
 void step2d_fields(float *p, size_t n, SField &f);
-// Ring and record of step it into level lev (before the first backward step).
+// Ring and record of step it into level lev (before a backward run that starts with it).
 int launch_step2d_restore(const SStep &a, int it, int lev, cudaStream_t s);
 // angle tables (device), and the source window of SK_CPU
 int load_step2d_angles(const float *thr, const float *cs, cudaStream_t s);

@@ -27,6 +27,7 @@ struct State {
     size_t in_use = 0, peak = 0, limit = ~size_t(0);
     std::map<std::string, long> launches, blocks_max;
     std::string refused;   // launches that a device would refuse
+    void (*on_launch)(const std::string &, void **) = nullptr;
 };
 inline State &st() {
     static State *s = new State;
@@ -50,6 +51,7 @@ inline cudaError_t launch(const void *f, dim3 grid, void **args, size_t smem) {
         st().refused += n + " on device " + std::to_string(device) + "\n";
         return err(cudaErrorInvalidValue);
     }
+    if (st().on_launch) st().on_launch(n, args);
     const unsigned v = 0x44fa0000u;   // 2000.0f
     if (n.find("k_raw_stats") != n.npos) {
         struct View { const float *a[4]; int nx, nz; } *r = (View *)args[0];

@@ -3,6 +3,7 @@
 #include "fake_cuda.h"
 #include "geofd.h"
 #include "step2d.cuh"
+#include "march2d.cuh"
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -165,6 +166,46 @@ static void check_batch_spread() {
         }
 }
 
+// The detector of non-finite values sees what a backward step computed: the
+// next step's lines and records go in after a scan, not before it.
+static int scans, late_scans, lines_of, lines_in;
+static void watch_order(const std::string &n, void **args) {
+    static int inject = -1;
+    auto is = [&](const char *k) { return n.find(k) != n.npos; };
+    if (is("k_march2d")) {
+        const auto &st = *static_cast<const geo::MarchStep *>(args[3]);
+        const bool fwd = is("k_march2dILi0E");
+        if (!fwd && lines_in != st.it) late_scans++;   // its own lines are in the level it reads
+        lines_in = inject = fwd ? -1 : st.inject;
+    } else if (is("k_march_inject")) {
+        lines_in = *static_cast<const int *>(args[1]);
+    } else if (is("k_march_watch")) {
+        scans++;
+        if (inject >= 0) late_scans++;
+    } else if (is("k_step2d_restore")) {
+        lines_of = *static_cast<const int *>(args[1]);
+    } else if (is("k_step2dILi3E")) {   // backward: a run starts with its lines put in by the launch before
+        if (lines_of != static_cast<const geo::SStep *>(args[1])->it0) late_scans++;
+    }
+}
+static void check_watch_order() {
+    const int nx = 40, nz = 30, n2 = nx * nz, xs[2] = {18, 20}, ws[2] = {9, 11};
+    auto v = filled(n2, 2000), e = filled(n2, 0.1f), d = filled(n2, 0.05f), th = filled(n2, 10);
+    std::vector<float> img(n2);
+    setenv("GEO_WATCH_EVERY", "3", 1);
+    fake::st().on_launch = watch_order;
+    geo_rtm2d_desc B{};
+    B.nx = nx; B.nz = nz; B.npd = 8; B.nt = 11; B.dx = B.dz = 10; B.dt_ms = 1; B.favg = 20; B.pfac = 10; B.zs = 2;
+    B.ns = 2; B.shot_x = xs; B.shot_nxs = ws;
+    OK(geo_rtm2d_batch(&B, v.data(), e.data(), d.data(), img.data(), nullptr, GEO_MEM_HOST, nullptr));
+    geo_rtm2d_gpu_desc G{};
+    G.nx = nx; G.nz = nz; G.npml = 8; G.nt = 11; G.dx = G.dz = 10; G.dt = 1e-3f; G.favg = 20; G.pfac = 10; G.wtype = 1;
+    G.ns = 2; G.fs = 20; G.zs = 1; G.mute_tt = 20; G.nangle = 60; G.dangle = 1;
+    OK(geo_rtm2d_gpu(&G, v.data(), e.data(), d.data(), nullptr, img.data(), nullptr, nullptr, nullptr, nullptr, GEO_MEM_HOST, nullptr));
+    OK(geo_rtm2d_tti(&G, v.data(), e.data(), d.data(), th.data(), nullptr, img.data(), nullptr, nullptr, nullptr, GEO_MEM_HOST, nullptr));
+    if (scans != 8 || late_scans) { printf("%d scans of the batch, %d steps or scans out of order\n", scans, late_scans); failures++; }
+}
+
 // Scratch of the codec that could not grow: the calls after it, of any size,
 // find buffers again.
 static void check_codec_growth() {
@@ -236,6 +277,7 @@ int main(int argc, char **argv) {
     else if (check == "codec_growth") check_codec_growth();
     else if (check == "codec_memory") check_codec_memory();
     else if (check == "batch_spread") check_batch_spread();
+    else if (check == "watch_order") check_watch_order();
     else return 2;
     return failures ? 1 : 0;
 }

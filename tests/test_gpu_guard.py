@@ -173,3 +173,19 @@ def test_2d_model_check_names_the_first_bad_cell(geo, array, value, text):
             with pytest.raises(geo.GeoError) as err:
                 call(a)
             assert text in str(err.value), str(err.value)
+
+
+@pytest.mark.parametrize("widths", [[3], [5, 31]])
+def test_batch_backward_overflow_found_at_the_first_scan(geo, widths):
+    """Overflow in cells that the next step's lines replace (a window of three
+    columns has no others at its sides) is found by the scan after the step
+    that computed it, not at the end of the pass."""
+    nx, nz = 80, 40
+    g = np.random.default_rng(4)
+    v = (2000 + 900 * g.random((nx, nz))).astype(np.float32)
+    r = ((v - 2000) / 2000).astype(np.float32)
+    kw = dict(npd=5, nt=330, dx=10.0, dz=10.0, dt_ms=1.0, favg=20.0, pfac=3e38, zs=1, shot_x=[41] * len(widths),
+              shot_nxs=widths)
+    with pytest.raises(geo.GeoError) as err:
+        geo.rtm2d_batch(v, 0.3 * r, 0.15 * r, **kw)
+    assert "pass: wavefield non-finite by time step 100" in str(err.value)

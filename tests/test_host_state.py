@@ -57,3 +57,7 @@ def test_codec_scratch_is_what_its_kernels_use(check):
 
 def test_small_batch_spreads_over_the_warps(check):
     check("batch_spread")
+
+
+def test_detector_scans_before_the_next_lines_go_in(check):
+    check("watch_order")
