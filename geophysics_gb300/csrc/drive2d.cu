@@ -767,7 +767,7 @@ extern "C" int geo_rtm2d_batch_adcig(const geo_rtm2d_desc *desc, const float *v,
         // graphs scan every shot's P; the verdict follows each pass
         auto watched = [&](int k) { return wd.every > 0 && ((k + 1) % wd.every == 0 || k == nt - 1); };
         auto watch = [&](int k, int nf, int lev) {
-            return watched(k) ? launch_march_watch(d_M, n, nf, lev, wd.d, k + 1, ss.cs) : (int)GEO_OK;
+            return watched(k) ? launch_march_watch(d_M, n, nf, lev, wd.word(), k + 1, ss.cs) : (int)GEO_OK;
         };
         // forward: source side only, with records and edge lines
         {

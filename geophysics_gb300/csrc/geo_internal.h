@@ -109,6 +109,7 @@ int watch_every();
 struct Watchdog {
     int *h = nullptr, *d = nullptr;
     int every = 100;
+    bool in_flight = false;   // scans since the last verdict
     Watchdog() = default;
     Watchdog(const Watchdog &) = delete;
     Watchdog &operator=(const Watchdog &) = delete;
@@ -116,6 +117,10 @@ struct Watchdog {
     int open();
     void close();
     void arm();
+    int *word() {   // for scans that the caller launches
+        in_flight = true;
+        return d;
+    }
     bool tripped() const;
     int check(const float *a, size_t n, int it, bool last, cudaStream_t s);
     int scan(const float *a, size_t n, int tag, cudaStream_t s);

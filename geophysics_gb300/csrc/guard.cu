@@ -74,8 +74,10 @@ int watch_every() {
 // The words come from one page of mapped pinned memory, taken on first use
 // and kept (an allocation and a free per call were 0.35 ms of a 2D shot's
 // 2.5 ms); runs beyond its 1024 words get their own.  A word goes back only
-// once the device is idle, so no scan still in flight can set it for its
-// next owner.
+// after a verdict, which waits for its scans, so none in flight can set it for
+// its next owner; a run that failed between a scan and its verdict keeps its
+// word out of use.  (Waiting for the whole device instead is not allowed while
+// another host thread captures a graph: it fails, and the capture with it.)
 namespace {
 constexpr int kWords = 1024;
 std::mutex g_words_mu;
@@ -105,12 +107,12 @@ int Watchdog::open() {
 
 void Watchdog::close() {
     if (h) {
-        cudaDeviceSynchronize();
         std::lock_guard<std::mutex> lock(g_words_mu);
-        if (g_words && h >= g_words && h < g_words + kWords) g_words_free.push_back((int)(h - g_words));
-        else cudaFreeHost(h);
+        if (!g_words || h < g_words || h >= g_words + kWords) cudaFreeHost(h);   // waits for its scans
+        else if (!in_flight) g_words_free.push_back((int)(h - g_words));
     }
     h = d = nullptr;
+    in_flight = false;
 }
 
 void Watchdog::arm() {
@@ -123,7 +125,7 @@ bool Watchdog::tripped() const { return h && *(volatile const int *)h != 0; }
 int Watchdog::check(const float *a, size_t n, int it, bool last, cudaStream_t s) {
     if (!h || every <= 0 || ((it + 1) % every && !last)) return GEO_OK;
     const int grid = (int)std::min<size_t>((n + 255) / 256, 152 * 8);
-    k_watch<<<grid, 256, 0, s>>>(a, n, d, it + 1);
+    k_watch<<<grid, 256, 0, s>>>(a, n, word(), it + 1);
     GEO_TRY(check_launch("watch"));
     return tripped() ? GEO_ERR_NAN : GEO_OK;
 }
@@ -131,13 +133,14 @@ int Watchdog::check(const float *a, size_t n, int it, bool last, cudaStream_t s)
 int Watchdog::scan(const float *a, size_t n, int tag, cudaStream_t s) {
     if (!h || every <= 0) return GEO_OK;
     const int grid = (int)std::min<size_t>((n + 255) / 256, 152 * 8);
-    k_watch<<<grid, 256, 0, s>>>(a, n, d, tag);
+    k_watch<<<grid, 256, 0, s>>>(a, n, word(), tag);
     return check_launch("watch");
 }
 
 int Watchdog::verdict(cudaStream_t s, const char *what) {
     if (!h) return GEO_OK;
     GEO_CUDA(cudaStreamSynchronize(s));
+    in_flight = false;
     const int tag = *(volatile int *)h;
     if (tag > 0) return fail(GEO_ERR_NAN, "%s: wavefield non-finite by time step %d", what, tag);
     if (tag < 0) return fail(GEO_ERR_NAN, "%s: non-finite values in the result", what);

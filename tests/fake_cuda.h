@@ -27,6 +27,7 @@ struct State {
     size_t in_use = 0, peak = 0, limit = ~size_t(0);
     std::map<std::string, long> launches, blocks_max;
     std::string refused;   // launches that a device would refuse
+    int device_waits = 0;
     void (*on_launch)(const std::string &, void **) = nullptr;
 };
 inline State &st() {
@@ -172,7 +173,7 @@ FAKE cudaError_t cudaDeviceGetAttribute(int *v, enum cudaDeviceAttr a, int) {
     *v = a == cudaDevAttrMultiProcessorCount ? 152 : 1;
     return cudaSuccess;
 }
-FAKE cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
+FAKE cudaError_t cudaDeviceSynchronize() { fake::st().device_waits++; return cudaSuccess; }
 FAKE cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 FAKE cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { *s = nullptr; return cudaSuccess; }
 FAKE cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }

@@ -21,6 +21,14 @@ static int failures = 0;
 
 static std::vector<float> filled(size_t n, float v) { return std::vector<float>(n, v); }
 
+// Waits for the whole device are not allowed while another host thread captures
+// a graph, so the calls that run beside each other in threads make none.
+static int waits_of(const char *what) {
+    if (fake::st().device_waits) { printf("%s: %d waits for the device\n", what, fake::st().device_waits); failures++; }
+    fake::st().device_waits = 0;
+    return 0;
+}
+
 static geo_fd2d_desc fd2d_desc(int variant) {
     geo_fd2d_desc d{};
     d.nx = 40; d.nz = 30; d.npd = 8; d.nt = 3;
@@ -57,8 +65,10 @@ static void every_entry_point() {
     const int m = 20, n3 = m * m * m;
     auto v3 = filled(n3, 2000), e3 = filled(n3, 0.1f), d3 = filled(n3, 0.05f), t3 = filled(n3, 10);
     std::vector<float> o3(4 * n3);
+    waits_of("2D");
     geo_ae *ae = nullptr;
     OK(geo_ae_create(&ae, 1));
+    fake::st().device_waits = 0;
     for (int mode : {GEO_MODE_EXACT, GEO_MODE_FAST}) {
         geo_fd3d_desc F{};
         F.nx = F.ny = F.nz = m; F.npd = 8; F.nt = 8; F.dx = F.dy = F.dz = 10; F.dt = 1e-3f; F.favg = 20; F.pfac = 10; F.wtype = 1;
@@ -88,6 +98,7 @@ static void every_entry_point() {
                 for (int f32 = 0; f32 < 2; f32++)
                     OK(geo_tc_gemm_bf16(rows, w, K, A.data(), B.data(), nullptr, 0, o.data(), f32, nullptr));
             }
+    waits_of("3D and the codec");
     OK(geo_ae_destroy(ae));
 }
 

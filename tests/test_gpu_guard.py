@@ -189,3 +189,43 @@ def test_batch_backward_overflow_found_at_the_first_scan(geo, widths):
     with pytest.raises(geo.GeoError) as err:
         geo.rtm2d_batch(v, 0.3 * r, 0.15 * r, **kw)
     assert "pass: wavefield non-finite by time step 100" in str(err.value)
+
+
+def test_calls_in_threads_beside_captures(geo):
+    """Batched RTM captures its time loop; shots, RTM and 3D runs of other host
+    threads neither fail beside that nor break it."""
+    import threading
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(2)
+    v = 2000 + 800 * torch.rand((90, 70), generator=g, device="cuda")
+    m = (v, 0.3 * (v - 2000) / 2000, 0.15 * (v - 2000) / 2000)
+    v3 = 2000 + 800 * torch.rand((20, 22, 24), generator=g, device="cuda")
+    m3 = (v3, 0.3 * (v3 - 2000) / 2000, 0.15 * (v3 - 2000) / 2000)
+    kw = dict(nt=60, dx=10.0, dz=10.0, favg=20.0)
+    jobs = [lambda: geo.rtm2d_batch(*m, npd=10, dt_ms=1.0, pfac=10.0, zs=2, shot_x=[40, 50], shot_nxs=[31, 41], **kw),
+            lambda: geo.fd2d_shot(*m, npd=10, dt=1e-3, fs=40, zs=2, **kw),
+            lambda: geo.fd2d_shot(*m, npd=10, dt=1e-3, fs=40, zs=2, variant="mpi", **kw),
+            lambda: geo.rtm2d_gpu(*m, npml=10, dt=1e-3, fs=40, zs=2, **kw)["illum"],
+            lambda: geo.fd3d_shot(*m3, npd=8, dy=10.0, dt=1e-3, fsx=10, fsy=10, fsz=2, **kw)]
+    ref = [j() for j in jobs]
+    bad = []
+
+    def run(first):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for k in range(15):
+                i = (first + k) % len(jobs)
+                try:
+                    out = jobs[i]()
+                    torch.cuda.current_stream().synchronize()
+                    if not torch.equal(out, ref[i]):
+                        bad.append((i, "differs"))
+                except Exception as ex:
+                    bad.append((i, repr(ex)[:200]))
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=run, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad[:3]

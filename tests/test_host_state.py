@@ -35,7 +35,9 @@ def check(tmp_path_factory):
 
 def test_second_device_gets_tables_and_kernel_attributes(check):
     """Every entry point on one device, then on another: the same constant
-    tables are copied to both, the same kernels' shared-memory limits set."""
+    tables are copied to both, the same kernels' shared-memory limits set.
+    No call waits for the whole device (a graph that another host thread
+    captures would fail)."""
     check("devices")
 
 
