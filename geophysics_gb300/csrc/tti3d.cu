@@ -445,7 +445,7 @@ struct MapPair {
 std::map<MapKey, MapPair> g_maps;
 std::mutex g_maps_mu;
 
-int tti_maps(const Tti3DStep &t, const MapPair **out) {
+int tti_maps(const Tti3DStep &t, MapPair &out) {
     const Grid3D &g = t.g;
     MapKey key{};
     const void *ptrs[16] = {t.P0, t.Q0, t.u0, t.v0, t.w0, t.u1, t.v1, t.w1, t.ct, t.st, t.cp, t.sp, g.vp, g.e2, g.d2,
@@ -482,7 +482,7 @@ int tti_maps(const Tti3DStep &t, const MapPair **out) {
         for (int r = 0; r < 3; r++) GEO_TRY(encode_map(&m.s.m[r], md[r], nz, ld, nx, ny, TZ, TX));
         it = g_maps.emplace(key, m).first;
     }
-    *out = &it->second;
+    out = it->second;   // a copy: another thread's plans may clear the cache
     return GEO_OK;
 }
 
@@ -497,8 +497,8 @@ int launch_tti3d(const Tti3DStep &t, const StepArgs3D &args, cudaStream_t s) {
         k_tti3d_source<<<1, 1, 0, s>>>(const_cast<float *>(t.P0), const_cast<float *>(t.Q0), st.src, st.amp, t.save);
         GEO_TRY(check_launch("tti3d_source"));
     }
-    const MapPair *m = nullptr;
-    GEO_TRY(tti_maps(t, &m));
+    MapPair m;
+    GEO_TRY(tti_maps(t, m));
     GEO_TRY(allow_smem(vel, (const void *)k_tti3d_vel, VEL_SMEM));
     GEO_TRY(allow_smem(stress, (const void *)k_tti3d_stress, STR_SMEM));
     if ((long)g.sxy * g.nny >= (1L << 31)) return fail(GEO_ERR_ARG, "grid too large for 32-bit plane offsets");
@@ -519,9 +519,9 @@ int launch_tti3d(const Tti3DStep &t, const StepArgs3D &args, cudaStream_t s) {
     const int nchunks = (planes + G.chunk - 1) / G.chunk;
     G.err = t.err;
     const dim3 block(TZ, NW), grid(G.ntiles * nchunks);
-    GEO_CUDA(launch_early(k_tti3d_vel, grid.x, block, VEL_SMEM, s, m->v, G, t.u1, t.v1, t.w1));
+    GEO_CUDA(launch_early(k_tti3d_vel, grid.x, block, VEL_SMEM, s, m.v, G, t.u1, t.v1, t.w1));
     GEO_TRY(check_launch("tti3d_vel"));
-    GEO_CUDA(launch_early(k_tti3d_stress, grid.x, block, STR_SMEM, s, m->s, G, t.P1, t.Q1, t.save, st));
+    GEO_CUDA(launch_early(k_tti3d_stress, grid.x, block, STR_SMEM, s, m.s, G, t.P1, t.Q1, t.save, st));
     return check_launch("tti3d_stress");
 }
 

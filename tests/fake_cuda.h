@@ -200,6 +200,7 @@ inline CUresult fake_encode(CUtensorMap *m, CUtensorMapDataType, cuuint32_t, voi
                             const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                             CUtensorMapL2promotion, CUtensorMapFloatOOBfill) {
     memset(m, 0, sizeof *m);
+    memcpy(m, &base, sizeof base);
     if (!base) fake::st().refused += "tensor map of a null buffer\n";
     return CUDA_SUCCESS;
 }

@@ -217,6 +217,47 @@ static void check_watch_order() {
     if (scans != 8 || late_scans) { printf("%d scans of the batch, %d steps or scans out of order\n", scans, late_scans); failures++; }
 }
 
+// A plan's step keeps its tensor maps while steps of other plans (here between
+// its two launches, as from another thread) push the cache of maps over.
+static geo_fd3d_plan *tilted_plan() {
+    const int m = 12, n3 = m * m * m;
+    static auto v = filled(n3, 2000), e = filled(n3, 0.1f), d = filled(n3, 0.05f), t = filled(n3, 10);
+    geo_fd3d_desc F{};
+    F.nx = F.ny = F.nz = m; F.npd = 5; F.nt = 8; F.dx = F.dy = F.dz = 10; F.dt = 1e-3f; F.favg = 20; F.pfac = 10; F.wtype = 1;
+    F.mode = GEO_MODE_FAST; F.fsx = F.fsy = 6; F.fsz = 2; F.rec_iz = 5; F.drx = F.dry = 1; F.nrx = F.nry = m;
+    geo_fd3d_plan *p = nullptr;
+    OK(geo_fd3d_plan_create(&p, &F));
+    OK(geo_fd3d_set_model(p, v.data(), e.data(), d.data(), GEO_MEM_HOST, nullptr));
+    OK(geo_fd3d_set_tilt(p, t.data(), t.data(), GEO_MEM_HOST, nullptr));
+    return p;
+}
+static int bad_maps, stress_seen;
+static void others_step(const std::string &n, void **args) {
+    if (n.find("k_tti3d_vel") != n.npos) {
+        fake::st().on_launch = nullptr;
+        for (int k = 0; k < 40; k++) {
+            float ms;
+            OK(geo_fd3d_time_steps(tilted_plan(), 2, &ms, nullptr));   // plans stay: distinct buffers
+        }
+        fake::st().on_launch = others_step;
+    } else if (n.find("k_tti3d_stress") != n.npos && !stress_seen++) {
+        for (int k = 0; k < 15; k++) {
+            const CUtensorMap &m = static_cast<const CUtensorMap *>(args[0])[k];
+            char *base;
+            memcpy(&base, &m, sizeof base);
+            auto it = fake::st().blocks.upper_bound(base);   // the allocation it lies in
+            if (it == fake::st().blocks.begin() || base >= static_cast<char *>((--it)->first) + it->second) bad_maps++;
+        }
+    }
+}
+static void check_tti_maps() {
+    geo_fd3d_plan *p = tilted_plan();
+    fake::st().on_launch = others_step;
+    float ms;
+    OK(geo_fd3d_time_steps(p, 1, &ms, nullptr));
+    if (!stress_seen || bad_maps) { printf("%d of 15 maps of a step are not its own\n", bad_maps); failures++; }
+}
+
 // Scratch of the codec that could not grow: the calls after it, of any size,
 // find buffers again.
 static void check_codec_growth() {
@@ -289,6 +330,7 @@ int main(int argc, char **argv) {
     else if (check == "codec_memory") check_codec_memory();
     else if (check == "batch_spread") check_batch_spread();
     else if (check == "watch_order") check_watch_order();
+    else if (check == "tti_maps") check_tti_maps();
     else return 2;
     return failures ? 1 : 0;
 }

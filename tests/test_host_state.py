@@ -26,7 +26,9 @@ def check(tmp_path_factory):
                     "-Wl,-rpath," + PKG, "-Wl,--allow-shlib-undefined", "-lpthread"], check=True)
 
     def run(name):
-        r = subprocess.run([exe, name], capture_output=True, text=True, timeout=300)
+        # freed memory is overwritten
+        env = dict(os.environ, MALLOC_PERTURB_="165")
+        r = subprocess.run([exe, name], capture_output=True, text=True, timeout=300, env=env)
         assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-1000:]
         return r.stdout
 
@@ -63,3 +65,7 @@ def test_small_batch_spreads_over_the_warps(check):
 
 def test_detector_scans_before_the_next_lines_go_in(check):
     check("watch_order")
+
+
+def test_tilted_step_keeps_its_maps(check):
+    check("tti_maps")
