@@ -50,7 +50,7 @@ struct ShotSet {
     int read(const Raw2D &raw, cudaStream_t s);
     // profiles and taper box of shot k: offsets in `small`
     struct Off {
-        size_t xprof, zprof, te2, td2, tpw;   // xprof cx1 cx2 ax1 ax2; zprof cz1 cz2 az1 az2, ldz each
+        size_t xprof, zprof, te2, td2;        // xprof cx1 cx2 ax1 ax2; zprof cz1 cz2 az1 az2, ldz each
         Taper2D box;
         std::vector<float> vbox;              // v on the taper box
         std::vector<float> p[8];

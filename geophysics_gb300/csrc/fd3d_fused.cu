@@ -44,7 +44,6 @@
 #include "fd3d_fused.cuh"
 #include "tc_util.cuh"
 #include <cudaTypedefs.h>
-#include <type_traits>
 
 namespace geo {
 
@@ -84,39 +83,21 @@ constexpr unsigned kFull = (1u << kW) - 1;
 struct FV {
     float v[kW];
 };
-using VecT = std::conditional_t<kW == 4, float4, float2>;
-template <class T>
-__device__ __forceinline__ FV unpack(const T &t) {
-    FV r;
-    r.v[0] = t.x;
-    r.v[1] = t.y;
-    if constexpr (kW == 4) {
-        r.v[2] = t.z;
-        r.v[3] = t.w;
-    }
-    return r;
-}
-__device__ __forceinline__ FV ld_s(const float *p) { return unpack(*reinterpret_cast<const VecT *>(p)); }
+static_assert(kW == 2, "vectors are float2");
+__device__ __forceinline__ FV unpack(const float2 &t) { return FV{{t.x, t.y}}; }
+__device__ __forceinline__ FV ld_s(const float *p) { return unpack(*reinterpret_cast<const float2 *>(p)); }
 // Plain loads throughout, also of arrays that this launch only reads: its
 // blocks come up while the kernel before, which wrote them, still runs, and
 // ld.global.nc (__ldg) is defined only for what nobody writes while a kernel
 // lives and may be moved ahead of the wait for that kernel.
-__device__ __forceinline__ FV ld_g(const float *p) { return unpack(*reinterpret_cast<const VecT *>(p)); }
+__device__ __forceinline__ FV ld_g(const float *p) { return unpack(*reinterpret_cast<const float2 *>(p)); }
 __device__ __forceinline__ FV ld_g(const float *p, bool on) {
-    VecT t{};
-    if (on) t = *reinterpret_cast<const VecT *>(p);
+    float2 t{};
+    if (on) t = *reinterpret_cast<const float2 *>(p);
     return unpack(t);
 }
-template <class T = VecT>
 __device__ __forceinline__ void st_v(float *p, const FV &a) {
-    T t;
-    t.x = a.v[0];
-    t.y = a.v[1];
-    if constexpr (kW == 4) {
-        t.z = a.v[2];
-        t.w = a.v[3];
-    }
-    *reinterpret_cast<T *>(p) = t;
+    *reinterpret_cast<float2 *>(p) = make_float2(a.v[0], a.v[1]);
 }
 __device__ __forceinline__ void push(FV *q, const FV &a) {
 #pragma unroll

@@ -96,7 +96,7 @@ __device__ __forceinline__ int adcig_bin(float a1) {
 
 constexpr int kMarchThreads = 128;
 enum MarchMode { MM_FWD = 0, MM_BWD = 1, MM_ADCIG = 2 };   // forward; backward; backward with angle gathers
-constexpr int march_blocks(int) { return 3; }   // per SM
+constexpr int kMarchBlocks = 3;   // per SM
 // A warp's prefetch stage: rows of one column, 128 depths each (float4
 // units): Q with the four depths either side, then P (seven columns on), u
 // (three on), w, the split stresses, the model, the image row.
@@ -109,11 +109,11 @@ constexpr int march_xch(int mode) { return mode == MM_FWD ? 0 : mode == MM_BWD ?
 constexpr size_t march_smem(int mode) {
     return kMarchSmem + (size_t)(kMarchThreads / 64) * 2 * march_xch(mode) * 32 * 16;
 }
-static_assert(4 * (march_smem(MM_BWD) + 1024) <= 233472 && 3 * (march_smem(MM_ADCIG) + 1024) <= 233472, "blocks per SM");
+static_assert(kMarchBlocks * (march_smem(MM_ADCIG) + 1024) <= 233472, "blocks per SM");
 
 // I: type of element offsets, 32 bits while a shot's slots fit.
 template <int MODE, bool FAST, class I>
-__global__ void __launch_bounds__(kMarchThreads, march_blocks(MODE))
+__global__ void __launch_bounds__(kMarchThreads, kMarchBlocks)
     k_march2d(const March2D *__restrict__ shots, const int4 *__restrict__ items, int nitems, const MarchStep st) {
     constexpr bool BWD = MODE != MM_FWD;
     constexpr int XN = march_xch(MODE);

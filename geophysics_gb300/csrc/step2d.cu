@@ -345,23 +345,21 @@ __global__ void __launch_bounds__(kThreads, NC == 1 ? 3 : 2)
             } else {
                 // u on the tile's columns and its halos: NU consecutive columns a
                 // warp, column uc at x = x0 - 4 + uc, taps P box columns uc .. uc+7
-                                {
-                    const int u0 = warp * NU;
-                    float2 q[8];
+                const int u0 = warp * NU;
+                float2 pq[8];
 #pragma unroll
-                    for (int j = 0; j < 7; j++) q[j + 1] = lds2(sP + min(u0 + j, TX + 13) * kTz + zl);
+                for (int j = 0; j < 7; j++) pq[j + 1] = lds2(sP + min(u0 + j, TX + 13) * kTz + zl);
 #pragma unroll
-                    for (int j = 0; j < NU; j++) {
-                        const int uc = u0 + j, ix = x0 - 4 + uc;
+                for (int j = 0; j < NU; j++) {
+                    const int uc = u0 + j, ix = x0 - 4 + uc;
 #pragma unroll
-                        for (int m = 0; m < 7; m++) q[m] = q[m + 1];
-                        q[7] = lds2(sP + min(uc + 7, TX + 13) * kTz + zl);
-                        if (uc < TX + 7 && ix >= 4 && ix < g.nnx - 4) {
-                            const float c1 = cu1[j] * g.dtx, c2 = cu2[j];
-                            const float2 xx = dx8(q), uo = lds2(sU + uc * kTz + zl);
-                            sts2(sU + uc * kTz + zl,
-                                 make_float2(z0u ? c2 * uo.x - c1 * xx.x : uo.x, z1u ? c2 * uo.y - c1 * xx.y : uo.y));
-                        }
+                    for (int m = 0; m < 7; m++) pq[m] = pq[m + 1];
+                    pq[7] = lds2(sP + min(uc + 7, TX + 13) * kTz + zl);
+                    if (uc < TX + 7 && ix >= 4 && ix < g.nnx - 4) {
+                        const float c1 = cu1[j] * g.dtx, c2 = cu2[j];
+                        const float2 xx = dx8(pq), uo = lds2(sU + uc * kTz + zl);
+                        sts2(sU + uc * kTz + zl,
+                             make_float2(z0u ? c2 * uo.x - c1 * xx.x : uo.x, z1u ? c2 * uo.y - c1 * xx.y : uo.y));
                     }
                 }
                 // w of the own points, and of the four depths above and below
