@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <cstdio>
 #include <cstdint>
+#include <atomic>
 #include <mutex>
 #include <vector>
 #include <string>
@@ -48,21 +49,23 @@ struct DevBuf {
 
 // Set-up of what belongs to a device and not to the process (constant memory,
 // kernel attributes): f once per device, under a lock so that host threads
-// find it done, and again after a failure.  No heap use.
+// find it done, and again after a failure.  No heap use, no lock once it is
+// done (every launch asks).
 class OncePerDevice {
     static constexpr int kDevices = 64;   // set up on every call beyond
     std::mutex mu;
-    bool done[kDevices] = {};
+    std::atomic<bool> done[kDevices] = {};
 
 public:
     template <class F>
     int run(F &&f) {
         int dev = 0;
         GEO_CUDA(cudaGetDevice(&dev));
+        if (dev < kDevices && done[dev].load(std::memory_order_acquire)) return GEO_OK;
         std::lock_guard<std::mutex> lock(mu);
-        if (dev < kDevices && done[dev]) return GEO_OK;
+        if (dev < kDevices && done[dev].load(std::memory_order_relaxed)) return GEO_OK;
         GEO_TRY(f());
-        if (dev < kDevices) done[dev] = true;
+        if (dev < kDevices) done[dev].store(true, std::memory_order_release);
         return GEO_OK;
     }
 };

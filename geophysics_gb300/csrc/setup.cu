@@ -53,10 +53,13 @@ int DevBuf::zero(cudaStream_t s) {
 }
 
 int sm_count() {
+    constexpr int kDevices = 64;
+    static std::atomic<int> known[kDevices];
     int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1)
-        n = 152;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 152;
+    if (dev < kDevices && (n = known[dev].load(std::memory_order_relaxed))) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 152;
+    if (dev < kDevices) known[dev].store(n, std::memory_order_relaxed);
     return n;
 }
 
