@@ -8,7 +8,7 @@
 //   tc_gemm x2   E3, E4 on tcgen05 (the last one writes the bf16 code);
 //   tc_gemm x2   D4, D3 on tcgen05;
 //   k_ae_d21     D2 on tcgen05, D1 (16 -> 8) on CUDA cores, unscale, store the
-//                snapshot; or
+//                snapshot (a round trip); or, in an RTM run,
 //   tc_gemm, k_ae_d1_vol  D2, then D1 with the product with the receiver
 //                wavefield added to the image (or, for the escape check, the
 //                comparison with the field).
@@ -544,7 +544,8 @@ __global__ void __launch_bounds__(256, 2) k_ae_e12(const __grid_constant__ CUten
 // nodes (packed FP32 multiply-adds) and 16 four-depth stores.  D2's output, 16
 // KB a block, never leaves the SM.  Two CTAs per SM.  Waits are bounded.
 // A 512x512x384 snapshot takes 116 us, 5.1 TB/s; D2 and D1 one after the other
-// took 221 (101 + 120).
+// took 221 (101 + 120).  The round trip's decode; imaging and the escape check
+// take D2 as a GEMM and k_ae_d1_vol.
 struct D21Args {
     AeVolume vol;
     int nb, tiles;

@@ -274,13 +274,13 @@ static int alloc_fields(geo_fd3d_plan *p, int f) {
 // queues, so more chunks mean more blocks in flight and shorter tails at the
 // price of the fill.  The count is the one with the fewest rounds of resident
 // blocks (two per SM) times a chunk's planes, the fill counted as one; of those
-// within 1.5 % of it the largest, whose tail is shorter.  us a step of the
+// within 1.5 % of it the largest, whose tail is shorter.  us a bare step of the
 // exact / fast form with it and with the best of 1 to 24: 121x93x107 + 20 (11
-// chunks) 65 / 60 against 64 / 60; 176x160x144 + 20 (7) 137 / 121, the best; 250x200x150 + 20 (8)
-// 219 / 189, the best; 400^3 + 40 (8) 1706 / 1379 against 1702 / 1374;
-// 500x120x260 + 30 (6) 499 / 419, the best.  (Timing seven counts on the device
-// at the first set_model, which this replaces, took 24 to 28 steps and did not
-// try 7.)
+// chunks) 62.0 / 58.4 against 59.7 / 55.5 (5); 176x160x144 + 20 (7) 134 / 118,
+// the best; 250x200x150 + 20 (8) 218.6 / 187.9 against 218.5 / 187.1;
+// 400^3 + 40 (8) 1738 / 1396 against 1729 / 1386 (10); 500x120x260 + 30 (6)
+// 498 / 418 against 498 / 417.  (Timing seven counts on the device at the first
+// set_model, which this replaces, took 24 to 28 steps and did not try 7.)
 int march_chunks(int tiles, int planes) {
     const int slots = 2 * sm_count();
     long best = 0;

@@ -445,7 +445,9 @@ __global__ void __launch_bounds__(kMarchThreads, kMarchBlocks)
 #pragma unroll
                         for (int j = 0; j < 4; j++) {
                             if (gz0 + j < 0 || gz0 + j >= nz) continue;
-                            // a zero product adds nothing: the sums start at +0 and never become -0
+                            // a zero product changes no sum but the sign of a zero one (a negative
+                            // product below 2^-150 rounds to -0 there), and the shots' stack, which
+                            // starts at +0, keeps no -0
                             if (Pn.v[j] * sP[j] == 0.0f) continue;
                             const float sx = -sP[j] * su[j], sz = -sQ[j] * sw[j];
                             const float rx = Pn.v[j] * q[4].v[j], rz = Qn.v[j] * wn.v[j];

@@ -30,8 +30,11 @@ constexpr int kGM = 128, kGK = 64;
 // with fewer K slices than that gets as many stages as slices (ST), so that
 // more CTAs share an SM and more tiles are in flight: the skinny codec
 // levels (K = 64, 128) have one or two slices per tile.  The shared memory
-// is then padded so that no more CTAs fit than tensor memory holds
-// accumulators for (512 columns per SM), so no allocation ever waits.
+// is then padded so that no more of a launch's CTAs fit than tensor memory
+// holds accumulators for (512 columns per SM), so none of them waits for
+// another.  A CTA launched early can find its predecessor's CTAs still holding
+// columns and wait in its allocation; that ends, since every predecessor CTA
+// has allocated before it lets a successor come and needs nothing of it.
 constexpr int default_stages(int bn) { return bn >= 256 ? 2 : (bn >= 128 ? 3 : 4); }
 // GEMMs of few tiles take narrow ones with a deep ring instead (launch_bn_k).
 constexpr int kDeepStages = 8;

@@ -122,6 +122,9 @@ int geo_fd2d_shot(const geo_fd2d_desc *desc, const float *v, const float *e, con
  *     library keeps until exit; larger shots fail with GEO_ERR_ARG;
  *   - CPU and GPU variants (SV taper and GPU-form mute included), no
  *     snapshots;
+ *   - it steps by half-steps, two launches a step, where geo_fd2d_shot has
+ *     fused steps: 401x401, 2000 steps 28.8 ms against 10.7 (the MPI
+ *     variant's geo_fd2d_shot, also half-steps: 25.9);
  *   - the first call on a device resolves the array's device address,
  *     which is kept for the life of the process: do not call this on a
  *     device after cudaDeviceReset;
