@@ -318,7 +318,7 @@ int MarchBatch::work(bool backward) {
         chunk = (int)std::min(48L, std::max(8L, cols / (4L * res)));
     }
     if (const char *e = getenv("GEO_RTM2D_CHUNK"))
-        if (const int c = atoi(e); c > 0) chunk = c;
+        if (const int c = atoi(e); c > 0) chunk = std::min(c, 1 << 20);
     std::vector<int4> &v = items[backward];
     v.clear();
     for (int k = 0; k < ns; k++) {

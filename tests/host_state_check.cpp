@@ -258,6 +258,20 @@ static void check_tti_maps() {
     if (!stress_seen || bad_maps) { printf("%d of 15 maps of a step are not its own\n", bad_maps); failures++; }
 }
 
+static void check_chunk_override() {
+    const int nx = 60, nz = 40, n2 = nx * nz, xs[2] = {18, 20}, ws[2] = {9, 11};
+    auto v = filled(n2, 2000), e = filled(n2, 0.1f), d = filled(n2, 0.05f);
+    std::vector<float> img(n2);
+    geo_rtm2d_desc B{};
+    B.nx = nx; B.nz = nz; B.npd = 8; B.nt = 2; B.dx = B.dz = 10; B.dt_ms = 1; B.favg = 20; B.pfac = 10; B.zs = 2;
+    B.ns = 2; B.shot_x = xs; B.shot_nxs = ws;
+    OK(geo_rtm2d_batch(&B, v.data(), e.data(), d.data(), img.data(), nullptr, GEO_MEM_HOST, nullptr));
+    long steps = 0;
+    for (const auto &kv : fake::st().launches)
+        if (kv.first.find("k_march2d") != std::string::npos) steps += kv.second;
+    if (steps != 4) { printf("%ld of 4 steps launched\n", steps); failures++; }
+}
+
 // Scratch of the codec that could not grow: the calls after it, of any size,
 // find buffers again.
 static void check_codec_growth() {
@@ -323,7 +337,11 @@ static void check_plans() {
 
 int main(int argc, char **argv) {
     const std::string check = argc > 1 ? argv[1] : "";
-    if (check == "devices") check_devices();
+    if (check == "batch_chunk_override") {
+        // any length leaves every window at least one chunk
+        setenv("GEO_RTM2D_CHUNK", "2147483647", 1);
+        check_chunk_override();
+    } else if (check == "devices") check_devices();
     else if (check == "batch_memory") check_batch_memory();
     else if (check == "plans") check_plans();
     else if (check == "codec_growth") check_codec_growth();

@@ -69,3 +69,7 @@ def test_detector_scans_before_the_next_lines_go_in(check):
 
 def test_tilted_step_keeps_its_maps(check):
     check("tti_maps")
+
+
+def test_any_chunk_override_covers_the_windows(check):
+    check("batch_chunk_override")
